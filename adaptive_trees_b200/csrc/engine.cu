@@ -35,6 +35,7 @@
 #include "binlevel.cuh"
 #include "levelbuild.cuh"
 #include "rebalance.cuh"
+#include "sort_repair.cuh"
 #include "tree_view.cuh"
 
 namespace aot
@@ -422,27 +423,39 @@ BinaryGeometry makeGeometry(const double *b, unsigned maxDepth, int real)
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Where a key generation leaves the digit counts of the sort that follows
+// (hist == nullptr: nowhere).
+struct KeygenSort
+{
+    u32 *hist = nullptr, *bins = nullptr;
+    sort::SortControl *ctl = nullptr;
+    const sort::PlanArgs *plan = nullptr;  // make the plan first
+};
+
 template <class Real, Curve C>
 void launchKeygenT(const Real *x, const Real *y, const Real *z, size_t n, const KeygenParams<Real> &prm, u64 *keys,
-                   u32 *hist, int passes, cudaStream_t s)
+                   const KeygenSort &ks, cudaStream_t s)
 {
+    if (ks.plan)
+        planKernel<Real, C><<<ceilDiv(ks.plan->samples, sort::kPlanThreads), sort::kPlanThreads, 0, s>>>(
+            x, y, z, n, prm, *ks.plan, ks.ctl, ks.hist), noteLaunch();
     const bool vec = aligned16(x) && aligned16(y) && aligned16(z);
     constexpr int V = sizeof(Real) == 4 ? 4 : 2;
     const size_t groups = vec ? n / V : n;
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(std::max<size_t>(groups, 1), kKeygenThreads),
                                                              unsigned(smCount()) * 8u));
-    if (vec) keygenKernel<Real, C, V><<<blocks, kKeygenThreads, 0, s>>>(x, y, z, n, prm, keys, hist, passes), noteLaunch();
-    else keygenKernel<Real, C, 1><<<blocks, kKeygenThreads, 0, s>>>(x, y, z, n, prm, keys, hist, passes), noteLaunch();
+    if (vec) keygenKernel<Real, C, V><<<blocks, kKeygenThreads, 0, s>>>(x, y, z, n, prm, keys, ks.hist, ks.bins, ks.ctl), noteLaunch();
+    else keygenKernel<Real, C, 1><<<blocks, kKeygenThreads, 0, s>>>(x, y, z, n, prm, keys, ks.hist, ks.bins, ks.ctl), noteLaunch();
     AOT_LAUNCH_CHECK();
 }
 
 template <class Real>
 void launchKeygen(int kind, bool hilbert, const Real *x, const Real *y, const Real *z, size_t n,
-                  const KeygenParams<Real> &prm, u64 *keys, u32 *hist, int passes, cudaStream_t s)
+                  const KeygenParams<Real> &prm, u64 *keys, const KeygenSort &ks, cudaStream_t s)
 {
-    if (kind == 1) launchKeygenT<Real, Curve::Binary>(x, y, z, n, prm, keys, hist, passes, s);
-    else if (hilbert) launchKeygenT<Real, Curve::Hilbert>(x, y, z, n, prm, keys, hist, passes, s);
-    else launchKeygenT<Real, Curve::Morton>(x, y, z, n, prm, keys, hist, passes, s);
+    if (kind == 1) launchKeygenT<Real, Curve::Binary>(x, y, z, n, prm, keys, ks, s);
+    else if (hilbert) launchKeygenT<Real, Curve::Hilbert>(x, y, z, n, prm, keys, ks, s);
+    else launchKeygenT<Real, Curve::Morton>(x, y, z, n, prm, keys, ks, s);
 }
 
 __global__ void iotaKernel(u32 *perm, size_t n)
@@ -451,60 +464,72 @@ __global__ void iotaKernel(u32 *perm, size_t n)
         perm[i] = u32(i);
 }
 
-// Sort scratch layout: hist[kPassSlots][256] | bins[kPassSlots][256] |
-// tileCounters[kPassSlots] (u32), then look-back status words (u64): passes x
-// tiles x 256 of configuration `config`, or room for every configuration
-// (config < 0: kPassSlots passes of the smallest tiles).
-struct SortArena
-{
-    DevMem counters, status;
-    void ensure(size_t n, int config, cudaStream_t owner)
-    {
-        counters.reserve((2 * sort::kPassSlots * sort::kRadix + sort::kPassSlots) * sizeof(u32), owner);
-        const size_t words = config < 0
-                                 ? size_t(sort::kPassSlots) * std::max<size_t>(1, (n + sort::kMinTile - 1) / sort::kMinTile)
-                                 : size_t(sort::configPasses(config)) *
-                                       std::max<size_t>(1, (n + sort::configTile(config) - 1) / sort::configTile(config));
-        status.reserve(words * sort::kRadix * sizeof(u64), owner);
-    }
-    u32 *hist() const { return counters.as<u32>(); }
-    u32 *bins() const { return counters.as<u32>() + sort::kPassSlots * sort::kRadix; }
-    u32 *tileCounters() const { return counters.as<u32>() + 2 * sort::kPassSlots * sort::kRadix; }
-};
-
 size_t configTiles(int cfg, size_t n) { return std::max<size_t>(1, (n + sort::configTile(cfg) - 1) / sort::configTile(cfg)); }
 
-// Onesweep passes of configuration `cfg` over (k[0], v[0]) -> ... for bits
-// [beginBit, endBit); the counts must already be in hist.  valsAreIndices:
-// the first pass generates the values.  Returns the index (0/1) of the
-// buffers holding the result.
-int runPasses(int cfg, cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int beginBit, int endBit, bool valsAreIndices,
-              SortArena &a, int *error)
+// Sort scratch in one block: the control block, the plan's counters,
+// hist[kPassSlots][256] and bins[kPassSlots][256]; the look-back status words
+// (u64) of one pass, with room for every configuration (their tags tell the
+// passes apart); and for a planned sort the list of long runs and the
+// plan's table.
+struct SortArena
+{
+    DevMem mem;
+    size_t longAt = 0, tableAt = 0;
+    sort::PlanArgs plan{};
+    static size_t up(size_t b) { return (b + 255) & ~size_t(255); }
+    static constexpr size_t kPlanAt = (sizeof(sort::SortControl) + 15) & ~size_t(15);
+    static constexpr size_t kHistAt = (kPlanAt + sizeof(sort::PlanCounters) + 255) & ~size_t(255);
+    static constexpr size_t kHistWords = size_t(sort::kPassSlots) * sort::kRadix;
+    static constexpr size_t kStatusAt = kHistAt + 2 * kHistWords * sizeof(u32);
+    void ensure(size_t n, cudaStream_t owner, bool planned)
+    {
+        const size_t tiles = std::max<size_t>(1, (n + sort::kMinTile - 1) / sort::kMinTile);
+        longAt = up(kStatusAt + tiles * sort::kRadix * sizeof(u64));
+        tableAt = up(longAt + (planned ? sort::longRunSlots(n) * sizeof(u32) : 0));
+        const void *before = mem.p;
+        mem.reserve(tableAt + (planned ? sort::planTableBytes(n) : 0), owner);
+        // words left by another owner of the block could carry a tag this
+        // arena will use: a new block starts cleared
+        if (mem.p != before) AOT_CHECK(cudaMemsetAsync(mem.p, 0, mem.bytes, owner));
+        if (!planned) return;
+        plan.table = reinterpret_cast<u64 *>(at(tableAt));
+        plan.counters = reinterpret_cast<sort::PlanCounters *>(at(kPlanAt));
+        plan.samples = sort::planSamples(n);
+        plan.slotBits = sort::planSlotBits(n);
+    }
+    unsigned char *at(size_t offset) const { return mem.as<unsigned char>() + offset; }
+    sort::SortControl *ctl() const { return mem.as<sort::SortControl>(); }
+    u32 *hist() const { return reinterpret_cast<u32 *>(at(kHistAt)); }
+    u32 *bins() const { return hist() + kHistWords; }
+    u64 *status() const { return reinterpret_cast<u64 *>(at(kStatusAt)); }
+    u32 *longRuns() const { return reinterpret_cast<u32 *>(at(longAt)); }
+};
+
+// The passes of configuration `cfg` over (k[0], v[0]) -> ... for bits [0,
+// endBit), the input indices as values; the digit starts must be in bins.
+// Without a plan all passes run, and the index (0/1) of the buffers holding
+// the result is returned; with one, the repair puts it into buffers 0
+// (and writes the sample).
+int runPasses(int cfg, cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int endBit, SortArena &a, int *error, bool plan,
+              u64 *sample = nullptr)
 {
     sort::setPassSmemAll();
     const int bitsPer = sort::kSortConfigs[cfg].bits;
-    const int passes = (endBit - beginBit + bitsPer - 1) / bitsPer;
-    const size_t tiles = configTiles(cfg, n);
-    sort::binsKernel<<<1, sort::kRadix, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
-    AOT_LAUNCH_CHECK();
-    for (int p = 0; p < passes; ++p)
+    const int passes = (endBit + bitsPer - 1) / bitsPer;
+    sort::PassArgs p{k[0], nullptr, {k[0], k[1]}, {v[0], v[1]}, n, a.bins(), a.ctl(), a.status(), error,
+                     0, endBit, passes, false};
+    for (int slot = 0; slot < passes; ++slot)
     {
-        const int in = p & 1, out = in ^ 1;
-        const int shift = beginBit + p * bitsPer;
-        sort::launchPass(cfg, s, k[in], (p == 0 && valsAreIndices) ? nullptr : v[in], k[out], v[out], n, shift,
-                         a.bins() + p * sort::kRadix, a.tileCounters() + p,
-                         a.status.as<u64>() + size_t(p) * tiles * sort::kRadix, error, std::min(bitsPer, endBit - shift)),
-            noteLaunch();
+        sort::launchPass(cfg, s, p, slot), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
-    return passes & 1;
-}
-
-// Zeroes the counters and the status words configuration `cfg` reads.
-void clearArena(int cfg, cudaStream_t s, SortArena &a, size_t n, int passes)
-{
-    AOT_CHECK(cudaMemsetAsync(a.counters.p, 0, a.counters.bytes, s));
-    AOT_CHECK(cudaMemsetAsync(a.status.p, 0, size_t(passes) * configTiles(cfg, n) * sort::kRadix * sizeof(u64), s));
+    if (!plan) return passes & 1;
+    const sort::RepairArgs r{{k[0], k[1]}, {v[0], v[1]}, n, a.ctl(), a.longRuns(), sample, error,
+                             0, passes, ~u64(0), false, true, true};
+    sort::repairKernel<true><<<sort::repairTiles(n), sort::kRepairThreads, 0, s>>>(r), noteLaunch();
+    sort::longRunKernel<<<unsigned(smCount()) * 2u, sort::kLongThreads, 0, s>>>(r), noteLaunch();
+    AOT_LAUNCH_CHECK();
+    return 0;
 }
 
 // Generic stable sort of (keys, identity indices) by bits [0, 8*passes),
@@ -513,12 +538,13 @@ int sortWithIndices(cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int passes, 
 {
     if (n == 0) return 0;
     const int cfg = sort::kDefaultSortConfig;
-    a.ensure(n, cfg, s);
-    clearArena(cfg, s, a, n, passes);
+    a.ensure(n, s, false);
+    sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
     sort::launchHistogram(cfg, s, blocks, k[0], n, 0, passes, a.hist(), 8 * passes), noteLaunch();
+    sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
     AOT_LAUNCH_CHECK();
-    return runPasses(cfg, s, k, v, n, 0, 8 * passes, true, a, error);
+    return runPasses(cfg, s, k, v, n, 8 * passes, a, error, false);
 }
 
 }  // namespace
@@ -651,11 +677,12 @@ struct PairSortLayout
     // altKeys | altVals | counters | status, each part 256-byte aligned.  The
     // counters part starts with the error word (and 3 pad words), so its
     // offset depends on n only and ao_sort_pairs_check can find it whatever
-    // configuration ran; then hist[passes][256], bins[passes][256] and the
-    // passes' tile counters.
+    // configuration ran; then the control block, hist[passes][256] and
+    // bins[passes][256].
     size_t altKeys = 0, altVals = 0, counters = 0, status = 0, total = 0, tiles = 0;
     int passes = 0;
     static constexpr size_t kCounterHead = 4;  // error word + padding (u32 words)
+    static constexpr size_t kCtlWords = (sizeof(sort::SortControl) / sizeof(u32) + 3) & ~size_t(3);
     static size_t up(size_t b) { return (b + 255) & ~size_t(255); }
     static size_t countersOffset(size_t n) { return up(up(n * sizeof(u64)) + n * sizeof(u32)); }
     PairSortLayout(size_t n, int cfg)
@@ -666,9 +693,9 @@ struct PairSortLayout
         altVals = up(altKeys + n * sizeof(u64));
         counters = countersOffset(n);
         status = up(counters + counterWords() * sizeof(u32));
-        total = up(status + size_t(passes) * tiles * sort::kRadix * sizeof(u64));
+        total = up(status + tiles * sort::kRadix * sizeof(u64));
     }
-    size_t counterWords() const { return kCounterHead + 2 * size_t(passes) * sort::kRadix + passes; }
+    size_t counterWords() const { return kCounterHead + kCtlWords + 2 * size_t(passes) * sort::kRadix; }
 };
 }  // namespace
 
@@ -720,11 +747,10 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     u32 *altV = reinterpret_cast<u32 *>(base + lay.altVals);
     u32 *head = reinterpret_cast<u32 *>(base + lay.counters);
     int *error = reinterpret_cast<int *>(head);
-    u32 *ctr = head + PairSortLayout::kCounterHead;  // hist
+    sort::SortControl *ctl = reinterpret_cast<sort::SortControl *>(head + PairSortLayout::kCounterHead);
+    u32 *hist = head + PairSortLayout::kCounterHead + PairSortLayout::kCtlWords;
+    u32 *bins = hist + size_t(lay.passes) * sort::kRadix;
     u64 *status = reinterpret_cast<u64 *>(base + lay.status);
-    const int slots = lay.passes;  // rows of hist and bins
-    u32 *bins = ctr + size_t(slots) * sort::kRadix;
-    u32 *tileCounters = ctr + 2 * size_t(slots) * sort::kRadix;
     const int bitsPer = sort::kSortConfigs[cfg].bits;
     const int passes = (endBit - beginBit + bitsPer - 1) / bitsPer;
     if (passes == 0)
@@ -737,29 +763,20 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
         return;
     }
     AOT_CHECK(cudaMemsetAsync(head, 0, lay.counterWords() * sizeof(u32), s));
-    AOT_CHECK(cudaMemsetAsync(status, 0, size_t(passes) * lay.tiles * sort::kRadix * sizeof(u64), s));
+    AOT_CHECK(cudaMemsetAsync(status, 0, lay.tiles * sort::kRadix * sizeof(u64), s));
+    sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(ctl, nullptr), noteLaunch();
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
-    sort::launchHistogram(cfg, s, blocks, reinterpret_cast<const u64 *>(keysIn), n, beginBit, passes, ctr, endBit),
+    sort::launchHistogram(cfg, s, blocks, reinterpret_cast<const u64 *>(keysIn), n, beginBit, passes, hist, endBit),
         noteLaunch();
-    sort::binsKernel<<<1, sort::kRadix, 0, s>>>(ctr, bins, passes), noteLaunch();
+    sort::binsKernel<<<1, sort::kThreads, 0, s>>>(hist, bins, passes), noteLaunch();
     AOT_LAUNCH_CHECK();
     sort::setPassSmemAll();
-    const u64 *kin = reinterpret_cast<const u64 *>(keysIn);
-    const u32 *vin = valsIn;
-    for (int p = 0; p < passes; ++p)
+    const sort::PassArgs p{reinterpret_cast<const u64 *>(keysIn), valsIn, {reinterpret_cast<u64 *>(keysOut), altK},
+                           {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes, true};
+    for (int slot = 0; slot < passes; ++slot)
     {
-        // the last pass writes keysOut; earlier passes alternate backwards from it
-        const bool toOut = ((passes - 1 - p) & 1) == 0;
-        u64 *kout = toOut ? reinterpret_cast<u64 *>(keysOut) : altK;
-        u32 *vout = toOut ? valsOut : altV;
-        const int shift = beginBit + p * bitsPer;
-        const int bits = std::min(bitsPer, endBit - shift);
-        sort::launchPass(cfg, s, kin, vin, kout, vout, n, shift, bins + p * sort::kRadix, tileCounters + p,
-                         status + size_t(p) * lay.tiles * sort::kRadix, error, bits),
-            noteLaunch();
+        sort::launchPass(cfg, s, p, slot), noteLaunch();
         AOT_LAUNCH_CHECK();
-        kin = kout;
-        vin = vout;
     }
 }
 
@@ -782,6 +799,7 @@ void TreeEngine::sortPairsPreload()
 {
     cudaFuncAttributes a;
     AOT_CHECK(cudaFuncGetAttributes(&a, iotaKernel));
+    AOT_CHECK(cudaFuncGetAttributes(&a, sort::beginSortKernel));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::binsKernel));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<8>));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<7>));
@@ -868,7 +886,7 @@ struct TreeEngine::Impl
     size_t bytes() const
     {
         const DevMem *all[] = {&P[0],        &P[1],        &Perm[0],        &Perm[1],      &sample,
-                               &sortArena.counters, &sortArena.status, &stMem, &history, &K[0],
+                               &sortArena.mem, &stMem, &history, &K[0],
                                &K[1],        &B[0],        &B[1],           &NF[0],        &NF[1],
                                &N[0],        &N[1],        &G[0],           &G[1],         &offs,
                                &dirty,       &scan,        &vBox,           &vSplit,       &vDepth,
@@ -877,7 +895,7 @@ struct TreeEngine::Impl
                                &vCandStart,  &vCandLevel,  &vLvKeys[0],     &vLvKeys[1],   &vLvVals[0],
                                &vLvVals[1],  &vLayKeys[0], &vLayKeys[1],    &vLayVals[0],  &vLayVals[1],
                                &vIntStartSfc, &vIntLevelSfc, &vIntM,        &vIntStartLay, &vIntLevelLay,
-                               &viewSort.counters, &viewSort.status, &nodeRows, &lvRows, &lvVal, &lvChild,
+                               &viewSort.mem, &nodeRows, &lvRows, &lvVal, &lvChild,
                                &lvLeaves, &lvOffset, &lvCtl, &lvNbr, &lvParent};
         size_t s = 0;
         for (const DevMem *d : all) s += d->bytes;
@@ -988,7 +1006,7 @@ TreeEngine::TreeEngine(const void *x, const void *y, const void *z, size_t n, co
             m_->Perm[k].reserve(n * sizeof(u32));
         }
         m_->sample.reserve(((n + kSampleStride - 1) >> kSampleShift) * sizeof(u64));
-        m_->sortArena.ensure(n, sort::kDefaultSortConfig, cfg.stream);
+        m_->sortArena.ensure(n, cfg.stream, true);
     }
     ensurePhysical(16);
     if (cfg.kind == 0)
@@ -1129,7 +1147,6 @@ void TreeEngine::sortParticles()
         // timed run are the sorted keys
         if (!m_->tuneStart) AOT_CHECK(cudaEventCreate(&m_->tuneStart));
         if (!m_->tuneEnd) AOT_CHECK(cudaEventCreate(&m_->tuneEnd));
-        m_->sortArena.ensure(n_, -1, s);
         auto time = [](int c, void *ctx) -> float {
             TreeEngine &e = *static_cast<TreeEngine *>(ctx);
             AOT_CHECK(cudaEventRecord(e.m_->tuneStart, e.cfg_.stream));
@@ -1140,11 +1157,7 @@ void TreeEngine::sortParticles()
             AOT_CHECK(cudaEventElapsedTime(&ms, e.m_->tuneStart, e.m_->tuneEnd));
             return ms;
         };
-        const int best = sortTune(false, n_, time, this);
-        // keep only the chosen configuration's status words
-        waitStream(s);
-        m_->sortArena.status.release();
-        m_->sortArena.ensure(n_, best, s);
+        sortTune(false, n_, time, this);
     }
     else if (capture != cudaStreamCaptureStatusNone && sortConfig_ >= 0)
     {
@@ -1152,43 +1165,41 @@ void TreeEngine::sortParticles()
     }
     else
     {
-        const int config = sortTuning(false, n_).config;
-        m_->sortArena.ensure(n_, config, s);
-        sortKeys(config);
+        sortKeys(sortTuning(false, n_).config);
     }
-    const KeyIndex idx = m_->keyIndex(n_);
-    rb::sampleKeysKernel<<<gridFor(idx.ns, 256), 256, 0, s>>>(m_->P[0].as<u64>(), n_, m_->sample.as<u64>(), idx.ns),
-        noteLaunch();
-    AOT_LAUNCH_CHECK();
 }
 
 // Keys of every particle, then the stable (key, slot) sort with sort
-// configuration `config`; the result lands in P[0] / Perm[0].
+// configuration `config`; the result lands in P[0] / Perm[0], every 32nd key
+// in the sample.
 void TreeEngine::sortKeys(int config)
 {
     cudaStream_t s = cfg_.stream;
     SortArena &a = m_->sortArena;
     const int passes = sort::configPasses(config);
     if (passes & 1) throw std::logic_error("adaptive_octree: sort configurations must have an even pass count");
-    clearArena(config, s, a, n_, passes);
     u64 *k[2] = {m_->P[0].as<u64>(), m_->P[1].as<u64>()};
     u32 *v[2] = {m_->Perm[0].as<u32>(), m_->Perm[1].as<u32>()};
-    // 8-bit digits: the histogram comes with the keys; otherwise a pass of its own
-    const bool fused = sort::kSortConfigs[config].bits == sort::kRadixBits;
-    const int histPasses = fused ? sort::kMaxPasses : 0;
+    // 8-bit digits: a plan, and the digit counts come with the keys; otherwise
+    // every pass, and the counts by a kernel of their own
+    const bool planned = sort::kSortConfigs[config].bits == sort::kRadixBits;
+    const KeygenSort ks = planned ? KeygenSort{a.hist(), a.bins(), a.ctl(), &a.plan} : KeygenSort{};
     if (cfg_.real == 0)
         launchKeygen<float>(cfg_.kind, cfg_.hilbert, static_cast<const float *>(x_), static_cast<const float *>(y_),
-                            static_cast<const float *>(z_), n_, m_->kpf, k[0], a.hist(), histPasses, s);
+                            static_cast<const float *>(z_), n_, m_->kpf, k[0], ks, s);
     else
         launchKeygen<double>(cfg_.kind, cfg_.hilbert, static_cast<const double *>(x_), static_cast<const double *>(y_),
-                             static_cast<const double *>(z_), n_, m_->kpd, k[0], a.hist(), histPasses, s);
-    if (!fused)
+                             static_cast<const double *>(z_), n_, m_->kpd, k[0], ks, s);
+    if (!planned)
     {
+        sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
         const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n_, sort::kThreads), unsigned(smCount()) * 8u));
         sort::launchHistogram(config, s, blocks, k[0], n_, 0, passes, a.hist(), 64), noteLaunch();
+        sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
-    runPasses(config, s, k, v, n_, 0, 64, true, a, &m_->st->error);  // an even pass count ends in buffer 0
+    // (without a plan the repair finds all passes run and writes the sample alone)
+    runPasses(config, s, k, v, n_, 64, a, &m_->st->error, true, m_->sample.as<u64>());
     sortConfig_ = config;
 }
 
@@ -1207,10 +1218,10 @@ void TreeEngine::computeKeys(int kind, int real, const void *x, const void *y, c
     pf.h = pd.h = hilbertTables();
     if (real == 0)
         launchKeygen<float>(kind, hilbert, static_cast<const float *>(x), static_cast<const float *>(y),
-                            static_cast<const float *>(z), n, pf, reinterpret_cast<u64 *>(keys), nullptr, 0, s);
+                            static_cast<const float *>(z), n, pf, reinterpret_cast<u64 *>(keys), {}, s);
     else
         launchKeygen<double>(kind, hilbert, static_cast<const double *>(x), static_cast<const double *>(y),
-                             static_cast<const double *>(z), n, pd, reinterpret_cast<u64 *>(keys), nullptr, 0, s);
+                             static_cast<const double *>(z), n, pd, reinterpret_cast<u64 *>(keys), {}, s);
     if (perm)
     {
         iotaKernel<<<gridFor(n, 256), 256, 0, s>>>(perm, n), noteLaunch();
@@ -2190,7 +2201,7 @@ void TreeEngine::prepareViews(size_t capacity, const adaptive_octree::ViewConfig
     m.vIntM.reserve(std::max<size_t>(I, 1) * 4, s);
     m.vIntStartLay.reserve(std::max<size_t>(I, 1) * 8, s);
     m.vIntLevelLay.reserve(std::max<size_t>(I, 1), s);
-    m.viewSort.ensure(L, sort::kDefaultSortConfig, s);
+    m.viewSort.ensure(L, s, false);
 }
 
 void TreeEngine::syncViewSizes()

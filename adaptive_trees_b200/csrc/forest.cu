@@ -425,7 +425,7 @@ void ForestEngine::sortKeys(int config)
                                        m.bins.as<u32>() + size_t(p) * m.S * sort::kRadix};
         sort::launchSegmentPass(config, s, m.numTiles, tiles, k[in], p == 0 ? nullptr : v[in], k[out], v[out], shift,
                                 m.tileCounters.as<u32>() + p, m.status.as<u64>() + size_t(p) * m.numTiles * sort::kRadix,
-                                &m.st.as<forest::State>()->error, std::min(bitsPer, 64 - shift)),
+                                sort::passTag(1), &m.st.as<forest::State>()->error, std::min(bitsPer, 64 - shift)),
             noteLaunch();
         AOT_LAUNCH_CHECK();
     }

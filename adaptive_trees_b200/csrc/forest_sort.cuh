@@ -60,7 +60,7 @@ __device__ __forceinline__ void sortPass(const SortArgs &p)
         sort::SegmentTiles{p.tiles.tileSeg, p.tiles.tileBegin, p.tiles.tileEnd, p.tiles.segFirstTile, p.tiles.segBase,
                            p.bins + size_t(Q) * p.f.numSystems * sort::kRadix},
         p.keys[Q & 1], Q == 0 ? nullptr : p.vals[Q & 1], p.keys[(Q & 1) ^ 1], p.vals[(Q & 1) ^ 1], shift,
-        p.tileCounters + Q, p.status + size_t(Q) * p.numTiles * sort::kRadix, p.error, bits, sort::kLookbackSpins,
+        p.tileCounters + Q, p.status + size_t(Q) * p.numTiles * sort::kRadix, sort::passTag(1), p.error, bits, sort::kLookbackSpins,
         p.numTiles))
         __syncthreads();
 }

@@ -4,13 +4,15 @@
 // computeSfcKeysBinaryKernel (kdtree3d_rebalance.cuh:247-273).  Each CTA
 // streams coordinates with 128-bit loads (4 floats or 2 doubles per axis per
 // thread step), writes the keys with 128-bit stores and accumulates the digit
-// counts of all eight radix passes in shared memory, so the sort never
+// counts of the sort's passes in shared memory, so the sort never
 // re-reads the keys for its histogram.  The identity permutation is not
-// written: the first sort pass generates it from the input index.
+// written: the first sort pass generates it from the input index.  A plan
+// kernel before it (planKernel) samples the keys and picks the passes; the
+// last CTA to add its counts turns them into the passes' digit starts.
 #pragma once
 
-#include "radix_sort.cuh"
 #include "sfc.cuh"
+#include "sort_plan.cuh"
 
 namespace aot
 {
@@ -46,34 +48,54 @@ __device__ __forceinline__ u64 particleKey(Real x, Real y, Real z, const KeygenP
 
 constexpr int kKeygenThreads = 256;
 
+// The two-level Hilbert table in shared memory, from the one-level tables.
+template <class Real>
+__device__ __forceinline__ void loadPairTable(const KeygenParams<Real> &prm, unsigned short *sPair)
+{
+    __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8];
+    for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x)
+    {
+        sEnc[i] = prm.h.enc[i];
+        sNext[i] = prm.h.encNext[i];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kHilbertPairEntries; i += blockDim.x) sPair[i] = hilbertPairEntry(i, sEnc, sNext);
+}
+
+// Start of a planned sort: the control block, zeroed digit counts and the
+// plan, from the keys of particles at random positions.
+template <class Real, Curve C>
+static __global__ void __launch_bounds__(sort::kPlanThreads)
+    planKernel(const Real *__restrict__ x, const Real *__restrict__ y, const Real *__restrict__ z, size_t n,
+               const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist)
+{
+    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    __syncthreads();
+    const auto keyAt = [&](size_t i, u32 &) { return particleKey<Real, C>(x[i], y[i], z[i], prm, sPair); };
+    sort::planSort(keyAt, n, plan, ctl, hist, size_t(sort::kPassSlots) * sort::kRadix);
+}
+
 // Vec: particles per thread step (4 for float4, 2 for double2, 1 scalar).
+// hist (with bins and ctl) or nullptr: the digit counts of the plan's passes
+// and their starts.
 template <class Real, Curve C, int Vec>
 static __global__ void __launch_bounds__(kKeygenThreads)
     keygenKernel(const Real *__restrict__ x, const Real *__restrict__ y, const Real *__restrict__ z, size_t n,
-                 const KeygenParams<Real> prm, u64 *__restrict__ keys, u32 *__restrict__ hist, int histPasses)
+                 const KeygenParams<Real> prm, u64 *__restrict__ keys, u32 *__restrict__ hist,
+                 u32 *__restrict__ bins, sort::SortControl *ctl)
 {
     __shared__ u32 sh[sort::kMaxPasses][sort::kRadix];
     __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
-    if constexpr (C == Curve::Hilbert)
-    {
-        // the one-level tables staged in shared memory, then the pair table from them
-        __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8];
-        for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x)
-        {
-            sEnc[i] = prm.h.enc[i];
-            sNext[i] = prm.h.encNext[i];
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < kHilbertPairEntries; i += blockDim.x)
-            sPair[i] = hilbertPairEntry(i, sEnc, sNext);
-    }
+    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    const int firstPass = hist ? int(ctl->first) : sort::kMaxPasses;
     __syncthreads();
 
     auto count = [&](u64 k) {
 #pragma unroll
         for (int p = 0; p < sort::kMaxPasses; ++p)
-            if (p < histPasses) atomicAdd(&sh[p][(k >> (p * sort::kRadixBits)) & (sort::kRadix - 1)], 1u);
+            if (p >= firstPass) atomicAdd(&sh[p][(k >> (p * sort::kRadixBits)) & (sort::kRadix - 1)], 1u);
     };
 
     const size_t groups = n / Vec;
@@ -135,12 +157,22 @@ static __global__ void __launch_bounds__(kKeygenThreads)
         keys[i] = k;
         count(k);
     }
+    if (!hist) return;
     __syncthreads();
-    for (int i = threadIdx.x; i < histPasses * sort::kRadix; i += blockDim.x)
+    for (int i = firstPass * sort::kRadix + threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x)
     {
         const u32 v = (&sh[0][0])[i];
         if (v) atomicAdd(hist + i, v);
     }
+    // the last CTA: the digit starts of every pass
+    __shared__ bool sLast;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sLast = atomicAdd(&ctl->keygenDone, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!sLast) return;
+    __threadfence();
+    sort::scanBins(hist, bins, firstPass, sort::kMaxPasses);
 }
 
 }  // namespace aot

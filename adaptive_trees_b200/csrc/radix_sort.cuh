@@ -18,6 +18,11 @@
 // The digit width and the keys per thread are template parameters; the
 // configurations compiled in are listed in kSortConfigs, and the sort tuner
 // (sortTune in engine.cu) picks one per device and problem size by timing them.
+//
+// A sort that has a plan (sort_plan.cuh) runs only the passes of its high
+// digits and leaves the rest to a repair of the short runs of equal high
+// digits (sort_repair.cuh).  Every pass is launched and reads the plan on the
+// device; the ones it leaves out return at once.
 // The look-back wait is bounded: after kLookbackSpins polls it records
 // kErrLookback in the device error word and proceeds, so a broken invariant
 // surfaces as an error status instead of a hung GPU.
@@ -40,7 +45,14 @@ constexpr int kPassSlots = 10;              // most passes of any configuration 
 constexpr int kMinTile = kThreads * 8;      // smallest tile of any configuration
 constexpr u64 kFlagAgg = u64(1) << 62;
 constexpr u64 kFlagPrefix = u64(2) << 62;
-constexpr u64 kValueMask = (u64(1) << 62) - 1;
+constexpr u64 kFlagMask = u64(3) << 62;
+// A status word is flag (2 bits) | tag (30 bits) | count (32 bits).  The tag
+// numbers the pass that wrote it, so one array serves every pass of every
+// sort without being cleared between them: a word of another pass reads as
+// not published.  (Cleared arrays of 8 passes were 107 MB of writes and 28 us
+// of a 16Mi sort; one pass' words are 13 MB and stay in L2.)
+constexpr u64 kTagMask = ((u64(1) << 30) - 1) << 32;
+__host__ __device__ constexpr u64 passTag(u32 number) { return (u64(number) << 32) & kTagMask; }
 constexpr unsigned kLookbackSpins = 1u << 22;
 constexpr int kLookbackWindow = 8;
 
@@ -61,18 +73,31 @@ __device__ __forceinline__ unsigned laneMaskLt()
     return m;
 }
 
-// Per-sort scratch laid out by the host (see SortScratch):
-//   hist[kMaxPasses][256] u32 counts, bins[kMaxPasses][256] u32 exclusive
-//   starts, tileCounters[kMaxPasses] u32, status[kMaxPasses][tiles][256] u64.
-struct Scratch
+// Control block of one sort, in device memory.
+struct SortControl
 {
-    u32 *hist;
-    u32 *bins;
-    u32 *tileCounters;
-    u64 *status;
-    int *error;
-    size_t tiles;
+    u32 first;      // the passes run are first .. passes - 1 (0: all of them)
+    u32 epoch;      // number of the sort: pass slot j writes tag epoch + j
+    u32 longRuns;   // runs the repair left to the long-run kernel
+    u32 keygenDone; // CTAs of the key generation that have added their digit counts
+    u32 tileCounters[kPassSlots];
 };
+constexpr u32 kEpochStep = 16;  // tags per sort (>= kPassSlots)
+
+// Start of a sort without a plan: every pass runs.
+static __global__ void __launch_bounds__(kThreads) beginSortKernel(SortControl *ctl, u32 *hist)
+{
+    if (hist)
+        for (int i = threadIdx.x; i < kPassSlots * kRadix; i += blockDim.x) hist[i] = 0;
+    if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
+    if (threadIdx.x == 0)
+    {
+        ctl->first = 0;
+        ctl->epoch += kEpochStep;
+        ctl->longRuns = 0;
+        ctl->keygenDone = 0;
+    }
+}
 
 // Histogram of the Bits-wide digits of keys[0, n) for passes covering
 // [beginBit, endBit); pass p's counts go to hist[p * kRadix + digit].
@@ -103,27 +128,42 @@ static __global__ void __launch_bounds__(kThreads) histogramKernel(const u64 *__
 }
 
 // Exclusive scan of each pass' 256 digit counts (a narrower radix leaves the
-// upper counts zero, so their starts are unused).
-static __global__ void __launch_bounds__(kRadix) binsKernel(const u32 *__restrict__ hist, u32 *__restrict__ bins, int passes)
+// upper counts zero, so their starts are unused).  A warp per pass, eight
+// counts per lane.  __ldcg: the counts may come from other CTAs' atomics.
+__device__ __forceinline__ void scanBins(const u32 *hist, u32 *bins, int firstPass, int passes)
 {
-    __shared__ u32 s[kRadix];
-    const int d = threadIdx.x;
-    for (int p = 0; p < passes; ++p)
+    static_assert(kRadix == 256, "eight counts per lane");
+    const int lane = threadIdx.x & 31;
+    for (int p = firstPass + int(threadIdx.x >> 5); p < passes; p += int(blockDim.x >> 5))
     {
-        const u32 v = hist[p * kRadix + d];
-        s[d] = v;
-        __syncthreads();
-        // Hillis-Steele inclusive scan over 256 entries
-        for (int off = 1; off < kRadix; off <<= 1)
+        const uint4 *h = reinterpret_cast<const uint4 *>(hist + p * kRadix) + lane * 2;
+        const uint4 a = __ldcg(h), b = __ldcg(h + 1);
+        const u32 c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        u32 sum = 0, e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
         {
-            const u32 t = d >= off ? s[d - off] : 0u;
-            __syncthreads();
-            s[d] += t;
-            __syncthreads();
+            e[i] = sum;
+            sum += c[i];
         }
-        bins[p * kRadix + d] = s[d] - v;
-        __syncthreads();
+        u32 inc = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += t;
+        }
+        const u32 base = inc - sum;
+        uint4 *o = reinterpret_cast<uint4 *>(bins + p * kRadix) + lane * 2;
+        o[0] = make_uint4(base + e[0], base + e[1], base + e[2], base + e[3]);
+        o[1] = make_uint4(base + e[4], base + e[5], base + e[6], base + e[7]);
     }
+}
+
+static __global__ void __launch_bounds__(kThreads) binsKernel(const u32 *__restrict__ hist, u32 *__restrict__ bins,
+                                                              int passes)
+{
+    scanBins(hist, bins, 0, passes);
 }
 
 template <int Bits, int Items>
@@ -267,7 +307,7 @@ template <int Bits, int Items, class Tiles>
 __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__restrict__ keysIn,
                                              const u32 *__restrict__ valsIn, u64 *__restrict__ keysOut,
                                              u32 *__restrict__ valsOut, int shift, u32 *tileCounter, u64 *status,
-                                             int *error, int bits, unsigned spinLimit = kLookbackSpins,
+                                             u64 tag, int *error, int bits, unsigned spinLimit = kLookbackSpins,
                                              u32 numTiles = 0xffffffffu)
 {
     using Smem = SharedPass<Bits, Items>;
@@ -367,7 +407,7 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
     {
         const int d = tid;
         const u32 cnt = d < R ? sm.count[d] : 0u;
-        if (d < R) stRelaxed(status + tile * R + d, (tiles.chainStart(tile) ? kFlagPrefix : kFlagAgg) | u64(cnt));
+        if (d < R) stRelaxed(status + tile * R + d, (tiles.chainStart(tile) ? kFlagPrefix : kFlagAgg) | tag | u64(cnt));
         // exclusive scan of the tile's digit counts -> local starts
         u32 v = cnt;
 #pragma unroll
@@ -421,8 +461,8 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
     if (tid < R)
     {
         const int d = tid;
-        const u64 total = sm.count[d];
-        u64 excl = 0;
+        const u32 total = sm.count[d];
+        u32 excl = 0;  // keys are fewer than 2^32
         if (!tiles.chainStart(tile))
         {
             // Walk back over earlier tiles, eight status words per round trip,
@@ -435,15 +475,14 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
                 u64 w8[kLookbackWindow];
 #pragma unroll
                 for (int k = 0; k < kLookbackWindow; ++k)
-                    w8[k] = j - k >= 0 ? ldRelaxed(status + size_t(j - k) * R + d) : kFlagPrefix;
+                    w8[k] = j - k >= 0 ? ldRelaxed(status + size_t(j - k) * R + d) : (kFlagPrefix | tag);
                 int k = 0;
                 bool done = false;
                 for (; k < kLookbackWindow; ++k)
                 {
-                    const u64 flag = w8[k] & ~kValueMask;
-                    if (flag == 0) break;
-                    excl += w8[k] & kValueMask;
-                    if (flag == kFlagPrefix)
+                    if ((w8[k] & kTagMask) != tag) break;  // not published in this pass
+                    excl += u32(w8[k]);
+                    if ((w8[k] & kFlagMask) == kFlagPrefix)
                     {
                         done = true;
                         break;
@@ -461,10 +500,10 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
                     if (spins > 64) __nanosleep(64);
                 }
             }
-            stRelaxed(status + tile * R + d, kFlagPrefix | (excl + total));
+            stRelaxed(status + tile * R + d, kFlagPrefix | tag | u64(excl + total));
         }
         // modulo 2^32: gstart + j is exact for every key of digit d
-        sm.gstart[d] = tiles.digitBase(tile)[d] + u32(excl) - sm.localStart[d];
+        sm.gstart[d] = tiles.digitBase(tile)[d] + excl - sm.localStart[d];
     }
     __syncthreads();
     const size_t remain = tiles.end(tile) - tileBase;
@@ -495,17 +534,38 @@ constexpr int passMinBlocks()
     return Items <= 12 ? 4 : 3;
 }
 
-// One onesweep pass over keys[0, n): digit at bit `shift` (`bits` wide).
-// valsIn == nullptr means values are the input indices (first pass).  The
-// look-back status holds one word per tile and digit of the radix.
-template <int Bits, int Items>
-static __global__ void __launch_bounds__(kThreads, passMinBlocks<Bits, Items>())
-    onesweepKernel(const u64 *__restrict__ keysIn, const u32 *__restrict__ valsIn, u64 *__restrict__ keysOut,
-                   u32 *__restrict__ valsOut, size_t n, int shift, const u32 *__restrict__ bins, u32 *tileCounter,
-                   u64 *status, int *error, int bits)
+// One contiguous sort: the passes of digits [beginBit, endBit) over n keys.
+// Slot j runs pass first + j, from the keys of slot j - 1 (slot 0: keysIn and
+// valsIn, or the input indices as values where valsIn is nullptr).  Slot j
+// writes buffer (j + 1) & 1; with endsIn0 the buffers alternate backwards from
+// the last pass instead, which then writes buffer 0.
+struct PassArgs
 {
-    onesweepTile<Bits, Items>(ContiguousTiles<kThreads * Items>{n, bins}, keysIn, valsIn, keysOut, valsOut, shift,
-                              tileCounter, status, error, bits);
+    const u64 *keysIn;
+    const u32 *valsIn;
+    u64 *k[2];
+    u32 *v[2];
+    size_t n;
+    const u32 *bins;
+    SortControl *ctl;
+    u64 *status;  // one word per tile and digit of the radix
+    int *error;
+    int beginBit, endBit, passes;
+    bool endsIn0;
+};
+
+template <int Bits, int Items>
+static __global__ void __launch_bounds__(kThreads, passMinBlocks<Bits, Items>()) onesweepKernel(PassArgs p, int slot)
+{
+    const int first = int(p.ctl->first), pass = first + slot;
+    if (pass >= p.passes) return;
+    const int out = (p.endsIn0 ? p.passes - 1 - pass : slot + 1) & 1;
+    const int shift = p.beginBit + pass * Bits;
+    const u64 *keysIn = slot ? (out ? p.k[0] : p.k[1]) : p.keysIn;
+    const u32 *valsIn = slot ? (out ? p.v[0] : p.v[1]) : p.valsIn;
+    onesweepTile<Bits, Items>(ContiguousTiles<kThreads * Items>{p.n, p.bins + pass * kRadix}, keysIn, valsIn,
+                              out ? p.k[1] : p.k[0], out ? p.v[1] : p.v[0], shift, p.ctl->tileCounters + slot,
+                              p.status, passTag(p.ctl->epoch + u32(slot)), p.error, min(Bits, p.endBit - shift));
 }
 
 // One onesweep pass over the segments of a forest: every segment is sorted
@@ -514,9 +574,9 @@ template <int Bits, int Items>
 static __global__ void __launch_bounds__(kThreads, passMinBlocks<Bits, Items>())
     segmentOnesweepKernel(SegmentTiles tiles, const u64 *__restrict__ keysIn, const u32 *__restrict__ valsIn,
                           u64 *__restrict__ keysOut, u32 *__restrict__ valsOut, int shift, u32 *tileCounter,
-                          u64 *status, int *error, int bits)
+                          u64 *status, u64 tag, int *error, int bits)
 {
-    onesweepTile<Bits, Items>(tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, error, bits);
+    onesweepTile<Bits, Items>(tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, tag, error, bits);
 }
 
 // ---------------------------------------------------------------------------
@@ -555,18 +615,14 @@ static inline void setPassSmemAll()
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
 
-// One contiguous pass of configuration c over n keys.
-static inline void launchPass(int c, cudaStream_t s, const u64 *keysIn, const u32 *valsIn, u64 *keysOut, u32 *valsOut,
-                       size_t n, int shift, const u32 *bins, u32 *tileCounter, u64 *status, int *error, int bits)
+// Pass slot `slot` of a contiguous sort with configuration c.
+static inline void launchPass(int c, cudaStream_t s, const PassArgs &p, int slot)
 {
-    const unsigned tiles = unsigned((n + size_t(configTile(c)) - 1) / size_t(configTile(c)));
+    const unsigned tiles = unsigned((p.n + size_t(configTile(c)) - 1) / size_t(configTile(c)));
     switch (c)
     {
 #define AOT_CASE(i, B, I)                                                                                        \
-    case i:                                                                                                      \
-        onesweepKernel<B, I><<<tiles, kThreads, sizeof(SharedPass<B, I>), s>>>(                                  \
-            keysIn, valsIn, keysOut, valsOut, n, shift, bins, tileCounter, status, error, bits);                 \
-        break;
+    case i: onesweepKernel<B, I><<<tiles, kThreads, sizeof(SharedPass<B, I>), s>>>(p, slot); break;
         AOT_SORT_CONFIGS(AOT_CASE)
 #undef AOT_CASE
     default: throw std::invalid_argument("sort: unknown configuration");
@@ -576,14 +632,14 @@ static inline void launchPass(int c, cudaStream_t s, const u64 *keysIn, const u3
 // One segmented pass of configuration c over `numTiles` tiles.
 static inline void launchSegmentPass(int c, cudaStream_t s, unsigned numTiles, const SegmentTiles &tiles, const u64 *keysIn,
                               const u32 *valsIn, u64 *keysOut, u32 *valsOut, int shift, u32 *tileCounter,
-                              u64 *status, int *error, int bits)
+                              u64 *status, u64 tag, int *error, int bits)
 {
     switch (c)
     {
 #define AOT_CASE(i, B, I)                                                                                        \
     case i:                                                                                                      \
         segmentOnesweepKernel<B, I><<<numTiles, kThreads, sizeof(SharedPass<B, I>), s>>>(                       \
-            tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, error, bits);                   \
+            tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, tag, error, bits);              \
         break;
         AOT_SORT_CONFIGS(AOT_CASE)
 #undef AOT_CASE

@@ -1349,12 +1349,5 @@ static __global__ void beginPassKernel(DeviceState *st)
     st->dirtyCount = 0;
 }
 
-// Sample every kSampleStride-th key for KeyIndex.
-static __global__ void sampleKeysKernel(const u64 *P, size_t n, u64 *sample, size_t ns)
-{
-    for (size_t j = blockIdx.x * size_t(blockDim.x) + threadIdx.x; j < ns; j += size_t(gridDim.x) * blockDim.x)
-        sample[j] = P[j << kSampleShift];
-}
-
 }  // namespace rb
 }  // namespace aot

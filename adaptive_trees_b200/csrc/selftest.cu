@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(sort::kThreads, 1)
                         u64 *status, int *error, unsigned spinLimit)
 {
     sort::onesweepTile<8, kProbeItems>(sort::ContiguousTiles<kProbeTile>{n, bins}, keysIn, nullptr, keysOut,
-                                       valsOut, 0, tileCounter, status, error, 8, spinLimit);
+                                       valsOut, 0, tileCounter, status, sort::passTag(1), error, 8, spinLimit);
 }
 
 __global__ void scanWaitProbeKernel(u64 *status, int *error, unsigned spinLimit, i64 *prefix)

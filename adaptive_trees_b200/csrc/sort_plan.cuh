@@ -1,0 +1,181 @@
+// sort_plan.cuh -- which digits of the keys a sort has to pass over.
+//
+// A radix sort of all 64 bits makes 8 passes, but n keys in space-filling
+// curve order are told apart by their high digits: 16Mi Plummer particles by
+// the first 32 bits, up to runs of a few dozen keys.  A sort with a plan
+// passes over the last D digits only (an LSD sort of the high 8 D bits,
+// stable), and the repair (sort_repair.cuh) orders the keys inside each run
+// of equal high digits.  The result is the sort's whatever the plan is; the
+// plan decides the time alone.
+//
+// The cost of the repair grows with the mean length of the run a key is in,
+// R_D = sum of (run length)^2 / n.  It is estimated from M keys at random
+// positions: two of them fall into the same run with probability R_D / n, so
+// M keys hold about M^2 / 2n x R_D pairs that share their high digits.  Pairs
+// of equal keys need no repair and are taken off (also positions drawn
+// twice); keys that repeat so often that their runs would be long send the
+// sort to all passes.
+#pragma once
+
+#include "radix_sort.cuh"
+
+namespace aot
+{
+namespace sort
+{
+constexpr int kPlanThreads = 256;      // a sampled key per thread
+constexpr u32 kPlanMaxSamples = 8192;
+constexpr int kPlanMinPasses = 2;
+constexpr int kPlanMaxPasses = 6;
+constexpr int kPlanSets = kPlanMaxPasses - kPlanMinPasses + 2;  // a set of prefixes per choice, one of whole keys
+// Cost in passes: the repair's fixed part and its part per key of the mean
+// run.
+constexpr float kRepairCost = 0.5f;
+constexpr float kRunCost = 0.05f;
+// mean run of equal keys above which all passes run (a long run is a CTA's
+// work in the repair)
+constexpr float kMaxRepeats = 64.f;
+
+// splitmix64's finaliser
+__host__ __device__ __forceinline__ u64 mix64(u64 x)
+{
+    x ^= x >> 30;
+    x *= 0xBF58476D1CE4E5B9ull;
+    x ^= x >> 27;
+    x *= 0x94D049BB133111EBull;
+    return x ^ (x >> 31);
+}
+
+// Keys sampled of n: about n / 4 pairs, so that a mean run of one key more
+// is seen two or three times (n up to 16Mi).
+inline u32 planSamples(size_t n)
+{
+    u32 m = 64;
+    while (m < kPlanMaxSamples && u64(m) * m < 4 * u64(n)) m += 64;
+    return m;
+}
+// slots of one set of the sampled prefixes (2^k, at least four per sample)
+inline u32 planSlotBits(size_t n)
+{
+    u32 bits = 8;
+    while ((u32(1) << bits) < 4 * planSamples(n)) ++bits;
+    return bits;
+}
+inline size_t planTableBytes(size_t n) { return (size_t(kPlanSets) << planSlotBits(n)) * sizeof(u64); }
+
+// Counters of one plan (zero between sorts: the last CTA clears them).
+struct PlanCounters
+{
+    u32 repeats[kPlanSets];  // sampled keys whose prefix another one holds already
+    u32 done;                // CTAs that have counted
+};
+
+// The sample and its sets.
+struct PlanArgs
+{
+    u64 *table;  // [kPlanSets][1 << slotBits]: sort number << 32 | the last prefix hashed there
+    PlanCounters *counters;
+    u32 samples, slotBits;
+};
+
+// The first pass to run (0: all 8) for n keys, from the repeats in each set
+// (set 0: whole keys; set s: prefixes of kPlanMinPasses + s - 1 digits).
+__device__ __forceinline__ u32 planFirst(const u32 *repeats, u32 m, size_t n)
+{
+    const float perPair = 2.f * float(n) / (float(m) * float(m));  // mean run per repeated key
+    const u32 equal = repeats[0];
+    if (float(equal) * perPair > kMaxRepeats) return 0;
+    float best = float(kMaxPasses);
+    u32 first = 0;
+    for (int d = kPlanMinPasses; d <= kPlanMaxPasses; ++d)
+    {
+        const u32 r = repeats[d - kPlanMinPasses + 1];
+        const float run = float(r > equal ? r - equal : 0u) * perPair;
+        const float cost = float(d) + kRepairCost + kRunCost * run;
+        if (cost < best)
+        {
+            best = cost;
+            first = u32(kMaxPasses - d);
+        }
+    }
+    return first;
+}
+
+// Position of sampled key i among n: drawn at random, so that the order the
+// keys are stored in (often along the curve already) does not matter.
+__device__ __forceinline__ size_t planPosition(u32 i, size_t n)
+{
+    return size_t(__umul64hi(mix64(u64(i) * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull), u64(n)));
+}
+
+// Start of a sort of n keys: the control block and the digit counts are set
+// up and the plan is made by the last CTA.  keyAt(i, group) is the key at
+// position i and the segment it is sorted in.  A sample per thread, over many
+// CTAs (one CTA took 84 us for 8192: its random loads and shared-memory
+// atomics go through one SM), and one exchange per sample and set, all of a
+// thread's in flight together: a slot holds the last prefix that was hashed
+// to it, so a repeat is missed where another prefix took the slot in between
+// (at most a quarter of the slots are used), which an estimate can bear;
+// sets with probing took 34-48 us in chains of L2 round trips.  Words of
+// earlier sorts match no prefix of this one, so nothing is cleared.
+template <class KeyAt>
+__device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const PlanArgs &a, SortControl *ctl, u32 *hist,
+                                         size_t histWords)
+{
+    __shared__ u32 sRepeats[kPlanSets];
+    __shared__ bool sLast;
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    const u64 epoch = u64(ctl->epoch + kEpochStep) << 32;  // this sort's number (set at the end)
+    if (threadIdx.x < kPlanSets) sRepeats[threadIdx.x] = 0;
+    __syncthreads();
+    for (size_t k = i; k < histWords; k += size_t(gridDim.x) * blockDim.x) hist[k] = 0;
+    u32 group = 0;
+    u64 key = 0;
+    const bool valid = i < a.samples;
+    if (valid) key = keyAt(planPosition(i, n), group);
+    u64 old[kPlanSets], word[kPlanSets];
+#pragma unroll
+    for (int set = 0; set < kPlanSets; ++set)
+    {
+        const int shift = set == 0 ? 0 : 64 - (kPlanMinPasses + set - 1) * kRadixBits;
+        const u64 h = mix64((key >> shift) * 0x9E3779B97F4A7C15ull + group);
+        word[set] = epoch | u32(h);  // the low half stands for the prefix, the high bits pick the slot
+        old[set] = 0;
+        if (valid)
+            old[set] = atomicExch(
+                reinterpret_cast<unsigned long long *>(a.table + (size_t(set) << a.slotBits) + (h >> (64 - a.slotBits))),
+                (unsigned long long)word[set]);
+    }
+#pragma unroll
+    for (int set = 0; set < kPlanSets; ++set)
+    {
+        const u32 c = u32(__popc(__ballot_sync(0xffffffffu, old[set] == word[set])));
+        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sRepeats[set], c);
+    }
+    __syncthreads();
+    if (threadIdx.x < kPlanSets && sRepeats[threadIdx.x])
+        atomicAdd(&a.counters->repeats[threadIdx.x], sRepeats[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sLast = atomicAdd(&a.counters->done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!sLast) return;
+    __threadfence();
+    if (threadIdx.x < kPlanSets)
+    {
+        sRepeats[threadIdx.x] = __ldcg(&a.counters->repeats[threadIdx.x]);
+        a.counters->repeats[threadIdx.x] = 0;
+    }
+    if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        a.counters->done = 0;
+        ctl->first = planFirst(sRepeats, a.samples, n);
+        ctl->epoch += kEpochStep;
+        ctl->longRuns = 0;
+        ctl->keygenDone = 0;
+    }
+}
+}  // namespace sort
+}  // namespace aot

@@ -1,0 +1,100 @@
+"""The planned sort of the particle keys against a stable numpy sort.
+
+The passes cover only the keys' high digits and a repair orders the runs that
+share them, so the cases are runs of every kind: none, short ones that straddle
+the repair's tiles, runs longer than its window, equal keys, escaped particles,
+and inputs on which every pass runs.  All results are integers: equality.
+"""
+import numpy as np
+import pytest
+
+from tests import scenarios as S
+
+pytestmark = pytest.mark.gpu
+
+TILE, RUN = 2048, 256  # the repair's tile and its longest run
+
+
+def uniform(n, seed):
+    return S.uniform_cube(n, seed=seed)
+
+
+def with_cluster(n, members, width, seed):
+    """Uniform particles of which `members` lie within `width` of one point."""
+    x = [a.copy() for a in S.uniform_cube(n, seed=seed)]
+    r = np.random.default_rng(seed + 1)
+    at = r.permutation(n)[:members]
+    for a in x:
+        a[at] = 0.3123456789 + width * r.random(members)
+    return x
+
+
+def stacked(n, copies, seed):
+    """Every particle `copies` times, at shuffled positions."""
+    base = S.uniform_cube(-(-n // copies), seed=seed)
+    order = np.random.default_rng(seed + 1).permutation(-(-n // copies) * copies)[:n]
+    return [np.repeat(a, copies)[order] for a in base]
+
+
+def escaped(n, every, seed):
+    x = [a.copy() for a in S.uniform_cube(n, seed=seed)]
+    for a in x:
+        a[::every] = S.ESC64
+    return x
+
+
+def in_order(n, seed):
+    """Particles already stored along the curve (Morton order of a fine grid)."""
+    x = S.uniform_cube(n, seed=seed)
+    q = [(a * 1024).astype(np.int64) for a in x]
+    key = np.zeros(n, np.int64)
+    for b in range(10):
+        for k, a in enumerate(q):
+            key |= ((a >> b) & 1) << (3 * b + 2 - k)
+    order = np.argsort(key, kind="stable")
+    return [a[order] for a in x]
+
+
+CASES = {
+    "one": uniform(1, 1), "two": uniform(2, 2), "31": uniform(31, 3), "tile-1": uniform(TILE - 1, 4),
+    "tile": uniform(TILE, 5), "tile+1": uniform(TILE + 1, 6), "tile+run": uniform(TILE + RUN, 7),
+    "3tiles+run+1": uniform(3 * TILE + RUN + 1, 8), "40k": uniform(40_009, 9), "700k": uniform(700_001, 10),
+    "plummer": S.plummer_sphere(500_003, seed=11, dtype=np.float32),
+    "run of 200": with_cluster(300_000, 200, 1e-9, 12), "run of 256": with_cluster(300_000, RUN, 1e-9, 13),
+    "run of 257": with_cluster(300_000, RUN + 1, 1e-9, 14), "run of 700": with_cluster(300_000, 700, 1e-9, 15),
+    "run of 3000": with_cluster(1_000_000, 3000, 1e-6, 16), "run of 20000": with_cluster(4_000_000, 20_000, 1e-6, 17),
+    "one cluster": with_cluster(100_000, 100_000, 1e-5, 18),
+    "pairs": stacked(200_000, 2, 19), "stacks of 100": stacked(200_000, 100, 20), "one point": stacked(50_000, 50_000, 21),
+    "escaped": escaped(100_001, 3, 22), "all escaped": escaped(5_000, 1, 23), "few escaped": escaped(500_000, 1000, 24),
+    "in order": in_order(600_000, 25),
+}
+
+
+@pytest.fixture(autouse=True, scope="module")
+def untuned_afterwards():
+    yield
+    import adaptive_trees_b200 as ab
+    ab.forget_sort_tuning()  # other tests start from an untuned library
+
+
+@pytest.mark.parametrize("kind,hilbert", [(0, False), (0, True), (1, False)])
+@pytest.mark.parametrize("name", list(CASES))
+def test_planned_sort_is_the_stable_sort(name, kind, hilbert):
+    import torch
+
+    import adaptive_trees_b200 as ab
+    xs = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in CASES[name]]
+    curve = ab.SfcKind.Hilbert if hilbert else ab.SfcKind.Morton
+    keys = ab.compute_sfc_keys(kind, *xs, sfc_kind=curve).view(torch.int64).cpu().numpy().view(np.uint64)
+    order = np.argsort(keys, kind="stable")
+    t = ab.Tree(kind, *xs, ab.TreeConfig(sfcKind=curve))
+    for step in range(3):  # the first build times the sort configurations; the control block is used again
+        t.build()
+        got_k = t.get("particleKeys_d").view(torch.int64).cpu().numpy().view(np.uint64)
+        got_p = t.get("perm_d").view(torch.int32).cpu().numpy().view(np.uint32)
+        assert np.array_equal(got_k, keys[order]), (name, step)
+        assert np.array_equal(got_p, order.astype(np.uint32)), (name, step)
+        counts = t.get("leafCounts_d").view(torch.int32).cpu().numpy().view(np.uint32)
+        corner = t.get("cornerstone_d").view(torch.int64).cpu().numpy().view(np.uint64)
+        assert np.array_equal(np.diff(np.searchsorted(keys[order], corner)), counts.astype(np.int64)), (name, step)
+    t.close()
