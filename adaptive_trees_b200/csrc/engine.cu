@@ -485,7 +485,7 @@ struct SortArena
     {
         const size_t tiles = std::max<size_t>(1, (n + sort::kMinTile - 1) / sort::kMinTile);
         longAt = up(kStatusAt + tiles * sort::kRadix * sizeof(u64));
-        tableAt = up(longAt + (planned ? sort::longRunSlots(n) * sizeof(u32) : 0));
+        tableAt = up(longAt + (planned ? sort::longRunWords(n) * sizeof(u32) : 0));
         const void *before = mem.p;
         mem.reserve(tableAt + (planned ? sort::planTableBytes(n) : 0), owner);
         // words left by another owner of the block could carry a tag this
@@ -532,12 +532,11 @@ int runPasses(int cfg, cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int endBi
     return 0;
 }
 
-// Generic stable sort of (keys, identity indices) by bits [0, 8*passes),
-// default configuration.
+// Generic stable sort of (keys, identity indices) by bits [0, 8*passes).
 int sortWithIndices(cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int passes, SortArena &a, int *error)
 {
     if (n == 0) return 0;
-    const int cfg = sort::kDefaultSortConfig;
+    const int cfg = sort::defaultSortConfig(n);
     a.ensure(n, s, false);
     sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
@@ -602,7 +601,7 @@ SortTuning sortTuning(bool segmented, size_t n)
         r.tuned = true;
         return r;
     }
-    return sortConfigInfo(sort::kDefaultSortConfig);
+    return sortConfigInfo(sort::defaultSortConfig(n));
 }
 
 bool sortNeedsTuning(bool segmented, size_t n)

@@ -37,7 +37,10 @@ struct ForestEngine::Impl
     int tileConfig = -1;
     cudaEvent_t tuneStart = nullptr, tuneEnd = nullptr;  // sort tuner timing
     DevMem systemsD, tileSys, tileBegin, tileEnd, segFirstTile, segBase;
-    DevMem P[2], Perm[2], hist, bins, tileCounters, status;
+    DevMem P[2], Perm[2], hist, bins, status;
+    DevMem sortCtl;  // SortControl, PlanCounters, GridBarrier, list of long runs, plan table
+    sort::PlanArgs plan{};
+    u32 *longRuns = nullptr;
     // leaf arrays (entries = all systems' leaves + sentinels)
     size_t entryCap = 0;
     DevMem K[2], B[2], SEG[2], N, ops, offs, dirty, scanStatus, scanTile;
@@ -51,7 +54,7 @@ struct ForestEngine::Impl
     std::vector<size_t> leafCap;
     bool built = false;
     // build by levels: the unit arena, the key sample and the control words
-    DevMem lvRows, lvChild, lvLeaves, lvOffset, lvUsys, lvSysRoot, lvBins, lvCtl, sample, sortBar;
+    DevMem lvRows, lvChild, lvLeaves, lvOffset, lvUsys, lvSysRoot, lvBins, lvCtl, sample;
     size_t lvCap = 0;
     size_t lastEntries = 0;  // entries of the last build (the first guess of the next)
     int buildMode = 0;
@@ -101,8 +104,54 @@ struct ForestEngine::Impl
         upload(segFirstTile, first.data(), first.size() * 4);
         upload(segBase, base.data(), base.size() * 4);
         status.release();
-        status.reserve(std::max<size_t>(numTiles, 1) * sort::configPasses(config) * sort::kRadix * 8);
+        status.reserve(std::max<size_t>(numTiles, 1) * sort::kRadix * 8);
+        // words of another owner of the block could carry a tag to come
+        AOT_CHECK(cudaMemsetAsync(status.p, 0, status.bytes, stream));
         tileConfig = config;
+    }
+
+    // The control block's parts: the words after the epoch up to the long
+    // runs' list are cleared before a persistent sort.
+    static constexpr size_t kPlanAt = (sizeof(sort::SortControl) + 15) & ~size_t(15);
+    static constexpr size_t kBarAt = (kPlanAt + sizeof(sort::PlanCounters) + 15) & ~size_t(15);
+    static constexpr size_t kListAt = (kBarAt + sizeof(GridBarrier) + 255) & ~size_t(255);
+    static constexpr size_t kClearFrom = sizeof(u32);  // SortControl::epoch stays
+    static_assert(offsetof(sort::SortControl, epoch) == 0, "the epoch leads the control block");
+    void prepareSortControl(cudaStream_t stream)
+    {
+        const size_t tableAt = (kListAt + sort::longRunWords(total) * sizeof(u32) + 255) & ~size_t(255);
+        sortCtl.reserve(tableAt + sort::planTableBytes(total));
+        AOT_CHECK(cudaMemsetAsync(sortCtl.p, 0, sortCtl.bytes, stream));
+        unsigned char *base = sortCtl.as<unsigned char>();
+        longRuns = reinterpret_cast<u32 *>(base + kListAt);
+        plan.table = reinterpret_cast<u64 *>(base + tableAt);
+        plan.counters = reinterpret_cast<sort::PlanCounters *>(base + kPlanAt);
+        plan.samples = sort::planSamples(total);
+        plan.slotBits = sort::planSlotBits(total);
+    }
+    sort::SortControl *ctl() const { return sortCtl.as<sort::SortControl>(); }
+    GridBarrier *sortBar() const { return reinterpret_cast<GridBarrier *>(sortCtl.as<unsigned char>() + kBarAt); }
+    sort::SegmentTiles segmentTiles() const
+    {
+        return sort::SegmentTiles{tileSys.as<u32>(),      tileBegin.as<u32>(), tileEnd.as<u32>(),
+                                  segFirstTile.as<u32>(), segBase.as<u32>(),   bins.as<u32>()};
+    }
+    sort::RepairArgs repairArgs() const
+    {
+        sort::RepairArgs r{};
+        for (int k = 0; k < 2; ++k)
+        {
+            r.k[k] = P[k].as<u64>();
+            r.v[k] = Perm[k].as<u32>();
+        }
+        r.n = total;
+        r.ctl = ctl();
+        r.longList = longRuns;
+        r.error = &st.as<forest::State>()->error;
+        r.passes = sort::kMaxPasses;
+        r.keyMask = ~u64(0);
+        r.aligned = r.escapes = true;
+        return r;
     }
 
     forest::Bufs bufs() const
@@ -176,7 +225,7 @@ ForestEngine::ForestEngine(const void *const *x, const void *const *y, const voi
     }
     m.hist.reserve(size_t(numSystems) * sort::kPassSlots * sort::kRadix * 4);
     m.bins.reserve(size_t(numSystems) * sort::kPassSlots * sort::kRadix * 4);
-    m.tileCounters.reserve(sort::kPassSlots * 4);
+    m.prepareSortControl(cfg.stream);
     m.st.reserve(sizeof(forest::State));
     AOT_CHECK(cudaMemsetAsync(m.st.p, 0, sizeof(forest::State), cfg.stream));
     m.sys.reserve(size_t(numSystems) * sizeof(forest::SysState));
@@ -288,8 +337,24 @@ void ForestEngine::sortParticles(bool withSample)
     AOT_LAUNCH_CHECK();
 }
 
-// Keys of every system into P[0] (hist: with the 8-bit digit histograms).
-void ForestEngine::launchKeygen(bool hist)
+namespace
+{
+// Real and curve of a forest's keys: fn(Real{}, integral_constant of the curve).
+template <class Fn>
+void forKeys(const EngineConfig &cfg, Fn fn)
+{
+    using Hil = std::integral_constant<Curve, Curve::Hilbert>;
+    using Mor = std::integral_constant<Curve, Curve::Morton>;
+    if (cfg.real == 0 && cfg.hilbert) fn(float{}, Hil{});
+    else if (cfg.real == 0) fn(float{}, Mor{});
+    else if (cfg.hilbert) fn(double{}, Hil{});
+    else fn(double{}, Mor{});
+}
+}  // namespace
+
+// Keys of every system into P[0] (hist: with the digit counts of the plan's
+// passes, or without a plan yet of the passes from forest::kCountedFrom on).
+void ForestEngine::launchKeygen(bool hist, bool planned)
 {
     Impl &m = *m_;
     cudaStream_t s = m.cfg.stream;
@@ -297,23 +362,21 @@ void ForestEngine::launchKeygen(bool hist)
     u64 *keys = m.P[0].as<u64>();
     u32 *keygenHist = hist ? m.hist.as<u32>() : nullptr;
     const Impl &cm = m;
-    auto launch = [&](auto real) {
+    forKeys(m.cfg, [&](auto real, auto curve) {
         using Real = decltype(real);
         const KeygenParams<Real> &prm = [&]() -> const KeygenParams<Real> & {
             if constexpr (sizeof(Real) == 4) return cm.kpf;
             else return cm.kpd;
         }();
-        if (m.cfg.hilbert)
-            forest::keygenKernel<Real, Curve::Hilbert><<<grid, forest::kThreads, 0, s>>>(
-                m.systemsD.as<forest::System>(), m.tileSys.as<u32>(), m.tileBegin.as<u32>(), m.tileEnd.as<u32>(),
-                m.numTiles, prm, keys, keygenHist), noteLaunch();
-        else
-            forest::keygenKernel<Real, Curve::Morton><<<grid, forest::kThreads, 0, s>>>(
-                m.systemsD.as<forest::System>(), m.tileSys.as<u32>(), m.tileBegin.as<u32>(), m.tileEnd.as<u32>(),
-                m.numTiles, prm, keys, keygenHist), noteLaunch();
-    };
-    if (m.cfg.real == 0) launch(float{});
-    else launch(double{});
+        if (planned)
+            forest::planKernel<Real, curve.value>
+                <<<ceilDiv(m.plan.samples, sort::kPlanThreads), sort::kPlanThreads, 0, s>>>(
+                    m.systemsD.as<forest::System>(), m.S, m.segBase.as<u32>(), m.total, prm, m.plan, m.ctl(),
+                    m.hist.as<u32>(), size_t(m.S) * sort::kPassSlots * sort::kRadix), noteLaunch();
+        forest::keygenKernel<Real, curve.value><<<grid, forest::kThreads, 0, s>>>(
+            m.systemsD.as<forest::System>(), m.tileSys.as<u32>(), m.tileBegin.as<u32>(), m.tileEnd.as<u32>(),
+            m.numTiles, prm, keys, keygenHist, planned ? m.ctl() : nullptr, forest::kCountedFrom), noteLaunch();
+    });
     AOT_LAUNCH_CHECK();
 }
 
@@ -335,15 +398,15 @@ bool ForestEngine::sortPersistent(int config)
     {
     case 8:
         fn = reinterpret_cast<const void *>(&forest::sortKernel<8>);
-        smem = sizeof(sort::SharedPass<8, 8>);
+        smem = sizeof(forest::SortShared<8>);
         break;
     case 10:
         fn = reinterpret_cast<const void *>(&forest::sortKernel<10>);
-        smem = sizeof(sort::SharedPass<8, 10>);
+        smem = sizeof(forest::SortShared<10>);
         break;
     case 16:
         fn = reinterpret_cast<const void *>(&forest::sortKernel<16>);
-        smem = sizeof(sort::SharedPass<8, 16>);
+        smem = sizeof(forest::SortShared<16>);
         break;
     default: return false;
     }
@@ -352,33 +415,24 @@ bool ForestEngine::sortPersistent(int config)
     AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, sort::kThreads, smem));
     if (perSm <= 0) return false;
     const unsigned grid = unsigned(perSm) * unsigned(smCount());
-    const int passes = sort::configPasses(config);
     const size_t ns = (m.total + kSampleStride - 1) >> kSampleShift;
     m.sample.reserve(std::max<size_t>(ns, 1) * sizeof(u64), s);
-    m.sortBar.reserve(sizeof(GridBarrier), s);
     AOT_CHECK(cudaMemsetAsync(m.hist.p, 0, size_t(m.S) * sort::kPassSlots * sort::kRadix * 4, s));
-    AOT_CHECK(cudaMemsetAsync(m.tileCounters.p, 0, sort::kPassSlots * 4, s));
-    AOT_CHECK(cudaMemsetAsync(m.status.p, 0, size_t(m.numTiles) * passes * sort::kRadix * 8, s));
-    AOT_CHECK(cudaMemsetAsync(m.sortBar.p, 0, sizeof(GridBarrier), s));
-    launchKeygen(true);
+    AOT_CHECK(cudaMemsetAsync(m.sortCtl.as<unsigned char>() + Impl::kClearFrom, 0, Impl::kListAt - Impl::kClearFrom, s));
+    launchKeygen(true, false);
     forest::SortArgs p{};
     p.f = m.bufs();
-    p.tiles = sort::SegmentTiles{m.tileSys.as<u32>(),      m.tileBegin.as<u32>(), m.tileEnd.as<u32>(),
-                                 m.segFirstTile.as<u32>(), m.segBase.as<u32>(),  nullptr};
+    p.tiles = m.segmentTiles();
     p.numTiles = m.numTiles;
-    for (int k = 0; k < 2; ++k)
-    {
-        p.keys[k] = m.P[k].as<u64>();
-        p.vals[k] = m.Perm[k].as<u32>();
-    }
+    p.r = m.repairArgs();
+    p.plan = m.plan;
     p.hist = m.hist.as<u32>();
     p.bins = m.bins.as<u32>();
-    p.tileCounters = m.tileCounters.as<u32>();
     p.status = m.status.as<u64>();
     p.error = &m.st.as<forest::State>()->error;
     p.sample = m.sample.as<u64>();
     p.ns = ns;
-    p.bar = m.sortBar.as<GridBarrier>();
+    p.bar = m.sortBar();
     void *args[] = {&p};
     AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(sort::kThreads), args, smem, s));
     noteLaunch();
@@ -386,49 +440,74 @@ bool ForestEngine::sortPersistent(int config)
     return true;
 }
 
+namespace
+{
+template <int Tile>
+void launchSegmentRepair(unsigned numTiles, const sort::RepairArgs &r, const sort::SegmentTiles &tiles,
+                         const forest::System *systems, cudaStream_t s)
+{
+    constexpr int smem = int(sizeof(sort::RepairShared<Tile>));
+    AOT_CHECK(cudaFuncSetAttribute(forest::segmentRepairKernel<Tile>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    forest::segmentRepairKernel<Tile><<<numTiles, sort::kRepairThreads, smem, s>>>(r, tiles, systems), noteLaunch();
+}
+}  // namespace
+
 // Keys of every system and the segmented sort with sort configuration
 // `config`, whose tile table must be in place; the result lands in P[0] /
-// Perm[0] (an even pass count).
+// Perm[0].
 void ForestEngine::sortKeys(int config)
 {
     Impl &m = *m_;
     cudaStream_t s = m.cfg.stream;
     if (config != m.tileConfig) throw std::logic_error("forest: the tile table is not the sort configuration's");
-    const int bitsPer = sort::kSortConfigs[config].bits;
     const int passes = sort::configPasses(config);
     if (passes & 1) throw std::logic_error("forest: sort configurations must have an even pass count");
-    AOT_CHECK(cudaMemsetAsync(m.hist.p, 0, size_t(m.S) * sort::kPassSlots * sort::kRadix * 4, s));
-    AOT_CHECK(cudaMemsetAsync(m.tileCounters.p, 0, sort::kPassSlots * 4, s));
-    AOT_CHECK(cudaMemsetAsync(m.status.p, 0, size_t(m.numTiles) * passes * sort::kRadix * 8, s));
-    u64 *keys = m.P[0].as<u64>();
-    // 8-bit digits: the histograms come with the keys; otherwise a pass of their own
-    const bool fused = bitsPer == sort::kRadixBits;
-    launchKeygen(fused);
-    if (!fused)
+    // 8-bit digits: a plan, and the digit counts come with the keys; otherwise
+    // every pass, and the counts by a kernel of their own
+    const bool planned = sort::kSortConfigs[config].bits == sort::kRadixBits;
+    launchKeygen(planned, planned);
+    if (!planned)
+    {
+        sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(m.ctl(), nullptr), noteLaunch();
+        AOT_CHECK(cudaMemsetAsync(m.hist.p, 0, size_t(m.S) * sort::kPassSlots * sort::kRadix * 4, s));
         forest::segHistKernel<7><<<m.numTiles, forest::kThreads, 0, s>>>(m.tileSys.as<u32>(), m.tileBegin.as<u32>(),
-                                                                      m.tileEnd.as<u32>(), keys, passes,
+                                                                      m.tileEnd.as<u32>(), m.P[0].as<u64>(), passes,
                                                                       m.hist.as<u32>()),
             noteLaunch();
+    }
     forest::binsKernel<<<unsigned(m.S), sort::kRadix, 0, s>>>(m.systemsD.as<forest::System>(), m.S, m.hist.as<u32>(),
-                                                              m.bins.as<u32>(), passes),
+                                                              m.bins.as<u32>(), m.ctl(), passes),
         noteLaunch();
     AOT_LAUNCH_CHECK();
     sort::setPassSmemAll();
-    u64 *k[2] = {m.P[0].as<u64>(), m.P[1].as<u64>()};
-    u32 *v[2] = {m.Perm[0].as<u32>(), m.Perm[1].as<u32>()};
-    for (int p = 0; p < passes; ++p)
+    const sort::RepairArgs r = m.repairArgs();
+    const sort::SegmentTiles tiles = m.segmentTiles();
+    sort::PassArgs p{};
+    for (int k = 0; k < 2; ++k)
     {
-        const int in = p & 1, out = in ^ 1;
-        const int shift = p * bitsPer;
-        const sort::SegmentTiles tiles{m.tileSys.as<u32>(),      m.tileBegin.as<u32>(), m.tileEnd.as<u32>(),
-                                       m.segFirstTile.as<u32>(), m.segBase.as<u32>(),
-                                       m.bins.as<u32>() + size_t(p) * m.S * sort::kRadix};
-        sort::launchSegmentPass(config, s, m.numTiles, tiles, k[in], p == 0 ? nullptr : v[in], k[out], v[out], shift,
-                                m.tileCounters.as<u32>() + p, m.status.as<u64>() + size_t(p) * m.numTiles * sort::kRadix,
-                                sort::passTag(1), &m.st.as<forest::State>()->error, std::min(bitsPer, 64 - shift)),
-            noteLaunch();
+        p.k[k] = r.k[k];
+        p.v[k] = r.v[k];
+    }
+    p.ctl = m.ctl();
+    p.status = m.status.as<u64>();
+    p.error = &m.st.as<forest::State>()->error;
+    p.passes = passes;
+    for (int slot = 0; slot < passes; ++slot)
+    {
+        sort::launchSegmentPass(config, s, m.numTiles, tiles, p, slot, m.S), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
+    if (!planned) return;
+    const forest::System *systems = m.systemsD.as<forest::System>();
+    switch (sort::kSortConfigs[config].items)
+    {
+    case 8: launchSegmentRepair<sort::kThreads * 8>(m.numTiles, r, tiles, systems, s); break;
+    case 10: launchSegmentRepair<sort::kThreads * 10>(m.numTiles, r, tiles, systems, s); break;
+    case 16: launchSegmentRepair<sort::kThreads * 16>(m.numTiles, r, tiles, systems, s); break;
+    default: throw std::logic_error("forest: no repair for the sort configuration's tiles");
+    }
+    sort::longRunKernel<<<unsigned(smCount()) * 2u, sort::kLongThreads, 0, s>>>(r), noteLaunch();
+    AOT_LAUNCH_CHECK();
 }
 
 // One decision round (build) or fixed pass (update) over all systems.

@@ -23,6 +23,7 @@
 
 #include "keygen.cuh"
 #include "rebalance.cuh"
+#include "sort_repair.cuh"
 
 namespace aot
 {
@@ -92,8 +93,44 @@ struct Bufs
 // --------------------------------------------------------------------------
 // keys and the segmented sort
 // --------------------------------------------------------------------------
+// The system that holds particle g (the last one that starts at or before it:
+// systems without particles start where the next one does).
+__device__ __forceinline__ u32 systemOf(const u32 *segBase, int numSystems, u32 g)
+{
+    u32 lo = 0, n = u32(numSystems);
+    while (n > 1)
+    {
+        const u32 half = n >> 1;
+        const bool right = __ldg(segBase + lo + half) <= g;
+        lo = right ? lo + half : lo;
+        n = right ? n - half : half;
+    }
+    return lo;
+}
+
+// Start of a planned sort (sort::planSort) from the keys of particles at
+// random positions of all systems.
+template <class Real, Curve C>
+static __global__ void __launch_bounds__(sort::kPlanThreads)
+    planKernel(const System *__restrict__ systems, int numSystems, const u32 *__restrict__ segBase, size_t total,
+               const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist, size_t histWords)
+{
+    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    __syncthreads();
+    const auto keyAt = [&](size_t g, u32 &group) {
+        group = systemOf(segBase, numSystems, u32(g));
+        const System sy = systems[group];
+        const size_t i = g - sy.base;
+        return particleKey<Real, C>(static_cast<const Real *>(sy.x)[i], static_cast<const Real *>(sy.y)[i],
+                                    static_cast<const Real *>(sy.z)[i], prm, sPair);
+    };
+    sort::planSort(keyAt, total, plan, ctl, hist, histWords);
+}
+
 // Keys of every system's particles and (hist != nullptr) the per-system
-// histograms of the eight 8-bit digits, hist[system][pass slot][digit].  Each
+// histograms of the 8-bit digits of passes firstPass to 7,
+// hist[system][pass slot][digit].  Each
 // CTA takes a contiguous range of tiles, so its shared histogram is flushed
 // only where the system changes.
 // The keys of tiles [t0, t1) (a CTA's share), with the digit histograms
@@ -103,7 +140,8 @@ template <class Real, Curve C>
 __device__ __forceinline__ void keygenTiles(const System *__restrict__ systems, const u32 *__restrict__ tileSys,
                                             const u32 *__restrict__ tileBegin, const u32 *__restrict__ tileEnd,
                                             u32 t0, u32 t1, const KeygenParams<Real> &prm, u64 *__restrict__ keys,
-                                            u32 *__restrict__ hist, u32 *sh, const unsigned short *sPair)
+                                            u32 *__restrict__ hist, int firstPass, u32 *sh,
+                                            const unsigned short *sPair)
 {
     int cur = -1;
     auto flush = [&]() {
@@ -111,7 +149,7 @@ __device__ __forceinline__ void keygenTiles(const System *__restrict__ systems, 
         if (cur >= 0 && hist)
         {
             u32 *h = hist + size_t(cur) * sort::kPassSlots * sort::kRadix;
-            for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x)
+            for (int i = firstPass * sort::kRadix + threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x)
             {
                 const u32 v = sh[i];
                 if (v)
@@ -145,7 +183,8 @@ __device__ __forceinline__ void keygenTiles(const System *__restrict__ systems, 
             {
 #pragma unroll
                 for (int p = 0; p < sort::kMaxPasses; ++p)
-                    atomicAdd(&sh[p * sort::kRadix + int((k >> (p * sort::kRadixBits)) & (sort::kRadix - 1))], 1u);
+                    if (p >= firstPass)
+                        atomicAdd(&sh[p * sort::kRadix + int((k >> (p * sort::kRadixBits)) & (sort::kRadix - 1))], 1u);
             }
         }
     }
@@ -156,28 +195,19 @@ template <class Real, Curve C>
 static __global__ void __launch_bounds__(kThreads)
     keygenKernel(const System *__restrict__ systems, const u32 *__restrict__ tileSys,
                  const u32 *__restrict__ tileBegin, const u32 *__restrict__ tileEnd, u32 numTiles,
-                 const KeygenParams<Real> prm, u64 *__restrict__ keys, u32 *__restrict__ hist)
+                 const KeygenParams<Real> prm, u64 *__restrict__ keys, u32 *__restrict__ hist,
+                 const sort::SortControl *ctl, int firstPass)
 {
+    if (ctl) firstPass = int(ctl->first);  // the plan's
     __shared__ u32 sh[sort::kMaxPasses * sort::kRadix];
     __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) sh[i] = 0;
-    if constexpr (C == Curve::Hilbert)
-    {
-        // the one-level tables staged in shared memory, then the pair table from them
-        __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8];
-        for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x)
-        {
-            sEnc[i] = prm.h.enc[i];
-            sNext[i] = prm.h.encNext[i];
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < kHilbertPairEntries; i += blockDim.x)
-            sPair[i] = hilbertPairEntry(i, sEnc, sNext);
-    }
+    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
     __syncthreads();
     const u32 per = (numTiles + gridDim.x - 1) / gridDim.x;
     const u32 t0 = blockIdx.x * per;
-    keygenTiles<Real, C>(systems, tileSys, tileBegin, tileEnd, t0, min(numTiles, t0 + per), prm, keys, hist, sh, sPair);
+    keygenTiles<Real, C>(systems, tileSys, tileBegin, tileEnd, t0, min(numTiles, t0 + per), prm, keys, hist, firstPass,
+                         sh, sPair);
 }
 
 // Per-system histograms of Bits-wide digits for `passes` passes, one CTA per
@@ -212,37 +242,71 @@ static __global__ void __launch_bounds__(kThreads)
     }
 }
 
-// Per system and pass: global start of each digit = base + exclusive scan of
-// the system's digit counts.  bins[pass][system][digit].  One CTA of kRadix
-// threads per system; s: kRadix words of shared scratch.
-__device__ __forceinline__ void systemBins(const System *__restrict__ systems, int numSystems, int sys,
-                                           const u32 *__restrict__ hist, u32 *__restrict__ bins, int passes, u32 *s)
+// Per system and pass [firstPass, passes): global start of each digit = base +
+// exclusive scan of the system's digit counts.  bins[pass][system][digit].
+// A warp per pass, eight counts per lane.
+__device__ __forceinline__ void systemBins(const System *__restrict__ systems, int numSystems, int sys, const u32 *hist,
+                                           u32 *bins, int firstPass, int passes)
 {
-    const int d = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const u32 base = systems[sys].base;
-    for (int p = 0; p < passes; ++p)
+    for (int p = firstPass + int(threadIdx.x >> 5); p < passes; p += int(blockDim.x >> 5))
     {
-        const u32 v = hist[(size_t(sys) * sort::kPassSlots + p) * sort::kRadix + d];
-        s[d] = v;
-        __syncthreads();
-        for (int off = 1; off < sort::kRadix; off <<= 1)
+        const uint4 *h = reinterpret_cast<const uint4 *>(hist + (size_t(sys) * sort::kPassSlots + p) * sort::kRadix) +
+                         lane * 2;
+        const uint4 a = __ldcg(h), b = __ldcg(h + 1);
+        const u32 c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        u32 sum = 0, e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
         {
-            const u32 t = d >= off ? s[d - off] : 0u;
-            __syncthreads();
-            s[d] += t;
-            __syncthreads();
+            e[i] = sum;
+            sum += c[i];
         }
-        bins[(size_t(p) * numSystems + sys) * sort::kRadix + d] = base + s[d] - v;
-        __syncthreads();
+        u32 inc = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += t;
+        }
+        const u32 at = base + inc - sum;
+        uint4 *o = reinterpret_cast<uint4 *>(bins + (size_t(p) * numSystems + sys) * sort::kRadix) + lane * 2;
+        o[0] = make_uint4(at + e[0], at + e[1], at + e[2], at + e[3]);
+        o[1] = make_uint4(at + e[4], at + e[5], at + e[6], at + e[7]);
     }
 }
 
 static __global__ void __launch_bounds__(sort::kRadix)
     binsKernel(const System *__restrict__ systems, int numSystems, const u32 *__restrict__ hist,
-               u32 *__restrict__ bins, int passes)
+               u32 *__restrict__ bins, const sort::SortControl *ctl, int passes)
 {
-    __shared__ u32 s[sort::kRadix];
-    systemBins(systems, numSystems, blockIdx.x, hist, bins, passes, s);
+    systemBins(systems, numSystems, blockIdx.x, hist, bins, int(ctl->first), passes);
+}
+
+// The repair (sort_repair.cuh) of one tile of the segmented sort.
+template <int Tile>
+__device__ __forceinline__ void repairSystemTile(const sort::RepairArgs &a, sort::RepairShared<Tile> &sm, u32 first,
+                                                 const sort::SegmentTiles &tiles, const System *__restrict__ systems,
+                                                 u32 tile)
+{
+    const bool inPlace = ((u32(a.passes) - first) & 1u) == 0;
+    const System sy = systems[tiles.tileSeg[tile]];
+    const size_t begin = tiles.tileBegin[tile], segBegin = sy.base, segEnd = size_t(sy.base) + sy.n;
+    if (first == 4) sort::repairTile<4>(a, sm, first, inPlace, begin, segBegin, segEnd);
+    else if (first < 4) sort::repairTile<3>(a, sm, first, inPlace, begin, segBegin, segEnd);
+    else sort::repairTile<0>(a, sm, first, inPlace, begin, segBegin, segEnd);
+}
+
+template <int Tile>
+static __global__ void __launch_bounds__(sort::kRepairThreads)
+    segmentRepairKernel(sort::RepairArgs a, sort::SegmentTiles tiles, const System *__restrict__ systems)
+{
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    if (*a.error) return;
+    const u32 first = a.ctl->first;
+    if (first == 0) return;
+    repairSystemTile(a, *reinterpret_cast<sort::RepairShared<Tile> *>(smemRaw), first, tiles, systems, blockIdx.x);
 }
 
 // With a sample array: also every 32nd key of the concatenated sorted keys

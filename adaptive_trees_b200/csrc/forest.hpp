@@ -63,7 +63,7 @@ private:
     std::unique_ptr<Impl> m_;
     void sortParticles(bool withSample);
     bool sortPersistent(int config);
-    void launchKeygen(bool hist);
+    void launchKeygen(bool hist, bool planned);
     bool levelBuild();
     void sortKeys(int config);
     void pass(bool build, const unsigned char *frozenDevice);

@@ -12,9 +12,21 @@
 //   2. a tiny kernel turns the counts into per-digit global start offsets;
 //   3. one onesweep kernel per digit: each CTA takes a tile of keys in
 //      arrival order (atomic tile counter), ranks them per warp with ballots,
-//      publishes its per-digit counts, resolves its global offsets by
-//      decoupled look-back over earlier tiles, reorders the tile in shared
-//      memory and writes digit runs out contiguously.
+//      publishes its per-digit counts, reorders the keys in shared memory,
+//      resolves its global offsets by decoupled look-back over earlier tiles
+//      (while the tile's values are on their way), reorders the values and
+//      writes digit runs out contiguously.
+// What bounds a pass is the shared-memory pipe and the issue slots, not HBM
+// (16Mi pairs, ncu: shared memory 81 % busy with an atomic-or match, DRAM
+// 32 %): about 40 shared-memory wavefronts and 100 instructions per 32 keys.
+// Measured at 16Mi pairs, per pass: 156 us before, with the values staged by a
+// bulk copy, the ballots left to the compiler and the tile's bounds checked
+// for every key; 147 us with the values loaded behind the key reorder; 136 us
+// with one lookup for a key's place instead of two and tiles of 3584 keys;
+// 120 us with the ballots written out (peerLanes) and tiles of 4096; 117.5 us
+// with the warp's counter read by all lanes instead of shuffled (3.4 TB/s).
+// Not faster: __match_any_sync (182 us), matching by shared atomic-or (133-138),
+// 512 threads (138), tiles of 4608-6144 keys (117-124).
 // The digit width and the keys per thread are template parameters; the
 // configurations compiled in are listed in kSortConfigs, and the sort tuner
 // (sortTune in engine.cu) picks one per device and problem size by timing them.
@@ -76,8 +88,8 @@ __device__ __forceinline__ unsigned laneMaskLt()
 // Control block of one sort, in device memory.
 struct SortControl
 {
+    u32 epoch;      // number of the sort: pass slot j writes tag epoch + j (the only word kept between sorts)
     u32 first;      // the passes run are first .. passes - 1 (0: all of them)
-    u32 epoch;      // number of the sort: pass slot j writes tag epoch + j
     u32 longRuns;   // runs the repair left to the long-run kernel
     u32 keygenDone; // CTAs of the key generation that have added their digit counts
     u32 tileCounters[kPassSlots];
@@ -173,13 +185,9 @@ struct SharedPass
     static constexpr int T = kThreads * Items;
     u64 keys[T];
     u32 vals[T];
-    u32 stage[T];              // the tile's input values, staged by one bulk copy (16-byte aligned)
-    u64 valuesReady;           // mbarrier of that copy
-    u32 staged;                // values in `stage` (a multiple of 4)
-    u32 warpHist[kWarps][R];   // per-warp digit counts, then exclusive warp offsets
+    u32 warpStart[kWarps][R];  // per-warp digit counts, then the tile-local start of each warp's digit
     u32 localStart[R];
     u32 gstart[R];             // global position of local index 0 of each digit (mod 2^32)
-    u32 count[R];
     u32 warpSums[kWarps];
     u32 tile;
 };
@@ -195,114 +203,90 @@ struct SortConfig
 constexpr SortConfig kSortConfigs[] = {{8, 10}, {8, 16}, {8, 8}, {7, 12}, {7, 16}};
 constexpr int kNumSortConfigs = int(sizeof(kSortConfigs) / sizeof(kSortConfigs[0]));
 constexpr int kDefaultSortConfig = 0;
+// The configuration of a sort no tuning has chosen one for: tiles of 4096
+// keys from a million keys on (64-bit pair sorts: 700k keys 108 us with 2560,
+// 112 with 4096; 1M 125 and 118; 4M 309 and 276; 16Mi 1135 and 1018).
+constexpr int defaultSortConfig(size_t n) { return n >= (size_t(1) << 20) ? 1 : kDefaultSortConfig; }
 constexpr int configTile(int c) { return kThreads * kSortConfigs[c].items; }
 constexpr int configPasses(int c, int bits = 64)
 {
     return (bits + kSortConfigs[c].bits - 1) / kSortConfigs[c].bits;
 }
 
-// Lanes of the warp whose (valid) digit equals this lane's: eight ballots, one
-// per digit bit, instead of __match_any_sync.
-__device__ __forceinline__ unsigned peerLanes(unsigned digit, int bits, unsigned validMask)
+// Lanes of the warp whose Bits-wide digit equals this lane's: a ballot per
+// digit bit.  Written out as test, ballot, select and one three-input AND-XOR
+// per bit: the compiler's version of the same took 16 us more of a 136 us pass.
+template <int Bits>
+__device__ __forceinline__ unsigned peerLanes(unsigned digit)
 {
-    unsigned peers = validMask;
+    unsigned peers = 0xffffffffu;
 #pragma unroll
-    for (int b = 0; b < kRadixBits; ++b)
+    for (int b = 0; b < Bits; ++b)
     {
-        if (b < bits)
-        {
-            const bool set = (digit >> b) & 1u;
-            const unsigned m = __ballot_sync(0xffffffffu, set);
-            peers &= set ? m : ~m;
-        }
+        unsigned lanes, other;  // lanes with the bit set; zero (this lane has it) or all ones
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t"
+            "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\tselp.b32 %1, 0, 0xffffffff, p;\n\t}"
+            : "=r"(lanes), "=r"(other)
+            : "r"(digit), "r"(1u << b));
+        asm("lop3.b32 %0, %0, %1, %2, 0x60;" : "+r"(peers) : "r"(lanes), "r"(other));  // peers & (lanes ^ other)
     }
     return peers;
 }
 
-// Shared-memory address of a pointer into shared memory.
-__device__ __forceinline__ unsigned smemAddr(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
+// A tile: the keys [base, base + count) (at most Tile), whether it starts a
+// look-back chain (publishes an inclusive prefix at once), the global start
+// of each digit, and what is subtracted from a generated value's key index.
+struct TileRange
+{
+    u32 base, count;
+    bool chainStart;
+    const u32 *digitBase;
+    u32 valueOffset;
+};
 
-// mbarrier and bulk-copy helpers (PTX ISA: mbarrier, cp.async.bulk)
-__device__ __forceinline__ void mbarInit(u64 *bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fenceMbarInit() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbarArriveExpectTx(u64 *bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbarArrive(u64 *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smemAddr(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbarTryWait(u64 *bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smemAddr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Global -> shared copy of `bytes` (a multiple of 16; both addresses 16-byte
-// aligned) that completes on `bar`.  No multicast: the source is this GPU's memory.
-__device__ __forceinline__ void bulkLoad(void *dst, const void *src, unsigned bytes, u64 *bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smemAddr(dst)),
-                 "l"(src), "r"(bytes), "r"(smemAddr(bar))
-                 : "memory");
-}
-constexpr unsigned kStageSpins = 1u << 22;  // bounded wait for the staged values
-
-// Tile geometry of a pass over one contiguous key array keys[0, n).  The
-// accessors are cheap and recomputed where used, so that nothing extra stays
-// live in registers across the pass.
+// Tiles of a pass over one contiguous key array keys[0, n).
 template <int Tile>
 struct ContiguousTiles
 {
-    static constexpr bool kStageValues = true;  // tiles start at multiples of Tile (16-byte aligned values)
     size_t n;
     const u32 *bins;  // [radix] global start of each digit
-    // the tile's keys are [base(t), min(base(t) + Tile, end(t)))
-    __device__ __forceinline__ size_t base(size_t tile) const { return tile * size_t(Tile); }
-    __device__ __forceinline__ size_t end(size_t) const { return n; }
-    // the tile publishes an inclusive prefix without look-back
-    __device__ __forceinline__ bool chainStart(size_t tile) const { return tile == 0; }
-    __device__ __forceinline__ const u32 *digitBase(size_t) const { return bins; }
-    // generated first-pass value of the key at global index i: i - valueOffset
-    __device__ __forceinline__ u32 valueOffset(size_t) const { return 0; }
+    __device__ __forceinline__ TileRange at(u32 tile) const
+    {
+        const size_t b = size_t(tile) * Tile, left = n - b;
+        return {u32(b), left < size_t(Tile) ? u32(left) : u32(Tile), tile == 0, bins, 0u};
+    }
 };
 
-// Tile geometry of a segmented pass (the systems of a forest): tile t holds
+// Tiles of a segmented pass (the systems of a forest): tile t holds
 // the keys [tileBegin[t], tileEnd[t]) of segment tileSeg[t] (at most one tile,
 // never straddling segments); a look-back chain ends at the segment's first
 // tile; digit starts are per segment, and generated values are indices within
 // the segment.
 struct SegmentTiles
 {
-    static constexpr bool kStageValues = false;  // tiles start anywhere: plain loads
     const u32 *tileSeg, *tileBegin, *tileEnd, *segFirstTile, *segBase;
     const u32 *bins;  // [segments][kRadix] global start of each digit of this pass
-    __device__ __forceinline__ size_t base(size_t tile) const { return tileBegin[tile]; }
-    __device__ __forceinline__ size_t end(size_t tile) const { return tileEnd[tile]; }
-    __device__ __forceinline__ bool chainStart(size_t tile) const { return u32(tile) == segFirstTile[tileSeg[tile]]; }
-    __device__ __forceinline__ const u32 *digitBase(size_t tile) const { return bins + size_t(tileSeg[tile]) * kRadix; }
-    __device__ __forceinline__ u32 valueOffset(size_t tile) const { return segBase[tileSeg[tile]]; }
+    __device__ __forceinline__ TileRange at(u32 tile) const
+    {
+        const u32 seg = __ldg(tileSeg + tile), b = __ldg(tileBegin + tile);
+        return {b, __ldg(tileEnd + tile) - b, tile == __ldg(segFirstTile + seg), bins + size_t(seg) * kRadix,
+                __ldg(segBase + seg)};
+    }
 };
 
-// One onesweep pass: the Bits-wide digit at bit `shift` (`bits` <= Bits
-// wide) of the tiles of `tiles`, Items keys per thread.  valsIn == nullptr
+// One onesweep pass: the digit at bit `shift` (`bits` <= Bits wide) of a tile
+// of `tiles`, Items keys per thread.  valsIn == nullptr
 // means values are generated (first pass).  Threads below the radix own one
-// digit each in the per-digit steps.  A look-back that polls an unpublished
+// digit each in the per-digit steps.  The places behind a short tile's keys
+// hold the largest digit, so that they rank last, and are not written; their
+// counts reach no later tile (a short tile ends its chain).  A look-back that polls an unpublished
 // tile more than spinLimit times records kErrLookback and goes on with the
 // prefix it has: every write stays inside the output, the result is wrong
-// and the host reports the error.  A persistent CTA calls it until it returns
+// and the host reports the error.  A persistent CTA calls it, with a
+// __syncthreads between, until it returns
 // false: the tile counter has passed numTiles (which a launch of one CTA per
-// tile never reaches).  Persistent use needs unstaged values
-// (Tiles::kStageValues false): the staging barrier is not set up again.
+// tile never reaches).
 template <int Bits, int Items, class Tiles>
 __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__restrict__ keysIn,
                                              const u32 *__restrict__ valsIn, u64 *__restrict__ keysOut,
@@ -314,102 +298,73 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
     constexpr int R = Smem::R;
     constexpr int T = Smem::T;
     static_assert(R <= kThreads && R <= kRadix, "one digit per thread");
-    static_assert(Items % 2 == 0, "ranks are packed in pairs");
+    static_assert(Items % 2 == 0 && T <= 0x10000, "ranks and places are packed in pairs");
     const unsigned dmask = (1u << bits) - 1;
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Smem &sm = *reinterpret_cast<Smem *>(smemRaw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-    const bool stage = Tiles::kStageValues && valsIn != nullptr;
-    for (int i = tid; i < kWarps * R; i += kThreads) (&sm.warpHist[0][0])[i] = 0;
-    if (tid == 0)
-    {
-        sm.tile = atomicAdd(tileCounter, 1u);
-        if (stage)
-        {
-            mbarInit(&sm.valuesReady, 1);
-            fenceMbarInit();
-        }
-    }
+    for (int i = tid; i < kWarps * R; i += kThreads) (&sm.warpStart[0][0])[i] = 0;
+    if (tid == 0) sm.tile = atomicAdd(tileCounter, 1u);
     __syncthreads();
-    const size_t tile = sm.tile;
+    const u32 tile = sm.tile;
     if (tile >= numTiles) return false;
-    const size_t tileBase = tiles.base(tile);
-    const size_t warpBase = tileBase + size_t(warp) * (32 * Items);
-    if (stage && tid == 0)
+    const TileRange r = tiles.at(tile);
+    const u32 at = u32(warp) * (32 * Items) + u32(lane);  // this lane's first key in the tile, then every 32nd
+    const bool full = r.count == u32(T);
+
+    u64 key[Items];
     {
-        // the values travel to shared memory while the keys are ranked
-        const size_t end = tiles.end(tile);
-        const u32 count = u32((end - tileBase) < size_t(T) ? end - tileBase : size_t(T));
-        const bool aligned = (reinterpret_cast<uintptr_t>(valsIn + tileBase) & 15u) == 0;
-        const u32 bulk = aligned ? (count & ~3u) : 0u;
-        sm.staged = bulk;
-        if (bulk)
+        const u64 *in = keysIn + r.base + at;
+        if (full)
         {
-            mbarArriveExpectTx(&sm.valuesReady, bulk * 4u);
-            bulkLoad(sm.stage, valsIn + tileBase, bulk * 4u, &sm.valuesReady);
+#pragma unroll
+            for (int i = 0; i < Items; ++i) key[i] = __ldcs(in + i * 32);
         }
         else
         {
-            mbarArrive(&sm.valuesReady);
-        }
-    }
-
-    u64 key[Items];
 #pragma unroll
-    for (int i = 0; i < Items; ++i)
-    {
-        const size_t idx = warpBase + size_t(i) * 32 + lane;
-        key[i] = idx < tiles.end(tile) ? __ldcs(keysIn + idx) : 0ull;
+            for (int i = 0; i < Items; ++i) key[i] = at + u32(i) * 32 < r.count ? __ldcs(in + i * 32) : ~u64(0);
+        }
     }
     // Rank within the warp, items in memory order (item-major, lane-minor):
-    // the lowest lane of each digit group adds the group size to the warp's
-    // counter and broadcasts the old value.
-    u32 *wh = sm.warpHist[warp];
+    // every lane reads its digit's counter of the warp, then the first lane
+    // of each digit group adds the group's size.
+    u32 *warpCount = sm.warpStart[warp];
     const unsigned ltMask = laneMaskLt();
-    u32 rank2[Items / 2];
+    u32 place2[Items / 2];  // rank, later place in the tile: two of 16 bits
 #pragma unroll
     for (int i = 0; i < Items; ++i)
     {
-        const size_t idx = warpBase + size_t(i) * 32 + lane;
-        const bool valid = idx < tiles.end(tile);
-        const unsigned validMask = __ballot_sync(0xffffffffu, valid);
         const unsigned d = unsigned(key[i] >> shift) & dmask;
-        const unsigned peers = peerLanes(d, bits, validMask);
-        const int leader = __ffs(peers) - 1;
-        u32 base = 0;
-        if (valid && lane == leader) base = atomicAdd(&wh[d], u32(__popc(peers)));
-        base = __shfl_sync(0xffffffffu, base, leader < 0 ? 0 : leader);
+        const unsigned peers = peerLanes<Bits>(d);
+        const u32 before = warpCount[d];
         __syncwarp();
-        const u32 r = base + __popc(peers & ltMask);
-        if (i & 1) rank2[i >> 1] |= r << 16;
-        else rank2[i >> 1] = r;
+        const u32 inGroup = __popc(peers & ltMask);
+        if (inGroup == 0) warpCount[d] = before + __popc(peers);
+        __syncwarp();
+        const u32 rank = before + inGroup;
+        if (i & 1) place2[i >> 1] |= rank << 16;
+        else place2[i >> 1] = rank;
     }
     __syncthreads();
-    // Per digit: warp exclusive offsets and tile total (thread = digit).
-    if (tid < R)
+    // Per digit (thread = digit): the tile's count, published at once (a
+    // chain's first tile publishes final prefixes; the look-back comes last,
+    // so earlier tiles have had time to publish theirs); the tile-local start
+    // of the digit and of each warp's part of it.
+    u32 count = 0;
     {
         const int d = tid;
-        u32 acc = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w)
+        u32 c[kWarps];
+        if (d < R)
         {
-            const u32 c = sm.warpHist[w][d];
-            sm.warpHist[w][d] = acc;
-            acc += c;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) c[w] = sm.warpStart[w][d];
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) count += c[w];
+            stRelaxed(status + size_t(tile) * R + d, (r.chainStart ? kFlagPrefix : kFlagAgg) | tag | u64(count));
         }
-        sm.count[d] = acc;
-    }
-    __syncthreads();
-    // Publish this tile's digit counts early (a chain's first tile publishes
-    // final prefixes), then build the tile-local order; the look-back comes
-    // last so earlier tiles have had time to publish inclusive prefixes.
-    {
-        const int d = tid;
-        const u32 cnt = d < R ? sm.count[d] : 0u;
-        if (d < R) stRelaxed(status + tile * R + d, (tiles.chainStart(tile) ? kFlagPrefix : kFlagAgg) | tag | u64(cnt));
-        // exclusive scan of the tile's digit counts -> local starts
-        u32 v = cnt;
+        u32 v = count;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1)
         {
@@ -418,52 +373,60 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
         }
         if (lane == 31) sm.warpSums[warp] = v;
         __syncthreads();
-        u32 wOff = 0;
+        u32 run = v - count;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w)
-            if (w < warp) wOff += sm.warpSums[w];
-        if (d < R) sm.localStart[d] = wOff + v - cnt;
-    }
-    __syncthreads();
-    // Reorder the tile in shared memory.
-    u32 staged = 0;
-    bool copyPending = false;
-    if (stage)
-    {
-        unsigned spins = 0;
-        while (!mbarTryWait(&sm.valuesReady, 0))
+            if (w < warp) run += sm.warpSums[w];
+        if (d < R)
         {
-            if (++spins > kStageSpins)
+            sm.localStart[d] = run;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w)
             {
-                atomicExch(error, kErrLookback);
-                copyPending = true;
-                break;
+                sm.warpStart[w][d] = run;
+                run += c[w];
             }
         }
-        staged = copyPending ? 0u : sm.staged;
     }
+    __syncthreads();
+    // Reorder the keys in shared memory; the values are loaded behind them and
+    // arrive during the look-back.
 #pragma unroll
     for (int i = 0; i < Items; ++i)
     {
-        const size_t idx = warpBase + size_t(i) * 32 + lane;
-        if (idx < tiles.end(tile))
+        const unsigned d = unsigned(key[i] >> shift) & dmask;
+        const u32 rank = (place2[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+        const u32 place = warpCount[d] + rank;
+        sm.keys[place] = key[i];
+        if (i & 1) place2[i >> 1] = (place2[i >> 1] & 0xffffu) | (place << 16);
+        else place2[i >> 1] = (place2[i >> 1] & 0xffff0000u) | place;
+    }
+    u32 val[Items];
+    if (valsIn)
+    {
+        const u32 *in = valsIn + r.base + at;
+        if (full)
         {
-            const unsigned d = unsigned(key[i] >> shift) & dmask;
-            const u32 r = (rank2[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
-            const u32 pos = sm.localStart[d] + sm.warpHist[warp][d] + r;
-            sm.keys[pos] = key[i];
-            const u32 li = u32(idx - tileBase);
-            sm.vals[pos] = valsIn ? (li < staged ? sm.stage[li] : __ldcs(valsIn + idx))
-                                  : u32(idx) - tiles.valueOffset(tile);
+#pragma unroll
+            for (int i = 0; i < Items; ++i) val[i] = __ldcs(in + i * 32);
         }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < Items; ++i) val[i] = at + u32(i) * 32 < r.count ? __ldcs(in + i * 32) : 0u;
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int i = 0; i < Items; ++i) val[i] = r.base + at + u32(i) * 32 - r.valueOffset;
     }
     // Look-back: global start of each digit for this tile.
     if (tid < R)
     {
         const int d = tid;
-        const u32 total = sm.count[d];
         u32 excl = 0;  // keys are fewer than 2^32
-        if (!tiles.chainStart(tile))
+        if (!r.chainStart)
         {
             // Walk back over earlier tiles, eight status words per round trip,
             // summing aggregates until an inclusive prefix is found (the
@@ -478,6 +441,7 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
                     w8[k] = j - k >= 0 ? ldRelaxed(status + size_t(j - k) * R + d) : (kFlagPrefix | tag);
                 int k = 0;
                 bool done = false;
+#pragma unroll
                 for (; k < kLookbackWindow; ++k)
                 {
                     if ((w8[k] & kTagMask) != tag) break;  // not published in this pass
@@ -500,28 +464,34 @@ __device__ __forceinline__ bool onesweepTile(const Tiles &tiles, const u64 *__re
                     if (spins > 64) __nanosleep(64);
                 }
             }
-            stRelaxed(status + tile * R + d, kFlagPrefix | tag | u64(excl + total));
+            stRelaxed(status + size_t(tile) * R + d, kFlagPrefix | tag | u64(excl + count));
         }
         // modulo 2^32: gstart + j is exact for every key of digit d
-        sm.gstart[d] = tiles.digitBase(tile)[d] + excl - sm.localStart[d];
+        sm.gstart[d] = r.digitBase[d] + excl - sm.localStart[d];
     }
+#pragma unroll
+    for (int i = 0; i < Items; ++i) sm.vals[(place2[i >> 1] >> ((i & 1) * 16)) & 0xffffu] = val[i];
     __syncthreads();
-    const size_t remain = tiles.end(tile) - tileBase;
-    const int valid = remain < size_t(T) ? int(remain) : T;
+    if (full)
+    {
 #pragma unroll 4
-    for (int j = tid; j < valid; j += kThreads)
-    {
-        const u64 k = sm.keys[j];
-        const unsigned d = unsigned(k >> shift) & dmask;
-        const u32 out = sm.gstart[d] + u32(j);
-        keysOut[out] = k;
-        valsOut[out] = sm.vals[j];
-    }
-    if (copyPending)
-    {
-        // the CTA does not leave with its copy still in flight (bounded again)
-        for (unsigned spins = 0; spins < kStageSpins && !mbarTryWait(&sm.valuesReady, 0); ++spins)
+        for (int i = 0; i < Items; ++i)
         {
+            const int j = tid + i * kThreads;
+            const u64 k = sm.keys[j];
+            const u32 out = sm.gstart[unsigned(k >> shift) & dmask] + u32(j);
+            keysOut[out] = k;
+            valsOut[out] = sm.vals[j];
+        }
+    }
+    else
+    {
+        for (int j = tid; j < int(r.count); j += kThreads)
+        {
+            const u64 k = sm.keys[j];
+            const u32 out = sm.gstart[unsigned(k >> shift) & dmask] + u32(j);
+            keysOut[out] = k;
+            valsOut[out] = sm.vals[j];
         }
     }
     return true;
@@ -568,15 +538,21 @@ static __global__ void __launch_bounds__(kThreads, passMinBlocks<Bits, Items>())
                               p.status, passTag(p.ctl->epoch + u32(slot)), p.error, min(Bits, p.endBit - shift));
 }
 
-// One onesweep pass over the segments of a forest: every segment is sorted
-// on its own (stable within the segment), in place in the global arrays.
+// Pass slot `slot` over the segments of a forest (`passes` in all): every
+// segment is sorted on its own (stable within the segment), in place in the
+// global arrays.  tiles.bins: [pass][segment][kRadix].
 template <int Bits, int Items>
 static __global__ void __launch_bounds__(kThreads, passMinBlocks<Bits, Items>())
-    segmentOnesweepKernel(SegmentTiles tiles, const u64 *__restrict__ keysIn, const u32 *__restrict__ valsIn,
-                          u64 *__restrict__ keysOut, u32 *__restrict__ valsOut, int shift, u32 *tileCounter,
-                          u64 *status, u64 tag, int *error, int bits)
+    segmentOnesweepKernel(SegmentTiles tiles, PassArgs p, int slot, int segments)
 {
-    onesweepTile<Bits, Items>(tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, tag, error, bits);
+    const int pass = int(p.ctl->first) + slot;
+    if (pass >= p.passes) return;
+    tiles.bins += size_t(pass) * size_t(segments) * kRadix;
+    const int shift = pass * Bits;
+    const bool odd = slot & 1;
+    onesweepTile<Bits, Items>(tiles, odd ? p.k[1] : p.k[0], slot == 0 ? nullptr : odd ? p.v[1] : p.v[0],
+                              odd ? p.k[0] : p.k[1], odd ? p.v[0] : p.v[1], shift, p.ctl->tileCounters + slot,
+                              p.status, passTag(p.ctl->epoch + u32(slot)), p.error, min(Bits, 64 - shift));
 }
 
 // ---------------------------------------------------------------------------
@@ -629,17 +605,16 @@ static inline void launchPass(int c, cudaStream_t s, const PassArgs &p, int slot
     }
 }
 
-// One segmented pass of configuration c over `numTiles` tiles.
-static inline void launchSegmentPass(int c, cudaStream_t s, unsigned numTiles, const SegmentTiles &tiles, const u64 *keysIn,
-                              const u32 *valsIn, u64 *keysOut, u32 *valsOut, int shift, u32 *tileCounter,
-                              u64 *status, u64 tag, int *error, int bits)
+// Pass slot `slot` of a segmented sort with configuration c over `numTiles` tiles.
+static inline void launchSegmentPass(int c, cudaStream_t s, unsigned numTiles, const SegmentTiles &tiles,
+                                     const PassArgs &p, int slot, int segments)
 {
     switch (c)
     {
 #define AOT_CASE(i, B, I)                                                                                        \
     case i:                                                                                                      \
-        segmentOnesweepKernel<B, I><<<numTiles, kThreads, sizeof(SharedPass<B, I>), s>>>(                       \
-            tiles, keysIn, valsIn, keysOut, valsOut, shift, tileCounter, status, tag, error, bits);              \
+        segmentOnesweepKernel<B, I><<<numTiles, kThreads, sizeof(SharedPass<B, I>), s>>>(tiles, p, slot,         \
+                                                                                         segments);              \
         break;
         AOT_SORT_CONFIGS(AOT_CASE)
 #undef AOT_CASE

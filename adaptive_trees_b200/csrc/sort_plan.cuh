@@ -29,9 +29,10 @@ constexpr int kPlanMinPasses = 2;
 constexpr int kPlanMaxPasses = 6;
 constexpr int kPlanSets = kPlanMaxPasses - kPlanMinPasses + 2;  // a set of prefixes per choice, one of whole keys
 // Cost in passes: the repair's fixed part and its part per key of the mean
-// run.
-constexpr float kRepairCost = 0.5f;
-constexpr float kRunCost = 0.05f;
+// run.  Measured at 16Mi keys (a pass 120 us): repairs of mean runs of 3.8,
+// 4.7 and 14.4 keys took 116, 130 and 272 us.
+constexpr float kRepairCost = 0.55f;
+constexpr float kRunCost = 0.11f;
 // mean run of equal keys above which all passes run (a long run is a CTA's
 // work in the repair)
 constexpr float kMaxRepeats = 64.f;
@@ -108,27 +109,23 @@ __device__ __forceinline__ size_t planPosition(u32 i, size_t n)
     return size_t(__umul64hi(mix64(u64(i) * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull), u64(n)));
 }
 
-// Start of a sort of n keys: the control block and the digit counts are set
-// up and the plan is made by the last CTA.  keyAt(i, group) is the key at
-// position i and the segment it is sorted in.  A sample per thread, over many
+// This CTA's part of the sample: keyAt(i, group) is the key at position i and
+// the segment it is sorted in.  A sample per thread, over many
 // CTAs (one CTA took 84 us for 8192: its random loads and shared-memory
 // atomics go through one SM), and one exchange per sample and set, all of a
 // thread's in flight together: a slot holds the last prefix that was hashed
 // to it, so a repeat is missed where another prefix took the slot in between
 // (at most a quarter of the slots are used), which an estimate can bear;
 // sets with probing took 34-48 us in chains of L2 round trips.  Words of
-// earlier sorts match no prefix of this one, so nothing is cleared.
+// earlier sorts (epoch: the number of this one) match no prefix of this one,
+// so nothing is cleared.
 template <class KeyAt>
-__device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const PlanArgs &a, SortControl *ctl, u32 *hist,
-                                         size_t histWords)
+__device__ __forceinline__ void planSample(const KeyAt &keyAt, size_t n, const PlanArgs &a, u32 epoch)
 {
     __shared__ u32 sRepeats[kPlanSets];
-    __shared__ bool sLast;
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 epoch = u64(ctl->epoch + kEpochStep) << 32;  // this sort's number (set at the end)
     if (threadIdx.x < kPlanSets) sRepeats[threadIdx.x] = 0;
     __syncthreads();
-    for (size_t k = i; k < histWords; k += size_t(gridDim.x) * blockDim.x) hist[k] = 0;
     u32 group = 0;
     u64 key = 0;
     const bool valid = i < a.samples;
@@ -139,7 +136,7 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     {
         const int shift = set == 0 ? 0 : 64 - (kPlanMinPasses + set - 1) * kRadixBits;
         const u64 h = mix64((key >> shift) * 0x9E3779B97F4A7C15ull + group);
-        word[set] = epoch | u32(h);  // the low half stands for the prefix, the high bits pick the slot
+        word[set] = (u64(epoch) << 32) | u32(h);  // the low half stands for the prefix, the high bits pick the slot
         old[set] = 0;
         if (valid)
             old[set] = atomicExch(
@@ -155,6 +152,20 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     __syncthreads();
     if (threadIdx.x < kPlanSets && sRepeats[threadIdx.x])
         atomicAdd(&a.counters->repeats[threadIdx.x], sRepeats[threadIdx.x]);
+}
+
+// Start of a sort of n keys: the digit counts are cleared and the keys
+// sampled by all CTAs, the plan made and the control block set up by the last.
+template <class KeyAt>
+__device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const PlanArgs &a, SortControl *ctl, u32 *hist,
+                                         size_t histWords)
+{
+    __shared__ u32 sTotal[kPlanSets];
+    __shared__ bool sLast;
+    const u32 epoch = ctl->epoch + kEpochStep;  // this sort's number (set at the end)
+    for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < histWords; k += size_t(gridDim.x) * blockDim.x)
+        hist[k] = 0;
+    planSample(keyAt, n, a, epoch);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) sLast = atomicAdd(&a.counters->done, 1u) == gridDim.x - 1;
@@ -163,7 +174,7 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     __threadfence();
     if (threadIdx.x < kPlanSets)
     {
-        sRepeats[threadIdx.x] = __ldcg(&a.counters->repeats[threadIdx.x]);
+        sTotal[threadIdx.x] = __ldcg(&a.counters->repeats[threadIdx.x]);
         a.counters->repeats[threadIdx.x] = 0;
     }
     if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
@@ -171,8 +182,8 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     if (threadIdx.x == 0)
     {
         a.counters->done = 0;
-        ctl->first = planFirst(sRepeats, a.samples, n);
-        ctl->epoch += kEpochStep;
+        ctl->first = planFirst(sTotal, a.samples, n);
+        ctl->epoch = epoch;
         ctl->longRuns = 0;
         ctl->keygenDone = 0;
     }

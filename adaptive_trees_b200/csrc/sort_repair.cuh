@@ -25,12 +25,12 @@ namespace aot
 namespace sort
 {
 constexpr int kRepairThreads = 256;
-constexpr int kRepairTile = kRepairThreads * 8;
+constexpr int kRepairTile = kRepairThreads * 8;  // keys per CTA of the contiguous sort's repair
 constexpr int kMaxRun = 256;  // longest run the tile kernel orders
-constexpr int kRepairWindow = kRepairTile + 2 * kMaxRun;
 constexpr int kLongThreads = 512;
 
-__host__ __device__ constexpr size_t longRunSlots(size_t n) { return n / kMaxRun + 1; }
+// words of the list of long runs: start and end of its segment for each
+__host__ __device__ constexpr size_t longRunWords(size_t n) { return 2 * (n / kMaxRun + 1); }
 
 struct RepairArgs
 {
@@ -38,7 +38,7 @@ struct RepairArgs
     u32 *v[2];
     size_t n;
     SortControl *ctl;
-    u32 *longList;  // starts of the long runs [longRunSlots(n)]
+    u32 *longList;  // the long runs: start, end of the segment [longRunWords(n)]
     u64 *sample;    // every 32nd sorted key (KeyIndex), or nullptr
     const int *error;  // a look-back gave up: the passes' order cannot be relied on
     int beginBit, passes;
@@ -48,43 +48,49 @@ struct RepairArgs
     bool escapes;   // keys of escaped particles (all bits set) share their high digits with no other key
 };
 
+template <int Tile>
 struct RepairShared
 {
-    u32 lo[kRepairWindow], hi[kRepairWindow];  // the words of the window's keys
-    u32 val[kRepairWindow];
-    u32 mark[kRepairWindow / 32];
-    int before[kRepairWindow / 32];  // last mark before the word's second key (kNoMark: none)
-    int after[kRepairWindow / 32];   // first mark after the word (-kNoMark: none)
+    static constexpr int kWindow = Tile + 2 * kMaxRun;
+    u32 lo[kWindow], hi[kWindow];  // the words of the window's keys
+    u32 val[kWindow];
+    u32 mark[kWindow / 32];
+    int before[kWindow / 32];  // last mark before the word's second key (kNoMark: none)
+    int after[kWindow / 32];   // first mark after the word (-kNoMark: none)
 };
 // Far enough from every position that a run to or from it is too long.
 constexpr int kNoMark = -(1 << 20);
 
-// The runs that start in tile blockIdx.x.  First: the plan's first pass, with
-// all 64 bits sorted, so that what tells runs apart and what orders a run are
-// known words; or 0: any plan, and the sorted bits are those of keyMask.
+// The runs that start in the tile of (at most) Tile keys from `begin`, in the
+// segment [segBegin, segEnd) of keys that are sorted together.  First: the
+// plan's first pass, with all 64 bits sorted, so that what tells runs apart
+// and what orders a run are known words; or 0: any plan, and the sorted bits
+// are those of keyMask.
 //
-// Window position w is key base - kMaxRun + w.  The warps take the window's
+// Window position w is key begin - kMaxRun + w.  The warps take the window's
 // words of 32 marks in turn; the runs of a word's keys start and end in the
 // word or, the same for all its lanes, at the last mark before it and the
 // first one after it (found for all words by two warps first).
-template <int First>
-__device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm, u32 first, bool inPlace)
+template <int First, int Tile>
+__device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared<Tile> &sm, u32 first, bool inPlace,
+                                           size_t begin, size_t segBegin, size_t segEnd)
 {
-    constexpr int kWords = kRepairWindow / 32, kSide = kMaxRun / 32;
+    constexpr int kWindow = Tile + 2 * kMaxRun, kWords = kWindow / 32, kSide = kMaxRun / 32;
+    static_assert(Tile % (2 * kRepairThreads) == 0 && 2 * kMaxRun % (2 * kRepairThreads) == 0, "whole rounds of loads");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // pointers to the key of window position 0 (used for positions [wBegin, wEnd) only)
-    const long long origin = (long long)blockIdx.x * kRepairTile - kMaxRun;
+    const long long origin = (long long)begin - kMaxRun;
     const u64 *src = (inPlace ? a.k[0] : a.k[1]) + origin;
     const u32 *srcV = (inPlace ? a.v[0] : a.v[1]) + origin;
     u64 *dst = a.k[0] + origin;
     u32 *dstV = a.v[0] + origin;
-    const size_t left = a.n - size_t(blockIdx.x) * kRepairTile;
-    const int wBegin = origin < 0 ? kMaxRun : 0;
-    const int wEnd = left < size_t(kRepairTile + kMaxRun) ? int(left) + kMaxRun : kRepairWindow;
-    if (a.aligned && wBegin == 0 && wEnd == kRepairWindow)
+    const int wBegin = (long long)segBegin > origin ? int((long long)segBegin - origin) : 0;
+    const bool atStart = (long long)segBegin >= origin;  // the window's first key starts the segment
+    const int wEnd = (long long)segEnd - origin < kWindow ? int((long long)segEnd - origin) : kWindow;
+    if (a.aligned && wBegin == 0 && wEnd == kWindow && (begin & 1) == 0)
     {
 #pragma unroll
-        for (int i = 0; i < kRepairWindow / (2 * kRepairThreads); ++i)
+        for (int i = 0; i < kWindow / (2 * kRepairThreads); ++i)
         {
             const int w = 2 * (tid + i * kRepairThreads);  // origin and w are even
             const uint4 k = *reinterpret_cast<const uint4 *>(src + w);
@@ -93,11 +99,22 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
             *reinterpret_cast<uint2 *>(sm.val + w) = *reinterpret_cast<const uint2 *>(srcV + w);
         }
     }
+    else if (wBegin == 0 && wEnd == kWindow)
+    {
+#pragma unroll
+        for (int i = 0; i < kWindow / kRepairThreads; ++i)
+        {
+            const int w = tid + i * kRepairThreads;
+            const u64 k = src[w];
+            sm.lo[w] = u32(k);
+            sm.hi[w] = u32(k >> 32);
+            sm.val[w] = srcV[w];
+        }
+    }
     else
     {
-        for (int w = tid; w < kRepairWindow; w += kRepairThreads)
+        for (int w = wBegin + tid; w < wEnd; w += kRepairThreads)
         {
-            if (w < wBegin || w >= wEnd) continue;
             const u64 k = src[w];
             sm.lo[w] = u32(k);
             sm.hi[w] = u32(k >> 32);
@@ -123,7 +140,7 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
         }
         else if (w == wBegin)
         {
-            mark = wBegin != 0;
+            mark = atStart;
         }
         const u32 m = __ballot_sync(0xffffffffu, mark);
         if (lane == 0) sm.mark[word] = m;
@@ -163,7 +180,7 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
     for (int word = kSide + warp; word < kWords; word += kRepairThreads / 32)
     {
         const u32 marks = sm.mark[word];
-        if (word >= kSide + kRepairTile / 32 && (marks & 1u)) break;  // past the last run of the tile
+        if (word >= kSide + Tile / 32 && (marks & 1u)) break;  // past the last run of the tile
         const int w0 = word * 32, w = w0 + lane;
         if (w >= wEnd) break;
         const u32 mh = marks & le, me = marks & ~le;
@@ -176,13 +193,17 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
             // part of a long run: its first key's CTA lists it, every key of
             // the tile is brought over as it is (escaped particles are equal
             // keys: nothing to sort)
-            if (w >= kMaxRun + kRepairTile) continue;
+            if (w >= kMaxRun + Tile) continue;
             if (h == w && !(a.escapes && (lo & sm.hi[w]) == 0xffffffffu))
-                a.longList[atomicAdd(&a.ctl->longRuns, 1u)] = u32(origin + w);
+            {
+                const u32 slot = atomicAdd(&a.ctl->longRuns, 1u);
+                a.longList[2 * slot] = u32(origin + w);
+                a.longList[2 * slot + 1] = u32(segEnd);
+            }
         }
         else
         {
-            if (unsigned(h - kMaxRun) >= unsigned(kRepairTile)) continue;  // another CTA's run
+            if (unsigned(h - kMaxRun) >= unsigned(Tile)) continue;  // another CTA's run
             if (e - h > 1)
             {
                 to = h;
@@ -220,9 +241,9 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
     for (int word = kSide + tid; word < kWords; word += kRepairThreads)
     {
         const int w = word * 32, h = sm.before[word];
-        const bool inTile = word < kSide + kRepairTile / 32;
+        const bool inTile = word < kSide + Tile / 32;
         if (w >= wEnd) continue;
-        const bool mine = unsigned(h - kMaxRun) < unsigned(kRepairTile);
+        const bool mine = unsigned(h - kMaxRun) < unsigned(Tile);
         const u32 later = sm.mark[word] & ~1u;
         const bool isLong = (later ? w + __ffs(int(later)) - 1 : sm.after[word]) - h > kMaxRun;
         if (isLong ? inTile : mine) a.sample[(origin + w) >> kSampleShift] = dst[w];
@@ -233,7 +254,7 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared &sm
 template <bool Whole>
 static __global__ void __launch_bounds__(kRepairThreads) repairKernel(RepairArgs a)
 {
-    __shared__ __align__(16) RepairShared sm;
+    __shared__ __align__(16) RepairShared<kRepairTile> sm;
     if (*a.error) return;
     const u32 first = a.ctl->first;
     if (first == 0)
@@ -246,33 +267,37 @@ static __global__ void __launch_bounds__(kRepairThreads) repairKernel(RepairArgs
         return;
     }
     const bool inPlace = a.endsIn0 || ((u32(a.passes) - first) & 1u) == 0;
-    if (Whole && first == 4) repairTile<4>(a, sm, first, inPlace);
-    else if (Whole && first < 4) repairTile<3>(a, sm, first, inPlace);
-    else repairTile<0>(a, sm, first, inPlace);
+    const size_t begin = size_t(blockIdx.x) * kRepairTile;
+    if (Whole && first == 4) repairTile<4>(a, sm, first, inPlace, begin, 0, a.n);
+    else if (Whole && first < 4) repairTile<3>(a, sm, first, inPlace, begin, 0, a.n);
+    else repairTile<0>(a, sm, first, inPlace, begin, 0, a.n);
 }
+
+template <int Threads>
+struct LongShared
+{
+    u32 start[kRadix];
+    u32 warp[Threads / 32][kRadix];
+    u32 end, same;
+};
 
 // A long run per CTA: an LSD radix sort of its remaining digits between its
 // stretch of buffer 0 and the same stretch of buffer 1.  Digits all keys
 // share are left out.
-static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs a)
+template <int Threads>
+__device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Threads> &sm, int first, u32 runs)
 {
-    constexpr int W = kLongThreads / 32;
-    __shared__ u32 sStart[kRadix];
-    __shared__ u32 sWarp[W][kRadix];
-    __shared__ u32 sEnd, sSame;
-    if (*a.error) return;
-    const u32 runs = a.ctl->longRuns;
+    constexpr int W = Threads / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int first = int(a.ctl->first);
     const int prefix = a.beginBit + first * kRadixBits;
     for (u32 r = blockIdx.x; r < runs; r += gridDim.x)
     {
-        const u32 h = a.longList[r];
+        const u32 h = a.longList[2 * r], limit = a.longList[2 * r + 1];
         if (warp == 0)
         {
             // end of the run: first key whose high digits are larger
             const u64 mine = (a.k[0][h] & a.keyMask) >> prefix;
-            u32 lo = h + 1, hi = u32(a.n);
+            u32 lo = h + 1, hi = limit;
             while (lo < hi)
             {
                 const u32 len = hi - lo;
@@ -284,10 +309,10 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
                 if (c > 0) lo = pLow + 1;
                 if (c < 32) hi = pHigh;
             }
-            if (lane == 0) sEnd = lo;
+            if (lane == 0) sm.end = lo;
         }
         __syncthreads();
-        const u32 e = sEnd;
+        const u32 e = sm.end;
         int at = 0;  // buffer that holds the run
         for (int d = 0; d < first; ++d)
         {
@@ -296,15 +321,15 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
             const u32 *inV = at ? a.v[1] : a.v[0];
             u64 *out = at ? a.k[0] : a.k[1];
             u32 *outV = at ? a.v[0] : a.v[1];
-            if (tid < kRadix) sStart[tid] = 0;
-            if (tid == 0) sSame = 0;
+            if (tid < kRadix) sm.start[tid] = 0;
+            if (tid == 0) sm.same = 0;
             __syncthreads();
-            for (u32 i = h + tid; i < e; i += kLongThreads)
-                atomicAdd(&sStart[unsigned(in[i] >> shift) & (kRadix - 1)], 1u);
+            for (u32 i = h + tid; i < e; i += Threads)
+                atomicAdd(&sm.start[unsigned(in[i] >> shift) & (kRadix - 1)], 1u);
             __syncthreads();
-            if (tid < kRadix && sStart[tid] == e - h) sSame = 1;
+            if (tid < kRadix && sm.start[tid] == e - h) sm.same = 1;
             __syncthreads();
-            const bool same = sSame != 0;
+            const bool same = sm.same != 0;
             if (same)
             {
                 __syncthreads();
@@ -317,7 +342,7 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                 {
-                    c[k] = sStart[lane * 8 + k];
+                    c[k] = sm.start[lane * 8 + k];
                     sum += c[k];
                 }
                 u32 inc = sum;
@@ -331,13 +356,13 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                 {
-                    sStart[lane * 8 + k] = run;
+                    sm.start[lane * 8 + k] = run;
                     run += c[k];
                 }
             }
-            for (u32 i0 = h; i0 < e; i0 += kLongThreads)
+            for (u32 i0 = h; i0 < e; i0 += Threads)
             {
-                for (int k = tid; k < W * kRadix; k += kLongThreads) (&sWarp[0][0])[k] = 0;
+                for (int k = tid; k < W * kRadix; k += Threads) (&sm.warp[0][0])[k] = 0;
                 __syncthreads();
                 const u32 i = i0 + tid;
                 const bool valid = i < e;
@@ -345,26 +370,26 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
                 const u32 val = valid ? inV[i] : 0;
                 const unsigned digit = unsigned(key >> shift) & (kRadix - 1);
                 const unsigned validMask = __ballot_sync(0xffffffffu, valid);
-                const unsigned peers = peerLanes(digit, kRadixBits, validMask);
+                const unsigned peers = peerLanes<kRadixBits>(digit) & validMask;
                 const unsigned rank = __popc(peers & laneMaskLt());
-                if (valid && rank == 0) sWarp[warp][digit] = __popc(peers);
+                if (valid && rank == 0) sm.warp[warp][digit] = __popc(peers);
                 __syncthreads();
                 if (tid < kRadix)
                 {
-                    u32 acc = sStart[tid];
+                    u32 acc = sm.start[tid];
 #pragma unroll
                     for (int w = 0; w < W; ++w)
                     {
-                        const u32 c = sWarp[w][tid];
-                        sWarp[w][tid] = acc;
+                        const u32 c = sm.warp[w][tid];
+                        sm.warp[w][tid] = acc;
                         acc += c;
                     }
-                    sStart[tid] = acc;
+                    sm.start[tid] = acc;
                 }
                 __syncthreads();
                 if (valid)
                 {
-                    const u32 to = sWarp[warp][digit] + rank;
+                    const u32 to = sm.warp[warp][digit] + rank;
                     out[to] = key;
                     outV[to] = val;
                 }
@@ -373,7 +398,7 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
             at ^= 1;
         }
         __syncthreads();
-        for (u32 i = h + tid; i < e; i += kLongThreads)
+        for (u32 i = h + tid; i < e; i += Threads)
         {
             u64 key;
             if (at)
@@ -390,6 +415,13 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
         }
         __syncthreads();
     }
+}
+
+static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs a)
+{
+    __shared__ LongShared<kLongThreads> sm;
+    if (*a.error) return;
+    sortLongRuns(a, sm, int(a.ctl->first), a.ctl->longRuns);
 }
 
 // The repair of a planned sort (after its passes).

@@ -98,3 +98,46 @@ def test_planned_sort_is_the_stable_sort(name, kind, hilbert):
         corner = t.get("cornerstone_d").view(torch.int64).cpu().numpy().view(np.uint64)
         assert np.array_equal(np.diff(np.searchsorted(keys[order], corner)), counts.astype(np.int64)), (name, step)
     t.close()
+
+
+SYSTEMS = {
+    "odd sizes": [uniform(n, 100 + n) for n in (1, 0, 31, 2048, 2049, 7, 0, 5000, 257)],
+    "the same system again": [with_cluster(30_000, 400, 1e-9, 31)] * 3,  # equal keys on both sides of a boundary
+    "clusters": [with_cluster(60_000, 3000, 1e-7, 32), uniform(100_001, 33), with_cluster(9_000, 9_000, 1e-6, 34)],
+    "points and escapes": [stacked(20_000, 300, 35), escaped(30_000, 2, 36), escaped(500, 1, 37), uniform(64, 38)],
+    "one cluster each": [with_cluster(8_000, 8_000, 1e-5, 40 + k) for k in range(6)],
+}
+
+
+@pytest.mark.parametrize("hilbert", [False, True])
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_planned_sort_of_a_batch_is_each_systems_stable_sort(name, hilbert):
+    import torch
+
+    import adaptive_trees_b200 as ab
+    curve = ab.SfcKind.Hilbert if hilbert else ab.SfcKind.Morton
+    dev = [[torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in x] for x in SYSTEMS[name]]
+    b = ab.Batch(*[[d[k] for d in dev] for k in range(3)], ab.TreeConfig(sfcKind=curve))
+
+    def check(step):
+        for s, d in enumerate(dev):
+            if not d[0].numel():
+                continue
+            keys = ab.compute_sfc_keys(0, *d, sfc_kind=curve).view(torch.int64).cpu().numpy().view(np.uint64)
+            order = np.argsort(keys, kind="stable")
+            got_k = b.get(s, "particleKeys_d").view(torch.int64).cpu().numpy().view(np.uint64)
+            got_p = b.get(s, "perm_d").view(torch.int32).cpu().numpy().view(np.uint32)
+            assert np.array_equal(got_k, keys[order]), (name, s, step)
+            assert np.array_equal(got_p, order.astype(np.uint32)), (name, s, step)
+
+    for step in ("first build (timed configurations)", "build in one launch", "build in one launch again"):
+        b.build()
+        check(step)
+    for d in dev:  # an update sorts launch by launch
+        for a in d:
+            a.copy_(torch.where(a < 1, (a + 1e-3) % 1.0, a))
+    torch.cuda.synchronize()
+    b.update()
+    b.doBuffersNeedResize()
+    check("update")
+    b.close()
