@@ -115,15 +115,16 @@ static __global__ void __launch_bounds__(sort::kPlanThreads)
     planKernel(const System *__restrict__ systems, int numSystems, const u32 *__restrict__ segBase, size_t total,
                const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist, size_t histWords)
 {
-    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
     __syncthreads();
+    const KeyMaker<Real, C> make(prm, sPair);
     const auto keyAt = [&](size_t g, u32 &group) {
         group = systemOf(segBase, numSystems, u32(g));
         const System sy = systems[group];
         const size_t i = g - sy.base;
-        return particleKey<Real, C>(static_cast<const Real *>(sy.x)[i], static_cast<const Real *>(sy.y)[i],
-                                    static_cast<const Real *>(sy.z)[i], prm, sPair);
+        return make(static_cast<const Real *>(sy.x)[i], static_cast<const Real *>(sy.y)[i],
+                    static_cast<const Real *>(sy.z)[i]);
     };
     sort::planSort(keyAt, total, plan, ctl, hist, histWords);
 }
@@ -141,8 +142,9 @@ __device__ __forceinline__ void keygenTiles(const System *__restrict__ systems, 
                                             const u32 *__restrict__ tileBegin, const u32 *__restrict__ tileEnd,
                                             u32 t0, u32 t1, const KeygenParams<Real> &prm, u64 *__restrict__ keys,
                                             u32 *__restrict__ hist, int firstPass, u32 *sh,
-                                            const unsigned short *sPair)
+                                            const u32 *sPair)
 {
+    const KeyMaker<Real, C> make(prm, sPair);
     int cur = -1;
     auto flush = [&]() {
         __syncthreads();
@@ -174,17 +176,28 @@ __device__ __forceinline__ void keygenTiles(const System *__restrict__ systems, 
         const Real *y = static_cast<const Real *>(sy.y);
         const Real *z = static_cast<const Real *>(sy.z);
         const u32 end = tileEnd[t];
-        for (u32 g = tileBegin[t] + threadIdx.x; g < end; g += blockDim.x)
+        // four particles a thread in flight (the loads of one at a time left
+        // the kernel waiting: systems start anywhere, so loads are scalar)
+        constexpr int V = 4;
+        for (u32 g0 = tileBegin[t] + threadIdx.x; g0 < end; g0 += V * blockDim.x)
         {
-            const u32 l = g - sy.base;
-            const u64 k = particleKey<Real, C>(x[l], y[l], z[l], prm, sPair);
-            keys[g] = k;
-            if (hist)
-            {
+            Real vx[V], vy[V], vz[V];
 #pragma unroll
-                for (int p = 0; p < sort::kMaxPasses; ++p)
-                    if (p >= firstPass)
-                        atomicAdd(&sh[p * sort::kRadix + int((k >> (p * sort::kRadixBits)) & (sort::kRadix - 1))], 1u);
+            for (int j = 0; j < V; ++j)
+            {
+                const u32 g = g0 + u32(j) * blockDim.x, l = (g < end ? g : g0) - sy.base;
+                vx[j] = __ldcs(x + l);
+                vy[j] = __ldcs(y + l);
+                vz[j] = __ldcs(z + l);
+            }
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+            {
+                const u32 g = g0 + u32(j) * blockDim.x;
+                if (g >= end) break;
+                const u64 k = make(vx[j], vy[j], vz[j]);
+                keys[g] = k;
+                if (hist) countDigits(k, firstPass, sh);
             }
         }
     }
@@ -200,7 +213,7 @@ static __global__ void __launch_bounds__(kThreads)
 {
     if (ctl) firstPass = int(ctl->first);  // the plan's
     __shared__ u32 sh[sort::kMaxPasses * sort::kRadix];
-    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) sh[i] = 0;
     if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
     __syncthreads();

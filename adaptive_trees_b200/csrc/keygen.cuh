@@ -26,23 +26,49 @@ struct KeygenParams
     HilbertTables h;
 };
 
-// sPair: the two-level Hilbert table (hilbertPairEntry) in shared memory.
+// What a thread keeps for the keys of its particles.  sPair: the two-level
+// Hilbert table (hilbertPairEntry) in shared memory.
 template <class Real, Curve C>
-__device__ __forceinline__ u64 particleKey(Real x, Real y, Real z, const KeygenParams<Real> &p,
-                                           const unsigned short *sPair)
+struct KeyMaker
 {
-    if constexpr (C == Curve::Binary)
+    QuantAxis<Real> x, y, z;
+    const u32 *sPair;
+    const BinaryGeometry &g;
+    __device__ __forceinline__ KeyMaker(const KeygenParams<Real> &p, const u32 *pair)
+        : x(quantAxis(p.q.xmin, p.q.ilx, p.q.bx)), y(quantAxis(p.q.ymin, p.q.ily, p.q.by)),
+          z(quantAxis(p.q.zmin, p.q.ilz, p.q.bz)), sPair(pair), g(p.g)
     {
-        return binaryKey<Real>(x, y, z, p.g);
     }
-    else
+    __device__ __forceinline__ u64 operator()(Real px, Real py, Real pz) const
     {
-        if (isEscaped<Real>(x, y, z)) return kInvalidKey;
-        const u32 ix = quantise(x, p.q.xmin, p.q.ilx, p.q.bx);
-        const u32 iy = quantise(y, p.q.ymin, p.q.ily, p.q.by);
-        const u32 iz = quantise(z, p.q.zmin, p.q.ilz, p.q.bz);
-        if constexpr (C == Curve::Hilbert) return hilbertKeyPairs(ix, iy, iz, sPair);
-        else return mortonKey(ix, iy, iz);
+        if constexpr (C == Curve::Binary)
+        {
+            return binaryKey<Real>(px, py, pz, g);
+        }
+        else
+        {
+            const u32 ix = quantise(px, x), iy = quantise(py, y), iz = quantise(pz, z);
+            u64 k;
+            if constexpr (C == Curve::Hilbert) k = hilbertKeyPairs(ix, iy, iz, sPair);
+            else k = mortonKey(ix, iy, iz);
+            return isEscaped<Real>(px, py, pz) ? kInvalidKey : k;
+        }
+    }
+};
+
+// Counts the digits of passes firstPass to 7 of a key in
+// sh[kMaxPasses][kRadix] (shared memory).
+__device__ __forceinline__ void countDigits(u64 k, int firstPass, u32 *sh)
+{
+    static_assert(sort::kMaxPasses == 8 && sort::kRadixBits == 8, "a byte per digit");
+    const u32 half[2] = {u32(k), u32(k >> 32)};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        if (firstPass >= 4 * (h + 1)) continue;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (4 * h + b >= firstPass) atomicAdd(sh + (4 * h + b) * sort::kRadix + ((half[h] >> (8 * b)) & 0xffu), 1u);
     }
 }
 
@@ -50,7 +76,7 @@ constexpr int kKeygenThreads = 256;
 
 // The two-level Hilbert table in shared memory, from the one-level tables.
 template <class Real>
-__device__ __forceinline__ void loadPairTable(const KeygenParams<Real> &prm, unsigned short *sPair)
+__device__ __forceinline__ void loadPairTable(const KeygenParams<Real> &prm, u32 *sPair)
 {
     __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8];
     for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x)
@@ -69,10 +95,11 @@ static __global__ void __launch_bounds__(sort::kPlanThreads)
     planKernel(const Real *__restrict__ x, const Real *__restrict__ y, const Real *__restrict__ z, size_t n,
                const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist)
 {
-    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
     __syncthreads();
-    const auto keyAt = [&](size_t i, u32 &) { return particleKey<Real, C>(x[i], y[i], z[i], prm, sPair); };
+    const KeyMaker<Real, C> make(prm, sPair);
+    const auto keyAt = [&](size_t i, u32 &) { return make(x[i], y[i], z[i]); };
     sort::planSort(keyAt, n, plan, ctl, hist, size_t(sort::kPassSlots) * sort::kRadix);
 }
 
@@ -86,18 +113,13 @@ static __global__ void __launch_bounds__(kKeygenThreads)
                  u32 *__restrict__ bins, sort::SortControl *ctl)
 {
     __shared__ u32 sh[sort::kMaxPasses][sort::kRadix];
-    __shared__ unsigned short sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
+    __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
     if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
     const int firstPass = hist ? int(ctl->first) : sort::kMaxPasses;
     __syncthreads();
 
-    auto count = [&](u64 k) {
-#pragma unroll
-        for (int p = 0; p < sort::kMaxPasses; ++p)
-            if (p >= firstPass) atomicAdd(&sh[p][(k >> (p * sort::kRadixBits)) & (sort::kRadix - 1)], 1u);
-    };
-
+    const KeyMaker<Real, C> make(prm, sPair);
     const size_t groups = n / Vec;
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     for (size_t gi = blockIdx.x * size_t(blockDim.x) + threadIdx.x; gi < groups; gi += stride)
@@ -132,8 +154,8 @@ static __global__ void __launch_bounds__(kKeygenThreads)
 #pragma unroll
         for (int j = 0; j < Vec; ++j)
         {
-            k[j] = particleKey<Real, C>(vx[j], vy[j], vz[j], prm, sPair);
-            count(k[j]);
+            k[j] = make(vx[j], vy[j], vz[j]);
+            countDigits(k[j], firstPass, &sh[0][0]);
         }
         if constexpr (Vec == 4)
         {
@@ -153,9 +175,9 @@ static __global__ void __launch_bounds__(kKeygenThreads)
     // tail particles that do not fill a vector
     for (size_t i = groups * Vec + blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += stride)
     {
-        const u64 k = particleKey<Real, C>(x[i], y[i], z[i], prm, sPair);
+        const u64 k = make(x[i], y[i], z[i]);
         keys[i] = k;
-        count(k);
+        countDigits(k, firstPass, &sh[0][0]);
     }
     if (!hist) return;
     __syncthreads();

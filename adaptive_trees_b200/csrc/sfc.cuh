@@ -19,15 +19,23 @@ namespace aot
 // --------------------------------------------------------------------------
 // Morton (iMorton / decodeMorton, sfc_keys.cuh:174-237)
 // --------------------------------------------------------------------------
-__host__ __device__ __forceinline__ u64 spread3(u64 v)
+// The 10 low bits of v, three places apart.  A multiplication adds the
+// shifted copy (the bits do not overlap), which leaves half of the work to the
+// multiply-add pipe: key generation is bound by the integer ALU, and 64-bit
+// spreads by shifts took half of its instructions.
+__host__ __device__ __forceinline__ u32 spread10(u32 v)
 {
-    u64 x = v & 0x1fffffull;
-    x = (x | x << 32) & 0x001f00000000ffffull;
-    x = (x | x << 16) & 0x001f0000ff0000ffull;
-    x = (x | x << 8) & 0x100f00f00f00f00full;
-    x = (x | x << 4) & 0x10c30c30c30c30c3ull;
-    x = (x | x << 2) & 0x1249249249249249ull;
-    return x;
+    v &= 0x3ffu;
+    v = (v * 0x00010001u) & 0xff0000ffu;
+    v = (v * 0x00000101u) & 0x0f00f00fu;
+    v = (v * 0x00000011u) & 0xc30c30c3u;
+    v = (v * 0x00000005u) & 0x49249249u;
+    return v;
+}
+// Ten levels of octants (x << 2 | y << 1 | z, the highest first) in 30 bits.
+__host__ __device__ __forceinline__ u32 interleave10(u32 x, u32 y, u32 z)
+{
+    return spread10(x) * 4u + spread10(y) * 2u + spread10(z);
 }
 __host__ __device__ __forceinline__ u32 compact3(u64 v)
 {
@@ -39,9 +47,11 @@ __host__ __device__ __forceinline__ u32 compact3(u64 v)
     v = (v ^ (v >> 32)) & 0x00000000001fffffull;
     return u32(v);
 }
+// x, y, z: 21-bit words.
 __host__ __device__ __forceinline__ u64 mortonKey(u32 x, u32 y, u32 z)
 {
-    return (spread3(x) << 2) | (spread3(y) << 1) | spread3(z);
+    const u32 last = ((x & 1u) << 2) | ((y & 1u) << 1) | (z & 1u);
+    return (u64(interleave10(x >> 11, y >> 11, z >> 11)) << 33) | (u64(interleave10(x >> 1, y >> 1, z >> 1)) << 3) | last;
 }
 
 // --------------------------------------------------------------------------
@@ -130,38 +140,50 @@ __host__ __device__ __forceinline__ u64 hilbertPrefix(u32 x, u32 y, u32 z, unsig
     return key << (3u * (kOctLevels - levels));
 }
 
-// Two levels per lookup: pair[state * 64 + (o1 << 3 | o2)] = the two emitted
-// digits (d1 << 3 | d2) | the state after both << 6, for the original octants
-// o1, o2 of two consecutive levels.  3072 entries built from enc / encNext.
+// Two levels per lookup: pair[state * 64 + (o1 << 3 | o2)] = the state after
+// both << 8 | the two emitted digits (d1 << 3 | d2) << 2, for the original
+// octants o1, o2 of two consecutive levels.  3072 entries built from enc /
+// encNext.  An entry's upper bits are the byte offset of its state's entries,
+// so the next lookup's offset is one bit selection between the entry and the
+// octants.
 constexpr int kHilbertPairEntries = 48 * 64;
-__host__ __device__ __forceinline__ unsigned short hilbertPairEntry(int i, const unsigned char *enc,
-                                                                   const unsigned char *encNext)
+__host__ __device__ __forceinline__ u32 hilbertPairEntry(int i, const unsigned char *enc, const unsigned char *encNext)
 {
     const int s = i >> 6, o1 = (i >> 3) & 7, o2 = i & 7;
     const int a = s * 8 + o1;
     const int b = int(encNext[a]) * 8 + o2;
-    return (unsigned short)((enc[a] << 3) | enc[b] | (encNext[b] << 6));
+    return (u32(encNext[b]) << 8) | (u32((enc[a] << 3) | enc[b]) << 2);
 }
 
 // The full 21-level Hilbert key of (x, y, z) with the pair table: the Morton
 // interleave of the words puts each level's original octant (x << 2 | y << 1
-// | z) in consecutive bits, so two levels are one 6-bit field.  Equal to
+// | z) in consecutive bits, so two levels are one 6-bit field (ten levels
+// from one 32-bit word; the last level alone).  Equal to
 // hilbertPrefix(x, y, z, kOctLevels, ...).
-__host__ __device__ __forceinline__ u64 hilbertKeyPairs(u32 x, u32 y, u32 z, const unsigned short *sPair)
+__host__ __device__ __forceinline__ u64 hilbertKeyPairs(u32 x, u32 y, u32 z, const u32 *sPair)
 {
-    const u64 m = mortonKey(x, y, z);
-    u64 key = 0;
-    unsigned s = kHilbertStart;
+    constexpr u32 kField = 0xfcu;  // a field's place in an entry and in its byte offset
+    const char *table = reinterpret_cast<const char *>(sPair);
+    const auto lookup = [&](u32 entry, u32 field) {
+        return *reinterpret_cast<const u32 *>(table + ((entry & ~kField) | (field & kField)));
+    };
+    const u32 w0 = interleave10(x >> 11, y >> 11, z >> 11), w1 = interleave10(x >> 1, y >> 1, z >> 1);
+    u32 v = u32(kHilbertStart) << 8, k0 = 0, k1 = 0;  // digits times 4
 #pragma unroll
-    for (int i = 0; i < int(kOctLevels) / 2; ++i)  // levels 2i and 2i + 1 from the top
+    for (int i = 0; i < 5; ++i)
     {
-        const unsigned v = sPair[s * 64 + (unsigned(m >> (3 * (kOctLevels - 2 - 2 * i))) & 63u)];
-        key = (key << 6) | (v & 63u);
-        s = v >> 6;
+        v = lookup(v, i < 4 ? w0 >> (22 - 6 * i) : w0 << 2);
+        k0 = k0 * 64u + (v & kField);
     }
-    // the last level alone: the first digit of the entry with o2 = 0
-    const unsigned v = sPair[s * 64 + ((unsigned(m) & 7u) << 3)];
-    return (key << 3) | ((v >> 3) & 7u);
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+    {
+        v = lookup(v, i < 4 ? w1 >> (22 - 6 * i) : w1 << 2);
+        k1 = k1 * 64u + (v & kField);
+    }
+    // the last level: the first digit of the entry with o2 = 0
+    v = lookup(v, ((x & 1u) << 7) | ((y & 1u) << 6) | ((z & 1u) << 5));
+    return (u64(k0) << 31) | (u64(k1) << 1) | ((v >> 5) & 7u);
 }
 
 // Decode the top `levels` levels of a Hilbert key to the cell's corner in
@@ -193,26 +215,39 @@ struct QuantBox
     unsigned bx, by, bz;  // bits per axis (21 minus the axis' shortening)
 };
 
+// One axis of it: cells per unit length m = 2^bits / length, the box' start
+// and the last cell.  Set up once per thread, not per particle.
+template <class T>
+struct QuantAxis
+{
+    T m, vmin;
+    int top;
+};
+__device__ __forceinline__ QuantAxis<float> quantAxis(float vmin, float il, unsigned bits)
+{
+    return {__fmul_rn(float(1u << bits), il), vmin, int(1u << bits) - 1};
+}
+__device__ __forceinline__ QuantAxis<double> quantAxis(double vmin, double il, unsigned bits)
+{
+    return {__dmul_rn(double(1u << bits), il), vmin, int(1u << bits) - 1};
+}
+
 // floor(v*m) - vmin*m with the subtraction fused (as nvcc contracts it in the
 // reference kernel), truncated with saturation and clamped to the top cell.
-__device__ __forceinline__ u32 quantise(float v, float vmin, float il, unsigned bits)
+__device__ __forceinline__ u32 quantise(float v, const QuantAxis<float> &a)
 {
-    const float m = __fmul_rn(float(1u << bits), il);
-    const float f = floorf(__fmul_rn(v, m));
-    const float q = __fmaf_rn(-vmin, m, f);
+    const float f = floorf(__fmul_rn(v, a.m));
+    const float q = __fmaf_rn(-a.vmin, a.m, f);
     int i = __float2int_rz(q);
-    const int top = int(1u << bits) - 1;
-    i = i < top ? i : top;
+    i = i < a.top ? i : a.top;
     return u32(i) & 0x1fffffu;
 }
-__device__ __forceinline__ u32 quantise(double v, double vmin, double il, unsigned bits)
+__device__ __forceinline__ u32 quantise(double v, const QuantAxis<double> &a)
 {
-    const double m = __dmul_rn(double(1u << bits), il);
-    const double f = floor(__dmul_rn(v, m));
-    const double q = __fma_rn(-vmin, m, f);
+    const double f = floor(__dmul_rn(v, a.m));
+    const double q = __fma_rn(-a.vmin, a.m, f);
     int i = __double2int_rz(q);
-    const int top = int(1u << bits) - 1;
-    i = i < top ? i : top;
+    i = i < a.top ? i : a.top;
     return u32(i) & 0x1fffffu;
 }
 
@@ -252,13 +287,20 @@ __device__ __forceinline__ u64 fixed63(double v)
     return k < kMaxKey - 1 ? k : kMaxKey - 1;
 }
 
+// d / side.  A side of 1 (the unit box; the same for all threads) needs no
+// division: d / 1 is d.
+__device__ __forceinline__ double sideFraction(double d, double side)
+{
+    return side == 1.0 ? d : __ddiv_rn(d, side);
+}
+
 template <class T>
 __device__ __forceinline__ u64 binaryKey(T x, T y, T z, const BinaryGeometry &g)
 {
     if (isEscaped<T>(x, y, z)) return kInvalidKey;
-    const double vx = __ddiv_rn(__dsub_rn(double(x), g.xmin), __dsub_rn(g.xmax, g.xmin));
-    const double vy = __ddiv_rn(__dsub_rn(double(y), g.ymin), __dsub_rn(g.ymax, g.ymin));
-    const double vz = __ddiv_rn(__dsub_rn(double(z), g.zmin), __dsub_rn(g.zmax, g.zmin));
+    const double vx = sideFraction(__dsub_rn(double(x), g.xmin), __dsub_rn(g.xmax, g.xmin));
+    const double vy = sideFraction(__dsub_rn(double(y), g.ymin), __dsub_rn(g.ymax, g.ymin));
+    const double vz = sideFraction(__dsub_rn(double(z), g.zmin), __dsub_rn(g.zmax, g.zmin));
     u64 c[3] = {fixed63(vx), fixed63(vy), fixed63(vz)};
     if (g.mortonOrder)
     {
