@@ -540,7 +540,7 @@ int sortWithIndices(cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int passes, 
     a.ensure(n, s, false);
     sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
-    sort::launchHistogram(cfg, s, blocks, k[0], n, 0, passes, a.hist(), 8 * passes), noteLaunch();
+    sort::launchHistogram(cfg, s, blocks, k[0], n, 0, passes, a.hist(), 8 * passes, a.ctl()), noteLaunch();
     sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
     AOT_LAUNCH_CHECK();
     return runPasses(cfg, s, k, v, n, 8 * passes, a, error, false);
@@ -673,15 +673,18 @@ namespace
 {
 struct PairSortLayout
 {
-    // altKeys | altVals | counters | status, each part 256-byte aligned.  The
+    // altKeys | altVals | counters | status | plan table | long runs, each
+    // part 256-byte aligned; from the counters to the plan table they are
+    // cleared before a sort.  The
     // counters part starts with the error word (and 3 pad words), so its
     // offset depends on n only and ao_sort_pairs_check can find it whatever
-    // configuration ran; then the control block, hist[passes][256] and
-    // bins[passes][256].
-    size_t altKeys = 0, altVals = 0, counters = 0, status = 0, total = 0, tiles = 0;
+    // configuration ran; then the control block, the plan's counters,
+    // hist[passes][256] and bins[passes][256].
+    size_t altKeys = 0, altVals = 0, counters = 0, status = 0, table = 0, longRuns = 0, total = 0, tiles = 0;
     int passes = 0;
     static constexpr size_t kCounterHead = 4;  // error word + padding (u32 words)
-    static constexpr size_t kCtlWords = (sizeof(sort::SortControl) / sizeof(u32) + 3) & ~size_t(3);
+    static constexpr size_t kCtlWords = (sizeof(sort::SortControl) + 15) / 16 * 4;
+    static constexpr size_t kPlanWords = (sizeof(sort::PlanCounters) + 15) / 16 * 4;
     static size_t up(size_t b) { return (b + 255) & ~size_t(255); }
     static size_t countersOffset(size_t n) { return up(up(n * sizeof(u64)) + n * sizeof(u32)); }
     PairSortLayout(size_t n, int cfg)
@@ -692,9 +695,11 @@ struct PairSortLayout
         altVals = up(altKeys + n * sizeof(u64));
         counters = countersOffset(n);
         status = up(counters + counterWords() * sizeof(u32));
-        total = up(status + tiles * sort::kRadix * sizeof(u64));
+        table = up(status + tiles * sort::kRadix * sizeof(u64));
+        longRuns = up(table + sort::planTableBytes(n));
+        total = up(longRuns + sort::longRunWords(n) * sizeof(u32));
     }
-    size_t counterWords() const { return kCounterHead + kCtlWords + 2 * size_t(passes) * sort::kRadix; }
+    size_t counterWords() const { return kCounterHead + kCtlWords + kPlanWords + 2 * size_t(passes) * sort::kRadix; }
 };
 }  // namespace
 
@@ -747,7 +752,8 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     u32 *head = reinterpret_cast<u32 *>(base + lay.counters);
     int *error = reinterpret_cast<int *>(head);
     sort::SortControl *ctl = reinterpret_cast<sort::SortControl *>(head + PairSortLayout::kCounterHead);
-    u32 *hist = head + PairSortLayout::kCounterHead + PairSortLayout::kCtlWords;
+    u32 *planCounters = head + PairSortLayout::kCounterHead + PairSortLayout::kCtlWords;
+    u32 *hist = planCounters + PairSortLayout::kPlanWords;
     u32 *bins = hist + size_t(lay.passes) * sort::kRadix;
     u64 *status = reinterpret_cast<u64 *>(base + lay.status);
     const int bitsPer = sort::kSortConfigs[cfg].bits;
@@ -761,22 +767,46 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
         AOT_LAUNCH_CHECK();
         return;
     }
-    AOT_CHECK(cudaMemsetAsync(head, 0, lay.counterWords() * sizeof(u32), s));
-    AOT_CHECK(cudaMemsetAsync(status, 0, lay.tiles * sort::kRadix * sizeof(u64), s));
-    sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(ctl, nullptr), noteLaunch();
+    AOT_CHECK(cudaMemsetAsync(head, 0, lay.longRuns - lay.counters, s));
+    const u64 *in = reinterpret_cast<const u64 *>(keysIn);
+    u64 *out = reinterpret_cast<u64 *>(keysOut);
+    const u64 keyMask = (endBit - beginBit == 64 ? ~u64(0) : ((u64(1) << (endBit - beginBit)) - 1)) << beginBit;
+    // a plan for 8-bit digits, where it can leave passes out
+    const bool planned = bitsPer == sort::kRadixBits && passes > sort::kPlanMinPasses;
+    if (planned)
+    {
+        const sort::PlanArgs plan{reinterpret_cast<u64 *>(base + lay.table),
+                                  reinterpret_cast<sort::PlanCounters *>(planCounters), sort::planSamples(n),
+                                  sort::planSlotBits(n)};
+        sort::planPairsKernel<<<ceilDiv(plan.samples, sort::kPlanThreads), sort::kPlanThreads, 0, s>>>(
+            in, n, beginBit, passes, keyMask, plan, ctl), noteLaunch();
+    }
+    else
+    {
+        sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(ctl, nullptr), noteLaunch();
+    }
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
-    sort::launchHistogram(cfg, s, blocks, reinterpret_cast<const u64 *>(keysIn), n, beginBit, passes, hist, endBit),
-        noteLaunch();
+    sort::launchHistogram(cfg, s, blocks, in, n, beginBit, passes, hist, endBit, ctl), noteLaunch();
     sort::binsKernel<<<1, sort::kThreads, 0, s>>>(hist, bins, passes), noteLaunch();
     AOT_LAUNCH_CHECK();
     sort::setPassSmemAll();
-    const sort::PassArgs p{reinterpret_cast<const u64 *>(keysIn), valsIn, {reinterpret_cast<u64 *>(keysOut), altK},
-                           {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes, true};
+    const sort::PassArgs p{in, valsIn, {out, altK}, {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes,
+                           true};
     for (int slot = 0; slot < passes; ++slot)
     {
         sort::launchPass(cfg, s, p, slot), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
+    if (!planned) return;
+    const bool aligned = aligned16(out) && (reinterpret_cast<uintptr_t>(valsOut) & 7u) == 0;
+    const sort::RepairArgs r{{out, altK}, {valsOut, altV}, n, ctl, reinterpret_cast<u32 *>(base + lay.longRuns), nullptr,
+                             error, beginBit, passes, keyMask, true, aligned, false};
+    if (keyMask == ~u64(0))
+        sort::repairKernel<true><<<sort::repairTiles(n), sort::kRepairThreads, 0, s>>>(r), noteLaunch();
+    else
+        sort::repairKernel<false><<<sort::repairTiles(n), sort::kRepairThreads, 0, s>>>(r), noteLaunch();
+    sort::longRunKernel<<<unsigned(smCount()) * 2u, sort::kLongThreads, 0, s>>>(r), noteLaunch();
+    AOT_LAUNCH_CHECK();
 }
 
 // Waits for `stream` and reads the error word of a pair sort of n items
@@ -800,6 +830,10 @@ void TreeEngine::sortPairsPreload()
     AOT_CHECK(cudaFuncGetAttributes(&a, iotaKernel));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::beginSortKernel));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::binsKernel));
+    AOT_CHECK(cudaFuncGetAttributes(&a, sort::planPairsKernel));
+    AOT_CHECK(cudaFuncGetAttributes(&a, sort::repairKernel<true>));
+    AOT_CHECK(cudaFuncGetAttributes(&a, sort::repairKernel<false>));
+    AOT_CHECK(cudaFuncGetAttributes(&a, sort::longRunKernel));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<8>));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<7>));
 #define AOT_CASE(i, B, I) AOT_CHECK(cudaFuncGetAttributes(&a, sort::onesweepKernel<B, I>));
@@ -1193,7 +1227,7 @@ void TreeEngine::sortKeys(int config)
     {
         sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
         const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n_, sort::kThreads), unsigned(smCount()) * 8u));
-        sort::launchHistogram(config, s, blocks, k[0], n_, 0, passes, a.hist(), 64), noteLaunch();
+        sort::launchHistogram(config, s, blocks, k[0], n_, 0, passes, a.hist(), 64, a.ctl()), noteLaunch();
         sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
         AOT_LAUNCH_CHECK();
     }

@@ -111,12 +111,14 @@ static __global__ void __launch_bounds__(kThreads) beginSortKernel(SortControl *
     }
 }
 
-// Histogram of the Bits-wide digits of keys[0, n) for passes covering
-// [beginBit, endBit); pass p's counts go to hist[p * kRadix + digit].
+// Histogram of the Bits-wide digits of keys[0, n) for the passes run of those
+// covering [beginBit, endBit); pass p's counts go to hist[p * kRadix + digit].
 template <int Bits = kRadixBits>
 static __global__ void __launch_bounds__(kThreads) histogramKernel(const u64 *__restrict__ keys, size_t n, int beginBit,
-                                                             int passes, u32 *__restrict__ hist, int endBit = 64)
+                                                             int passes, u32 *__restrict__ hist, int endBit,
+                                                             const SortControl *ctl)
 {
+    const int first = int(ctl->first);
     constexpr int R = 1 << Bits;
     __shared__ u32 sh[kPassSlots][R];
     for (int i = threadIdx.x; i < kPassSlots * R; i += kThreads) (&sh[0][0])[i] = 0;
@@ -124,7 +126,7 @@ static __global__ void __launch_bounds__(kThreads) histogramKernel(const u64 *__
     for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n; i += size_t(gridDim.x) * kThreads)
     {
         const u64 k = __ldg(keys + i);
-        for (int p = 0; p < passes; ++p)
+        for (int p = first; p < passes; ++p)
         {
             const int shift = beginBit + p * Bits;
             const int bits = endBit - shift < Bits ? endBit - shift : Bits;
@@ -624,12 +626,12 @@ static inline void launchSegmentPass(int c, cudaStream_t s, unsigned numTiles, c
 
 // Histogram of configuration c's digits.
 static inline void launchHistogram(int c, cudaStream_t s, unsigned blocks, const u64 *keys, size_t n, int beginBit, int passes,
-                            u32 *hist, int endBit)
+                            u32 *hist, int endBit, const SortControl *ctl)
 {
     if (kSortConfigs[c].bits == 8)
-        histogramKernel<8><<<blocks, kThreads, 0, s>>>(keys, n, beginBit, passes, hist, endBit);
+        histogramKernel<8><<<blocks, kThreads, 0, s>>>(keys, n, beginBit, passes, hist, endBit, ctl);
     else
-        histogramKernel<7><<<blocks, kThreads, 0, s>>>(keys, n, beginBit, passes, hist, endBit);
+        histogramKernel<7><<<blocks, kThreads, 0, s>>>(keys, n, beginBit, passes, hist, endBit, ctl);
 }
 
 }  // namespace sort

@@ -38,11 +38,10 @@ namespace aot
 {
 namespace
 {
-// Scratch layout of the pair sort for kNoAllocMaxItems items: alternate keys
-// (8 B/item), alternate values (4 B/item), counters (error word and 3 pad
-// words, 2 x 8 passes x 256 digits, 8 tile counters), look-back status
-// (8 passes x tiles of kSortTileItems items x 256 digits x 8 B), each part
-// rounded up to 256 bytes.  The call checks the sort's own size query against
+// Scratch of the pair sort for kNoAllocMaxItems items: alternate keys
+// (8 B/item) and values (4 B/item), counters, look-back status, plan table and
+// list of long runs, about 14.3 MB; the array keeps the room that look-back
+// words for 8 passes took.  The call checks the sort's own size query against
 // this before using the array.
 constexpr size_t kNoAllocMaxItems = size_t(1) << 20;
 constexpr size_t up256(size_t b) { return (b + 255) & ~size_t(255); }

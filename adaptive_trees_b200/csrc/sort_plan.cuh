@@ -79,16 +79,16 @@ struct PlanArgs
     u32 samples, slotBits;
 };
 
-// The first pass to run (0: all 8) for n keys, from the repeats in each set
-// (set 0: whole keys; set s: prefixes of kPlanMinPasses + s - 1 digits).
-__device__ __forceinline__ u32 planFirst(const u32 *repeats, u32 m, size_t n)
+// The first pass to run (0: all `passes`) for n keys, from the repeats in each
+// set (set 0: whole keys; set s: prefixes of kPlanMinPasses + s - 1 digits).
+__device__ __forceinline__ u32 planFirst(const u32 *repeats, u32 m, size_t n, int passes = kMaxPasses)
 {
     const float perPair = 2.f * float(n) / (float(m) * float(m));  // mean run per repeated key
     const u32 equal = repeats[0];
     if (float(equal) * perPair > kMaxRepeats) return 0;
-    float best = float(kMaxPasses);
+    float best = float(passes);
     u32 first = 0;
-    for (int d = kPlanMinPasses; d <= kPlanMaxPasses; ++d)
+    for (int d = kPlanMinPasses; d <= kPlanMaxPasses && d < passes; ++d)
     {
         const u32 r = repeats[d - kPlanMinPasses + 1];
         const float run = float(r > equal ? r - equal : 0u) * perPair;
@@ -96,7 +96,7 @@ __device__ __forceinline__ u32 planFirst(const u32 *repeats, u32 m, size_t n)
         if (cost < best)
         {
             best = cost;
-            first = u32(kMaxPasses - d);
+            first = u32(passes - d);
         }
     }
     return first;
@@ -158,7 +158,7 @@ __device__ __forceinline__ void planSample(const KeyAt &keyAt, size_t n, const P
 // sampled by all CTAs, the plan made and the control block set up by the last.
 template <class KeyAt>
 __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const PlanArgs &a, SortControl *ctl, u32 *hist,
-                                         size_t histWords)
+                                         size_t histWords, int passes = kMaxPasses)
 {
     __shared__ u32 sTotal[kPlanSets];
     __shared__ bool sLast;
@@ -182,11 +182,22 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     if (threadIdx.x == 0)
     {
         a.counters->done = 0;
-        ctl->first = planFirst(sTotal, a.samples, n);
+        ctl->first = planFirst(sTotal, a.samples, n, passes);
         ctl->epoch = epoch;
         ctl->longRuns = 0;
         ctl->keygenDone = 0;
     }
+}
+
+// Start of a planned pair sort by bits [beginBit, beginBit + 8 passes) of
+// keyMask: the digits sampled are those of the passes.
+static __global__ void __launch_bounds__(kPlanThreads)
+    planPairsKernel(const u64 *__restrict__ keys, size_t n, int beginBit, int passes, u64 keyMask, PlanArgs plan,
+                    SortControl *ctl)
+{
+    const int up = 64 - passes * kRadixBits;
+    const auto keyAt = [&](size_t i, u32 &) { return ((keys[i] & keyMask) >> beginBit) << up; };
+    planSort(keyAt, n, plan, ctl, nullptr, 0, passes);
 }
 }  // namespace sort
 }  // namespace aot

@@ -141,3 +141,47 @@ def test_planned_sort_of_a_batch_is_each_systems_stable_sort(name, hilbert):
     b.doBuffersNeedResize()
     check("update")
     b.close()
+
+
+def pair_keys(kind, n, seed):
+    r = np.random.default_rng(seed)
+    k = r.integers(0, 2 ** 64 - 1, size=n, dtype=np.uint64, endpoint=True)
+    if kind == "low bits only":
+        k &= np.uint64(0xFFFF)
+    elif kind == "runs":  # high digits repeat, low ones tell apart; the all-ones prefix among them
+        k = (k & np.uint64(0xFFFFFF)) | (np.uint64(0xFFFFFFFFFF) - (k >> np.uint64(40)) % np.uint64(max(1, n // 40)) << np.uint64(24))
+    elif kind == "long run":
+        k[: n // 3] = (k[: n // 3] & np.uint64(0xFFFFFFFF)) | np.uint64(0x1234567800000000)
+        k = k[r.permutation(n)]
+    elif kind == "equal":
+        k[:] = k[0]
+    return k
+
+
+@pytest.mark.parametrize("begin,end", [(0, 64), (5, 50), (0, 32), (40, 64), (0, 17), (3, 11)])
+@pytest.mark.parametrize("kind", ["random", "low bits only", "runs", "long run", "equal"])
+@pytest.mark.parametrize("n,offset", [(1, 0), (2047, 0), (2305, 1), (60_001, 0), (600_000, 1)])
+def test_planned_pair_sort_is_the_stable_sort(n, offset, kind, begin, end):
+    import ctypes
+
+    import torch
+
+    from adaptive_trees_b200 import _capi as C
+    lib = C.load()
+    k = pair_keys(kind, n, n + begin)
+    keys = torch.from_numpy(k.view(np.int64)).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda") * 7
+    out_k = torch.zeros(n + 1, dtype=torch.int64, device="cuda")[offset:offset + n]  # 8-byte aligned only
+    out_v = torch.zeros(n + 1, dtype=torch.int32, device="cuda")[offset:offset + n]
+    size = ctypes.c_size_t()
+    C.check(lib.ao_sort_pairs(None, ctypes.byref(size), None, None, None, None, n, begin, end, None))
+    scratch = torch.full((size.value,), 0xA5, dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    mask = np.uint64((((1 << (end - begin)) - 1) << begin) & (2 ** 64 - 1))
+    order = np.argsort(k & mask, kind="stable")
+    for _ in range(2):  # the second call finds the first one's words in the scratch
+        C.check(lib.ao_sort_pairs(scratch.data_ptr(), ctypes.byref(size), keys.data_ptr(), out_k.data_ptr(),
+                                  vals.data_ptr(), out_v.data_ptr(), n, begin, end, stream))
+        C.check(lib.ao_sort_pairs_check(scratch.data_ptr(), n, stream))
+        assert np.array_equal(out_k.cpu().numpy().view(np.uint64), k[order])
+        assert np.array_equal(out_v.cpu().numpy(), order.astype(np.int32) * 7)
