@@ -857,10 +857,6 @@ struct TreeEngine::Impl
     size_t hstBytes = 0;
     cudaStream_t d2h = nullptr;
     cudaEvent_t ready = nullptr;
-    // level build: the neighbour references of a level run on `side` beside
-    // the expansion of the same level (neither needs the other)
-    cudaStream_t side = nullptr;
-    cudaEvent_t sideFork = nullptr, sideJoin = nullptr;
     int device = 0;  // the device of the pooled streams and events
     cudaEvent_t marks[8] = {};              // stage events (profiling)
     cudaEvent_t tuneStart = nullptr, tuneEnd = nullptr;  // sort tuner timing
@@ -870,7 +866,7 @@ struct TreeEngine::Impl
     DevMem K[2], B[2], NF[2], N[2], G[2], offs, dirty, scan;
     DevMem nodeRows;  // node table of the near-field refresh (NFCount)
     // converged build by levels (levelbuild.cuh): unit arena and its control
-    DevMem lvRows, lvVal, lvChild, lvLeaves, lvOffset, lvCtl, lvNbr, lvParent;
+    DevMem lvRows, lvVal, lvChild, lvLeaves, lvOffset, lvCtl, lvNbr, lvParent, lvRec;
     size_t lvCap = 0;
     int lvLevels = int(kOctLevels);  // levels the last level build needed, with one to spare
     DevMem mergeSplits;              // merge-path cuts of the full begin refresh
@@ -910,9 +906,6 @@ struct TreeEngine::Impl
         if (tuneEnd) cudaEventDestroy(tuneEnd);
         for (cudaEvent_t e : nfMarks) cudaEventDestroy(e);
         blockcache::giveStream(d2h, device);
-        blockcache::giveEvent(sideFork, device);
-        blockcache::giveEvent(sideJoin, device);
-        blockcache::giveStream(side, device);
     }
 
     // device bytes held by this tree
@@ -929,7 +922,7 @@ struct TreeEngine::Impl
                                &vLvVals[1],  &vLayKeys[0], &vLayKeys[1],    &vLayVals[0],  &vLayVals[1],
                                &vIntStartSfc, &vIntLevelSfc, &vIntM,        &vIntStartLay, &vIntLevelLay,
                                &viewSort.mem, &nodeRows, &lvRows, &lvVal, &lvChild,
-                               &lvLeaves, &lvOffset, &lvCtl, &lvNbr, &lvParent};
+                               &lvLeaves, &lvOffset, &lvCtl, &lvNbr, &lvParent, &lvRec};
         size_t s = 0;
         for (const DevMem *d : all) s += d->bytes;
         return s;
@@ -1101,7 +1094,6 @@ TreeEngine::~TreeEngine()
     {
         (void)cudaStreamSynchronize(cfg_.stream);
         if (m_->d2h) (void)cudaStreamSynchronize(m_->d2h);
-        if (m_->side) (void)cudaStreamSynchronize(m_->side);
     }
 }
 
@@ -1673,6 +1665,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             m.lvVal.reserve(cap * 8 * sizeof(u32), s);
             m.lvNbr.reserve(cap * 27 * sizeof(u32), s);
             m.lvParent.reserve(cap * sizeof(u32), s);
+            m.lvRec.reserve(cap * sizeof(u64), s);
         }
         m.lvChild.reserve(cap * 8 * sizeof(u32), s);
         m.lvLeaves.reserve(cap * sizeof(u32), s);
@@ -1684,6 +1677,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         a.val = nf ? m.lvVal.as<u32>() : nullptr;
         a.nbr = nf ? m.lvNbr.as<u32>() : nullptr;
         a.parent = nf ? m.lvParent.as<u32>() : nullptr;
+        a.rec = nf ? m.lvRec.as<u64>() : nullptr;
         a.usys = nullptr;
         a.sysRoot = nullptr;
         a.child = m.lvChild.as<u32>();
@@ -1703,40 +1697,19 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         // placement; one readback at the end checks that no deeper level
         // was left out.
         const int levels = std::max(1, std::min(int(kOctLevels), m.lvLevels));
-        const bool useSide = nf;
-        if (useSide && !m.side)
-        {
-            m.side = blockcache::takeStream();
-            m.sideFork = blockcache::takeEvent();
-            m.sideJoin = blockcache::takeEvent();
-        }
         for (int l = 0; l < levels; ++l)
         {
-            const bool fork = nf && l > 0 && useSide;
-            if (fork)
-            {
-                // the neighbour references of level l need level l - 1 only
-                AOT_CHECK(cudaEventRecord(m.sideFork, s));
-                AOT_CHECK(cudaStreamWaitEvent(m.side, m.sideFork, 0));
-                if (cfg_.hilbert) lb::nbrKernel<true><<<blocks * 2, lb::kThreads, 0, m.side>>>(a, l, m.kpd.h), noteLaunch();
-                else lb::nbrKernel<false><<<blocks * 2, lb::kThreads, 0, m.side>>>(a, l, m.kpd.h), noteLaunch();
-                AOT_CHECK(cudaEventRecord(m.sideJoin, m.side));
-            }
-            lb::expandKernel<<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
-            if (fork) AOT_CHECK(cudaStreamWaitEvent(s, m.sideJoin, 0));
+            if (!nf)
+                lb::expandKernel<false, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+            else if (cfg_.hilbert)
+                lb::expandKernel<true, true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+            else
+                lb::expandKernel<true, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
             if (nf)
             {
                 markNearField(true);
-                if (cfg_.hilbert)
-                {
-                    if (l > 0 && !fork) lb::nbrKernel<true><<<blocks * 2, lb::kThreads, 0, s>>>(a, l, m.kpd.h), noteLaunch();
-                    lb::nearFieldKernel<true><<<blocks / 4 * 5, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
-                }
-                else
-                {
-                    if (l > 0 && !fork) lb::nbrKernel<false><<<blocks * 2, lb::kThreads, 0, s>>>(a, l, m.kpd.h), noteLaunch();
-                    lb::nearFieldKernel<false><<<blocks / 4 * 5, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
-                }
+                if (cfg_.hilbert) lb::nearFieldKernel<true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+                else lb::nearFieldKernel<false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
                 markNearField(false);
                 if (cfg_.hilbert)
                     lb::classifyKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket, m.kpd.h), noteLaunch();
@@ -1756,13 +1729,18 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             const rb::TreeBufs tb = m.bufs();
             for (int l = 0; l < levels; ++l)
             {
-                if (nf)
-                    lb::placeKernel<true><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0], l, levels,
-                                                                          u32(physCap_)),
+                const u32 cap32 = u32(physCap_);
+                if (nf && cfg_.hilbert)
+                    lb::placeKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
+                                                                                 l, levels, cap32, m.kpd.h),
+                        noteLaunch();
+                else if (nf)
+                    lb::placeKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
+                                                                                  l, levels, cap32, m.kpd.h),
                         noteLaunch();
                 else
-                    lb::placeKernel<false><<<blocks, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], l, levels,
-                                                                           u32(physCap_)),
+                    lb::placeKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], l,
+                                                                            levels, cap32, m.kpd.h),
                         noteLaunch();
             }
             AOT_LAUNCH_CHECK();

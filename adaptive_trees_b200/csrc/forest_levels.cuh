@@ -118,9 +118,10 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         const u32 start = vload(c.levelStart[l]), count = vload(c.levelCount[l]);
         if (vload(c.overflow) | vload(c.late) || count == 0) break;
         deepest = l;
-        expandUnits(a, p.idx, l, start, count, rank, size);
+        expandUnits<false, false>(a, p.idx, l, start, count, rank, size, nullptr);
         if (!gridBarrier(&ls->bar)) return;
-        classifyUnits<false, Hilbert, true>(a, l, p.bucket, start, count, sNext, sDec, nullptr, nullptr, rank, size);
+        classifyUnits<false, Hilbert, true>(a, l, p.bucket, start, count, sNext, sDec, nullptr, nullptr, nullptr, rank,
+                                              size);
         if (!gridBarrier(&ls->bar)) return;
     }
     if (vload(c.overflow) | vload(c.late)) return;
@@ -243,8 +244,8 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
     // placement, shallowest level first (a unit's first entry comes from its parent)
     for (int l = 0; l <= deepest; ++l)
     {
-        placeUnits<false>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], l, vload(c.levelStart[l]),
-                          vload(c.levelCount[l]), p.capacity, rank, size);
+        placeUnits<false, false>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], l, vload(c.levelStart[l]),
+                          vload(c.levelCount[l]), p.capacity, rank, size, nullptr);
         if (!gridBarrier(&ls->bar)) return;
     }
     const i64 E = vload(ls->entries);

@@ -11,11 +11,11 @@
 // bucket and its level is below 21.  This file builds that tree one level at
 // a time, without the rounds:
 //   expand    the internal cells ("units") of level l get the begin indices
-//             of their 8 children in the sorted keys (and, for NFCount, a row
-//             in the node table of the near-field lookups);
-//   nearField NFCount: the near-field counts of the children of the level-l
-//             units, one unit per parent cell as in the refresh of the
-//             rounds (octNearFieldKernel);
+//             of their 8 children in the sorted keys (and, for NFCount, the
+//             8 child counts as bytes);
+//   nearField NFCount: the 27 cells around each level-l unit, from those
+//             around its parent, and from their child counts the near-field
+//             counts of the unit's children;
 //   classify  the children whose value exceeds the bucket become the units of
 //             level l + 1 (slots taken by warp-aggregated atomics); the
 //             others are leaves of the tree;
@@ -68,11 +68,12 @@ struct Arena
 {
     u32 *rows;       // [cap][kRow]
     u32 *val;        // [cap][8] value of each child (NF or count)
-    u32 *child;      // [cap][8] unit index of an internal child, or kLeaf
+    u32 *child;      // [cap][8] unit index of an internal child, or kLeaf (LeafCount: by digit, NFCount: by octant)
     u32 *leaves;     // [cap] leaves in the unit's subtree
     u32 *offset;     // [cap] cornerstone index of the unit's first leaf
     u32 *nbr;        // NFCount: [cap][27] the cells around each unit (nbrRef)
-    u32 *parent;     // NFCount: [cap] parent unit * 8 + the unit's digit in it
+    u32 *parent;     // NFCount: [cap] parent unit * 8 + the unit's octant in it
+    u64 *rec;        // NFCount: [cap] child counts of a unit, a byte per octant (kBigRec: one does not fit)
     u32 *usys;       // batch of trees: [cap] the tree (system) of each unit
     u32 *sysRoot;    // batch of trees: [systems] each system's root unit, or kLeaf
     Control *ctl;
@@ -98,9 +99,11 @@ __device__ __forceinline__ u32 unitLevelOf(u32 w) { return (w >> 19) & 0x1fu; }
 __device__ __forceinline__ u32 unitStateOf(u32 w) { return (w >> 24) & 0x3fu; }
 
 // A cell around a unit, at the unit's level: a unit index when the cell is an
-// internal node, else kLeafRef | (parent unit * 8 + digit) naming the leaf
+// internal node, else kLeafRef | (parent unit * 8 + octant) naming the leaf
 // of the tree that holds the cell (the cell itself or a coarser leaf).
 constexpr u32 kLeafRef = 0x80000000u;
+// Child counts of which one is 255 or more.
+constexpr u64 kBigRec = ~u64(0);
 
 // Levels a leaf of value x at level m splits by (calculateNodeOp,
 // octree_rebalance.cuh:188-249: 8, 64, 512 or 4096 children), given that it
@@ -274,15 +277,19 @@ __device__ __forceinline__ u32 boundaryIn(const KeyIndex &idx, u32 lo, u32 hi, u
 // 9 child begins of the units of level l: one thread per unit (the 7 inner
 // ones by innerBegins), one lane per inner boundary on levels of fewer units,
 // one warp per inner boundary on levels of few units.
+// Rec: also the units' child counts as bytes (not on levels of few units,
+// whose counts do not fit and which do without), by octant: dec[state * 8 +
+// digit] for the Hilbert curve.
 // `rank` and `size` number the threads taking part (a grid, or the grid of a
 // persistent kernel).
+template <bool Rec, bool Hilbert>
 __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx, int l, u32 start, u32 count, u32 rank,
-                                            u32 size)
+                                            u32 size, const unsigned char *dec)
 {
     const u64 cr = octRange(unsigned(l) + 1);
+    const int lane = threadIdx.x & 31;
     if (count <= kWideUnits)
     {
-        const int lane = threadIdx.x & 31;
         for (u32 w = rank >> 5; w < count * 7; w += size >> 5)
         {
             const u32 i = w / 7, d = w - i * 7;
@@ -302,12 +309,26 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
     }
     if (count <= kLaneUnits)
     {
-        for (u32 e = rank; e < count * 8; e += size)
+        for (u32 e = rank; e < count * 8; e += size)  // the 8 lanes of a unit together
         {
             const u32 i = e >> 3, d = e & 7;
-            if (d == 7) continue;
             u32 *row = a.rows + size_t(start + i) * kRow;
-            row[3 + d] = boundaryIn(idx, row[2], row[10], rowKey(row) + u64(d + 1) * cr);
+            const u32 lo = row[2], hi = row[10];
+            u32 end = hi;  // of child d
+            if (d < 7)
+            {
+                end = boundaryIn(idx, lo, hi, rowKey(row) + u64(d + 1) * cr);
+                row[3 + d] = end;
+            }
+            if constexpr (Rec)
+            {
+                const unsigned group = 0xffu << (lane & 24);
+                const u32 prev = __shfl_up_sync(group, end, 1, 8);
+                const u32 cnt = end - (d ? prev : lo);
+                const bool big = __any_sync(group, cnt >= 255u);
+                const u32 oct = Hilbert ? u32(dec[unitStateOf(row[11]) * 8 + d]) : d;
+                reinterpret_cast<unsigned char *>(a.rec + (start + i))[oct] = big ? 255 : (unsigned char)cnt;
+            }
         }
         return;
     }
@@ -315,77 +336,70 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
     {
         u32 *row = a.rows + size_t(start + i) * kRow;
         u32 b[7];
-        innerBegins(idx, row[2], row[10], rowKey(row), cr, b);
+        const u32 lo = row[2], hi = row[10];
+        innerBegins(idx, lo, hi, rowKey(row), cr, b);
 #pragma unroll
         for (int d = 0; d < 7; ++d) row[3 + d] = b[d];
+        if constexpr (Rec)
+        {
+            const u32 st = unitStateOf(row[11]);
+            u64 rec = 0;
+            bool big = false;
+#pragma unroll
+            for (int d = 0; d < 8; ++d)
+            {
+                const u32 cnt = (d < 7 ? b[d] : hi) - (d ? b[d - 1] : lo);
+                big |= cnt >= 255u;
+                const u32 oct = Hilbert ? u32(dec[st * 8 + d]) : u32(d);
+                rec |= u64(cnt & 0xffu) << (8 * oct);
+            }
+            a.rec[start + i] = big ? kBigRec : rec;
+        }
     }
 }
 
-static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyIndex idx, int l)
+template <bool Rec, bool Hilbert>
+static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyIndex idx, int l, HilbertTables h)
 {
+    __shared__ unsigned char sDec[48 * 8];
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
-    expandUnits(a, idx, l, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x,
-                gridDim.x * blockDim.x);
-}
-
-// The 27 cells around every unit of level l >= 1, from those around its
-// parent U: the cell at offset (dx, dy, dz) of the unit (octant o in U) is
-// child o' of the cell at offset floor((o + d) / 2) around U, o' =
-// (o + d) mod 2 per axis.  That cell is a unit (the child of a unit around
-// U, if internal) or lies in a leaf: a leaf child of a unit around U, or the
-// leaf that already holds U's cell.
-template <bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) nbrKernel(Arena a, int l, HilbertTables h)
-{
-    __shared__ unsigned char sEnc[48 * 8], sDec[48 * 8];
-    const Control &c = *a.ctl;
-    if (c.overflow | c.late | c.error) return;
-    const u32 start = c.levelStart[l], count = c.levelCount[l];
-    const size_t total = size_t(count) * 27;
-    if (total <= size_t(blockIdx.x) * blockDim.x) return;
-    if constexpr (Hilbert)
+    if constexpr (Rec && Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
-        {
-            sEnc[k] = h.enc[k];
-            sDec[k] = h.decOct[k];
-        }
+        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x) sDec[k] = h.decOct[k];
         __syncthreads();
     }
-    for (size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += size_t(gridDim.x) * blockDim.x)
-    {
-        const u32 g = start + u32(e / 27);
-        const int q = int(e - size_t(e / 27) * 27);
-        const u32 pr = a.parent[g];
-        const u32 U = pr >> 3, d = pr & 7u;
-        const u32 stU = unitStateOf(a.rows[size_t(U) * kRow + 11]);
-        const int o = Hilbert ? int(sDec[stU * 8 + d]) : int(d);
-        const int tx = (o >> 2) + q % 3 - 1, ty = ((o >> 1) & 1) + (q / 3) % 3 - 1, tz = (o & 1) + q / 9 - 1;
-        const int qp = ((tx + 2) / 2) + 3 * ((ty + 2) / 2) + 9 * ((tz + 2) / 2);  // offset around U
-        const u32 r = a.nbr[size_t(U) * 27 + qp];
-        u32 ref = r;
-        if (!(r & kLeafRef))
-        {
-            const int oc = ((tx & 1) << 2) | ((ty & 1) << 1) | (tz & 1);
-            const u32 stV = unitStateOf(a.rows[size_t(r) * kRow + 11]);
-            const u32 dv = Hilbert ? u32(sEnc[stV * 8 + oc]) : u32(oc);
-            const u32 ch = a.child[size_t(r) * 8 + dv];
-            ref = ch != kLeaf ? ch : (kLeafRef | (r * 8 + dv));
-        }
-        a.nbr[size_t(g) * 27 + q] = ref;
-    }
+    expandUnits<Rec, Hilbert>(a, idx, l, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x,
+                              gridDim.x * blockDim.x, sDec);
 }
 
-// Near-field counts of the children of the level-l units: per unit, the 27
-// parent-level cells Q around it (nbrKernel) give the 4 x 4 x 4 block of
-// child counts -- from the 9 child begins of Q when Q is a unit, counted
-// within the keys of the leaf that holds Q otherwise -- and each child sums
-// its 3 x 3 x 3 sub-block (octNearFieldKernel's unit, with the cells around
-// it known instead of looked up).
-// Per-warp scratch of the units in flight (the refresh's scratch without the
-// group-flag populations, which leaves more of the SM's shared storage to L1).
-struct UnitScratch
+// Near-field counts of the children of the level-l units, a warp per
+// kUnitBatch units at a time.
+//
+// The 27 cells around a unit come from those around its parent U: the cell at
+// offset (dx, dy, dz) of the unit (octant o in U) is child o' of the cell at
+// offset floor((o + d) / 2) around U, o' = (o + d) mod 2 per axis.  That cell
+// is a unit (the child of a unit around U, if internal) or lies in a leaf: a
+// leaf child of a unit around U, or the leaf that already holds U's cell.
+// (Children are kept by octant, so no curve state is needed on the way.)
+//
+// The children of those 27 cells form a 6 x 6 x 6 block of cells, a unit's
+// own children in its middle; each child's population is its 3 x 3 x 3
+// sub-block's.  Cells that are units bring their 8 child counts as one 8-byte
+// record, a byte per octant; those in a leaf (one of eight at 16Mi Plummer
+// particles, a few keys each) have the leaf's keys counted.  A lane sums two
+// children from the record words by byte dot products.  Units around which a
+// count does not fit a byte, and levels of few units, take the path by rows
+// (nearFieldByRows).
+//
+// Before: the 27 cells by a kernel of their own, a 48-byte row of begin
+// indices and a curve state per cell here, scattered into 4 x 4 x 4 blocks of
+// words that eight lanes a unit summed: 387 us (beside the expansion) and
+// 786 us for the 1.8 M units of a 16Mi Plummer build, bound by L1 and
+// shared memory (79 %).
+
+// Per-warp scratch of the path by rows: the units in flight.
+struct RowScratch
 {
     u64 pStart[rb::kUnitBatch];
     int childState[rb::kUnitBatch];
@@ -394,148 +408,339 @@ struct UnitScratch
     unsigned short slowItem[rb::kUnitBatch * 27];
     int nSlow;
 };
+// Per-warp scratch of the path by records.
+struct RecScratch
+{
+    u64 rec[rb::kUnitBatch * 27];  // child counts of the cells around the units: [unit][27]
+    u32 parent[rb::kUnitBatch];
+    u32 slowRef[rb::kUnitBatch * 27];
+    unsigned short slowItem[rb::kUnitBatch * 27];
+};
+union NearScratch
+{
+    RowScratch rows;
+    RecScratch recs;
+};
+struct NearTables
+{
+    unsigned char enc[48 * 8], next[48 * 8], dec[48 * 8];
+    unsigned char step[8 * 27];  // [octant of the unit][offset]: offset around the parent << 3 | octant there
+};
 
-// 5 CTAs per SM (48 registers, 29.6 KB of scratch each): 0.7 % faster builds
-// at 16 Mi than 4.
+// Key range of the leaf `ref` (kLeafRef removed) and, for a cell at level l
+// and offset q around the unit with key start `pStart` that lies in it, the
+// cell's key and curve state.
 template <bool Hilbert>
-static __global__ void __launch_bounds__(kThreads, 5)
+__device__ __forceinline__ void leafCell(const Arena &a, const NearTables &t, u32 ref, int l, u64 pStart, int q, u32 &lo,
+                                         u32 &hi, u64 &qKey, int &qState)
+{
+    const u32 o = ref & 7u;
+    const u32 *row = a.rows + size_t(ref >> 3) * kRow;
+    const u32 reg = row[11], st = unitStateOf(reg);
+    const u32 d = Hilbert ? u32(t.enc[st * 8 + o]) : o;
+    lo = row[2 + d];
+    hi = row[3 + d];
+    if (unitLevelOf(reg) + 1 == unsigned(l))
+    {
+        // the leaf is the cell itself: child o of its parent unit
+        qKey = rowKey(row) + u64(d) * octRange(unsigned(l));
+        qState = Hilbert ? int(t.next[st * 8 + o]) : kHilbertStart;
+    }
+    else if (lo < hi)
+    {
+        const rb::CellPath path = rb::decodeCell<Hilbert>(pStart, unsigned(l), t.next, t.dec);
+        qKey = rb::neighbourCellOf<Hilbert>(path, pStart, unsigned(l), q, qState, t.enc, t.next);
+    }
+    else
+    {
+        qKey = 0;
+        qState = kHilbertStart;
+    }
+}
+
+// The units [first, first + nb) of level l by rows: any counts.
+template <bool Hilbert>
+__device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx, int l, u32 first, int nb, RowScratch &w,
+                                             const NearTables &t)
+{
+    const unsigned m = unsigned(l) + 1;
+    const int lane = threadIdx.x & 31;
+    const unsigned ltMask = (1u << lane) - 1u;
+    if (lane < nb)
+    {
+        // the cell's path is decoded only where a neighbour lies inside a
+        // coarser leaf (phase B); the children's curve state is in the row
+        const u32 *row = a.rows + size_t(first + u32(lane)) * kRow;
+        w.pStart[lane] = rowKey(row);
+        w.childState[lane] = int(unitStateOf(row[11]));
+    }
+    if (lane == 0) w.nSlow = 0;
+    __syncwarp();
+    // phase A: (unit, Q) pairs over the lanes; a Q that is a unit gives
+    // its children's counts from its row
+    const int items = nb * 27;
+    for (int ib = 0; ib < items; ib += 32)
+    {
+        const int it = ib + lane;
+        const int u = it / 27, q = it - (it / 27) * 27;
+        u32 ref = 0;
+        bool slow = false;
+        if (it < items)
+        {
+            ref = a.nbr[size_t(first) * 27 + it];
+            if (ref & kLeafRef)
+            {
+                slow = true;
+            }
+            else
+            {
+                const uint4 *vr = reinterpret_cast<const uint4 *>(a.rows + size_t(ref) * kRow);
+                const uint4 r0 = vr[0], r1 = vr[1], r2 = vr[2];
+                const u32 gb[rb::kGroupBegins] = {r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z};
+                rb::childrenFromPacked<Hilbert>(gb, q, int(unitStateOf(r2.w)), w.block[u]);
+            }
+        }
+        const unsigned slowMask = __ballot_sync(0xffffffffu, slow);
+        if (slow)
+        {
+            const int k = w.nSlow + __popc(slowMask & ltMask);
+            w.slowRef[k] = ref;
+            w.slowItem[k] = (unsigned short)it;
+        }
+        __syncwarp();
+        if (lane == 0) w.nSlow += __popc(slowMask);
+        __syncwarp();
+    }
+    // phase B: Q in a leaf: its children counted among the leaf's keys
+    const int nSlow = w.nSlow;
+    for (int k = lane; k < nSlow; k += 32)
+    {
+        const int it = w.slowItem[k];
+        const int u = it / 27, q = it - u * 27;
+        u32 lo, hi;
+        u64 qKey;
+        int qState;
+        leafCell<Hilbert>(a, t, w.slowRef[k] & ~kLeafRef, l, w.pStart[u], q, lo, hi, qKey, qState);
+        u32 begins[rb::kGroupBegins];
+        rb::childBeginsWithin(idx.keys, lo, hi, qKey, m, begins);
+        rb::childrenFromPacked<Hilbert>(begins, q, qState, w.block[u]);
+    }
+    __syncwarp();
+    // phase C: the 8 children of each unit, two per lane
+    for (int e = lane; e < nb * 8; e += 32)
+    {
+        const int u = e >> 3, d = e & 7;
+        const u32 g = first + u32(u);
+        const u32 *row = a.rows + size_t(g) * kRow;
+        const u32 cnt = row[2 + d + 1] - row[2 + d];
+        u32 out = 0;
+        if (cnt)
+        {
+            const unsigned o = Hilbert ? unsigned(t.dec[w.childState[u] * 8 + d]) : unsigned(d);
+            const u32 *sub = w.block[u] + (o >> 2) * 16 + ((o >> 1) & 1u) * 4 + (o & 1u);
+            u64 pop = 0;
+            if (m > 1)
+            {
+                u32 p32 = 0;
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+#pragma unroll
+                    for (int y = 0; y < 3; ++y)
+#pragma unroll
+                        for (int z = 0; z < 3; ++z) p32 += sub[x * 16 + y * 4 + z];
+                pop = p32;
+            }
+            else
+            {
+                // level 1: the periodic wrap repeats cells, the sum may exceed 2^32
+                for (int x = 0; x < 3; ++x)
+                    for (int y = 0; y < 3; ++y)
+                        for (int z = 0; z < 3; ++z) pop += sub[x * 16 + y * 4 + z];
+            }
+            const u64 v = u64(cnt) * pop;
+            out = v > 0xffffffffull ? 0xffffffffu : u32(v);
+        }
+        a.val[size_t(g) * 8 + d] = out;
+    }
+    __syncwarp();
+}
+
+// Child counts of the level-l cell [qKey, qKey + 8 cr) among the keys
+// P[lo, hi) (cr: its children's range), a byte per octant, or kBigRec.
+template <bool Hilbert>
+__device__ __forceinline__ u64 countedRec(const u64 *P, u32 lo, u32 hi, u64 qKey, int qState, int l,
+                                          const unsigned char *dec)
+{
+    if (hi - lo >= 255u) return kBigRec;
+    const unsigned shift = 3u * (kOctLevels - unsigned(l) - 1);
+    u64 rec = 0;
+    for (u32 k = lo; k < hi; ++k)
+    {
+        const u64 d = (__ldg(P + k) - qKey) >> shift;  // 8 or more: outside the cell
+        if (d < 8) rec += u64(1) << (8 * (Hilbert ? unsigned(dec[qState * 8 + int(d)]) : unsigned(d)));
+    }
+    return rec;
+}
+
+template <bool Hilbert>
+static __global__ void __launch_bounds__(kThreads, 4)
     nearFieldKernel(Arena a, KeyIndex idx, int l, HilbertTables h)
 {
     using rb::kUnitBatch;
-    __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8], sDec[48 * 8];
-    __shared__ UnitScratch sWarp[kThreads / 32];
+    __shared__ NearTables t;
+    __shared__ NearScratch sWarp[kThreads / 32];
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     const u32 start = c.levelStart[l], count = c.levelCount[l];
-    if (count <= blockIdx.x * u32(kThreads / 32) * u32(rb::kUnitBatch)) return;  // no units for this CTA
+    if (count <= blockIdx.x * u32(kThreads / 32) * u32(kUnitBatch)) return;  // no units for this CTA
     if constexpr (Hilbert)
     {
         for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
         {
-            sEnc[k] = h.enc[k];
-            sNext[k] = h.encNext[k];
-            sDec[k] = h.decOct[k];
+            t.enc[k] = h.enc[k];
+            t.next[k] = h.encNext[k];
+            t.dec[k] = h.decOct[k];
         }
     }
+    for (int k = threadIdx.x; k < 8 * 27; k += blockDim.x)
+    {
+        const int o = k / 27, q = k - o * 27;
+        const int tx = (o >> 2) + q % 3 - 1, ty = ((o >> 1) & 1) + (q / 3) % 3 - 1, tz = (o & 1) + q / 9 - 1;
+        const int qp = ((tx + 2) / 2) + 3 * ((ty + 2) / 2) + 9 * ((tz + 2) / 2);  // offset around the parent
+        t.step[k] = (unsigned char)(qp << 3 | ((tx & 1) << 2) | ((ty & 1) << 1) | (tz & 1));
+    }
     __syncthreads();
-    const unsigned m = unsigned(l) + 1;
-    UnitScratch &w = sWarp[threadIdx.x >> 5];
+    constexpr int kRounds = (kUnitBatch * 27 + 31) / 32;
     const int lane = threadIdx.x & 31;
     const unsigned ltMask = (1u << lane) - 1u;
+    const bool byRecs = count > kWideUnits;
+    RecScratch &w = sWarp[threadIdx.x >> 5].recs;
     const u32 warpsTotal = gridDim.x * (blockDim.x / 32);
     const u32 w0 = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     for (u32 base = w0 * kUnitBatch; base < count; base += warpsTotal * kUnitBatch)
     {
-        const int nb = int(min(u32(kUnitBatch), count - base));
-        if (lane < nb)
+        const int nb = int(min(u32(kUnitBatch), count - base)), items = nb * 27;
+        const u32 first = start + base;
+        // the cells around the units, (unit, cell) pairs over the lanes: all
+        // loads of a step in flight together
+        u32 ref[kRounds];
+        if (l > 0)
         {
-            // the cell's path is decoded only where a neighbour lies inside a
-            // coarser leaf (phase B); the children's curve state is in the row
-            const u32 *row = a.rows + size_t(start + base + u32(lane)) * kRow;
-            w.pStart[lane] = rowKey(row);
-            w.childState[lane] = int(unitStateOf(row[11]));
-        }
-        if (lane == 0) w.nSlow = 0;
-        __syncwarp();
-        // phase A: (unit, Q) pairs over the lanes; a Q that is a unit gives
-        // its children's counts from its row
-        const int items = nb * 27;
-        for (int ib = 0; ib < items; ib += 32)
-        {
-            const int it = ib + lane;
-            const int u = it / 27, q = it - (it / 27) * 27;
-            u32 ref = 0;
-            bool slow = false;
-            if (it < items)
+            if (lane < nb) w.parent[lane] = a.parent[first + u32(lane)];
+            __syncwarp();
+            u32 oct[kRounds];
+#pragma unroll
+            for (int i = 0; i < kRounds; ++i)
             {
-                ref = a.nbr[size_t(start + base + u32(u)) * 27 + q];
-                if (ref & kLeafRef)
+                const int it = i * 32 + lane, u = it / 27, q = it - u * 27;
+                ref[i] = kLeafRef;
+                oct[i] = 0;
+                if (it < items)
                 {
-                    slow = true;
-                }
-                else
-                {
-                    const uint4 *vr = reinterpret_cast<const uint4 *>(a.rows + size_t(ref) * kRow);
-                    const uint4 r0 = vr[0], r1 = vr[1], r2 = vr[2];
-                    const u32 gb[rb::kGroupBegins] = {r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z};
-                    rb::childrenFromPacked<Hilbert>(gb, q, int(unitStateOf(r2.w)), w.block[u]);
+                    const u32 p = w.parent[u], step = t.step[(p & 7u) * 27 + q];
+                    ref[i] = a.nbr[size_t(p >> 3) * 27 + (step >> 3)];
+                    oct[i] = step & 7u;
                 }
             }
-            const unsigned slowMask = __ballot_sync(0xffffffffu, slow);
-            if (slow)
+            u32 ch[kRounds];
+#pragma unroll
+            for (int i = 0; i < kRounds; ++i)
+                ch[i] = ref[i] & kLeafRef ? kLeaf : a.child[size_t(ref[i]) * 8 + oct[i]];
+#pragma unroll
+            for (int i = 0; i < kRounds; ++i)
             {
-                const int k = w.nSlow + __popc(slowMask & ltMask);
-                w.slowRef[k] = ref;
-                w.slowItem[k] = (unsigned short)it;
+                if (!(ref[i] & kLeafRef)) ref[i] = ch[i] != kLeaf ? ch[i] : (kLeafRef | (ref[i] * 8 + oct[i]));
+                const int it = i * 32 + lane;
+                if (it < items) a.nbr[size_t(first) * 27 + it] = ref[i];
+            }
+        }
+        bool big = !byRecs;
+        if (byRecs)
+        {
+            u64 rec[kRounds];
+#pragma unroll
+            for (int i = 0; i < kRounds; ++i)
+                rec[i] = i * 32 + lane < items && !(ref[i] & kLeafRef) ? a.rec[ref[i]] : 0;
+            int nSlow = 0;
+#pragma unroll
+            for (int i = 0; i < kRounds; ++i)
+            {
+                const int it = i * 32 + lane;
+                const bool slow = it < items && (ref[i] & kLeafRef);
+                const unsigned slowMask = __ballot_sync(0xffffffffu, slow);
+                if (slow)
+                {
+                    const int k = nSlow + __popc(slowMask & ltMask);
+                    w.slowRef[k] = ref[i];
+                    w.slowItem[k] = (unsigned short)it;
+                }
+                else if (it < items)
+                {
+                    big |= rec[i] == kBigRec;
+                    w.rec[it] = rec[i];
+                }
+                nSlow += __popc(slowMask);
             }
             __syncwarp();
-            if (lane == 0) w.nSlow += __popc(slowMask);
-            __syncwarp();
-        }
-        // phase B: Q in a leaf: its children counted among the leaf's keys
-        const int nSlow = w.nSlow;
-        for (int k = lane; k < nSlow; k += 32)
-        {
-            const int it = w.slowItem[k];
-            const int u = it / 27, q = it - u * 27;
-            const u32 lr = w.slowRef[k] & ~kLeafRef;
-            const u32 P = lr >> 3, d = lr & 7u;
-            const u32 *prow = a.rows + size_t(P) * kRow;
-            const u32 preg = prow[11];
-            u64 qKey;
-            int qState;
-            if (unitLevelOf(preg) + 1 == unsigned(l))
+            for (int k = lane; k < nSlow; k += 32)
             {
-                // the leaf is Q itself: child d of its parent unit
-                qKey = rowKey(prow) + u64(d) * octRange(unsigned(l));
-                const u32 stP = unitStateOf(preg);
-                qState = Hilbert ? int(sNext[stP * 8 + sDec[stP * 8 + d]]) : kHilbertStart;
+                const int it = w.slowItem[k], u = it / 27;
+                u32 lo, hi;
+                u64 qKey;
+                int qState;
+                leafCell<Hilbert>(a, t, w.slowRef[k] & ~kLeafRef, l, rowKey(a.rows + size_t(first + u32(u)) * kRow),
+                                  it - u * 27, lo, hi, qKey, qState);
+                const u64 r = countedRec<Hilbert>(idx.keys, lo, hi, qKey, qState, l, t.dec);
+                big |= r == kBigRec;
+                w.rec[it] = r;
             }
-            else
-            {
-                const rb::CellPath path = rb::decodeCell<Hilbert>(w.pStart[u], unsigned(l), sNext, sDec);
-                qKey = rb::neighbourCellOf<Hilbert>(path, w.pStart[u], unsigned(l), q, qState, sEnc, sNext);
-            }
-            u32 begins[rb::kGroupBegins];
-            rb::childBeginsWithin(idx.keys, prow[2 + d], prow[3 + d], qKey, m, begins);
-            rb::childrenFromPacked<Hilbert>(begins, q, qState, w.block[u]);
+            big = __any_sync(0xffffffffu, big);  // (also: the records are written)
         }
         __syncwarp();
-        // phase C: the 8 children of each unit, two per lane
-        for (int e = lane; e < nb * 8; e += 32)
+        if (big)
         {
-            const int u = e >> 3, d = e & 7;
-            const u32 g = start + base + u32(u);
-            const u32 *row = a.rows + size_t(g) * kRow;
-            const u32 cnt = row[2 + d + 1] - row[2 + d];
-            u32 out = 0;
-            if (cnt)
+            nearFieldByRows<Hilbert>(a, idx, l, first, nb, sWarp[threadIdx.x >> 5].rows, t);
+            continue;
+        }
+        // Four lanes a unit: lane (x0, y0) sums the children (x0, y0, 0) and
+        // (x0, y0, 1).  A record's word holds the cells (y, z) of one x of its
+        // cell: bytes (0,0) (0,1) (1,0) (1,1).  The sub-block's y range is the
+        // upper half of cell row 0 and row 1 (y0 = 0), or row 1 and the lower
+        // half of row 2; its z range likewise.
+        const int u = lane >> 2, x0 = (lane >> 1) & 1, y0 = lane & 1;
+        if (u < nb)
+        {
+            const u32 *words = reinterpret_cast<const u32 *>(w.rec + u * 27);
+            const u32 g = first + u32(u);
+            const u32 rowA = y0 ? 0x01010101u : 0x01010000u;  // bytes of the two cell rows the range takes
+            const u32 rowB = y0 ? 0x00000101u : 0x01010101u;
+            u32 z0 = 0, z1 = 0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
             {
-                const unsigned o = Hilbert ? unsigned(sDec[w.childState[u] * 8 + d]) : unsigned(d);
-                const u32 *sub = w.block[u] + (o >> 2) * 16 + ((o >> 1) & 1u) * 4 + (o & 1u);
-                u64 pop = 0;
-                if (m > 1)
+                const int x = x0 + 1 + i, qx = x >> 1, ox = x & 1;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
                 {
-                    u32 p32 = 0;
-#pragma unroll
-                    for (int x = 0; x < 3; ++x)
-#pragma unroll
-                        for (int y = 0; y < 3; ++y)
-#pragma unroll
-                            for (int z = 0; z < 3; ++z) p32 += sub[x * 16 + y * 4 + z];
-                    pop = p32;
+                    const u32 row = j ? rowB : rowA;
+                    const u32 *cell = words + 2 * (qx + 3 * (y0 + j)) + ox;
+                    const u32 below = cell[0], middle = cell[18], above = cell[36];
+                    const u32 both = __dp4a(middle, row, 0u);
+                    z0 += both + __dp4a(below, row & 0x01000100u, 0u);
+                    z1 += both + __dp4a(above, row & 0x00010001u, 0u);
                 }
-                else
-                {
-                    // level 1: the periodic wrap repeats cells, the sum may exceed 2^32
-                    for (int x = 0; x < 3; ++x)
-                        for (int y = 0; y < 3; ++y)
-                            for (int z = 0; z < 3; ++z) pop += sub[x * 16 + y * 4 + z];
-                }
-                const u64 v = u64(cnt) * pop;
-                out = v > 0xffffffffull ? 0xffffffffu : u32(v);
             }
-            a.val[size_t(g) * 8 + d] = out;
+            const u32 own = words[2 * 13 + x0] >> (16 * y0);
+            const u32 c0 = own & 0xffu, c1 = (own >> 8) & 0xffu;
+            u32 d0 = u32(x0 * 4 + y0 * 2), d1 = d0 + 1;
+            if constexpr (Hilbert)
+            {
+                const u32 st = unitStateOf(a.rows[size_t(g) * kRow + 11]);
+                d0 = t.enc[st * 8 + d0];
+                d1 = t.enc[st * 8 + d1];
+            }
+            a.val[size_t(g) * 8 + d0] = c0 * z0;  // at most 254 x 27 x 254
+            a.val[size_t(g) * 8 + d1] = c1 * z1;
         }
         __syncwarp();
     }
@@ -549,10 +754,12 @@ static __global__ void __launch_bounds__(kThreads, 5)
 // links, and the placement follows the digits).
 // Forest: the history counts go to the unit's system's bins in global memory
 // (sContrib / sLanded unused); otherwise to the CTA's shared bins.
+// NFCount: the child slots are kept by octant; sSlots[32 * 9] of the warp
+// turns them around and lets the warp write them coalesced.
 template <bool NF, bool Hilbert, bool Forest>
 __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bucket, u32 start, u32 count,
                                               const unsigned char *sNext, const unsigned char *sDec, u32 *sContrib,
-                                              u32 *sLanded, u32 rank, u32 size)
+                                              u32 *sLanded, u32 *sSlots, u32 rank, u32 size)
 {
     Control &c = *a.ctl;
     const u32 next = start + count;
@@ -604,7 +811,7 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
         u32 base = 0;
         if (lane == 31 && incl) base = atomicAdd(&c.levelCount[l + 1], incl);
         base = __shfl_sync(0xffffffffu, base, 31);
-        if (!valid) continue;
+        if (!NF && !valid) continue;
         const u32 aR = regionArrival(reg), lR = regionLevel(reg), kR = regionDepth(reg);
         const u32 j = m - lR;  // 1 <= j <= kR
         const u32 sys = Forest ? a.usys[g] : 0u;
@@ -613,6 +820,7 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
 #pragma unroll
         for (int d = 0; d < 8; ++d)
         {
+            if (NF && !valid) break;
             u32 slot = kLeaf;
             if (highMask & (1u << d))
             {
@@ -630,13 +838,14 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
                     }
                     if constexpr (Forest) a.usys[gc] = sys;
                     // the child's own level and the curve state ordering its children
-                    u32 cst = kHilbertStart;
+                    u32 cst = kHilbertStart, oct = u32(d);
                     if constexpr (Hilbert)
                     {
                         const u32 st = unitStateOf(reg);
-                        cst = sNext[st * 8 + sDec[st * 8 + d]];
+                        oct = sDec[st * 8 + d];
+                        cst = sNext[st * 8 + oct];
                     }
-                    if constexpr (NF) a.parent[gc] = g * 8 + u32(d);
+                    if constexpr (NF) a.parent[gc] = g * 8 + oct;
                     const u64 ck = key + u64(d) * cr;
                     uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
                     crow[0] = make_uint4(u32(ck), u32(ck >> 32), b[d], 0u);
@@ -656,11 +865,29 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
             {
                 atomicAdd(&sContrib[(aR * kJumps + kR) * kJumps + j], 1u);
             }
-            slots[d] = slot;
+            if constexpr (NF && Hilbert) sSlots[lane * 9 + sDec[unitStateOf(reg) * 8 + d]] = slot;
+            else if constexpr (NF) sSlots[lane * 9 + d] = slot;
+            else slots[d] = slot;
         }
-        uint4 *ch4 = reinterpret_cast<uint4 *>(a.child + size_t(g) * 8);
-        ch4[0] = make_uint4(slots[0], slots[1], slots[2], slots[3]);
-        ch4[1] = make_uint4(slots[4], slots[5], slots[6], slots[7]);
+        if constexpr (NF)
+        {
+            __syncwarp();
+            const u32 words = min(32u, count - i0) * 8;
+            u32 *out = a.child + size_t(start + i0) * 8;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+            {
+                const u32 e = u32(k) * 32 + u32(lane);
+                if (e < words) out[e] = sSlots[(e >> 3) * 9 + (e & 7)];
+            }
+            __syncwarp();
+        }
+        else
+        {
+            uint4 *ch4 = reinterpret_cast<uint4 *>(a.child + size_t(g) * 8);
+            ch4[0] = make_uint4(slots[0], slots[1], slots[2], slots[3]);
+            ch4[1] = make_uint4(slots[4], slots[5], slots[6], slots[7]);
+        }
     }
 }
 
@@ -670,6 +897,7 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
     __shared__ u32 sContrib[kContribBins];
     __shared__ u32 sLanded[kArrivals];
     __shared__ unsigned char sNext[48 * 8], sDec[48 * 8];
+    __shared__ u32 sSlots[NF ? (kThreads / 32) * 32 * 9 : 1];
     Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     const u32 start = c.levelStart[l], count = c.levelCount[l];
@@ -687,6 +915,7 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
     if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
     __syncthreads();
     classifyUnits<NF, Hilbert, false>(a, l, bucket, start, count, sNext, sDec, sContrib, sLanded,
+                                      sSlots + (NF ? (threadIdx.x >> 5) * 32 * 9 : 0),
                                       blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     __syncthreads();
     for (int k = threadIdx.x; k < kContribBins; k += kThreads)
@@ -726,10 +955,13 @@ static __global__ void leafCountKernel(Arena a, int l, int levels)
 // child: a segmented scan of the children's leaf counts gives each child's
 // position, so a warp writes the entries of four units at once.
 // K, B (and NF, N, SEG where given) are the cornerstone arrays written: N the
-// leaf counts, SEG each leaf's tree (system) in a batch of trees.
-template <bool NF>
+// leaf counts, SEG each leaf's tree (system) in a batch of trees.  dec: the
+// digit -> octant table of the Hilbert curve (NFCount trees keep their
+// children by octant).
+template <bool NF, bool Hilbert>
 __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, int l,
-                                           u32 start, u32 count, u32 capacity, u32 rank, u32 size)
+                                           u32 start, u32 count, u32 capacity, u32 rank, u32 size,
+                                           const unsigned char *dec)
 {
     Control &c = *a.ctl;
     const u64 cr = octRange(unsigned(l) + 1);
@@ -740,8 +972,15 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
         const size_t e = e0 + size_t(lane);
         const bool valid = e < total;
         const u32 g = start + u32(valid ? e >> 3 : 0);
-        const u32 ch = valid ? a.child[size_t(g) * 8 + d] : kLeaf;
-        const u32 mine = ch == kLeaf ? 1u : a.leaves[ch];
+        u32 ch = valid ? a.child[size_t(g) * 8 + d] : kLeaf;
+        u32 mine = ch == kLeaf ? 1u : a.leaves[ch];
+        if constexpr (NF && Hilbert)
+        {
+            // from octants to digits within the unit's 8 lanes
+            const int from = valid ? (lane & 24) | dec[unitStateOf(a.rows[size_t(g) * kRow + 11]) * 8 + d] : lane;
+            ch = __shfl_sync(0xffffffffu, ch, from);
+            mine = __shfl_sync(0xffffffffu, mine, from);
+        }
         // exclusive prefix of the leaf counts within the unit's 8 lanes
         u32 inc = mine;
 #pragma unroll
@@ -772,13 +1011,20 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
     }
 }
 
-template <bool NF>
-static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int l, int levels, u32 capacity)
+template <bool NF, bool Hilbert>
+static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int l, int levels, u32 capacity,
+                                   HilbertTables h)
 {
+    __shared__ unsigned char sDec[48 * 8];
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    placeUnits<NF>(a, K, B, NFo, N, nullptr, l, c.levelStart[l], c.levelCount[l], capacity,
-                   blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if constexpr (NF && Hilbert)
+    {
+        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x) sDec[k] = h.decOct[k];
+        __syncthreads();
+    }
+    placeUnits<NF, Hilbert>(a, K, B, NFo, N, nullptr, l, c.levelStart[l], c.levelCount[l], capacity,
+                            blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sDec);
 }
 
 // The finished tree: sentinel boundary and the state of a converged build
