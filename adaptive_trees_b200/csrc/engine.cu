@@ -383,12 +383,6 @@ int smCount()
     return sms;
 }
 
-const HilbertTables &hilbertTables()
-{
-    static const HilbertTables t = makeHilbertTables();
-    return t;
-}
-
 namespace
 {
 // makeBinaryGeometry (binary_node.cuh:17-40): the longest side is halved at
@@ -1011,8 +1005,6 @@ TreeEngine::TreeEngine(const void *x, const void *y, const void *z, size_t n, co
             "adaptive_octree: particle count exceeds 32-bit permutation index range");
     m_->kpf.q = makeQuantBox<float>(cfg.box);
     m_->kpd.q = makeQuantBox<double>(cfg.box);
-    m_->kpf.h = hilbertTables();
-    m_->kpd.h = hilbertTables();
     prepared_ = cfg.views;
 
     // stream-ordered set-up: nothing here synchronises the device
@@ -1240,7 +1232,6 @@ void TreeEngine::computeKeys(int kind, int real, const void *x, const void *y, c
     if (kind == 1) pd.g = pf.g = makeGeometry(box, maxDepth, real);
     pf.q = makeQuantBox<float>(box);
     pd.q = makeQuantBox<double>(box);
-    pf.h = pd.h = hilbertTables();
     if (real == 0)
         launchKeygen<float>(kind, hilbert, static_cast<const float *>(x), static_cast<const float *>(y),
                             static_cast<const float *>(z), n, pf, reinterpret_cast<u64 *>(keys), {}, s);
@@ -1369,43 +1360,6 @@ void TreeEngine::refreshAll()
     }
 }
 
-// The digit -> block position table of the near-field kernel, once per device.
-static void ensureDigitPos()
-{
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    AOT_CHECK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= 64 || done[dev]) return;
-    const HilbertTables h = makeHilbertTables();
-    std::vector<unsigned long long> t(2 * 27 * 48);
-    for (int hil = 0; hil < 2; ++hil)
-        for (int q = 0; q < 27; ++q)
-            for (int st = 0; st < 48; ++st)
-            {
-                unsigned long long packed = 0;
-                for (int d = 0; d < 8; ++d)
-                {
-                    // block coordinate 2 * offset + child bit + 1 per axis, where Q touches P
-                    const int o = hil ? h.decOct[st * 8 + d] : d;
-                    const int dq[3] = {q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1};
-                    const int bit[3] = {o >> 2, (o >> 1) & 1, o & 1};
-                    bool ok = true;
-                    int p = 0;
-                    for (int ax = 0; ax < 3; ++ax)
-                    {
-                        if ((dq[ax] < 0 && bit[ax] == 0) || (dq[ax] > 0 && bit[ax] == 1)) ok = false;
-                        p = p * 4 + (2 * dq[ax] + bit[ax] + 1);
-                    }
-                    packed |= (unsigned long long)(ok ? p : 0xff) << (8 * d);
-                }
-                t[(hil * 27 + q) * 48 + st] = packed;
-            }
-    AOT_CHECK(cudaMemcpyToSymbol(rb::gDigitPos, t.data(), t.size() * sizeof(unsigned long long)));
-    done[dev] = true;
-}
-
 // Per-leaf quantities of the active octree: begin indices, then (NFCount)
 // near-field counts and group-merge flags.  all = every leaf, else the work
 // lists of the last materialisation.
@@ -1430,9 +1384,7 @@ void TreeEngine::refreshCounts(bool all, unsigned blocks)
     }
     if (cfg_.nf)
     {
-        const HilbertTables &h = m_->kpd.h;
         const rb::NodeTable gt{m_->nodeRows.as<u32>(), m_->nodeSlots};
-        ensureDigitPos();
         // a cleared table takes the nodes of every leaf, else those of the new leaves
         const bool fill = all || m_->nodeStale;
         if (m_->nodeStale)
@@ -1444,13 +1396,13 @@ void TreeEngine::refreshCounts(bool all, unsigned blocks)
         else rb::nodeTableKernel<false><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, gt), noteLaunch();
         markNearField(true);
         if (all && cfg_.hilbert)
-            rb::octNearFieldKernel<true, true><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, h, gt), noteLaunch();
+            rb::octNearFieldKernel<true, true><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, gt), noteLaunch();
         else if (all)
-            rb::octNearFieldKernel<false, true><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, h, gt), noteLaunch();
+            rb::octNearFieldKernel<false, true><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, gt), noteLaunch();
         else if (cfg_.hilbert)
-            rb::octNearFieldKernel<true, false><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, h, gt), noteLaunch();
+            rb::octNearFieldKernel<true, false><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, gt), noteLaunch();
         else
-            rb::octNearFieldKernel<false, false><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, h, gt), noteLaunch();
+            rb::octNearFieldKernel<false, false><<<blocks, rb::kRefreshThreads, 0, s>>>(tb, idx, cfg_.bucket, gt), noteLaunch();
         markNearField(false);
     }
     AOT_LAUNCH_CHECK();
@@ -1688,7 +1640,6 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         a.landed = a.contrib + lb::kContribBins;
         a.cap = u32(cap);
         AOT_CHECK(cudaMemsetAsync(m.lvCtl.p, 0, kCtlBytes, s));
-        if (nf) ensureDigitPos();
         lb::rootKernel<<<1, 32, 0, s>>>(a, m.bufs(), P, n_, cfg_.bucket, nf ? 1 : 0), noteLaunch();
         AOT_LAUNCH_CHECK();
         // Every kernel reads its level's size on the device, so the whole
@@ -1700,25 +1651,25 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         for (int l = 0; l < levels; ++l)
         {
             if (!nf)
-                lb::expandKernel<false, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+                lb::expandKernel<false, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
             else if (cfg_.hilbert)
-                lb::expandKernel<true, true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+                lb::expandKernel<true, true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
             else
-                lb::expandKernel<true, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+                lb::expandKernel<true, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
             if (nf)
             {
                 markNearField(true);
-                if (cfg_.hilbert) lb::nearFieldKernel<true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
-                else lb::nearFieldKernel<false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, m.kpd.h), noteLaunch();
+                if (cfg_.hilbert) lb::nearFieldKernel<true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
+                else lb::nearFieldKernel<false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
                 markNearField(false);
                 if (cfg_.hilbert)
-                    lb::classifyKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket, m.kpd.h), noteLaunch();
+                    lb::classifyKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
                 else
-                    lb::classifyKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket, m.kpd.h), noteLaunch();
+                    lb::classifyKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
             }
             else
             {
-                lb::classifyKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, l, cfg_.bucket, m.kpd.h), noteLaunch();
+                lb::classifyKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
             }
             AOT_LAUNCH_CHECK();
         }
@@ -1732,15 +1683,15 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
                 const u32 cap32 = u32(physCap_);
                 if (nf && cfg_.hilbert)
                     lb::placeKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
-                                                                                 l, levels, cap32, m.kpd.h),
+                                                                                 l, levels, cap32),
                         noteLaunch();
                 else if (nf)
                     lb::placeKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
-                                                                                  l, levels, cap32, m.kpd.h),
+                                                                                  l, levels, cap32),
                         noteLaunch();
                 else
                     lb::placeKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], l,
-                                                                            levels, cap32, m.kpd.h),
+                                                                            levels, cap32),
                         noteLaunch();
             }
             AOT_LAUNCH_CHECK();

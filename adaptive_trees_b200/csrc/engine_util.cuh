@@ -15,8 +15,6 @@ void noteLaunch();
 int smCount();
 // Blocks of `threads` threads covering n items (at least 1).
 unsigned gridFor(size_t n, unsigned threads);
-// Hilbert encode/decode tables (generated once).
-const HilbertTables &hilbertTables();
 
 // Box<T> (sfc_keys.cuh:420-465): inverse lengths and per-axis bits in T.
 template <class T>

@@ -208,7 +208,6 @@ ForestEngine::ForestEngine(const void *const *x, const void *const *y, const voi
     m.total = total;
     m.kpf.q = makeQuantBox<float>(cfg.box);
     m.kpd.q = makeQuantBox<double>(cfg.box);
-    m.kpf.h = m.kpd.h = hilbertTables();
     m.capModel.assign(size_t(numSystems), OctreeCapacity{});
     m.leafCap.assign(size_t(numSystems), 0);
 
@@ -618,7 +617,6 @@ bool ForestEngine::levelBuild()
         p.capacity = u32(std::min<size_t>(m.entryCap, 0xffffffffu));
         p.bucket = m.cfg.bucket;
         p.maxDepth = int(m.cfg.maxDepth);
-        p.h = m.kpd.h;
         AOT_CHECK(cudaMemsetAsync(m.lvCtl.p, 0, kCtlBytes, s));
         void *args[] = {&p};
         AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(lb::kThreads), args, 0, s));

@@ -116,7 +116,7 @@ static __global__ void __launch_bounds__(sort::kPlanThreads)
                const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist, size_t histWords)
 {
     __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
-    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    if constexpr (C == Curve::Hilbert) loadPairTable(sPair);
     __syncthreads();
     const KeyMaker<Real, C> make(prm, sPair);
     const auto keyAt = [&](size_t g, u32 &group) {
@@ -215,7 +215,7 @@ static __global__ void __launch_bounds__(kThreads)
     __shared__ u32 sh[sort::kMaxPasses * sort::kRadix];
     __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) sh[i] = 0;
-    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    if constexpr (C == Curve::Hilbert) loadPairTable(sPair);
     __syncthreads();
     const u32 per = (numTiles + gridDim.x - 1) / gridDim.x;
     const u32 t0 = blockIdx.x * per;

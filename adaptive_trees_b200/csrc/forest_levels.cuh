@@ -54,14 +54,13 @@ struct LevelArgs
     u32 capacity;     // entries the leaf arrays hold
     unsigned bucket;
     int maxDepth;
-    HilbertTables h;
 };
 
 template <bool Hilbert>
 static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArgs p)
 {
     using namespace lb;
-    __shared__ unsigned char sNext[48 * 8], sDec[48 * 8];
+    __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
     __shared__ u32 sBin[kContribBins];
     __shared__ unsigned long long sVal[kContribBins];
     __shared__ int sBins, sRounds;
@@ -75,11 +74,8 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
     if (vload(p.f.st->error)) return;  // the sort gave up: the host reports it
     if constexpr (Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
-        {
-            sNext[k] = p.h.encNext[k];
-            sDec[k] = p.h.decOct[k];
-        }
+        copyTable(sNext, gHilbert.encNext);
+        copyTable(sDec, gHilbert.decOct);
     }
     // roots, and zeroed history bins
     for (size_t i = rank; i < size_t(S) * kContribBins; i += size) a.contrib[i] = 0;

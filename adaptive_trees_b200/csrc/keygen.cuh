@@ -23,11 +23,10 @@ struct KeygenParams
 {
     QuantBox<Real> q;
     BinaryGeometry g;
-    HilbertTables h;
 };
 
 // What a thread keeps for the keys of its particles.  sPair: the two-level
-// Hilbert table (hilbertPairEntry) in shared memory.
+// Hilbert table in shared memory.
 template <class Real, Curve C>
 struct KeyMaker
 {
@@ -74,18 +73,10 @@ __device__ __forceinline__ void countDigits(u64 k, int firstPass, u32 *sh)
 
 constexpr int kKeygenThreads = 256;
 
-// The two-level Hilbert table in shared memory, from the one-level tables.
-template <class Real>
-__device__ __forceinline__ void loadPairTable(const KeygenParams<Real> &prm, u32 *sPair)
+// The two-level Hilbert table to shared memory.
+__device__ __forceinline__ void loadPairTable(u32 *sPair)
 {
-    __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8];
-    for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x)
-    {
-        sEnc[i] = prm.h.enc[i];
-        sNext[i] = prm.h.encNext[i];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kHilbertPairEntries; i += blockDim.x) sPair[i] = hilbertPairEntry(i, sEnc, sNext);
+    for (int i = threadIdx.x; i < kHilbertPairEntries; i += blockDim.x) sPair[i] = __ldg(gHilbertPairs.entry + i);
 }
 
 // Start of a planned sort: the control block, zeroed digit counts and the
@@ -96,7 +87,7 @@ static __global__ void __launch_bounds__(sort::kPlanThreads)
                const KeygenParams<Real> prm, sort::PlanArgs plan, sort::SortControl *ctl, u32 *hist)
 {
     __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
-    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    if constexpr (C == Curve::Hilbert) loadPairTable(sPair);
     __syncthreads();
     const KeyMaker<Real, C> make(prm, sPair);
     const auto keyAt = [&](size_t i, u32 &) { return make(x[i], y[i], z[i]); };
@@ -115,7 +106,7 @@ static __global__ void __launch_bounds__(kKeygenThreads)
     __shared__ u32 sh[sort::kMaxPasses][sort::kRadix];
     __shared__ u32 sPair[C == Curve::Hilbert ? kHilbertPairEntries : 1];
     for (int i = threadIdx.x; i < sort::kMaxPasses * sort::kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
-    if constexpr (C == Curve::Hilbert) loadPairTable(prm, sPair);
+    if constexpr (C == Curve::Hilbert) loadPairTable(sPair);
     const int firstPass = hist ? int(ctl->first) : sort::kMaxPasses;
     __syncthreads();
 

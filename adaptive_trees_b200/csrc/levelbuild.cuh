@@ -359,14 +359,14 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
 }
 
 template <bool Rec, bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyIndex idx, int l, HilbertTables h)
+static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyIndex idx, int l)
 {
-    __shared__ unsigned char sDec[48 * 8];
+    __shared__ __align__(4) unsigned char sDec[48 * 8];
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     if constexpr (Rec && Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x) sDec[k] = h.decOct[k];
+        copyTable(sDec, gHilbert.decOct);
         __syncthreads();
     }
     expandUnits<Rec, Hilbert>(a, idx, l, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x,
@@ -421,7 +421,7 @@ union NearScratch
     RowScratch rows;
     RecScratch recs;
 };
-struct NearTables
+struct alignas(4) NearTables
 {
     unsigned char enc[48 * 8], next[48 * 8], dec[48 * 8];
     unsigned char step[8 * 27];  // [octant of the unit][offset]: offset around the parent << 3 | octant there
@@ -584,7 +584,7 @@ __device__ __forceinline__ u64 countedRec(const u64 *P, u32 lo, u32 hi, u64 qKey
 
 template <bool Hilbert>
 static __global__ void __launch_bounds__(kThreads, 4)
-    nearFieldKernel(Arena a, KeyIndex idx, int l, HilbertTables h)
+    nearFieldKernel(Arena a, KeyIndex idx, int l)
 {
     using rb::kUnitBatch;
     __shared__ NearTables t;
@@ -595,12 +595,9 @@ static __global__ void __launch_bounds__(kThreads, 4)
     if (count <= blockIdx.x * u32(kThreads / 32) * u32(kUnitBatch)) return;  // no units for this CTA
     if constexpr (Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
-        {
-            t.enc[k] = h.enc[k];
-            t.next[k] = h.encNext[k];
-            t.dec[k] = h.decOct[k];
-        }
+        copyTable(t.enc, gHilbert.enc);
+        copyTable(t.next, gHilbert.encNext);
+        copyTable(t.dec, gHilbert.decOct);
     }
     for (int k = threadIdx.x; k < 8 * 27; k += blockDim.x)
     {
@@ -892,11 +889,11 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
 }
 
 template <bool NF, bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l, unsigned bucket, HilbertTables h)
+static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l, unsigned bucket)
 {
     __shared__ u32 sContrib[kContribBins];
     __shared__ u32 sLanded[kArrivals];
-    __shared__ unsigned char sNext[48 * 8], sDec[48 * 8];
+    __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
     __shared__ u32 sSlots[NF ? (kThreads / 32) * 32 * 9 : 1];
     Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
@@ -905,11 +902,8 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
     if (count <= blockIdx.x * blockDim.x) return;
     if constexpr (Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
-        {
-            sNext[k] = h.encNext[k];
-            sDec[k] = h.decOct[k];
-        }
+        copyTable(sNext, gHilbert.encNext);
+        copyTable(sDec, gHilbert.decOct);
     }
     for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
     if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
@@ -1012,15 +1006,14 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
 }
 
 template <bool NF, bool Hilbert>
-static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int l, int levels, u32 capacity,
-                                   HilbertTables h)
+static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int l, int levels, u32 capacity)
 {
-    __shared__ unsigned char sDec[48 * 8];
+    __shared__ __align__(4) unsigned char sDec[48 * 8];
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
     if constexpr (NF && Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x) sDec[k] = h.decOct[k];
+        copyTable(sDec, gHilbert.decOct);
         __syncthreads();
     }
     placeUnits<NF, Hilbert>(a, K, B, NFo, N, nullptr, l, c.levelStart[l], c.levelCount[l], capacity,

@@ -984,15 +984,47 @@ __device__ __forceinline__ u64 neighbourCell(const Scratch &w, int u, int q, int
 // Where the children of the neighbour cell at offset q land in the unit's
 // 4 x 4 x 4 block, per child state and digit: [Morton, Hilbert][q][state],
 // 8 bits per digit (the block position, or 0xff for a child that does not
-// touch P).  Filled once per device from the host.
-__device__ u64 gDigitPos[2 * 27 * 48];
+// touch P).
+struct DigitPos
+{
+    u64 packed[2 * 27 * 48];
+};
+constexpr DigitPos makeDigitPos()
+{
+    const HilbertTables h = makeHilbertTables();
+    DigitPos t{};
+    for (int hil = 0; hil < 2; ++hil)
+        for (int q = 0; q < 27; ++q)
+            for (int st = 0; st < 48; ++st)
+            {
+                u64 packed = 0;
+                for (int d = 0; d < 8; ++d)
+                {
+                    // block coordinate 2 * offset + child bit + 1 per axis, where Q touches P
+                    const int o = hil ? h.decOct[st * 8 + d] : d;
+                    const int dq[3] = {q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1};
+                    const int bit[3] = {o >> 2, (o >> 1) & 1, o & 1};
+                    bool ok = true;
+                    int p = 0;
+                    for (int ax = 0; ax < 3; ++ax)
+                    {
+                        if ((dq[ax] < 0 && bit[ax] == 0) || (dq[ax] > 0 && bit[ax] == 1)) ok = false;
+                        p = p * 4 + (2 * dq[ax] + bit[ax] + 1);
+                    }
+                    packed |= u64(ok ? p : 0xff) << (8 * d);
+                }
+                t.packed[(hil * 27 + q) * 48 + st] = packed;
+            }
+    return t;
+}
+static __device__ const DigitPos gDigitPos = makeDigitPos();
 
 // Child counts of Q from its 9 begin indices (children in digit order) into
 // the unit's block.
 template <bool Hilbert>
 __device__ __forceinline__ void childrenFromPacked(const u32 (&b)[kGroupBegins], int q, int qState, u32 *block)
 {
-    const u64 packed = gDigitPos[(Hilbert ? 27 * 48 : 0) + q * 48 + qState];
+    const u64 packed = __ldg(&gDigitPos.packed[(Hilbert ? 27 * 48 : 0) + q * 48 + qState]);
 #pragma unroll
     for (int d = 0; d < 8; ++d)
     {
@@ -1007,20 +1039,17 @@ __device__ __forceinline__ void childrenFromPacked(const u32 (&b)[kGroupBegins],
 // always merge).
 template <bool Hilbert, bool All>
 static __global__ void __launch_bounds__(kRefreshThreads, 4)
-    octNearFieldKernel(TreeBufs tb, KeyIndex idx, unsigned bucket, HilbertTables h, NodeTable gt)
+    octNearFieldKernel(TreeBufs tb, KeyIndex idx, unsigned bucket, NodeTable gt)
 {
-    __shared__ unsigned char sEnc[48 * 8], sNext[48 * 8], sDec[48 * 8];
+    __shared__ __align__(4) unsigned char sEnc[48 * 8], sNext[48 * 8], sDec[48 * 8];
     __shared__ UnitScratch sWarp[kRefreshThreads / 32];
     DeviceState *st = tb.st;
     if (halted(st)) return;
     if constexpr (Hilbert)
     {
-        for (int k = threadIdx.x; k < 48 * 8; k += blockDim.x)
-        {
-            sEnc[k] = h.enc[k];
-            sNext[k] = h.encNext[k];
-            sDec[k] = h.decOct[k];
-        }
+        copyTable(sEnc, gHilbert.enc);
+        copyTable(sNext, gHilbert.encNext);
+        copyTable(sDec, gHilbert.decOct);
     }
     __syncthreads();
     const int a = st->activeBuffer;

@@ -59,7 +59,7 @@ __host__ __device__ __forceinline__ u64 mortonKey(u32 x, u32 y, u32 z)
 // --------------------------------------------------------------------------
 // Index = state * 8 + original octant (octant = x<<2 | y<<1 | z of the
 // original coordinates' bits at the level).
-struct HilbertTables
+struct alignas(4) HilbertTables
 {
     unsigned char enc[48 * 8];      // emitted octal digit
     unsigned char encNext[48 * 8];  // next state
@@ -67,20 +67,14 @@ struct HilbertTables
 };
 
 // Builds the tables from the reference's per-level rules (host only).
-inline HilbertTables makeHilbertTables()
+constexpr HilbertTables makeHilbertTables()
 {
     HilbertTables t{};
-    static const unsigned order[8] = {0, 1, 3, 2, 7, 6, 4, 5};  // sfc_keys.cuh:248-252
-    static const int perms[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-    auto stateOf = [&](const int p[3], const int f[3]) {
-        int pi = 0;
-        for (int k = 0; k < 6; ++k)
-            if (perms[k][0] == p[0] && perms[k][1] == p[1] && perms[k][2] == p[2]) pi = k;
-        return pi * 8 + (f[0] << 2) + (f[1] << 1) + f[2];
-    };
+    constexpr unsigned order[8] = {0, 1, 3, 2, 7, 6, 4, 5};  // sfc_keys.cuh:248-252
+    constexpr int perms[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
     for (int s = 0; s < 48; ++s)
     {
-        const int *perm = perms[s / 8];
+        const int perm[3] = {perms[s / 8][0], perms[s / 8][1], perms[s / 8][2]};
         const int flips[3] = {(s >> 2) & 1, (s >> 1) & 1, s & 1};
         for (unsigned o = 0; o < 8; ++o)
         {
@@ -97,25 +91,43 @@ inline HilbertTables makeHilbertTables()
             if (xi & (ny | zi)) wf[0] ^= 1;
             if ((xi & (yi | zi)) | (yi & nz)) wf[1] ^= 1;
             if ((xi & ny & nz) | (yi & nz)) wf[2] ^= 1;
+            const int p0 = wp[0], f0 = wf[0];
             if (zi)
             {
-                const int tp = wp[0], tf = wf[0];
                 wp[0] = wp[1]; wf[0] = wf[1];
                 wp[1] = wp[2]; wf[1] = wf[2];
-                wp[2] = tp; wf[2] = tf;
+                wp[2] = p0; wf[2] = f0;
             }
             else if (ny)
             {
-                std::swap(wp[0], wp[2]);
-                std::swap(wf[0], wf[2]);
+                wp[0] = wp[2]; wf[0] = wf[2];
+                wp[2] = p0; wf[2] = f0;
             }
-            const int next = stateOf(wp, wf);
+            int pi = 0;
+            for (int k = 0; k < 6; ++k)
+                if (perms[k][0] == wp[0] && perms[k][1] == wp[1] && perms[k][2] == wp[2]) pi = k;
+            const int next = pi * 8 + (wf[0] << 2) + (wf[1] << 1) + wf[2];
             t.enc[s * 8 + o] = (unsigned char)digit;
             t.encNext[s * 8 + o] = (unsigned char)next;
             t.decOct[s * 8 + digit] = (unsigned char)o;
         }
     }
     return t;
+}
+
+// The tables in device memory, set up at compile time.  Kernels copy them to
+// shared memory by words; as kernel parameters they were read byte by byte at
+// another address per lane, one lane at a time (1-2 us at the start of every
+// kernel).
+static __device__ const HilbertTables gHilbert = makeHilbertTables();
+static_assert(sizeof(HilbertTables) == 3 * 48 * 8, "tables without padding");
+
+// Copies the table of gHilbert that `from` names to shared memory (4-byte
+// aligned), by the CTA.
+__device__ __forceinline__ void copyTable(unsigned char *to, const unsigned char (&from)[48 * 8])
+{
+    for (int k = threadIdx.x; k < 48 * 8 / 4; k += blockDim.x)
+        reinterpret_cast<u32 *>(to)[k] = __ldg(reinterpret_cast<const u32 *>(from) + k);
 }
 
 // The identity state (permutation 0, no complements).
@@ -142,18 +154,29 @@ __host__ __device__ __forceinline__ u64 hilbertPrefix(u32 x, u32 y, u32 z, unsig
 
 // Two levels per lookup: pair[state * 64 + (o1 << 3 | o2)] = the state after
 // both << 8 | the two emitted digits (d1 << 3 | d2) << 2, for the original
-// octants o1, o2 of two consecutive levels.  3072 entries built from enc /
+// octants o1, o2 of two consecutive levels.  3072 entries made from enc /
 // encNext.  An entry's upper bits are the byte offset of its state's entries,
 // so the next lookup's offset is one bit selection between the entry and the
 // octants.
 constexpr int kHilbertPairEntries = 48 * 64;
-__host__ __device__ __forceinline__ u32 hilbertPairEntry(int i, const unsigned char *enc, const unsigned char *encNext)
+struct HilbertPairs
 {
-    const int s = i >> 6, o1 = (i >> 3) & 7, o2 = i & 7;
-    const int a = s * 8 + o1;
-    const int b = int(encNext[a]) * 8 + o2;
-    return (u32(encNext[b]) << 8) | (u32((enc[a] << 3) | enc[b]) << 2);
+    u32 entry[kHilbertPairEntries];
+};
+constexpr HilbertPairs makeHilbertPairs()
+{
+    const HilbertTables t = makeHilbertTables();
+    HilbertPairs p{};
+    for (int i = 0; i < kHilbertPairEntries; ++i)
+    {
+        const int s = i >> 6, o1 = (i >> 3) & 7, o2 = i & 7;
+        const int a = s * 8 + o1;
+        const int b = int(t.encNext[a]) * 8 + o2;
+        p.entry[i] = (u32(t.encNext[b]) << 8) | (u32((t.enc[a] << 3) | t.enc[b]) << 2);
+    }
+    return p;
 }
+static __device__ const HilbertPairs gHilbertPairs = makeHilbertPairs();
 
 // The full 21-level Hilbert key of (x, y, z) with the pair table: the Morton
 // interleave of the words puts each level's original octant (x << 2 | y << 1
