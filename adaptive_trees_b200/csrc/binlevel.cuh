@@ -13,8 +13,8 @@
 //             (a warp per unit on levels of few units), then its two
 //             children: those above the bucket become units of the next
 //             level (warp-aggregated slots), the others are leaves;
-//   leafCount subtree leaf counts, deepest level first;
-//   place     every leaf's K, B and count, shallowest level first.
+//   subtree   subtree leaf counts, bottom-up, all levels in one launch;
+//   place     every leaf's K, B and count, top-down, all levels in one launch.
 // Each pass of the reference splits one level, so the passes that change the
 // tree number the deepest unit's level + 1, and its leaf capacity, grown by
 // 25 % steps to the leaf count of every pass (commitIfLast, rebalance.cuh),
@@ -39,6 +39,8 @@ struct Control
     u32 levelCount[kLevels + 2];
     int overflow;       // the unit arena is too small
     int placeOverflow;  // more leaves than the leaf arrays hold
+    int error;          // a bounded wait gave up
+    u32 placeNext;      // next chunk of the placement
 };
 
 struct Arena
@@ -46,8 +48,9 @@ struct Arena
     uint4 *rows;    // [cap] key lo, key hi, begin, end
     u32 *mid;       // [cap] first key of the upper child
     u32 *child;     // [cap][2] unit index of an internal child, or kLeaf
-    u32 *leaves;    // [cap] leaves in the unit's subtree
-    u32 *offset;    // [cap] leaf index of the unit's first leaf
+    u32 *parent;    // [cap] parent unit
+    u64 *sub;       // [cap] leaves counted below the unit | children to come << lb::kSubShift
+    u32 *offset;    // [cap] leaf index of the unit's first leaf (lb::kPending before it is known)
     Control *ctl;
     u32 cap;
 };
@@ -111,6 +114,8 @@ static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex
             if (lane != 0) continue;
             a.mid[g] = m;
             const u32 cnt[2] = {m - r.z, r.w - m};
+            const u32 inner = (cnt[0] > bucket && deeper ? 1u : 0u) + (cnt[1] > bucket && deeper ? 1u : 0u);
+            a.sub[g] = (u64(inner) << lb::kSubShift) | (2u - inner);
             for (int s = 0; s < 2; ++s)
             {
                 u32 slot = kLeaf;
@@ -121,6 +126,8 @@ static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex
                     {
                         const u64 ck = key + u64(s) * half;
                         a.rows[gc] = make_uint4(u32(ck), u32(ck >> 32), s ? m : r.z, s ? r.w : m);
+                        a.parent[gc] = g;
+                        a.offset[gc] = lb::kPending;
                         slot = gc;
                     }
                     else
@@ -165,6 +172,7 @@ static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex
         if (lane == 31 && incl) base = atomicAdd(&c.levelCount[l + 1], incl);
         base = __shfl_sync(0xffffffffu, base, 31);
         if (!valid) continue;
+        a.sub[g] = (u64(nHigh) << lb::kSubShift) | (2u - nHigh);
         u32 rank = base + incl - nHigh;
         for (int s = 0; s < 2; ++s)
         {
@@ -176,6 +184,8 @@ static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex
                 {
                     const u64 ck = key + u64(s) * half;
                     a.rows[gc] = make_uint4(u32(ck), u32(ck >> 32), s ? m : r.z, s ? r.w : m);
+                    a.parent[gc] = g;
+                    a.offset[gc] = lb::kPending;
                     slot = gc;
                 }
                 else
@@ -188,57 +198,97 @@ static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex
     }
 }
 
-// Leaves below each unit of depth l (the units of depth l + 1 are counted).
-// `levels`: the depths the build expanded; units below them mean the build is
-// incomplete, and nothing is counted or placed.
-static __global__ void leafCountKernel(Arena a, int l, int levels)
+// The leaves below every unit (lb::subtreeKernel for two children): a unit of
+// two leaves starts, and the child of a unit that comes last takes the total
+// on.  `levels`: the depths the build expanded; units below them mean the
+// build is incomplete, and nothing is counted or placed.
+static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int levels)
 {
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow) return;
-    const u32 start = c.levelStart[l], count = c.levelCount[l];
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    const u32 total = c.levelStart[levels];
+    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
-        const u32 g = start + i;
-        const u32 c0 = a.child[size_t(g) * 2], c1 = a.child[size_t(g) * 2 + 1];
-        a.leaves[g] = (c0 == kLeaf ? 1u : a.leaves[c0]) + (c1 == kLeaf ? 1u : a.leaves[c1]);
+        // (a unit with internal children holds 3 leaves or more when they have come)
+        u64 n = sort::ldRelaxed(a.sub + g);
+        if (n != 2) continue;
+        for (u32 u = g; u != 0;)
+        {
+            u = a.parent[u];
+            const u64 old = atomicAdd(reinterpret_cast<unsigned long long *>(a.sub + u),
+                                      (unsigned long long)(n - (u64(1) << lb::kSubShift)));
+            if ((old >> lb::kSubShift) != 1) break;
+            n += old & ((u64(1) << lb::kSubShift) - 1);
+        }
     }
 }
 
-// K, B and the count of the leaf children of the depth-l units, and the
-// first leaf index of their internal children.
-static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *N, int l, int levels, u32 capacity)
+// K, B and the count of the leaf children of every unit, and the first leaf
+// index of the internal ones (lb::placeKernel for two children: chunks of one
+// depth's units in order, a thread per unit; a unit waits for its own place,
+// which its parent's chunk writes).
+constexpr u32 kPlaceChunk = kThreads;
+static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, int levels, u32 capacity)
 {
+    __shared__ u32 sChunk;
     Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow) return;
-    const u32 start = c.levelStart[l], count = c.levelCount[l];
-    const u64 half = depthRange(l + 1);
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    if (c.levelCount[levels] | c.overflow | c.error) return;
+    u32 level = 0, levelChunk = 0;  // chunks before `level`
+    for (;;)
     {
-        const u32 g = start + i;
+        __syncthreads();
+        // (after a wait that gave up: no more chunks)
+        if (threadIdx.x == 0)
+            sChunk = *static_cast<volatile int *>(&c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
+        __syncthreads();
+        const u32 chunk = sChunk;
+        u32 count = 0;
+        for (; level < u32(levels); ++level)
+        {
+            count = c.levelCount[level];
+            const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
+            if (chunk < levelChunk + chunks) break;
+            levelChunk += chunks;
+        }
+        if (level >= u32(levels)) return;
+        const u32 i = (chunk - levelChunk) * kPlaceChunk + threadIdx.x;
+        const bool valid = i < count;
+        const u32 g = c.levelStart[level] + (valid ? i : 0);
+        const u64 half = depthRange(int(level) + 1);
         const uint4 r = a.rows[g];
         const u64 key = (u64(r.y) << 32) | r.x;
         const u32 m = a.mid[g];
-        const u32 lo[2] = {r.z, m}, hi[2] = {m, r.w};
-        u32 o = a.offset[g];
-        for (int s = 0; s < 2; ++s)
+        const u32 ch[2] = {a.child[size_t(g) * 2], a.child[size_t(g) * 2 + 1]};
+        const u32 below = ch[0] == kLeaf ? 1u : u32(a.sub[ch[0]]);
+        u32 o = 0;
+        for (unsigned spins = 0;; ++spins)
         {
-            const u32 ch = a.child[size_t(g) * 2 + s];
-            if (ch != kLeaf)
+            o = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
+            if (!__any_sync(0xffffffffu, o == lb::kPending)) break;
+            if (spins > lb::kPlaceSpins)
             {
-                a.offset[ch] = o;
-                o += a.leaves[ch];
+                c.error = kErrLookback;
+                break;
+            }
+            if (spins > 64) __nanosleep(64);
+        }
+        if (!valid || o == lb::kPending) continue;
+        const u32 lo[2] = {r.z, m}, hi[2] = {m, r.w};
+        for (int s = 0; s < 2; ++s, o += below)
+        {
+            if (ch[s] != kLeaf)
+            {
+                *static_cast<volatile u32 *>(a.offset + ch[s]) = o;
             }
             else if (o >= capacity)
             {
                 c.placeOverflow = 1;  // the host grows the leaf arrays and places again
-                ++o;
             }
             else
             {
                 K[o] = key + u64(s) * half;
                 B[o] = lo[s];
                 N[o] = hi[s] - lo[s];
-                ++o;
             }
         }
     }

@@ -860,14 +860,14 @@ struct TreeEngine::Impl
     DevMem K[2], B[2], NF[2], N[2], G[2], offs, dirty, scan;
     DevMem nodeRows;  // node table of the near-field refresh (NFCount)
     // converged build by levels (levelbuild.cuh): unit arena and its control
-    DevMem lvRows, lvVal, lvChild, lvLeaves, lvOffset, lvCtl, lvNbr, lvParent, lvRec;
+    DevMem lvRows, lvVal, lvChild, lvSub, lvOffset, lvCtl, lvNbr, lvParent, lvRec;
     size_t lvCap = 0;
     int lvLevels = int(kOctLevels);  // levels the last level build needed, with one to spare
     DevMem mergeSplits;              // merge-path cuts of the full begin refresh
     unsigned char *lvHost = nullptr; // pinned: the level build's one readback
     size_t lvHostBytes = 0;
     // binary tree by levels (binlevel.cuh)
-    DevMem blRows, blMid, blChild, blLeaves, blOffset, blCtl;
+    DevMem blRows, blMid, blChild, blSub, blParent, blOffset, blCtl;
     size_t blCap = 0;
     int blLevels = bl::kLevels;      // depths the last binary build needed, with one to spare
     bl::Control *blHost = nullptr;   // pinned readback
@@ -916,7 +916,7 @@ struct TreeEngine::Impl
                                &vLvVals[1],  &vLayKeys[0], &vLayKeys[1],    &vLayVals[0],  &vLayVals[1],
                                &vIntStartSfc, &vIntLevelSfc, &vIntM,        &vIntStartLay, &vIntLevelLay,
                                &viewSort.mem, &nodeRows, &lvRows, &lvVal, &lvChild,
-                               &lvLeaves, &lvOffset, &lvCtl, &lvNbr, &lvParent, &lvRec};
+                               &lvSub, &lvOffset, &lvCtl, &lvNbr, &lvParent, &lvRec};
         size_t s = 0;
         for (const DevMem *d : all) s += d->bytes;
         return s;
@@ -1616,11 +1616,11 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         {
             m.lvVal.reserve(cap * 8 * sizeof(u32), s);
             m.lvNbr.reserve(cap * 27 * sizeof(u32), s);
-            m.lvParent.reserve(cap * sizeof(u32), s);
             m.lvRec.reserve(cap * sizeof(u64), s);
         }
         m.lvChild.reserve(cap * 8 * sizeof(u32), s);
-        m.lvLeaves.reserve(cap * sizeof(u32), s);
+        m.lvSub.reserve(cap * sizeof(u64), s);
+        m.lvParent.reserve(cap * sizeof(u32), s);
         m.lvOffset.reserve(cap * sizeof(u32), s);
         m.lvCtl.reserve(kCtlBytes, s);
         m.lvCap = cap;
@@ -1628,12 +1628,13 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         a.rows = m.lvRows.as<u32>();
         a.val = nf ? m.lvVal.as<u32>() : nullptr;
         a.nbr = nf ? m.lvNbr.as<u32>() : nullptr;
-        a.parent = nf ? m.lvParent.as<u32>() : nullptr;
+        a.parent = m.lvParent.as<u32>();
         a.rec = nf ? m.lvRec.as<u64>() : nullptr;
         a.usys = nullptr;
         a.sysRoot = nullptr;
         a.child = m.lvChild.as<u32>();
-        a.leaves = m.lvLeaves.as<u32>();
+        a.sub = m.lvSub.as<u64>();
+        a.leaves = nullptr;
         a.offset = m.lvOffset.as<u32>();
         a.ctl = m.lvCtl.as<lb::Control>();
         a.contrib = reinterpret_cast<unsigned long long *>(m.lvCtl.as<unsigned char>() + kHeadBytes);
@@ -1673,27 +1674,21 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             }
             AOT_LAUNCH_CHECK();
         }
-        for (int l = levels - 1; l >= 0; --l)
-            lb::leafCountKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, l, levels), noteLaunch();
+        lb::subtreeKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
         AOT_LAUNCH_CHECK();
         auto place = [&]() {
             const rb::TreeBufs tb = m.bufs();
-            for (int l = 0; l < levels; ++l)
-            {
-                const u32 cap32 = u32(physCap_);
-                if (nf && cfg_.hilbert)
-                    lb::placeKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
-                                                                                 l, levels, cap32),
-                        noteLaunch();
-                else if (nf)
-                    lb::placeKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0],
-                                                                                  l, levels, cap32),
-                        noteLaunch();
-                else
-                    lb::placeKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], l,
-                                                                            levels, cap32),
-                        noteLaunch();
-            }
+            const u32 room = u32(physCap_);
+            const unsigned grid = blocks * wide;
+            if (nf && cfg_.hilbert)
+                lb::placeKernel<true, true><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0], levels, room),
+                    noteLaunch();
+            else if (nf)
+                lb::placeKernel<true, false><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0], levels, room),
+                    noteLaunch();
+            else
+                lb::placeKernel<false, false><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], levels, room),
+                    noteLaunch();
             AOT_LAUNCH_CHECK();
         };
         place();
@@ -1701,7 +1696,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         // everything once
         // (with the device state: its active count, set by the root kernel)
         AOT_CHECK(cudaMemcpyAsync(host, m.lvCtl.p, kCtlBytes, cudaMemcpyDeviceToHost, s));
-        AOT_CHECK(cudaMemcpyAsync(host + kCtlBytes, a.leaves, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        AOT_CHECK(cudaMemcpyAsync(host + kCtlBytes, a.sub, sizeof(u32), cudaMemcpyDeviceToHost, s));  // the root's leaves
         AOT_CHECK(cudaMemcpyAsync(m.hst, m.st, sizeof(DeviceState), cudaMemcpyDeviceToHost, s));
         waitStream(s);
         u32 rootLeaves = 1;
@@ -1752,6 +1747,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         {
             ensurePhysical(rootLeaves);
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
+            AOT_CHECK(cudaMemsetAsync(&a.ctl->placeNext, 0, sizeof(u32), s));
             place();
         }
         hostLeaves_ = rootLeaves;
@@ -1855,7 +1851,8 @@ bool TreeEngine::binaryLevelBuild()
         m.blRows.reserve(cap * sizeof(uint4), s);
         m.blMid.reserve(cap * sizeof(u32), s);
         m.blChild.reserve(cap * 2 * sizeof(u32), s);
-        m.blLeaves.reserve(cap * sizeof(u32), s);
+        m.blSub.reserve(cap * sizeof(u64), s);
+        m.blParent.reserve(cap * sizeof(u32), s);
         m.blOffset.reserve(cap * sizeof(u32), s);
         m.blCtl.reserve(sizeof(bl::Control), s);
         m.blCap = cap;
@@ -1863,7 +1860,8 @@ bool TreeEngine::binaryLevelBuild()
         a.rows = m.blRows.as<uint4>();
         a.mid = m.blMid.as<u32>();
         a.child = m.blChild.as<u32>();
-        a.leaves = m.blLeaves.as<u32>();
+        a.sub = m.blSub.as<u64>();
+        a.parent = m.blParent.as<u32>();
         a.offset = m.blOffset.as<u32>();
         a.ctl = m.blCtl.as<bl::Control>();
         a.cap = u32(cap);
@@ -1874,24 +1872,21 @@ bool TreeEngine::binaryLevelBuild()
         const int levels = std::max(1, std::min(bl::kLevels, m.blLevels));
         for (int l = 0; l < levels; ++l)
             bl::levelKernel<<<blocks * 2, bl::kThreads, 0, s>>>(a, idx, l, cfg_.bucket, cfg_.maxDepth), noteLaunch();
-        for (int l = levels - 1; l >= 0; --l)
-            bl::leafCountKernel<<<blocks, bl::kThreads, 0, s>>>(a, l, levels), noteLaunch();
+        bl::subtreeKernel<<<blocks, bl::kThreads, 0, s>>>(a, levels), noteLaunch();
         auto place = [&]() {
             const rb::TreeBufs tb = m.bufs();
-            for (int l = 0; l < levels; ++l)
-                bl::placeKernel<<<blocks, bl::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.N[0], l, levels,
-                                                               u32(physCap_)),
-                    noteLaunch();
+            bl::placeKernel<<<blocks, bl::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.N[0], levels, u32(physCap_)), noteLaunch();
             AOT_LAUNCH_CHECK();
         };
         place();
         AOT_CHECK(cudaMemcpyAsync(m.blHost, m.blCtl.p, sizeof(bl::Control), cudaMemcpyDeviceToHost, s));
         unsigned char *leavesHost = reinterpret_cast<unsigned char *>(m.blHost) + kLeavesAt;
-        AOT_CHECK(cudaMemcpyAsync(leavesHost, a.leaves, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        AOT_CHECK(cudaMemcpyAsync(leavesHost, a.sub, sizeof(u32), cudaMemcpyDeviceToHost, s));  // the root's leaves
         AOT_CHECK(cudaMemcpyAsync(m.hst, m.st, sizeof(DeviceState), cudaMemcpyDeviceToHost, s));
         waitStream(s);
         u32 rootLeaves = 1;
-        if (m.hst->error) throw std::runtime_error("adaptive_octree: a device scan gave up waiting (bounded look-back)");
+        if (m.hst->error | hc.error)
+            throw std::runtime_error("adaptive_octree: a device scan gave up waiting (bounded look-back)");
         if (hc.overflow)
         {
             cap *= 2;
@@ -1910,6 +1905,7 @@ bool TreeEngine::binaryLevelBuild()
         {
             ensurePhysical(rootLeaves);
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
+            AOT_CHECK(cudaMemsetAsync(&a.ctl->placeNext, 0, sizeof(u32), s));
             place();
         }
         // one pass per depth of units; the capacity's 25 % steps end at the

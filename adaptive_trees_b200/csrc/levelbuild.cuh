@@ -19,8 +19,9 @@
 //   classify  the children whose value exceeds the bucket become the units of
 //             level l + 1 (slots taken by warp-aggregated atomics); the
 //             others are leaves of the tree;
-//   leafCount, place: subtree leaf counts bottom-up, then every leaf's
-//             position in the cornerstone array top-down.
+//   subtree, place: subtree leaf counts bottom-up, then every leaf's
+//             position in the cornerstone array top-down, a kernel each for
+//             all levels.
 //
 // The capacity the reference ends with depends on how many leaves each round
 // proposed (resizeWithHeadroom history, octree.cu:159-180 and 453-457).  That
@@ -58,8 +59,9 @@ struct Control
     u32 levelCount[kOctLevels + 2];
     int overflow;       // the unit arena is too small
     int late;           // an arrival round beyond the tracked ones
-    int error;          // reserved (the level build has no waits)
+    int error;          // a bounded wait gave up
     int placeOverflow;  // the tree has more leaves than the cornerstone buffers hold
+    u32 placeNext;      // next chunk of the placement
 };
 
 // The unit arena: units of all levels, level l at
@@ -69,10 +71,11 @@ struct Arena
     u32 *rows;       // [cap][kRow]
     u32 *val;        // [cap][8] value of each child (NF or count)
     u32 *child;      // [cap][8] unit index of an internal child, or kLeaf (LeafCount: by digit, NFCount: by octant)
-    u32 *leaves;     // [cap] leaves in the unit's subtree
-    u32 *offset;     // [cap] cornerstone index of the unit's first leaf
+    u64 *sub;        // single tree: [cap] leaves counted below the unit | children to come << 56
+    u32 *leaves;     // batch of trees: [cap] leaves in the unit's subtree
+    u32 *offset;     // [cap] cornerstone index of the unit's first leaf (single tree: kPending before it is known)
     u32 *nbr;        // NFCount: [cap][27] the cells around each unit (nbrRef)
-    u32 *parent;     // NFCount: [cap] parent unit * 8 + the unit's octant in it
+    u32 *parent;     // single tree: [cap] parent unit * 8 + the unit's place in its child slots
     u64 *rec;        // NFCount: [cap] child counts of a unit, a byte per octant (kBigRec: one does not fit)
     u32 *usys;       // batch of trees: [cap] the tree (system) of each unit
     u32 *sysRoot;    // batch of trees: [systems] each system's root unit, or kLeaf
@@ -104,6 +107,10 @@ __device__ __forceinline__ u32 unitStateOf(u32 w) { return (w >> 24) & 0x3fu; }
 constexpr u32 kLeafRef = 0x80000000u;
 // Child counts of which one is 255 or more.
 constexpr u64 kBigRec = ~u64(0);
+// A unit's first leaf is not known yet.
+constexpr u32 kPending = 0xffffffffu;
+constexpr int kSubShift = 56;
+constexpr unsigned kPlaceSpins = 1u << 22;  // polls of a parent's placement
 
 // Levels a leaf of value x at level m splits by (calculateNodeOp,
 // octree_rebalance.cuh:188-249: 8, 64, 512 or 4096 children), given that it
@@ -159,7 +166,6 @@ static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t
         {
             // every cell around the root is the root (periodic wrap)
             for (int q = 0; q < 27; ++q) a.nbr[q] = 0;
-            a.parent[0] = kLeaf;
         }
         st->numLeaves = 0;  // set when the tree is placed
     }
@@ -842,7 +848,11 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
                         oct = sDec[st * 8 + d];
                         cst = sNext[st * 8 + oct];
                     }
-                    if constexpr (NF) a.parent[gc] = g * 8 + oct;
+                    if constexpr (!Forest)
+                    {
+                        a.parent[gc] = g * 8 + oct;
+                        a.offset[gc] = kPending;
+                    }
                     const u64 ck = key + u64(d) * cr;
                     uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
                     crow[0] = make_uint4(u32(ck), u32(ck >> 32), b[d], 0u);
@@ -865,6 +875,10 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
             if constexpr (NF && Hilbert) sSlots[lane * 9 + sDec[unitStateOf(reg) * 8 + d]] = slot;
             else if constexpr (NF) sSlots[lane * 9 + d] = slot;
             else slots[d] = slot;
+        }
+        if constexpr (!Forest)
+        {
+            if (valid) a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
         }
         if constexpr (NF)
         {
@@ -918,9 +932,7 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
         atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
 }
 
-// Leaves below each unit of level l (the units of level l + 1 are done).
-// `levels` is the number of levels the build expanded: units below them mean
-// the build is incomplete, and nothing is counted.
+// Batch of trees: leaves below each unit of a level (the units of the next are done).
 __device__ __forceinline__ void leafCountUnits(const Arena &a, u32 start, u32 count, u32 rank, u32 size)
 {
     for (u32 i = rank; i < count; i += size)
@@ -937,11 +949,31 @@ __device__ __forceinline__ void leafCountUnits(const Arena &a, u32 start, u32 co
     }
 }
 
-static __global__ void leafCountKernel(Arena a, int l, int levels)
+// The leaves below every unit of a single tree, all levels in one launch: a
+// unit whose children are all leaves starts (8 leaves) and adds its count to
+// its parent's; the child that comes last takes the parent's total on.  (A
+// kernel per level cost its launch and tail 11 times at 300k particles, 2.5 us
+// and a gap each.)  `levels` is the number of levels the build expanded: units
+// below them mean the build is incomplete, and nothing is counted.
+static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int levels)
 {
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    leafCountUnits(a, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    const u32 total = c.levelStart[levels];
+    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
+    {
+        // (a unit with internal children holds 15 leaves or more when they have come)
+        u64 n = sort::ldRelaxed(a.sub + g);
+        if (n != 8) continue;
+        for (u32 u = g; u != 0;)
+        {
+            u = a.parent[u] >> 3;
+            const u64 old = atomicAdd(reinterpret_cast<unsigned long long *>(a.sub + u),
+                                      (unsigned long long)(n - (u64(1) << kSubShift)));
+            if ((old >> kSubShift) != 1) break;
+            n += old & ((u64(1) << kSubShift) - 1);
+        }
+    }
 }
 
 // Cornerstone entries of the leaf children of the level-l units, and the
@@ -952,7 +984,7 @@ static __global__ void leafCountKernel(Arena a, int l, int levels)
 // leaf counts, SEG each leaf's tree (system) in a batch of trees.  dec: the
 // digit -> octant table of the Hilbert curve (NFCount trees keep their
 // children by octant).
-template <bool NF, bool Hilbert>
+template <bool NF, bool Hilbert, bool Forest>
 __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, int l,
                                            u32 start, u32 count, u32 capacity, u32 rank, u32 size,
                                            const unsigned char *dec)
@@ -967,7 +999,7 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
         const bool valid = e < total;
         const u32 g = start + u32(valid ? e >> 3 : 0);
         u32 ch = valid ? a.child[size_t(g) * 8 + d] : kLeaf;
-        u32 mine = ch == kLeaf ? 1u : a.leaves[ch];
+        u32 mine = ch == kLeaf ? 1u : Forest ? a.leaves[ch] : u32(a.sub[ch]);
         if constexpr (NF && Hilbert)
         {
             // from octants to digits within the unit's 8 lanes
@@ -983,8 +1015,28 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
             if (d >= off) inc += t;
         }
+        u32 first = 0;  // the unit's first leaf
+        if constexpr (Forest)
+        {
+            if (valid) first = a.offset[g];
+        }
+        else
+        {
+            // placed by the unit's parent, in a chunk handed out before this one
+            for (unsigned spins = 0;; ++spins)
+            {
+                first = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
+                if (!__any_sync(0xffffffffu, first == kPending)) break;
+                if (spins > kPlaceSpins)
+                {
+                    c.error = kErrLookback;
+                    return;
+                }
+                if (spins > 64) __nanosleep(64);
+            }
+        }
         if (!valid) continue;
-        const u32 o = a.offset[g] + inc - mine;
+        const u32 o = first + inc - mine;
         if (ch == kLeaf && o >= capacity)
         {
             c.placeOverflow = 1;  // the host grows the buffers and places again
@@ -1000,24 +1052,51 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
         }
         else
         {
-            a.offset[ch] = o;
+            *static_cast<volatile u32 *>(a.offset + ch) = o;
         }
     }
 }
 
+// Units of a placement chunk (one level's, so a chunk's parents lie in
+// chunks before it).
+constexpr u32 kPlaceChunk = 128;
+
+// The placement of a single tree, all levels in one launch: CTAs take chunks
+// of units in level order from a counter; a unit waits for its own place,
+// which its parent's chunk writes.  Chunks are handed out in order to running
+// CTAs and wait for earlier ones only, so the waits end (they are bounded all
+// the same).  A kernel per level: 36 us and 11 gaps at 300k particles.
 template <bool NF, bool Hilbert>
-static __global__ void placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int l, int levels, u32 capacity)
+static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels,
+                                                               u32 capacity)
 {
     __shared__ __align__(4) unsigned char sDec[48 * 8];
-    const Control &c = *a.ctl;
+    __shared__ u32 sChunk;
+    Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    if constexpr (NF && Hilbert)
+    if constexpr (NF && Hilbert) copyTable(sDec, gHilbert.decOct);
+    u32 level = 0, levelChunk = 0;  // chunks before `level`
+    for (;;)
     {
-        copyTable(sDec, gHilbert.decOct);
         __syncthreads();
+        // (after a wait that gave up: no more chunks)
+        if (threadIdx.x == 0)
+            sChunk = *static_cast<volatile int *>(&c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
+        __syncthreads();
+        const u32 chunk = sChunk;
+        u32 count = 0;
+        for (; level < u32(levels); ++level)
+        {
+            count = c.levelCount[level];
+            const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
+            if (chunk < levelChunk + chunks) break;
+            levelChunk += chunks;
+        }
+        if (level >= u32(levels)) return;
+        const u32 base = (chunk - levelChunk) * kPlaceChunk;
+        placeUnits<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, int(level), c.levelStart[level] + base,
+                                       min(kPlaceChunk, count - base), capacity, threadIdx.x, kThreads, sDec);
     }
-    placeUnits<NF, Hilbert>(a, K, B, NFo, N, nullptr, l, c.levelStart[l], c.levelCount[l], capacity,
-                            blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sDec);
 }
 
 // The finished tree: sentinel boundary and the state of a converged build
@@ -1027,7 +1106,7 @@ static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int rounds, int le
     DeviceState *st = tb.st;
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error | c.placeOverflow) return;
-    const int leaves = c.levelCount[0] ? int(a.leaves[0]) : 1;
+    const int leaves = c.levelCount[0] ? int(u32(a.sub[0])) : 1;
     if (u32(leaves) > capacity) return;
     tb.K[0][leaves] = kMaxKey;
     tb.B[0][leaves] = st->numActiveParticles;
