@@ -394,9 +394,9 @@ static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyInde
 // sub-block's.  Cells that are units bring their 8 child counts as one 8-byte
 // record, a byte per octant; those in a leaf (one of eight at 16Mi Plummer
 // particles, a few keys each) have the leaf's keys counted.  A lane sums two
-// children from the record words by byte dot products.  Units around which a
-// count does not fit a byte, and levels of few units, take the path by rows
-// (nearFieldByRows).
+// children from the record words by byte dot products.  (Levels of few units
+// have no records; theirs are made from the rows.)  Units around which a
+// count does not fit a byte take the path by rows (nearFieldByRows).
 //
 // Before: the 27 cells by a kernel of their own, a 48-byte row of begin
 // indices and a curve state per cell here, scattered into 4 x 4 x 4 blocks of
@@ -462,6 +462,26 @@ __device__ __forceinline__ void leafCell(const Arena &a, const NearTables &t, u3
         qKey = 0;
         qState = kHilbertStart;
     }
+}
+
+// A unit's child counts as bytes, from its row.
+template <bool Hilbert>
+__device__ __forceinline__ u64 rowRec(const u32 *row, const unsigned char *dec)
+{
+    const uint4 *r4 = reinterpret_cast<const uint4 *>(row);
+    const uint4 r0 = r4[0], r1 = r4[1], r2 = r4[2];
+    const u32 b[rb::kGroupBegins] = {r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z};
+    const u32 st = unitStateOf(r2.w);
+    u64 rec = 0;
+    bool big = false;
+#pragma unroll
+    for (int d = 0; d < 8; ++d)
+    {
+        const u32 cnt = b[d + 1] - b[d];
+        big |= cnt >= 255u;
+        rec |= u64(cnt & 0xffu) << (8 * (Hilbert ? u32(dec[st * 8 + d]) : u32(d)));
+    }
+    return big ? kBigRec : rec;
 }
 
 // The units [first, first + nb) of level l by rows: any counts.
@@ -598,7 +618,7 @@ static __global__ void __launch_bounds__(kThreads, 4)
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     const u32 start = c.levelStart[l], count = c.levelCount[l];
-    if (count <= blockIdx.x * u32(kThreads / 32) * u32(kUnitBatch)) return;  // no units for this CTA
+    if (count <= blockIdx.x) return;  // no units for this CTA
     if constexpr (Hilbert)
     {
         copyTable(t.enc, gHilbert.enc);
@@ -619,10 +639,12 @@ static __global__ void __launch_bounds__(kThreads, 4)
     const bool byRecs = count > kWideUnits;
     RecScratch &w = sWarp[threadIdx.x >> 5].recs;
     const u32 warpsTotal = gridDim.x * (blockDim.x / 32);
-    const u32 w0 = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    for (u32 base = w0 * kUnitBatch; base < count; base += warpsTotal * kUnitBatch)
+    // levels that do not fill the warps' batches: fewer units per warp, shorter chains
+    const u32 per = min(u32(kUnitBatch), (count + warpsTotal - 1) / warpsTotal);
+    const u32 w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // (a level of few units spreads over the SMs)
+    for (u32 base = w0 * per; base < count; base += warpsTotal * per)
     {
-        const int nb = int(min(u32(kUnitBatch), count - base)), items = nb * 27;
+        const int nb = int(min(per, count - base)), items = nb * 27;
         const u32 first = start + base;
         // the cells around the units, (unit, cell) pairs over the lanes: all
         // loads of a step in flight together
@@ -657,13 +679,23 @@ static __global__ void __launch_bounds__(kThreads, 4)
                 if (it < items) a.nbr[size_t(first) * 27 + it] = ref[i];
             }
         }
-        bool big = !byRecs;
-        if (byRecs)
+        bool big = false;
+        if (!byRecs)
+        {
+            // without records: counts that cannot fit a byte are told by the units themselves
+            const u32 *row = a.rows + size_t(first + u32(lane < nb ? lane : 0)) * kRow;
+            big = l == 0 || __any_sync(0xffffffffu, row[10] - row[2] > 8 * 254u);
+        }
+        if (!big)
         {
             u64 rec[kRounds];
 #pragma unroll
             for (int i = 0; i < kRounds; ++i)
-                rec[i] = i * 32 + lane < items && !(ref[i] & kLeafRef) ? a.rec[ref[i]] : 0;
+            {
+                rec[i] = 0;
+                if (i * 32 + lane < items && !(ref[i] & kLeafRef))
+                    rec[i] = byRecs ? a.rec[ref[i]] : rowRec<Hilbert>(a.rows + size_t(ref[i]) * kRow, t.dec);
+            }
             int nSlow = 0;
 #pragma unroll
             for (int i = 0; i < kRounds; ++i)
