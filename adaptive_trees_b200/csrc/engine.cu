@@ -922,6 +922,28 @@ struct TreeEngine::Impl
         return s;
     }
 
+    // the unit arena (levelbuild.cuh)
+    static constexpr size_t kUnitHeadBytes = (sizeof(lb::Control) + 255) & ~size_t(255);
+    static constexpr size_t kUnitCtlBytes =
+        kUnitHeadBytes + (lb::kContribBins + lb::kArrivals) * sizeof(unsigned long long);
+    lb::Arena units() const
+    {
+        lb::Arena a{};
+        a.rows = lvRows.as<u32>();
+        a.val = lvVal.as<u32>();
+        a.nbr = lvNbr.as<u32>();
+        a.rec = lvRec.as<u64>();
+        a.child = lvChild.as<u32>();
+        a.sub = lvSub.as<u64>();
+        a.parent = lvParent.as<u32>();
+        a.offset = lvOffset.as<u32>();
+        a.ctl = lvCtl.as<lb::Control>();
+        a.contrib = reinterpret_cast<unsigned long long *>(lvCtl.as<unsigned char>() + kUnitHeadBytes);
+        a.landed = a.contrib + lb::kContribBins;
+        a.cap = u32(lvCap);
+        return a;
+    }
+
     rb::TreeBufs bufs() const
     {
         rb::TreeBufs t{};
@@ -1144,8 +1166,31 @@ void TreeEngine::ensurePhysical(size_t capacity)
             m_->nodeSlots = u32(slots);
             m_->nodeStale = true;
         }
+        // the refresh of update() takes a large tree's internal nodes as units
+        if (refreshByUnits() && c > 4096) ensureUnits(std::max(c / 7 + 1, n_ / 4 + 4096));
     }
     physCap_ = c;
+}
+
+// The unit arena for at least `cap` units.
+void TreeEngine::ensureUnits(size_t cap)
+{
+    Impl &m = *m_;
+    cudaStream_t s = cfg_.stream;
+    cap = std::max(cap, m.lvCap);
+    m.lvRows.reserve(cap * lb::kRow * sizeof(u32), s);
+    if (cfg_.nf)
+    {
+        m.lvVal.reserve(cap * 8 * sizeof(u32), s);
+        m.lvNbr.reserve(cap * 27 * sizeof(u32), s);
+        m.lvRec.reserve(cap * sizeof(u64), s);
+    }
+    m.lvChild.reserve(cap * 8 * sizeof(u32), s);
+    m.lvSub.reserve(cap * sizeof(u64), s);
+    m.lvParent.reserve(cap * sizeof(u32), s);
+    m.lvOffset.reserve(cap * sizeof(u32), s);
+    m.lvCtl.reserve(Impl::kUnitCtlBytes, s);
+    m.lvCap = cap;
 }
 
 // --------------------------------------------------------------------------
@@ -1385,6 +1430,11 @@ void TreeEngine::refreshCounts(bool all, unsigned blocks)
     if (cfg_.nf)
     {
         const rb::NodeTable gt{m_->nodeRows.as<u32>(), m_->nodeSlots};
+        if (all && refreshByUnits())
+        {
+            refreshUnits();
+            return;
+        }
         // a cleared table takes the nodes of every leaf, else those of the new leaves
         const bool fill = all || m_->nodeStale;
         if (m_->nodeStale)
@@ -1407,6 +1457,38 @@ void TreeEngine::refreshCounts(bool all, unsigned blocks)
     }
     AOT_LAUNCH_CHECK();
 }
+
+// The full refresh of a large NFCount tree: its internal nodes as units, their
+// near field level by level, and the node table of the passes from the units.
+// (Every level a tree can have is launched: a captured update() serves deeper
+// trees too.)
+void TreeEngine::refreshUnits()
+{
+    Impl &m = *m_;
+    cudaStream_t s = cfg_.stream;
+    const rb::TreeBufs tb = m.bufs();
+    const lb::Arena a = m.units();
+    const KeyIndex idx = m.keyIndex(n_);
+    const unsigned blocks = unsigned(smCount()) * 4u;
+    AOT_CHECK(cudaMemsetAsync(a.ctl, 0, sizeof(lb::Control), s));
+    lb::treeRootKernel<<<1, 1, 0, s>>>(a, tb), noteLaunch();
+    for (int l = 0; l < int(kOctLevels); ++l)
+        if (cfg_.hilbert) lb::treeUnitsKernel<true><<<blocks * 2, lb::kThreads, 0, s>>>(a, tb, l), noteLaunch();
+        else lb::treeUnitsKernel<false><<<blocks * 2, lb::kThreads, 0, s>>>(a, tb, l), noteLaunch();
+    markNearField(true);
+    for (int l = 0; l < int(kOctLevels); ++l)
+        if (cfg_.hilbert) lb::nearFieldKernel<true, false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, tb, cfg_.bucket), noteLaunch();
+        else lb::nearFieldKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, tb, cfg_.bucket), noteLaunch();
+    markNearField(false);
+    const rb::NodeTable gt{m.nodeRows.as<u32>(), m.nodeSlots};
+    AOT_CHECK(cudaMemsetAsync(gt.rows, 0, size_t(gt.slots) * rb::kGroupRow * sizeof(u32), s));
+    m.nodeStale = false;
+    lb::unitsToTableKernel<<<blocks * 2, lb::kThreads, 0, s>>>(a, gt), noteLaunch();
+    AOT_LAUNCH_CHECK();
+}
+
+// (The units' 42 launches cost about 150 us however small the tree is.)
+bool TreeEngine::refreshByUnits() const { return cfg_.kind == 0 && cfg_.nf && n_ >= kUnitRefreshParticles; }
 
 void TreeEngine::materializeCounts()
 {
@@ -1602,8 +1684,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
     const KeyIndex idx = m.keyIndex(n_);
     const u64 *P = m.P[0].as<u64>();
     size_t cap = std::max<size_t>(m.lvCap, n_ / 4 + 4096);
-    constexpr size_t kHeadBytes = (sizeof(lb::Control) + 255) & ~size_t(255);
-    constexpr size_t kCtlBytes = kHeadBytes + (lb::kContribBins + lb::kArrivals) * sizeof(unsigned long long);
+    constexpr size_t kHeadBytes = Impl::kUnitHeadBytes, kCtlBytes = Impl::kUnitCtlBytes;
     if (!m.lvHost)
         m.lvHost = static_cast<unsigned char *>(blockcache::takeHost(kCtlBytes + 16, &m.lvHostBytes));
     unsigned char *host = m.lvHost;
@@ -1611,35 +1692,8 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
     for (;;)
     {
         if (cap >= (size_t(1) << 28)) return false;  // neighbour references hold unit * 8 + digit in 31 bits
-        m.lvRows.reserve(cap * lb::kRow * sizeof(u32), s);
-        if (nf)
-        {
-            m.lvVal.reserve(cap * 8 * sizeof(u32), s);
-            m.lvNbr.reserve(cap * 27 * sizeof(u32), s);
-            m.lvRec.reserve(cap * sizeof(u64), s);
-        }
-        m.lvChild.reserve(cap * 8 * sizeof(u32), s);
-        m.lvSub.reserve(cap * sizeof(u64), s);
-        m.lvParent.reserve(cap * sizeof(u32), s);
-        m.lvOffset.reserve(cap * sizeof(u32), s);
-        m.lvCtl.reserve(kCtlBytes, s);
-        m.lvCap = cap;
-        lb::Arena a{};
-        a.rows = m.lvRows.as<u32>();
-        a.val = nf ? m.lvVal.as<u32>() : nullptr;
-        a.nbr = nf ? m.lvNbr.as<u32>() : nullptr;
-        a.parent = m.lvParent.as<u32>();
-        a.rec = nf ? m.lvRec.as<u64>() : nullptr;
-        a.usys = nullptr;
-        a.sysRoot = nullptr;
-        a.child = m.lvChild.as<u32>();
-        a.sub = m.lvSub.as<u64>();
-        a.leaves = nullptr;
-        a.offset = m.lvOffset.as<u32>();
-        a.ctl = m.lvCtl.as<lb::Control>();
-        a.contrib = reinterpret_cast<unsigned long long *>(m.lvCtl.as<unsigned char>() + kHeadBytes);
-        a.landed = a.contrib + lb::kContribBins;
-        a.cap = u32(cap);
+        ensureUnits(cap);
+        const lb::Arena a = m.units();
         AOT_CHECK(cudaMemsetAsync(m.lvCtl.p, 0, kCtlBytes, s));
         lb::rootKernel<<<1, 32, 0, s>>>(a, m.bufs(), P, n_, cfg_.bucket, nf ? 1 : 0), noteLaunch();
         AOT_LAUNCH_CHECK();
@@ -1660,8 +1714,8 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             if (nf)
             {
                 markNearField(true);
-                if (cfg_.hilbert) lb::nearFieldKernel<true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
-                else lb::nearFieldKernel<false><<<blocks, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
+                if (cfg_.hilbert) lb::nearFieldKernel<true, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
+                else lb::nearFieldKernel<false, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
                 markNearField(false);
                 if (cfg_.hilbert)
                     lb::classifyKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();

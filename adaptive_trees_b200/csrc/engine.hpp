@@ -25,6 +25,11 @@ struct DeviceState;
 
 // Keys per tile of the onesweep radix sort (threads x items per thread).
 constexpr size_t kSortTileItems = 2560;
+// NFCount trees of this many particles refresh by units (TreeEngine::refreshUnits).
+// An update() of n Plummer particles replayed from a graph, by units and by
+// leaves: 0.7M 740 and 620 us, 1.5M 883 and 800, 3M 1206 and 1240, 6M 1771 and
+// 2160; uniform: 3M 836 and 816, 6M 1231 and 1350.
+constexpr size_t kUnitRefreshParticles = size_t(1) << 22;
 
 // A CUDA runtime failure inside the engine.
 struct CudaError : std::runtime_error
@@ -244,6 +249,9 @@ private:
     void binaryPass(bool buildMode, long long limit);
     void refreshAll();
     void refreshCounts(bool all, unsigned blocks);
+    void refreshUnits();
+    bool refreshByUnits() const;
+    void ensureUnits(size_t cap);
     void prepareGraphBuffers(size_t capacity);
     void ensurePhysical(size_t capacity);
     void buildViews(const adaptive_octree::ViewConfig &v);

@@ -70,7 +70,8 @@ struct Arena
 {
     u32 *rows;       // [cap][kRow]
     u32 *val;        // [cap][8] value of each child (NF or count)
-    u32 *child;      // [cap][8] unit index of an internal child, or kLeaf (LeafCount: by digit, NFCount: by octant)
+    u32 *child;      // [cap][8] unit index of an internal child, or kLeaf; units of a standing tree: a leaf's
+                     // index | kLeafRef (LeafCount: by digit, NFCount: by octant)
     u64 *sub;        // single tree: [cap] leaves counted below the unit | children to come << 56
     u32 *leaves;     // batch of trees: [cap] leaves in the unit's subtree
     u32 *offset;     // [cap] cornerstone index of the unit's first leaf (single tree: kPending before it is known)
@@ -410,6 +411,7 @@ struct RowScratch
     u64 pStart[rb::kUnitBatch];
     int childState[rb::kUnitBatch];
     rb::UnitBlocks block;
+    unsigned long long pop[rb::kUnitBatch];  // population of the 27 cells around the unit
     u32 slowRef[rb::kUnitBatch * 27];
     unsigned short slowItem[rb::kUnitBatch * 27];
     int nSlow;
@@ -484,10 +486,27 @@ __device__ __forceinline__ u64 rowRec(const u32 *row, const unsigned char *dec)
     return big ? kBigRec : rec;
 }
 
+// Where the near-field counts go.  Build: into the units' values.  Else (the
+// units of a standing tree) to the leaves, with the group flags.
+struct NearOut
+{
+    u32 *NF;
+    u8 *G;
+    unsigned bucket;
+};
+
+// May the 8 leaf children of a unit with `own` particles and `pop` in the 27
+// cells around it merge (computeGroupCanMergeKernel, octree_rebalance.cuh:636-700)?
+__device__ __forceinline__ u8 canMerge(u64 own, u64 pop, unsigned bucket)
+{
+    // (pop is below 27 x 2^32: only a product of 37 and 32 bits or more can pass 2^64)
+    return own == 0 || (pop <= u64(bucket) && own * pop <= u64(bucket)) ? 1 : 0;
+}
+
 // The units [first, first + nb) of level l by rows: any counts.
-template <bool Hilbert>
+template <bool Hilbert, bool Build>
 __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx, int l, u32 first, int nb, RowScratch &w,
-                                             const NearTables &t)
+                                             const NearTables &t, const NearOut &out)
 {
     const unsigned m = unsigned(l) + 1;
     const int lane = threadIdx.x & 31;
@@ -501,6 +520,7 @@ __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx
         w.childState[lane] = int(unitStateOf(row[11]));
     }
     if (lane == 0) w.nSlow = 0;
+    if (!Build && lane < nb) w.pop[lane] = 0;
     __syncwarp();
     // phase A: (unit, Q) pairs over the lanes; a Q that is a unit gives
     // its children's counts from its row
@@ -524,6 +544,7 @@ __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx
                 const uint4 r0 = vr[0], r1 = vr[1], r2 = vr[2];
                 const u32 gb[rb::kGroupBegins] = {r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z};
                 rb::childrenFromPacked<Hilbert>(gb, q, int(unitStateOf(r2.w)), w.block[u]);
+                if (!Build) atomicAdd(&w.pop[u], (unsigned long long)(gb[8] - gb[0]));
             }
         }
         const unsigned slowMask = __ballot_sync(0xffffffffu, slow);
@@ -550,6 +571,7 @@ __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx
         u32 begins[rb::kGroupBegins];
         rb::childBeginsWithin(idx.keys, lo, hi, qKey, m, begins);
         rb::childrenFromPacked<Hilbert>(begins, q, qState, w.block[u]);
+        if (!Build) atomicAdd(&w.pop[u], (unsigned long long)(begins[8] - begins[0]));
     }
     __syncwarp();
     // phase C: the 8 children of each unit, two per lane
@@ -559,10 +581,10 @@ __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx
         const u32 g = first + u32(u);
         const u32 *row = a.rows + size_t(g) * kRow;
         const u32 cnt = row[2 + d + 1] - row[2 + d];
-        u32 out = 0;
+        const unsigned o = Hilbert ? unsigned(t.dec[w.childState[u] * 8 + d]) : unsigned(d);
+        u32 nf = 0;
         if (cnt)
         {
-            const unsigned o = Hilbert ? unsigned(t.dec[w.childState[u] * 8 + d]) : unsigned(d);
             const u32 *sub = w.block[u] + (o >> 2) * 16 + ((o >> 1) & 1u) * 4 + (o & 1u);
             u64 pop = 0;
             if (m > 1)
@@ -584,9 +606,21 @@ __device__ __noinline__ void nearFieldByRows(const Arena &a, const KeyIndex &idx
                         for (int z = 0; z < 3; ++z) pop += sub[x * 16 + y * 4 + z];
             }
             const u64 v = u64(cnt) * pop;
-            out = v > 0xffffffffull ? 0xffffffffu : u32(v);
+            nf = v > 0xffffffffull ? 0xffffffffu : u32(v);
         }
-        a.val[size_t(g) * 8 + d] = out;
+        if constexpr (Build)
+        {
+            a.val[size_t(g) * 8 + d] = nf;
+        }
+        else
+        {
+            const u32 ch = a.child[size_t(g) * 8 + o];
+            if (ch & kLeafRef) out.NF[ch & ~kLeafRef] = nf;
+            // the 8 lanes of a unit together: all its children leaves?
+            const unsigned group = 0xffu << (lane & 24);
+            if (__all_sync(group, (ch & kLeafRef) != 0) && d == 0)
+                out.G[ch & ~kLeafRef] = canMerge(row[10] - row[2], w.pop[u], out.bucket);
+        }
     }
     __syncwarp();
 }
@@ -608,9 +642,11 @@ __device__ __forceinline__ u64 countedRec(const u64 *P, u32 lo, u32 hi, u64 qKey
     return rec;
 }
 
-template <bool Hilbert>
+// Build: the values of a build's units; else the near-field counts and group
+// flags of the leaves of a standing tree (treeUnitsKernel).
+template <bool Hilbert, bool Build>
 static __global__ void __launch_bounds__(kThreads, 4)
-    nearFieldKernel(Arena a, KeyIndex idx, int l)
+    nearFieldKernel(Arena a, KeyIndex idx, int l, rb::TreeBufs tb, unsigned bucket)
 {
     using rb::kUnitBatch;
     __shared__ NearTables t;
@@ -618,6 +654,12 @@ static __global__ void __launch_bounds__(kThreads, 4)
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     const u32 start = c.levelStart[l], count = c.levelCount[l];
+    NearOut out{};
+    if constexpr (!Build)
+    {
+        const int active = tb.st->activeBuffer;
+        out = {tb.nf(active), tb.g(active), bucket};
+    }
     if (count <= blockIdx.x) return;  // no units for this CTA
     if constexpr (Hilbert)
     {
@@ -670,11 +712,11 @@ static __global__ void __launch_bounds__(kThreads, 4)
             u32 ch[kRounds];
 #pragma unroll
             for (int i = 0; i < kRounds; ++i)
-                ch[i] = ref[i] & kLeafRef ? kLeaf : a.child[size_t(ref[i]) * 8 + oct[i]];
+                ch[i] = ref[i] & kLeafRef ? kLeaf : a.child[size_t(ref[i]) * 8 + oct[i]];  // (kLeafRef is set in kLeaf)
 #pragma unroll
             for (int i = 0; i < kRounds; ++i)
             {
-                if (!(ref[i] & kLeafRef)) ref[i] = ch[i] != kLeaf ? ch[i] : (kLeafRef | (ref[i] * 8 + oct[i]));
+                if (!(ref[i] & kLeafRef)) ref[i] = ch[i] & kLeafRef ? kLeafRef | (ref[i] * 8 + oct[i]) : ch[i];
                 const int it = i * 32 + lane;
                 if (it < items) a.nbr[size_t(first) * 27 + it] = ref[i];
             }
@@ -734,7 +776,7 @@ static __global__ void __launch_bounds__(kThreads, 4)
         __syncwarp();
         if (big)
         {
-            nearFieldByRows<Hilbert>(a, idx, l, first, nb, sWarp[threadIdx.x >> 5].rows, t);
+            nearFieldByRows<Hilbert, Build>(a, idx, l, first, nb, sWarp[threadIdx.x >> 5].rows, t, out);
             continue;
         }
         // Four lanes a unit: lane (x0, y0) sums the children (x0, y0, 0) and
@@ -767,17 +809,218 @@ static __global__ void __launch_bounds__(kThreads, 4)
             }
             const u32 own = words[2 * 13 + x0] >> (16 * y0);
             const u32 c0 = own & 0xffu, c1 = (own >> 8) & 0xffu;
-            u32 d0 = u32(x0 * 4 + y0 * 2), d1 = d0 + 1;
+            const u32 o0 = u32(x0 * 4 + y0 * 2);
+            u32 d0 = o0, d1 = o0 + 1;
             if constexpr (Hilbert)
             {
                 const u32 st = unitStateOf(a.rows[size_t(g) * kRow + 11]);
                 d0 = t.enc[st * 8 + d0];
                 d1 = t.enc[st * 8 + d1];
             }
-            a.val[size_t(g) * 8 + d0] = c0 * z0;  // at most 254 x 27 x 254
-            a.val[size_t(g) * 8 + d1] = c1 * z1;
+            // near-field counts: at most 254 x 27 x 254
+            if constexpr (Build)
+            {
+                a.val[size_t(g) * 8 + d0] = c0 * z0;
+                a.val[size_t(g) * 8 + d1] = c1 * z1;
+            }
+            else
+            {
+                const uint2 ch = *reinterpret_cast<const uint2 *>(a.child + size_t(g) * 8 + o0);
+                if (ch.x & kLeafRef) out.NF[ch.x & ~kLeafRef] = c0 * z0;
+                if (ch.y & kLeafRef) out.NF[ch.y & ~kLeafRef] = c1 * z1;
+                // a complete group's flag: the unit's particles and those of the 27 cells
+                const unsigned group = 0xfu << (lane & 28);
+                if (__all_sync(group, (ch.x & ch.y & kLeafRef) != 0))
+                {
+                    u32 pop = 0;
+                    for (int k = lane & 3; k < 54; k += 4) pop = __dp4a(words[k], 0x01010101u, pop);
+                    pop += __shfl_xor_sync(group, pop, 1);
+                    pop += __shfl_xor_sync(group, pop, 2);
+                    const u32 mine = __dp4a(words[27], 0x01010101u, __dp4a(words[26], 0x01010101u, 0u));
+                    if (d0 == 0 || d1 == 0)
+                        out.G[(d0 == 0 ? ch.x : ch.y) & ~kLeafRef] = canMerge(mine, pop, out.bucket);
+                }
+            }
         }
         __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The units of a standing NFCount tree (the full refresh of update()): its
+// internal nodes, level by level from the leaf boundaries K, with the begin
+// indices B of the moved particles.  A level is one kernel: a node's 7 inner
+// child boundaries are found among its leaves, a child of more than one leaf is
+// a unit of the next level.  The near field then goes over the units as in a
+// build.
+// ---------------------------------------------------------------------------
+// The root (a tree of one leaf is refreshed here).
+static __global__ void treeRootKernel(Arena a, rb::TreeBufs tb)
+{
+    const DeviceState *st = tb.st;
+    if (rb::halted(st)) return;  // no units: the levels find none
+    const int active = st->activeBuffer, L = st->numLeaves;
+    if (L > 1)
+    {
+        u32 *row = a.rows;
+        row[0] = row[1] = row[2] = 0;
+        row[3] = 0;
+        row[4] = u32(L);
+        row[10] = st->numActiveParticles;
+        row[11] = withUnit(0, 0, kHilbertStart);
+        for (int q = 0; q < 27; ++q) a.nbr[q] = 0;  // every cell around the root is the root (periodic wrap)
+        a.ctl->levelCount[0] = 1;
+        return;
+    }
+    const u64 c = st->numActiveParticles, v = c * c > 0xffffffffull ? 0xffffffffull : c * c * 27ull;
+    tb.nf(active)[0] = v > 0xffffffffull ? 0xffffffffu : u32(v);
+}
+
+// Levels of at most this many units: a CTA per unit, a warp per boundary.
+constexpr u32 kTreeWideUnits = 2048;
+
+// Child d of unit g: leaves [j, jEnd), keys [b, bEnd).  Slots of the warp's
+// new units by one atomic add.  All lanes of the warp take part (act: this
+// lane holds a child; the 8 children of a unit in the lanes of an aligned
+// group of 8).
+template <bool Hilbert>
+__device__ __forceinline__ void treeChild(const Arena &a, int l, u32 next, bool act, u32 g, int d, u64 key, u32 st, u32 j,
+                                          u32 jEnd, u32 b, u32 bEnd, const unsigned char *sNext, const unsigned char *sDec)
+{
+    Control &c = *a.ctl;
+    const int lane = threadIdx.x & 31;
+    const unsigned m = unsigned(l) + 1;
+    const bool inner = act && jEnd - j > 1;
+    const unsigned innerMask = __ballot_sync(0xffffffffu, inner);
+    u32 base = 0;
+    if (lane == 0 && innerMask) base = atomicAdd(&c.levelCount[l + 1], u32(__popc(innerMask)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const unsigned big = __ballot_sync(0xffffffffu, act && bEnd - b >= 255u) & (0xffu << (lane & 24));
+    if (!act) return;
+    const u32 oct = Hilbert ? u32(sDec[st * 8 + d]) : u32(d);
+    u32 slot = kLeafRef | j;
+    if (inner)
+    {
+        const u32 gc = next + base + u32(__popc(innerMask & ((1u << lane) - 1u)));
+        if (gc < a.cap)
+        {
+            const u64 ck = key + u64(d) * octRange(m);
+            const u32 cst = Hilbert ? u32(sNext[st * 8 + oct]) : u32(kHilbertStart);
+            uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
+            crow[0] = make_uint4(u32(ck), u32(ck >> 32), b, j);
+            crow[1] = make_uint4(jEnd, 0u, 0u, 0u);
+            crow[2] = make_uint4(0u, 0u, bEnd, withUnit(0, m, cst));
+            a.parent[gc] = g * 8 + oct;
+            slot = gc;
+        }
+        else
+        {
+            c.overflow = 1;
+        }
+    }
+    a.child[size_t(g) * 8 + oct] = slot;
+    a.rows[size_t(g) * kRow + 2 + d] = b;
+    reinterpret_cast<unsigned char *>(a.rec + g)[oct] = big ? 255 : (unsigned char)(bEnd - b);
+}
+
+template <bool Hilbert>
+static __global__ void __launch_bounds__(kThreads) treeUnitsKernel(Arena a, rb::TreeBufs tb, int l)
+{
+    __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
+    __shared__ u32 sCut[9];
+    Control &c = *a.ctl;
+    if (c.overflow) return;
+    const u32 start = c.levelStart[l], count = c.levelCount[l], next = start + count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.levelStart[l + 1] = next;
+    const bool wide = count <= kTreeWideUnits;
+    if (wide ? count <= blockIdx.x : count * 8 <= blockIdx.x * kThreads) return;
+    if constexpr (Hilbert)
+    {
+        copyTable(sNext, gHilbert.encNext);
+        copyTable(sDec, gHilbert.decOct);
+    }
+    __syncthreads();
+    const int active = tb.st->activeBuffer;
+    const u64 *K = tb.k(active);
+    const u32 *B = tb.b(active);
+    const u64 cr = octRange(unsigned(l) + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (wide)
+    {
+        for (u32 i = blockIdx.x; i < count; i += gridDim.x)
+        {
+            const u32 g = start + i;
+            const u32 *row = a.rows + size_t(g) * kRow;
+            const u64 key = rowKey(row);
+            const u32 i0 = row[3], i1 = row[4], st = unitStateOf(row[11]);
+            u32 cut = warp == 0 ? i0 : i1;
+            if (warp > 0) cut = warpLowerBound(K, i0, i1, key + u64(warp) * cr, lane);
+            if (lane == 0) sCut[warp] = cut;
+            if (threadIdx.x == 0) sCut[8] = i1;
+            __syncthreads();  // (row[3] and row[4] are read by every warp)
+            if (warp == 0)
+            {
+                const bool act = lane < 8;
+                const u32 j = sCut[act ? lane : 8], jEnd = sCut[act ? lane + 1 : 8];
+                treeChild<Hilbert>(a, l, next, act, g, lane & 7, key, st, j, jEnd, B[j], B[jEnd], sNext, sDec);
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const u32 total = count * 8;
+    for (u32 e0 = blockIdx.x * kThreads + (threadIdx.x & ~31u); e0 < total; e0 += gridDim.x * kThreads)
+    {
+        const u32 e = e0 + u32(lane);
+        const bool act = e < total;
+        const int d = int(e & 7);
+        const u32 g = start + (act ? e >> 3 : 0);
+        const u32 *row = a.rows + size_t(g) * kRow;
+        const u64 key = rowKey(row);
+        const u32 i0 = row[3], i1 = row[4], bEnd = row[10], st = unitStateOf(row[11]);
+        // first leaf of child d
+        u32 j = i0;
+        if (d > 0)
+        {
+            const u64 t = key + u64(d) * cr;
+            u32 len = i1 - i0;
+            while (len)
+            {
+                const u32 half = len >> 1;
+                const bool less = __ldg(K + j + half) < t;
+                j = less ? j + half + 1 : j;
+                len = less ? len - half - 1 : half;
+            }
+        }
+        const u32 b = B[j];
+        __syncwarp();  // the group's lanes have read row[3] and row[4]
+        u32 jEnd = __shfl_down_sync(0xffffffffu, j, 1, 8), bNext = __shfl_down_sync(0xffffffffu, b, 1, 8);
+        if (d == 7)
+        {
+            jEnd = i1;
+            bNext = bEnd;
+        }
+        treeChild<Hilbert>(a, l, next, act, g, d, key, st, j, jEnd, b, bNext, sNext, sDec);
+    }
+}
+
+// Every unit into the (cleared) node table of the partial refreshes.
+static __global__ void __launch_bounds__(kThreads) unitsToTableKernel(Arena a, rb::NodeTable gt)
+{
+    const Control &c = *a.ctl;
+    if (c.overflow) return;
+    const u32 total = c.levelStart[kOctLevels];
+    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
+    {
+        const uint4 *r4 = reinterpret_cast<const uint4 *>(a.rows + size_t(g) * kRow);
+        const uint4 r0 = r4[0], r1 = r4[1], r2 = r4[2];
+        u32 *to = rb::nodeRow(gt, rb::cellCode((u64(r0.y) << 32) | r0.x, unitLevelOf(r2.w)));
+        if (!to) continue;
+        // (rows are 48 bytes: the two words of the code, then the 9 values)
+        *reinterpret_cast<uint2 *>(to) = make_uint2(r0.z, r0.w);
+        *reinterpret_cast<uint4 *>(to + 2) = r1;
+        *reinterpret_cast<uint2 *>(to + 6) = make_uint2(r2.x, r2.y);
+        to[8] = r2.z;
     }
 }
 
