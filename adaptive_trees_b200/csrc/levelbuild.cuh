@@ -444,14 +444,25 @@ __device__ __forceinline__ void leafCell(const Arena &a, const NearTables &t, u3
 {
     const u32 o = ref & 7u;
     const u32 *row = a.rows + size_t(ref >> 3) * kRow;
-    const u32 reg = row[11], st = unitStateOf(reg);
+    // the whole row at once: its words one after the other were three round
+    // trips (with four keys in flight in countedRec: 16Mi near field 586 to 542 us)
+    const uint4 *r4 = reinterpret_cast<const uint4 *>(row);
+    const uint4 r0 = r4[0], r1 = r4[1], r2 = r4[2];
+    const u32 reg = r2.w, st = unitStateOf(reg);
     const u32 d = Hilbert ? u32(t.enc[st * 8 + o]) : o;
-    lo = row[2 + d];
-    hi = row[3 + d];
+    const u32 b[rb::kGroupBegins] = {r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z};
+    lo = b[0];
+    hi = b[1];
+#pragma unroll
+    for (u32 k = 1; k < 8; ++k)
+    {
+        lo = d == k ? b[k] : lo;
+        hi = d == k ? b[k + 1] : hi;
+    }
     if (unitLevelOf(reg) + 1 == unsigned(l))
     {
         // the leaf is the cell itself: child o of its parent unit
-        qKey = rowKey(row) + u64(d) * octRange(unsigned(l));
+        qKey = ((u64(r0.y) << 32) | r0.x) + u64(d) * octRange(unsigned(l));
         qState = Hilbert ? int(t.next[st * 8 + o]) : kHilbertStart;
     }
     else if (lo < hi)
@@ -634,10 +645,17 @@ __device__ __forceinline__ u64 countedRec(const u64 *P, u32 lo, u32 hi, u64 qKey
     if (hi - lo >= 255u) return kBigRec;
     const unsigned shift = 3u * (kOctLevels - unsigned(l) - 1);
     u64 rec = 0;
-    for (u32 k = lo; k < hi; ++k)
+    for (u32 k = lo; k < hi; k += 4)  // four keys in flight
     {
-        const u64 d = (__ldg(P + k) - qKey) >> shift;  // 8 or more: outside the cell
-        if (d < 8) rec += u64(1) << (8 * (Hilbert ? unsigned(dec[qState * 8 + int(d)]) : unsigned(d)));
+        u64 key[4];
+#pragma unroll
+        for (u32 i = 0; i < 4; ++i) key[i] = __ldg(P + min(k + i, hi - 1));
+#pragma unroll
+        for (u32 i = 0; i < 4; ++i)
+        {
+            const u64 d = (key[i] - qKey) >> shift;  // 8 or more: outside the cell
+            if (k + i < hi && d < 8) rec += u64(1) << (8 * (Hilbert ? unsigned(dec[qState * 8 + int(d)]) : unsigned(d)));
+        }
     }
     return rec;
 }
