@@ -955,7 +955,7 @@ struct TreeEngine::Impl
             t.G[k] = G[k].as<u8>();
             t.N[k] = N[k].as<u32>();
         }
-        t.offs = offs.as<i64>();
+        t.offs = offs.as<u32>();
         t.dirty = dirty.as<int>();
         t.scanStatus = scan.as<u64>();
         t.scanTile = reinterpret_cast<u32 *>(scan.as<u64>() + scanTiles);
@@ -1146,7 +1146,7 @@ void TreeEngine::ensurePhysical(size_t capacity)
             m_->G[k].grow(16, m_->G[k].bytes, s);
         }
     }
-    m_->offs.reserve((c + 1) * sizeof(i64), s);
+    m_->offs.reserve((c + 1) * sizeof(u32), s);
     m_->dirty.reserve((c + 1) * sizeof(int), s);
     // the merge-path cuts of the full begin refresh (reserved here: an update
     // may run under stream capture, where nothing may be allocated)

@@ -514,7 +514,11 @@ static __global__ void __launch_bounds__(rb::kScanThreads) scanKernel(Bufs f)
     }
     i64 total;
     const i64 excl = rb::blockExclusiveScan(sum, sWarp, total);
-    if (threadIdx.x == 0) sPrefix = rb::lookback(f.scanStatus, tile, total, &st->error);
+    if (threadIdx.x < 32)
+    {
+        const i64 prefix = rb::lookback(f.scanStatus, tile, total, &st->error);
+        if (threadIdx.x == 0) sPrefix = prefix;
+    }
     __syncthreads();
     i64 run = sPrefix + excl;
 #pragma unroll

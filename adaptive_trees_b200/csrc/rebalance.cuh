@@ -43,7 +43,7 @@ struct TreeBufs
     u32 *NF[2];   // near-field counts (NFCount octrees)
     u8 *G[2];     // group-can-merge flag at each complete group's first leaf
     u32 *N[2];    // leaf counts, materialised for getters and views
-    i64 *offs;    // decision scan, capacity + 1
+    u32 *offs;    // decision scan (mod 2^32: an accepted proposal is smaller), capacity + 1
     int *dirty;   // new leaves that need a search (and NF)
     u64 *scanStatus;
     u32 *scanTile;
@@ -98,65 +98,78 @@ __device__ __forceinline__ i64 blockExclusiveScan(i64 v, i64 *sWarp, i64 &total)
     return wOff + inc - v;
 }
 
-// Decoupled look-back: returns the exclusive prefix of `tile` given its
-// aggregate.  Called by one thread.  Polling an unpublished tile more than
+// Decoupled look-back by one warp: returns the exclusive prefix of `tile`
+// given its aggregate, to every lane.  A lane per earlier tile, 32 a round
+// trip: a thread that walked 8 at a time made the 6,200 tiles of a 12.7 M leaf
+// scan wait 31 ns each for their turn.  Polling unpublished tiles more than
 // spinLimit times records kErrLookback and returns the prefix summed so far.
 __device__ __forceinline__ i64 lookback(u64 *status, u32 tile, i64 aggregate, int *error,
                                         unsigned spinLimit = kLookbackSpins)
 {
-    if (tile == 0)
-    {
-        stRelaxed(status, kFlagPrefix | u64(aggregate));
-        return 0;
-    }
-    stRelaxed(status + tile, kFlagAgg | u64(aggregate));
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) stRelaxed(status + tile, (tile == 0 ? kFlagPrefix : kFlagAgg) | u64(aggregate));
+    if (tile == 0) return 0;
     i64 excl = 0;
     long long j = (long long)tile - 1;
     unsigned spins = 0;
-    while (j >= 0)
+    for (;;)
     {
-        u64 v[8];
+        const u64 v = j - lane >= 0 ? ldRelaxed(status + (j - lane)) : kFlagPrefix;
+        const unsigned open = __ballot_sync(0xffffffffu, (v & ~kValueMask) == 0);  // not published
+        const unsigned whole = __ballot_sync(0xffffffffu, (v & ~kValueMask) == kFlagPrefix);
+        const int ready = open ? __ffs(int(open)) - 1 : 32;
+        const int last = whole ? __ffs(int(whole)) - 1 : 32;  // the nearest inclusive prefix
+        const bool done = last < ready;
+        i64 part = lane < (done ? last + 1 : ready) ? i64(v & kValueMask) : 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = j - k >= 0 ? ldRelaxed(status + (j - k)) : kFlagPrefix;
-        int k = 0;
-        bool done = false;
-        for (; k < 8; ++k)
-        {
-            const u64 flag = v[k] & ~kValueMask;
-            if (flag == 0) break;
-            excl += i64(v[k] & kValueMask);
-            if (flag == kFlagPrefix)
-            {
-                done = true;
-                break;
-            }
-        }
+        for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+        excl += part;
         if (done) break;
-        j -= k;
-        if (k < 8)
+        j -= ready;
+        if (ready < 32)
         {
             if (++spins > spinLimit)
             {
-                atomicExch(error, kErrLookback);
+                if (lane == 0) atomicExch(error, kErrLookback);
                 break;
             }
             if (spins > 64) __nanosleep(64);
         }
     }
-    stRelaxed(status + tile, kFlagPrefix | u64(excl + aggregate));
+    if (lane == 0) stRelaxed(status + tile, kFlagPrefix | u64(excl + aggregate));
     return excl;
 }
 
-// Generic single-pass decide+scan.  OpFn(i, L) returns the op code of leaf
-// i < L; entry L is 0.  Writes offs[0..L] (exclusive), state->proposal and
-// state->changed.
-template <class OpFn>
-__device__ void decideScan(const OpFn &opOf, TreeBufs tb)
+// Generic single-pass decide+scan.  Op::code returns the op code of leaf i < L
+// from the tile's leaf boundaries K, values V (begin indices or near-field
+// counts) and group flags in shared memory, of which it looks at Op::kBack
+// before to Op::kAhead behind the leaf; entry L is 0.  Writes offs[0..L]
+// (exclusive), state->proposal and state->changed.
+//
+// Bound by the latency of its loads (DRAM 12 % busy), so the tile is loaded
+// once, coalesced, with a thread's nine positions in flight together, and
+// leaves are taken by neighbouring lanes.  A thread that read its own 8 leaves
+// and their siblings from global memory took 205 us for the 12.7 M leaves of a
+// 16Mi Plummer NFCount tree and 13.5 us for an 8Mi k-d tree's 400 k; now 111
+// and 9.9 us.
+template <class Op>
+struct DecideShared
 {
-    __shared__ i64 sWarp[kScanThreads / 32];
-    __shared__ u32 sTile;
-    __shared__ i64 sPrefix;
-    __shared__ int sChanged;
+    static constexpr int kWindow = kScanTile + Op::kBack + Op::kAhead;
+    u64 K[kWindow];
+    u32 V[kWindow];
+    u8 G[Op::kFlags ? kWindow : 1];
+    __align__(16) unsigned short op[kScanTile];
+    i64 warp[kScanThreads / 32];
+    i64 prefix;
+    u32 tile;
+    int changed;
+};
+
+template <class Op>
+__device__ void decideScan(const Op &op, TreeBufs tb, const u64 *K, const u32 *V, const u8 *G)
+{
+    __shared__ DecideShared<Op> sm;
     DeviceState *st = tb.st;
     if (halted(st) || st->needsResize) return;
     const int L = st->numLeaves;
@@ -164,49 +177,95 @@ __device__ void decideScan(const OpFn &opOf, TreeBufs tb)
     const u32 numTiles = u32((entries + kScanTile - 1) / kScanTile);
     if (threadIdx.x == 0)
     {
-        sTile = atomicAdd(tb.scanTile, 1u);
-        sChanged = 0;
+        sm.tile = atomicAdd(tb.scanTile, 1u);
+        sm.changed = 0;
     }
     __syncthreads();
-    const u32 tile = sTile;
+    const u32 tile = sm.tile;
     if (tile >= numTiles) return;
-    const size_t first = size_t(tile) * kScanTile + size_t(threadIdx.x) * kScanItems;
-    int ops[kScanItems];
-    i64 sum = 0;
+    const long long base = (long long)tile * kScanTile, origin = base - Op::kBack;  // leaf of window position 0
+    {
+        // all loads in flight together (positions outside the tree repeat its ends)
+        constexpr int kRounds = (DecideShared<Op>::kWindow + kScanThreads - 1) / kScanThreads;
+        u64 k[kRounds];
+        u32 v[kRounds];
+        u8 f[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r)
+        {
+            const long long i = origin + int(threadIdx.x) + r * kScanThreads;
+            const int at = i < 0 ? 0 : i > L ? L : int(i);
+            k[r] = __ldg(K + at);
+            v[r] = __ldg(V + at);
+            if constexpr (Op::kFlags) f[r] = __ldg(G + at);
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r)
+        {
+            const int w = int(threadIdx.x) + r * kScanThreads;
+            if (w >= DecideShared<Op>::kWindow) continue;
+            sm.K[w] = k[r];
+            sm.V[w] = v[r];
+            if constexpr (Op::kFlags) sm.G[w] = f[r];
+        }
+    }
+    __syncthreads();
     bool changed = false;
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j)
     {
-        const size_t i = first + j;
-        int op = 0;
-        if (i < size_t(L))
+        const int t = int(threadIdx.x) + j * kScanThreads;
+        const long long i = base + t;
+        int code = 0;
+        if (i < L)
         {
-            op = opOf(int(i), L);
-            changed |= op != 1;
+            // (arrays indexed by leaf: position 0 of the window is leaf `origin`)
+            code = op.code(sm.K - origin, sm.V - origin, sm.G - (Op::kFlags ? origin : 0), int(i), L);
+            changed |= code != 1;
         }
-        ops[j] = op;
-        sum += op;
+        sm.op[t] = (unsigned short)code;
     }
-    if (changed) sChanged = 1;
+    if (changed) sm.changed = 1;
+    __syncthreads();
+    const uint4 packed = *reinterpret_cast<const uint4 *>(sm.op + threadIdx.x * kScanItems);
+    const u32 words[4] = {packed.x, packed.y, packed.z, packed.w};
+    static_assert(kScanItems == 8, "eight op codes per thread");
+    i64 sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += i64((words[j] & 0xffffu) + (words[j] >> 16));
     i64 total;
-    const i64 excl = blockExclusiveScan(sum, sWarp, total);
-    if (threadIdx.x == 0)
+    const i64 excl = blockExclusiveScan(sum, sm.warp, total);
+    if (threadIdx.x < 32)
     {
-        sPrefix = lookback(tb.scanStatus, tile, total, &st->error);
-        if (sChanged) atomicOr(&st->changed, 1);
+        const i64 prefix = lookback(tb.scanStatus, tile, total, &st->error);
+        if (threadIdx.x == 0)
+        {
+            sm.prefix = prefix;
+            if (sm.changed) atomicOr(&st->changed, 1);
+        }
     }
     __syncthreads();
-    i64 run = sPrefix + excl;
+    i64 run = sm.prefix + excl;
+    const long long first = base + (long long)threadIdx.x * kScanItems;
+    u32 out[kScanItems];
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j)
     {
-        const size_t i = first + j;
-        if (i <= size_t(L))
-        {
-            tb.offs[i] = run;
-            if (i == size_t(L)) st->proposal = run;
-        }
-        run += ops[j];
+        out[j] = u32(run);
+        if (first + j == L) st->proposal = run;
+        run += (words[j >> 1] >> (16 * (j & 1))) & 0xffffu;
+    }
+    if (first + kScanItems - 1 <= L)
+    {
+        uint4 *o = reinterpret_cast<uint4 *>(tb.offs + first);
+        o[0] = make_uint4(out[0], out[1], out[2], out[3]);
+        o[1] = make_uint4(out[4], out[5], out[6], out[7]);
+    }
+    else
+    {
+#pragma unroll
+        for (int j = 0; j < kScanItems; ++j)
+            if (first + j <= L) tb.offs[first + j] = out[j];
     }
 }
 
@@ -313,12 +372,11 @@ __device__ __forceinline__ int siblingIndex(const u64 *K, int L, int i, unsigned
 template <bool NF>
 struct OctreeOp
 {
-    const u64 *K;
-    const u32 *B;
-    const u32 *NFc;
-    const u8 *G;
+    static constexpr int kBack = 7, kAhead = 8;  // a leaf's sibling group and its end
+    static constexpr bool kFlags = NF;
     unsigned bucket;
-    __device__ __forceinline__ int operator()(int i, int L) const
+    // V: begin indices, or near-field counts (NF)
+    __device__ __forceinline__ int code(const u64 *K, const u32 *V, const u8 *G, int i, int L) const
     {
         unsigned level = 0;
         const int sib = siblingIndex(K, L, i, level);
@@ -327,10 +385,10 @@ struct OctreeOp
             if (sib > 0)
             {
                 const int first = i - sib;
-                const u64 parent = u64(B[first + 8] - B[first]);
+                const u64 parent = u64(V[first + 8] - V[first]);
                 if (parent <= u64(bucket)) return 0;
             }
-            const u32 c = B[i + 1] - B[i];
+            const u32 c = V[i + 1] - V[i];
             if (c > bucket * 512u && level + 3 < kOctLevels) return 4096;
             if (c > bucket * 64u && level + 2 < kOctLevels) return 512;
             if (c > bucket * 8u && level + 1 < kOctLevels) return 64;
@@ -344,7 +402,7 @@ struct OctreeOp
                 const int first = i - sib;
                 if (first + 8 <= L && G[first]) return sib == 0 ? 1 : 0;
             }
-            const u64 c = NFc[i], b = bucket;
+            const u64 c = V[i], b = bucket;
             if (c > b * 262144 && level + 3 < kOctLevels) return 4096;
             if (c > b * 4096 && level + 2 < kOctLevels) return 512;
             if (c > b * 64 && level + 1 < kOctLevels) return 64;
@@ -358,11 +416,11 @@ template <bool NF>
 static __global__ void __launch_bounds__(kScanThreads) octDecideScanKernel(TreeBufs tb, unsigned bucket)
 {
     const int a = tb.st->activeBuffer;
-    const OctreeOp<NF> op{tb.k(a), tb.b(a), tb.nf(a), tb.g(a), bucket};
-    decideScan(op, tb);
+    const OctreeOp<NF> op{bucket};
+    decideScan(op, tb, tb.k(a), NF ? tb.nf(a) : tb.b(a), tb.g(a));
 }
 
-__device__ __forceinline__ int opAt(const i64 *offs, int i) { return int(offs[i + 1] - offs[i]); }
+__device__ __forceinline__ int opAt(const u32 *offs, int i) { return int(offs[i + 1] - offs[i]); }
 
 // log8ceil of a split op code (octree_rebalance.cuh:349): 8->1, 64->2, 512->3, 4096->4
 __device__ __forceinline__ unsigned splitLevels(int op) { return op == 8 ? 1u : op == 64 ? 2u : op == 512 ? 3u : 4u; }
@@ -381,39 +439,49 @@ __device__ __forceinline__ void octScatterLeaf(const TreeBufs &tb, DeviceState *
     u64 *Kn = tb.k(b);
     if (i < L)
     {
+        // everything a kept leaf needs, in flight together (most leaves are kept)
         const u64 *K = tb.k(a);
-        const i64 *offs = tb.offs;
-        op = opAt(offs, i);
+        const u32 *offs = tb.offs;
+        const u32 o0 = offs[i], o1 = offs[i + 1], o2 = offs[i + 1 < L ? i + 2 : i + 1];
         start = K[i];
-        const unsigned level = octLevel(K[i + 1] - start);
-        ni = offs[i];
+        const u64 end = K[i + 1];
+        const u32 begin = tb.b(a)[i];
+        u32 nf = 0;
+        u8 flag = 0;
+        if constexpr (NF)
+        {
+            nf = tb.nf(a)[i];
+            flag = tb.g(a)[i];
+        }
+        op = int(o1 - o0);
+        ni = o0;
         u32 *Bn = tb.b(b);
         if (op == 1)
         {
             Kn[ni] = start;
-            Bn[ni] = tb.b(a)[i];
+            Bn[ni] = begin;
             if constexpr (NF)
             {
                 // a merge leader becomes a new leaf; a kept leaf keeps its NF
                 // and its group flag (both depend on the particles only; a
                 // group completed in this pass holds a new leaf, and the
                 // refresh of that leaf's parent rewrites the flag)
-                const bool leader = i + 1 < L && opAt(offs, i + 1) == 0;
+                const bool leader = i + 1 < L && o2 == o1;
                 if (leader)
                 {
                     nDirty = 1;
                 }
                 else
                 {
-                    tb.nf(b)[ni] = tb.nf(a)[i];
-                    tb.g(b)[ni] = tb.g(a)[i];
+                    tb.nf(b)[ni] = nf;
+                    tb.g(b)[ni] = flag;
                 }
             }
         }
         else if (op > 1)
         {
-            nr = octRange(level + splitLevels(op));
-            Bn[ni] = tb.b(a)[i];  // the first child starts where the parent did
+            nr = octRange(octLevel(end - start) + splitLevels(op));
+            Bn[ni] = begin;  // the first child starts where the parent did
             nDirty = NF ? op : op - 1;
         }
         if (i == 0)
@@ -422,6 +490,7 @@ __device__ __forceinline__ void octScatterLeaf(const TreeBufs &tb, DeviceState *
             tb.b(b)[total] = st->numActiveParticles;
         }
     }
+    if (!__any_sync(0xffffffffu, nDirty != 0)) return;  // 32 leaves that stay or go
     // work lists (warp-aggregated appends; list order is irrelevant)
     const int d0 = warpAppend(&st->dirtyCount, nDirty);
     if (nDirty && op == 1) tb.dirty[d0] = int(ni);
@@ -468,7 +537,10 @@ __device__ __forceinline__ void octScatterLeaf(const TreeBufs &tb, DeviceState *
 // work lists of the refresh: new leaves needing a search (and NF) and
 // candidate group leaders needing a parent NF.  Persistent grid: each warp
 // strides over the leaves 32 at a time, so every lane takes part in the
-// warp-aggregated appends.
+// warp-aggregated appends.  Bound by the latency of its loads: all that a kept
+// leaf (nearly every one) needs is loaded before the op code is known, and a
+// warp of kept leaves is done then; loads behind the op code and the flag took
+// 127 instead of 92 us for 12.7 M leaves.
 template <bool NF>
 static __global__ void __launch_bounds__(kScatterThreads)
     octScatterKernel(TreeBufs tb, long long limit, int mode, long long *history)
@@ -1265,19 +1337,19 @@ static __global__ void materializeCountsKernel(TreeBufs tb)
 // --------------------------------------------------------------------------
 struct BinaryOp
 {
-    const u64 *K;
-    const u32 *B;
+    static constexpr int kBack = 1, kAhead = 2;  // a leaf's possible siblings and their end
+    static constexpr bool kFlags = false;
     unsigned bucket, maxDepth;
-    __device__ __forceinline__ bool siblings(int L, int first) const  // binarySiblings, binary_node.cuh:91-98
+    __device__ __forceinline__ bool siblings(const u64 *K, int L, int first) const  // binarySiblings, binary_node.cuh:91-98
     {
         if (first < 0 || first + 1 >= L) return false;
         const u64 r = K[first + 1] - K[first];
         return !(K[first] & r) && K[first + 2] - K[first + 1] == r;
     }
-    __device__ __forceinline__ int operator()(int i, int L) const
+    __device__ __forceinline__ int code(const u64 *K, const u32 *B, const u8 *, int i, int L) const
     {
         const u32 ci = B[i + 1] - B[i];
-        const bool merge = i && siblings(L, i - 1) && u64(B[i] - B[i - 1]) + ci <= bucket;
+        const bool merge = i && siblings(K, L, i - 1) && u64(B[i] - B[i - 1]) + ci <= bucket;
         if (merge) return 0;
         return (ci > bucket && unsigned(clz64(K[i + 1] - K[i])) < maxDepth) ? 2 : 1;
     }
@@ -1286,8 +1358,8 @@ struct BinaryOp
 static __global__ void __launch_bounds__(kScanThreads) binDecideScanKernel(TreeBufs tb, unsigned bucket, unsigned maxDepth)
 {
     const int a = tb.st->activeBuffer;
-    const BinaryOp op{tb.k(a), tb.b(a), bucket, maxDepth};
-    decideScan(op, tb);
+    const BinaryOp op{bucket, maxDepth};
+    decideScan(op, tb, tb.k(a), tb.b(a), static_cast<const u8 *>(nullptr));
 }
 
 static __global__ void __launch_bounds__(kScatterThreads)

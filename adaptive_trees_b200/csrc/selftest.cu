@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(sort::kThreads, 1)
 
 __global__ void scanWaitProbeKernel(u64 *status, int *error, unsigned spinLimit, i64 *prefix)
 {
-    if (threadIdx.x == 0) prefix[blockIdx.x] = rb::lookback(status, blockIdx.x + 1, 1, error, spinLimit);
+    const i64 p = rb::lookback(status, blockIdx.x + 1, 1, error, spinLimit);
+    if (threadIdx.x == 0) prefix[blockIdx.x] = p;
 }
 
 // Device allocations of the probe, freed on every exit path.
