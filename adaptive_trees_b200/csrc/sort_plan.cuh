@@ -33,9 +33,11 @@ constexpr int kPlanSets = kPlanMaxPasses - kPlanMinPasses + 2;  // a set of pref
 // 4.7 and 14.4 keys took 116, 130 and 272 us.
 constexpr float kRepairCost = 0.55f;
 constexpr float kRunCost = 0.11f;
-// mean run of equal keys above which all passes run (a long run is a CTA's
-// work in the repair)
-constexpr float kMaxRepeats = 64.f;
+// Mean run of equal keys above which all passes run: they share their run with
+// keys that are not equal, and a long run is a CTA's work in the repair.  In
+// the sample a single stack of equal keys shows by its share of them, so this
+// is 32 of M sampled keys: 0.4 % of 16Mi keys, 4 % of 130k.
+constexpr float kMaxRepeats = 16.f;
 
 // splitmix64's finaliser
 __host__ __device__ __forceinline__ u64 mix64(u64 x)

@@ -278,16 +278,21 @@ struct LongShared
 {
     u32 start[kRadix];
     u32 warp[Threads / 32][kRadix];
-    u32 end, same;
+    u32 end;
+    u32 differ;  // digits in which the run's keys differ
 };
 
 // A long run per CTA: an LSD radix sort of its remaining digits between its
 // stretch of buffer 0 and the same stretch of buffer 1.  Digits all keys
-// share are left out.
+// share are left out: the run is read once, eight keys of a thread in flight,
+// to find them, and a run of equal keys is done then.  A run of 27k keys, most
+// of them equal, took 267 us with a digit counted to see that it is shared and
+// a key per thread and step; 17k such keys take 122 now, 50k 327.
 template <int Threads>
 __device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Threads> &sm, int first, u32 runs)
 {
     constexpr int W = Threads / 32;
+    constexpr int kLongItems = Threads == kLongThreads ? 4 : 2;  // keys per thread and step (2: no spills in the forest's sort)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int prefix = a.beginBit + first * kRadixBits;
     for (u32 r = blockIdx.x; r < runs; r += gridDim.x)
@@ -309,32 +314,53 @@ __device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Thr
                 if (c > 0) lo = pLow + 1;
                 if (c < 32) hi = pHigh;
             }
-            if (lane == 0) sm.end = lo;
+            if (lane == 0)
+            {
+                sm.end = lo;
+                sm.differ = 0;
+            }
         }
         __syncthreads();
         const u32 e = sm.end;
+        {
+            const u64 head = a.k[0][h];
+            u64 diff = 0;
+            for (u32 i = h + tid; i < e; i += 8 * Threads)
+            {
+                u64 k[8];
+#pragma unroll
+                for (u32 q = 0; q < 8; ++q) k[q] = a.k[0][min(i + q * Threads, e - 1)];
+#pragma unroll
+                for (u32 q = 0; q < 8; ++q) diff |= k[q] ^ head;
+            }
+            u32 digits = 0;
+            for (int d = 0; d < first; ++d)
+                if (((diff & a.keyMask) >> (a.beginBit + d * kRadixBits)) & (kRadix - 1)) digits |= 1u << d;
+            if (digits) atomicOr(&sm.differ, digits);
+        }
+        __syncthreads();
+        const u32 differ = sm.differ;
         int at = 0;  // buffer that holds the run
         for (int d = 0; d < first; ++d)
         {
+            if (!(differ & (1u << d))) continue;
             const int shift = a.beginBit + d * kRadixBits;
             const u64 *in = at ? a.k[1] : a.k[0];
             const u32 *inV = at ? a.v[1] : a.v[0];
             u64 *out = at ? a.k[0] : a.k[1];
             u32 *outV = at ? a.v[0] : a.v[1];
             if (tid < kRadix) sm.start[tid] = 0;
-            if (tid == 0) sm.same = 0;
             __syncthreads();
-            for (u32 i = h + tid; i < e; i += Threads)
-                atomicAdd(&sm.start[unsigned(in[i] >> shift) & (kRadix - 1)], 1u);
-            __syncthreads();
-            if (tid < kRadix && sm.start[tid] == e - h) sm.same = 1;
-            __syncthreads();
-            const bool same = sm.same != 0;
-            if (same)
+            for (u32 i = h + tid; i < e; i += 4 * Threads)
             {
-                __syncthreads();
-                continue;
+                u64 k[4];
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q) k[q] = in[min(i + q * Threads, e - 1)];
+#pragma unroll
+                for (u32 q = 0; q < 4; ++q)
+                    if (i + q * Threads < e) atomicAdd(&sm.start[unsigned(k[q] >> shift) & (kRadix - 1)], 1u);
             }
+            __syncthreads();
             if (warp == 0)
             {
                 // exclusive scan of the counts, eight per lane
@@ -360,19 +386,34 @@ __device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Thr
                     run += c[k];
                 }
             }
-            for (u32 i0 = h; i0 < e; i0 += Threads)
+            // tiles of kLongItems keys per thread, a warp's 32 x kLongItems in a row
+            for (u32 i0 = h; i0 < e; i0 += Threads * kLongItems)
             {
                 for (int k = tid; k < W * kRadix; k += Threads) (&sm.warp[0][0])[k] = 0;
+                u64 key[kLongItems];
+                u32 val[kLongItems], rank[kLongItems];
+                const u32 w0 = i0 + u32(warp) * 32 * kLongItems + lane;
+#pragma unroll
+                for (int q = 0; q < kLongItems; ++q)
+                {
+                    const u32 i = min(w0 + q * 32, e - 1);
+                    key[q] = in[i];
+                    val[q] = inV[i];
+                }
                 __syncthreads();
-                const u32 i = i0 + tid;
-                const bool valid = i < e;
-                const u64 key = valid ? in[i] : 0;
-                const u32 val = valid ? inV[i] : 0;
-                const unsigned digit = unsigned(key >> shift) & (kRadix - 1);
-                const unsigned validMask = __ballot_sync(0xffffffffu, valid);
-                const unsigned peers = peerLanes<kRadixBits>(digit) & validMask;
-                const unsigned rank = __popc(peers & laneMaskLt());
-                if (valid && rank == 0) sm.warp[warp][digit] = __popc(peers);
+#pragma unroll
+                for (int q = 0; q < kLongItems; ++q)
+                {
+                    const unsigned digit = unsigned(key[q] >> shift) & (kRadix - 1);
+                    const unsigned validMask = __ballot_sync(0xffffffffu, w0 + q * 32 < e);
+                    const unsigned peers = peerLanes<kRadixBits>(digit) & validMask;
+                    const u32 before = sm.warp[warp][digit];
+                    const unsigned under = __popc(peers & laneMaskLt());
+                    rank[q] = before + under;
+                    __syncwarp();
+                    if ((validMask >> lane & 1u) && under == 0) sm.warp[warp][digit] = before + __popc(peers);
+                    __syncwarp();
+                }
                 __syncthreads();
                 if (tid < kRadix)
                 {
@@ -387,31 +428,33 @@ __device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Thr
                     sm.start[tid] = acc;
                 }
                 __syncthreads();
-                if (valid)
+#pragma unroll
+                for (int q = 0; q < kLongItems; ++q)
                 {
-                    const u32 to = sm.warp[warp][digit] + rank;
-                    out[to] = key;
-                    outV[to] = val;
+                    if (w0 + q * 32 >= e) break;
+                    const u32 to = sm.warp[warp][unsigned(key[q] >> shift) & (kRadix - 1)] + rank[q];
+                    out[to] = key[q];
+                    outV[to] = val[q];
                 }
                 __syncthreads();
             }
             at ^= 1;
         }
         __syncthreads();
-        for (u32 i = h + tid; i < e; i += Threads)
+        if (at)
         {
-            u64 key;
-            if (at)
+            for (u32 i = h + tid; i < e; i += Threads)
             {
-                key = a.k[1][i];
+                const u64 key = a.k[1][i];
                 a.k[0][i] = key;
                 a.v[0][i] = a.v[1][i];
+                if (a.sample && (i & (kSampleStride - 1)) == 0) a.sample[i >> kSampleShift] = key;
             }
-            else
-            {
-                key = a.k[0][i];
-            }
-            if (a.sample && (i & (kSampleStride - 1)) == 0) a.sample[i >> kSampleShift] = key;
+        }
+        else if (a.sample)
+        {
+            for (u32 j = ((h + kSampleStride - 1) >> kSampleShift) + tid; (j << kSampleShift) < e; j += Threads)
+                a.sample[j] = a.k[0][j << kSampleShift];
         }
         __syncthreads();
     }

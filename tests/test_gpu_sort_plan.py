@@ -63,6 +63,8 @@ CASES = {
     "run of 200": with_cluster(300_000, 200, 1e-9, 12), "run of 256": with_cluster(300_000, RUN, 1e-9, 13),
     "run of 257": with_cluster(300_000, RUN + 1, 1e-9, 14), "run of 700": with_cluster(300_000, 700, 1e-9, 15),
     "run of 3000": with_cluster(1_000_000, 3000, 1e-6, 16), "run of 20000": with_cluster(4_000_000, 20_000, 1e-6, 17),
+    # steps of a long run's sort: 2048 keys
+    **{f"run of {k}": with_cluster(1_000_000, k, 1e-6, 50 + k) for k in (2047, 2048, 2049, 4097)},
     "one cluster": with_cluster(100_000, 100_000, 1e-5, 18),
     "pairs": stacked(200_000, 2, 19), "stacks of 100": stacked(200_000, 100, 20), "one point": stacked(50_000, 50_000, 21),
     "escaped": escaped(100_001, 3, 22), "all escaped": escaped(5_000, 1, 23), "few escaped": escaped(500_000, 1000, 24),
