@@ -1681,11 +1681,22 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
     cudaStream_t s = cfg_.stream;
     Impl &m = *m_;
     const bool nf = cfg_.nf;
-    // NFCount trees (deep levels of many units) classify, count and place
-    // with 8 CTAs per SM (an A/B at 16 Mi: 3.49 ms with 4, 3.40 ms with 8,
-    // 3.42 ms with 16); LeafCount trees keep 4
     const unsigned blocks = unsigned(smCount()) * 4u;
-    const unsigned wide = nf ? 2u : 1u;
+    // deep levels of many units classify, count and place with 8 CTAs per SM
+    // (an A/B at 16 Mi: 3.49 ms with 4, 3.40 ms with 8, 3.42 ms with 16)
+    const unsigned wide = 2u;
+    unsigned leafGrid = 0;
+    if (!nf)
+    {
+        // one cooperative launch: a CTA per unit of a typical level (2.5
+        // leaves per bucket of particles, 7 leaves per unit), as many as fit;
+        // few CTAs meet at a barrier sooner
+        int perSm = 0;
+        AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, lb::leafBuildKernel, lb::kThreads, 0));
+        if (perSm <= 0) return false;
+        leafGrid = unsigned(std::min<size_t>(size_t(std::min(perSm, 4)) * size_t(smCount()),
+                                             n_ / (2 * std::max<size_t>(cfg_.bucket, 1)) + 16));
+    }
     const KeyIndex idx = m.keyIndex(n_);
     const u64 *P = m.P[0].as<u64>();
     size_t cap = std::max<size_t>(m.lvCap, n_ / 4 + 4096);
@@ -1700,41 +1711,12 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         ensureUnits(cap);
         const lb::Arena a = m.units();
         AOT_CHECK(cudaMemsetAsync(m.lvCtl.p, 0, kCtlBytes, s));
-        lb::rootKernel<<<1, 32, 0, s>>>(a, m.bufs(), P, n_, cfg_.bucket, nf ? 1 : 0), noteLaunch();
-        AOT_LAUNCH_CHECK();
         // Every kernel reads its level's size on the device, so the whole
         // build is queued without a host wait: the levels the last build
         // needed (all 21 the first time), their subtree counts and the
         // placement; one readback at the end checks that no deeper level
         // was left out.
-        const int levels = std::max(1, std::min(int(kOctLevels), m.lvLevels));
-        for (int l = 0; l < levels; ++l)
-        {
-            if (!nf)
-                lb::expandKernel<false, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
-            else if (cfg_.hilbert)
-                lb::expandKernel<true, true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
-            else
-                lb::expandKernel<true, false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
-            if (nf)
-            {
-                markNearField(true);
-                if (cfg_.hilbert) lb::nearFieldKernel<true, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
-                else lb::nearFieldKernel<false, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
-                markNearField(false);
-                if (cfg_.hilbert)
-                    lb::classifyKernel<true, true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
-                else
-                    lb::classifyKernel<true, false><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
-            }
-            else
-            {
-                lb::classifyKernel<false, false><<<blocks, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
-            }
-            AOT_LAUNCH_CHECK();
-        }
-        lb::subtreeKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
-        AOT_LAUNCH_CHECK();
+        const int levels = nf ? std::max(1, std::min(int(kOctLevels), m.lvLevels)) : int(kOctLevels);
         auto place = [&]() {
             const rb::TreeBufs tb = m.bufs();
             const u32 room = u32(physCap_);
@@ -1750,16 +1732,52 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
                     noteLaunch();
             AOT_LAUNCH_CHECK();
         };
-        place();
-        // the round history is needed before finishKernel writes it; read
-        // everything once
-        // (with the device state: its active count, set by the root kernel)
-        AOT_CHECK(cudaMemcpyAsync(host, m.lvCtl.p, kCtlBytes, cudaMemcpyDeviceToHost, s));
-        AOT_CHECK(cudaMemcpyAsync(host + kCtlBytes, a.sub, sizeof(u32), cudaMemcpyDeviceToHost, s));  // the root's leaves
-        AOT_CHECK(cudaMemcpyAsync(m.hst, m.st, sizeof(DeviceState), cudaMemcpyDeviceToHost, s));
-        waitStream(s);
         u32 rootLeaves = 1;
-        std::memcpy(&rootLeaves, host + kCtlBytes, sizeof(u32));
+        if (nf)
+        {
+            lb::rootKernel<<<1, 32, 0, s>>>(a, m.bufs(), P, n_, cfg_.bucket), noteLaunch();
+            AOT_LAUNCH_CHECK();
+            for (int l = 0; l < levels; ++l)
+            {
+                if (cfg_.hilbert) lb::expandKernel<true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
+                else lb::expandKernel<false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
+                markNearField(true);
+                if (cfg_.hilbert) lb::nearFieldKernel<true, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
+                else lb::nearFieldKernel<false, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
+                markNearField(false);
+                if (cfg_.hilbert)
+                    lb::classifyKernel<true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
+                else
+                    lb::classifyKernel<false><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
+                AOT_LAUNCH_CHECK();
+            }
+            lb::subtreeKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
+            AOT_LAUNCH_CHECK();
+            place();
+            // the round history is needed before finishKernel writes it; read
+            // everything once
+            // (with the device state: its active count, set by the root kernel)
+            AOT_CHECK(cudaMemcpyAsync(host, m.lvCtl.p, kCtlBytes, cudaMemcpyDeviceToHost, s));
+            AOT_CHECK(cudaMemcpyAsync(host + kCtlBytes, a.sub, sizeof(u32), cudaMemcpyDeviceToHost, s));  // the root's leaves
+            AOT_CHECK(cudaMemcpyAsync(m.hst, m.st, sizeof(DeviceState), cudaMemcpyDeviceToHost, s));
+            waitStream(s);
+            std::memcpy(&rootLeaves, host + kCtlBytes, sizeof(u32));
+        }
+        else
+        {
+            lb::LeafBuildArgs p{a, idx, m.bufs(), P, n_, cfg_.bucket, cfg_.maxDepth, u32(physCap_)};
+            void *args[] = {&p};
+            AOT_CHECK(cudaLaunchCooperativeKernel(lb::leafBuildKernel, dim3(leafGrid), dim3(lb::kThreads), args, 0, s));
+            noteLaunch();
+            AOT_CHECK(cudaMemcpyAsync(host, m.lvCtl.p, kCtlBytes, cudaMemcpyDeviceToHost, s));
+            waitStream(s);
+            if (hc.bar.error) throw std::runtime_error("adaptive_octree: a grid barrier of the level build gave up waiting");
+            rootLeaves = hc.leaves;
+            // the device state's other words are set below, as the kernel set them
+            *m.hst = DeviceState{};
+            m.hst->numActiveParticles = hc.active;
+            m.hst->error = hc.stateError;
+        }
         if (hc.error) throw std::runtime_error("adaptive_octree: a device scan gave up waiting (bounded look-back)");
         if (hc.overflow)
         {
@@ -1767,7 +1785,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             continue;
         }
         if (hc.late) return false;
-        if (hc.levelCount[levels] != 0)
+        if (nf && hc.levelCount[levels] != 0)
         {
             m.lvLevels = int(kOctLevels);  // deeper than the last build: all levels again
             continue;
@@ -1811,8 +1829,11 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         }
         hostLeaves_ = rootLeaves;
         m.lvLevels = std::min(int(kOctLevels), deepest + 2);
-        lb::finishKernel<<<1, 1, 0, s>>>(a, m.bufs(), rounds, levels, u32(physCap_)), noteLaunch();
-        AOT_LAUNCH_CHECK();
+        if (nf || hc.placeOverflow)
+        {
+            lb::finishKernel<<<1, 1, 0, s>>>(a, m.bufs(), rounds, levels, u32(physCap_)), noteLaunch();
+            AOT_LAUNCH_CHECK();
+        }
         // the host mirror of what finishKernel writes (the readback above
         // brought the active count), so the build needs no second readback
         DeviceState &h = *m.hst;

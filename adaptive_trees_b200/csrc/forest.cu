@@ -54,7 +54,7 @@ struct ForestEngine::Impl
     std::vector<size_t> leafCap;
     bool built = false;
     // build by levels: the unit arena, the key sample and the control words
-    DevMem lvRows, lvChild, lvLeaves, lvOffset, lvUsys, lvSysRoot, lvBins, lvCtl, sample;
+    DevMem lvRows, lvChild, lvSub, lvParent, lvOffset, lvUsys, lvSysRoot, lvBins, lvCtl, sample;
     size_t lvCap = 0;
     size_t lastEntries = 0;  // entries of the last build (the first guess of the next)
     int buildMode = 0;
@@ -585,14 +585,14 @@ bool ForestEngine::levelBuild()
     Impl &m = *m_;
     cudaStream_t s = m.cfg.stream;
     if (u64(m.cfg.bucket) * 512u > 0xffffffffull) return false;
-    const bool hil = m.cfg.hilbert;
-    const void *fn = hil ? reinterpret_cast<const void *>(&forest::levelBuildKernel<true>)
-                         : reinterpret_cast<const void *>(&forest::levelBuildKernel<false>);
+    const void *fn = reinterpret_cast<const void *>(&forest::levelBuildKernel);
     int perSm = 0;
     AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, lb::kThreads, 0));
     if (perSm <= 0) return false;
-    const unsigned grid = unsigned(perSm) * unsigned(smCount());
+    // a CTA per system, and per unit of a typical level, as many as fit
     const size_t S = size_t(m.S);
+    const unsigned grid = unsigned(std::min<size_t>(size_t(perSm) * size_t(smCount()),
+                                                    S + m.total / (2 * std::max<size_t>(m.cfg.bucket, 1)) + 16));
     constexpr size_t kHeadBytes = (sizeof(lb::Control) + 255) & ~size_t(255);
     constexpr size_t kCtlBytes = kHeadBytes + sizeof(forest::LevelStatus);
     size_t cap = std::max<size_t>(m.lvCap, m.total / std::max(1u, m.cfg.bucket) + 4096);
@@ -604,7 +604,8 @@ bool ForestEngine::levelBuild()
         if (cap >= (size_t(1) << 31)) return false;
         m.lvRows.reserve(cap * lb::kRow * sizeof(u32), s);
         m.lvChild.reserve(cap * 8 * sizeof(u32), s);
-        m.lvLeaves.reserve(cap * sizeof(u32), s);
+        m.lvSub.reserve(cap * sizeof(u64), s);
+        m.lvParent.reserve(cap * sizeof(u32), s);
         m.lvOffset.reserve(cap * sizeof(u32), s);
         m.lvUsys.reserve(cap * sizeof(u32), s);
         m.lvSysRoot.reserve(S * sizeof(u32), s);
@@ -615,7 +616,8 @@ bool ForestEngine::levelBuild()
         lb::Arena &a = p.a;
         a.rows = m.lvRows.as<u32>();
         a.child = m.lvChild.as<u32>();
-        a.leaves = m.lvLeaves.as<u32>();
+        a.sub = m.lvSub.as<u64>();
+        a.parent = m.lvParent.as<u32>();
         a.offset = m.lvOffset.as<u32>();
         a.usys = m.lvUsys.as<u32>();
         a.sysRoot = m.lvSysRoot.as<u32>();
@@ -637,7 +639,7 @@ bool ForestEngine::levelBuild()
         AOT_CHECK(cudaMemcpyAsync(&hc, m.lvCtl.p, sizeof(hc), cudaMemcpyDeviceToHost, s));
         AOT_CHECK(cudaMemcpyAsync(&hl, p.ls, sizeof(hl), cudaMemcpyDeviceToHost, s));
         waitStream(s);
-        if (hl.bar.error) throw std::runtime_error("forest: a grid barrier of the level build gave up waiting");
+        if (hl.bar.error || hc.error) throw std::runtime_error("forest: a wait of the level build gave up");
         if (hc.overflow)
         {
             cap *= 2;

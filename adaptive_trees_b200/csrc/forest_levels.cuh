@@ -12,14 +12,14 @@
 // phase, separated by grid barriers:
 //   roots      a level-0 unit for every system with more than `bucket` active
 //              particles (the others are a single root leaf);
-//   levels     expand (child begins), barrier, classify (new units, history
-//              bins per system), barrier -- until a level has no units;
-//   leafCount  subtree leaf counts, deepest level first;
+//   levels     child begins, new units and history bins per system, barrier
+//              -- until a level has no units;
+//   subtree    subtree leaf counts, all levels at once;
 //   layout     CTA 0: each system's first entry (an exclusive scan of
 //              leaves + 1 over the systems), sentinels and root leaves, the
 //              per-system and forest-wide state;
 //   history    per system (one CTA each): leaves after every round;
-//   place      every leaf's entry, shallowest level first;
+//   place      every leaf's entry, all levels at once;
 //   counts     N = differences of B.
 // A barrier waits a bounded number of polls; a CTA that gives up records it
 // and every CTA returns at its next barrier.  The launch is cooperative, so
@@ -56,11 +56,10 @@ struct LevelArgs
     int maxDepth;
 };
 
-template <bool Hilbert>
 static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArgs p)
 {
     using namespace lb;
-    __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
+    __shared__ u32 sEnds[8], sChunk;
     __shared__ u32 sBin[kContribBins];
     __shared__ unsigned long long sVal[kContribBins];
     __shared__ int sBins, sRounds;
@@ -72,11 +71,6 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
     const u32 rank = blockIdx.x * blockDim.x + threadIdx.x, size = gridDim.x * blockDim.x;
     const int S = p.f.numSystems;
     if (vload(p.f.st->error)) return;  // the sort gave up: the host reports it
-    if constexpr (Hilbert)
-    {
-        copyTable(sNext, gHilbert.encNext);
-        copyTable(sDec, gHilbert.decOct);
-    }
     // roots, and zeroed history bins
     for (size_t i = rank; i < size_t(S) * kContribBins; i += size) a.contrib[i] = 0;
     for (size_t i = rank; i < size_t(S) * kArrivals; i += size) a.landed[i] = 0;
@@ -97,6 +91,7 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
                 row[10] = base + active;
                 row[11] = withUnit(regionWord(0, 0, splitDepth(false, active, p.bucket, 0)), 0, kHilbertStart);
                 a.usys[g] = s;
+                a.parent[g] = kLeaf;
                 root = g;
             }
             else
@@ -107,25 +102,19 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         a.sysRoot[s] = root;
     }
     if (!gridBarrier(&ls->bar)) return;
-    // levels: every CTA reads the same counts and flags after a barrier
-    int deepest = -1;
-    for (int l = 0; l < int(kOctLevels); ++l)
+    // levels: every CTA reads the same counts after a barrier (a flag may
+    // already be set by the next level's units)
+    int levels = 0;
+    for (; levels < int(kOctLevels); ++levels)
     {
-        const u32 start = vload(c.levelStart[l]), count = vload(c.levelCount[l]);
-        if (vload(c.overflow) | vload(c.late) || count == 0) break;
-        deepest = l;
-        expandUnits<false, false>(a, p.idx, l, start, count, rank, size, nullptr);
-        if (!gridBarrier(&ls->bar)) return;
-        classifyUnits<false, Hilbert, true>(a, l, p.bucket, start, count, sNext, sDec, nullptr, nullptr, nullptr, rank,
-                                              size);
+        const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
+        if (count == 0 || count > a.cap - start) break;
+        growUnits<true>(a, p.idx, levels, p.bucket, start, count, sEnds, nullptr, nullptr);
         if (!gridBarrier(&ls->bar)) return;
     }
     if (vload(c.overflow) | vload(c.late)) return;
-    for (int l = deepest; l >= 0; --l)
-    {
-        leafCountUnits(a, vload(c.levelStart[l]), vload(c.levelCount[l]), rank, size);
-        if (!gridBarrier(&ls->bar)) return;
-    }
+    countSubtrees<true>(a, levels ? vload(c.levelStart[levels]) : 0u);
+    if (!gridBarrier(&ls->bar)) return;
     // layout (CTA 0): systems one after the other, each followed by its sentinel
     if (blockIdx.x == 0)
     {
@@ -138,7 +127,7 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
             if (s < S)
             {
                 root = a.sysRoot[s];
-                leaves = root == kLeaf ? 1u : a.leaves[root];
+                leaves = root == kLeaf ? 1u : u32(a.sub[root]);
             }
             i64 total;
             const i64 excl = rb::blockExclusiveScan(s < S ? i64(leaves) + 1 : 0, sWarp, total);
@@ -178,7 +167,7 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         {
             const i64 entries = sCarry;
             ls->entries = entries;
-            ls->deepest = deepest;
+            ls->deepest = levels - 1;
             if (entries > i64(p.capacity)) ls->entriesOverflow = 1;
             State &st = *p.f.st;
             const int err = st.error;
@@ -237,13 +226,10 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         }
         __syncthreads();
     }
-    // placement, shallowest level first (a unit's first entry comes from its parent)
-    for (int l = 0; l <= deepest; ++l)
-    {
-        placeUnits<false, false, true>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], l, vload(c.levelStart[l]),
-                          vload(c.levelCount[l]), p.capacity, rank, size, nullptr);
-        if (!gridBarrier(&ls->bar)) return;
-    }
+    // placement (a unit's first entry comes from its parent)
+    placeChunks<false, false, true>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], levels, p.capacity, nullptr,
+                                    sChunk);
+    if (!gridBarrier(&ls->bar)) return;
     const i64 E = vload(ls->entries);
     for (i64 i = rank; i < E; i += size)
         p.f.N[i] = p.f.K[0][i] == kMaxKey ? 0u : p.f.B[0][i + 1] - p.f.B[0][i];

@@ -16,6 +16,7 @@ struct GridBarrier
 };
 
 constexpr u32 kBarrierSpins = 1u << 22;  // polls of about 128 ns: well over 0.5 s
+constexpr u32 kBarrierHot = 64;          // polls without a pause: most barriers open within a few hundred ns
 
 // Every CTA of the grid arrives; the last one opens the next generation.  A
 // CTA that polls more than kBarrierSpins times (or sees another CTA's error)
@@ -42,7 +43,8 @@ __device__ __forceinline__ bool gridBarrier(GridBarrier *b)
             u32 spins = 0;
             while (*gen == g)
             {
-                if (*err || ++spins > kBarrierSpins)
+                if (++spins <= kBarrierHot) continue;
+                if (*err || spins > kBarrierSpins)
                 {
                     atomicExch(&b->error, 1);
                     break;

@@ -20,8 +20,11 @@
 //             level l + 1 (slots taken by warp-aggregated atomics); the
 //             others are leaves of the tree;
 //   subtree, place: subtree leaf counts bottom-up, then every leaf's
-//             position in the cornerstone array top-down, a kernel each for
-//             all levels.
+//             position in the cornerstone array top-down.
+// A LeafCount build is one cooperative launch (leafBuildKernel): a unit's
+// counts are differences of its begins, so expand and classify are one step
+// (growUnits) with a grid barrier per level.  An NFCount build is a launch per
+// step and level, and one each for the subtree counts and the placement.
 //
 // The capacity the reference ends with depends on how many leaves each round
 // proposed (resizeWithHeadroom history, octree.cu:159-180 and 453-457).  That
@@ -39,6 +42,7 @@
 // per round; the host sums the leaf counts of every round from them.
 #pragma once
 
+#include "grid_barrier.cuh"
 #include "rebalance.cuh"
 
 namespace aot
@@ -62,6 +66,11 @@ struct Control
     int error;          // a bounded wait gave up
     int placeOverflow;  // the tree has more leaves than the cornerstone buffers hold
     u32 placeNext;      // next chunk of the placement
+    // one-launch build:
+    GridBarrier bar;
+    u32 leaves;         // leaves of the tree
+    u32 active;         // active particles
+    int stateError;     // DeviceState::error
 };
 
 // The unit arena: units of all levels, level l at
@@ -72,11 +81,10 @@ struct Arena
     u32 *val;        // [cap][8] value of each child (NF or count)
     u32 *child;      // [cap][8] unit index of an internal child, or kLeaf; units of a standing tree: a leaf's
                      // index | kLeafRef (LeafCount: by digit, NFCount: by octant)
-    u64 *sub;        // single tree: [cap] leaves counted below the unit | children to come << 56
-    u32 *leaves;     // batch of trees: [cap] leaves in the unit's subtree
-    u32 *offset;     // [cap] cornerstone index of the unit's first leaf (single tree: kPending before it is known)
+    u64 *sub;        // [cap] leaves counted below the unit | children to come << 56
+    u32 *offset;     // [cap] cornerstone index of the unit's first leaf (kPending before it is known)
     u32 *nbr;        // NFCount: [cap][27] the cells around each unit (nbrRef)
-    u32 *parent;     // single tree: [cap] parent unit * 8 + the unit's place in its child slots
+    u32 *parent;     // [cap] parent unit * 8 + the unit's place in its child slots (batch of trees: kLeaf for a root)
     u64 *rec;        // NFCount: [cap] child counts of a unit, a byte per octant (kBigRec: one does not fit)
     u32 *usys;       // batch of trees: [cap] the tree (system) of each unit
     u32 *sysRoot;    // batch of trees: [systems] each system's root unit, or kLeaf
@@ -139,7 +147,8 @@ __device__ __forceinline__ u64 rowKey(const u32 *row) { return (u64(row[1]) << 3
 // root: 27 x count^2, clamped, octree.cu:23-38), else the whole tree is the
 // root leaf, written straight to the cornerstone buffers.
 // One warp: the active count by a warp-wide search, then lane 0.
-static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t n, unsigned bucket, int nf)
+__device__ __forceinline__ void rootUnit(const Arena &a, const rb::TreeBufs &tb, const u64 *P, size_t n, unsigned bucket,
+                                         bool nf)
 {
     DeviceState *st = tb.st;
     const unsigned active = n ? warpLowerBound(P, 0, u32(n), kMaxKey, int(threadIdx.x & 31)) : 0u;
@@ -160,7 +169,7 @@ static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t
         row[1] = 0;
         row[2] = 0;
         row[10] = active;
-        row[11] = withUnit(regionWord(0, 0, splitDepth(nf != 0, x, bucket, 0)), 0, kHilbertStart);
+        row[11] = withUnit(regionWord(0, 0, splitDepth(nf, x, bucket, 0)), 0, kHilbertStart);
         c.levelCount[0] = 1;
         a.offset[0] = 0;
         if (nf)
@@ -181,6 +190,11 @@ static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t
         tb.N[0][0] = active;
         st->numLeaves = 1;
     }
+}
+
+static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t n, unsigned bucket)
+{
+    rootUnit(a, tb, P, n, bucket, true);
 }
 
 // Lower bounds of the 7 inner child boundaries key + (d + 1) * cr of a unit
@@ -281,15 +295,150 @@ __device__ __forceinline__ u32 boundaryIn(const KeyIndex &idx, u32 lo, u32 hi, u
     return b;
 }
 
-// 9 child begins of the units of level l: one thread per unit (the 7 inner
-// ones by innerBegins), one lane per inner boundary on levels of fewer units,
-// one warp per inner boundary on levels of few units.
-// Rec: also the units' child counts as bytes (not on levels of few units,
-// whose counts do not fit and which do without), by octant: dec[state * 8 +
-// digit] for the Hilbert curve.
-// `rank` and `size` number the threads taking part (a grid, or the grid of a
-// persistent kernel).
-template <bool Rec, bool Hilbert>
+// The same by a warp: first sampled key >= t among the samples inside [lo, hi),
+// then the window of at most 31 keys before it.
+__device__ __forceinline__ u32 warpBoundaryIn(const KeyIndex &idx, u32 lo, u32 hi, u64 t, int lane)
+{
+    const u32 jA = (lo + kSampleStride - 1) >> kSampleShift, jB = (hi + kSampleStride - 1) >> kSampleShift;
+    const u32 sIdx = warpLowerBound(idx.sample, jA, jB > jA ? jB : jA, t, lane);
+    const u32 wlo = sIdx > jA ? ((sIdx - 1) << kSampleShift) + 1 : lo;
+    const u32 whi = sIdx < jB ? (sIdx << kSampleShift) : hi;
+    return warpLowerBound(idx.keys, wlo, whi, t, lane);
+}
+
+// The children of units (LeafCount): lanes hold a child each, eight to a unit
+// g in digit order, of which `valid` ones take part (whole units; all lanes of
+// the warp call).  A child of more than `bucket` keys below level 21 becomes a
+// unit of level l + 1 (slots by an atomic add per warp; the order of a level's
+// units is free), the others are leaves, counted into the round history by
+// (arrival, depth, relative level): of the CTA (sContrib, sLanded) or, Forest,
+// of the unit's system.  key and reg: the unit's key and region word;
+// [begin, end): the child's keys; next: first unit of level l + 1.
+template <bool Forest>
+__device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned bucket, u32 next, u32 g, bool valid,
+                                             u32 begin, u32 end, u64 key, u32 reg, u32 *sContrib, u32 *sLanded)
+{
+    Control &c = *a.ctl;
+    const unsigned m = unsigned(l) + 1;
+    const int lane = threadIdx.x & 31, d = lane & 7;
+    const u32 x = end - begin;
+    const bool high = valid && x > bucket && m < kOctLevels;
+    const unsigned ballot = __ballot_sync(0xffffffffu, high);
+    u32 base = 0;
+    if (lane == 0 && ballot) base = atomicAdd(&c.levelCount[l + 1], u32(__popc(ballot)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (!valid) return;
+    const u32 aR = regionArrival(reg), lR = regionLevel(reg), kR = regionDepth(reg);
+    const u32 j = m - lR;  // 1 <= j <= kR
+    const u32 nHigh = u32(__popc((ballot >> (lane & 24)) & 0xffu));
+    const u32 sys = Forest ? a.usys[g] : 0u;
+    u32 slot = kLeaf;
+    if (high)
+    {
+        const u32 gc = next + base + u32(__popc(ballot & sort::laneMaskLt()));
+        if (gc < a.cap)
+        {
+            u32 creg = reg;
+            // a landed internal node: a leaf in round aR + 1, splitting at once
+            if (j == kR) creg = regionWord(min(aR + 1, u32(kArrivals) - 1), m, splitDepth(false, x, bucket, m));
+            if constexpr (Forest) a.usys[gc] = sys;
+            a.parent[gc] = g * 8 + u32(d);
+            a.offset[gc] = kPending;
+            const u64 ck = key + u64(d) * octRange(m);
+            uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
+            crow[0] = make_uint4(u32(ck), u32(ck >> 32), begin, 0u);
+            crow[2] = make_uint4(0u, 0u, end, withUnit(creg, m, kHilbertStart));
+            slot = gc;
+        }
+        else
+        {
+            c.overflow = 1;
+        }
+    }
+    a.child[size_t(g) * 8 + d] = slot;
+    if (d != 0) return;
+    a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
+    const u32 bin = (aR * kJumps + kR) * kJumps + j;
+    if (nHigh < 8)
+    {
+        if (Forest) atomicAdd(a.contrib + size_t(sys) * kContribBins + bin, 8ull - nHigh);
+        else atomicAdd(&sContrib[bin], 8u - nHigh);
+    }
+    if (j == kR && nHigh)
+    {
+        if (aR + 2 >= u32(kArrivals)) c.late = 1;
+        else if (Forest) atomicAdd(a.landed + size_t(sys) * kArrivals + aR + 1, (unsigned long long)nHigh);
+        else atomicAdd(&sLanded[aR + 1], nHigh);
+    }
+}
+
+// Expand and classify of a LeafCount level in one step, by a whole grid: on
+// levels of few units a CTA per unit, a warp per inner child boundary (sEnds:
+// 7 words of the CTA), else a lane per child.
+template <bool Forest>
+__device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, int l, unsigned bucket, u32 start,
+                                          u32 count, u32 *sEnds, u32 *sContrib, u32 *sLanded)
+{
+    const u32 next = start + count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u64 cr = octRange(unsigned(l) + 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->levelStart[l + 1] = next;
+    if (count <= kWideUnits)
+    {
+        static_assert(kThreads / 32 >= 7, "a warp per inner boundary");
+        for (u32 i = blockIdx.x; i < count; i += gridDim.x)
+        {
+            u32 *row = a.rows + size_t(start + i) * kRow;
+            const u32 lo = row[2], hi = row[10], reg = row[11];
+            const u64 key = rowKey(row);
+            if (warp < 7)
+            {
+                const u32 r = warpBoundaryIn(idx, lo, hi, key + u64(warp + 1) * cr, lane);
+                if (lane == 0)
+                {
+                    row[3 + warp] = r;
+                    sEnds[warp] = r;
+                }
+            }
+            __syncthreads();
+            if (warp == 0)
+            {
+                const int d = lane & 7;
+                growChildren<Forest>(a, l, bucket, next, start + i, lane < 8, d ? sEnds[d - 1] : lo, d < 7 ? sEnds[d] : hi,
+                                     key, reg, sContrib, sLanded);
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const size_t total = size_t(count) * 8;
+    for (size_t e0 = size_t(blockIdx.x) * kThreads + warp * 32; e0 < total; e0 += size_t(gridDim.x) * kThreads)
+    {
+        const size_t e = e0 + lane;
+        const bool valid = e < total;
+        const u32 g = start + u32(valid ? e >> 3 : 0);
+        const int d = lane & 7;
+        u32 *row = a.rows + size_t(g) * kRow;
+        const u32 lo = row[2], hi = row[10], reg = row[11];
+        const u64 key = rowKey(row);
+        u32 end = hi;
+        if (valid && d < 7)
+        {
+            end = boundaryIn(idx, lo, hi, key + u64(d + 1) * cr);
+            row[3 + d] = end;
+        }
+        const u32 prev = __shfl_up_sync(0xffffffffu, end, 1, 8);
+        growChildren<Forest>(a, l, bucket, next, g, valid, d ? prev : lo, end, key, reg, sContrib, sLanded);
+    }
+}
+
+// 9 child begins of the units of level l of an NFCount build: one thread per
+// unit (the 7 inner ones by innerBegins), one lane per inner boundary on
+// levels of fewer units, one warp per inner boundary on levels of few units;
+// and the units' child counts as bytes (not on levels of few units, whose
+// counts do not fit and which do without), by octant: dec[state * 8 + digit]
+// for the Hilbert curve.
+template <bool Hilbert>
 __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx, int l, u32 start, u32 count, u32 rank,
                                             u32 size, const unsigned char *dec)
 {
@@ -301,15 +450,7 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
         {
             const u32 i = w / 7, d = w - i * 7;
             u32 *row = a.rows + size_t(start + i) * kRow;
-            const u32 lo = row[2], hi = row[10];
-            const u64 t = rowKey(row) + u64(d + 1) * cr;
-            // first sampled key >= t among the samples inside [lo, hi), then
-            // the window of at most 31 keys before it
-            const u32 jA = (lo + kSampleStride - 1) >> kSampleShift, jB = (hi + kSampleStride - 1) >> kSampleShift;
-            const u32 sIdx = warpLowerBound(idx.sample, jA, jB > jA ? jB : jA, t, lane);
-            const u32 wlo = sIdx > jA ? ((sIdx - 1) << kSampleShift) + 1 : lo;
-            const u32 whi = sIdx < jB ? (sIdx << kSampleShift) : hi;
-            const u32 r = warpLowerBound(idx.keys, wlo, whi, t, lane);
+            const u32 r = warpBoundaryIn(idx, row[2], row[10], rowKey(row) + u64(d + 1) * cr, lane);
             if (lane == 0) row[3 + d] = r;
         }
         return;
@@ -327,15 +468,12 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
                 end = boundaryIn(idx, lo, hi, rowKey(row) + u64(d + 1) * cr);
                 row[3 + d] = end;
             }
-            if constexpr (Rec)
-            {
-                const unsigned group = 0xffu << (lane & 24);
-                const u32 prev = __shfl_up_sync(group, end, 1, 8);
-                const u32 cnt = end - (d ? prev : lo);
-                const bool big = __any_sync(group, cnt >= 255u);
-                const u32 oct = Hilbert ? u32(dec[unitStateOf(row[11]) * 8 + d]) : d;
-                reinterpret_cast<unsigned char *>(a.rec + (start + i))[oct] = big ? 255 : (unsigned char)cnt;
-            }
+            const unsigned group = 0xffu << (lane & 24);
+            const u32 prev = __shfl_up_sync(group, end, 1, 8);
+            const u32 cnt = end - (d ? prev : lo);
+            const bool big = __any_sync(group, cnt >= 255u);
+            const u32 oct = Hilbert ? u32(dec[unitStateOf(row[11]) * 8 + d]) : d;
+            reinterpret_cast<unsigned char *>(a.rec + (start + i))[oct] = big ? 255 : (unsigned char)cnt;
         }
         return;
     }
@@ -347,36 +485,33 @@ __device__ __forceinline__ void expandUnits(const Arena &a, const KeyIndex &idx,
         innerBegins(idx, lo, hi, rowKey(row), cr, b);
 #pragma unroll
         for (int d = 0; d < 7; ++d) row[3 + d] = b[d];
-        if constexpr (Rec)
-        {
-            const u32 st = unitStateOf(row[11]);
-            u64 rec = 0;
-            bool big = false;
+        const u32 st = unitStateOf(row[11]);
+        u64 rec = 0;
+        bool big = false;
 #pragma unroll
-            for (int d = 0; d < 8; ++d)
-            {
-                const u32 cnt = (d < 7 ? b[d] : hi) - (d ? b[d - 1] : lo);
-                big |= cnt >= 255u;
-                const u32 oct = Hilbert ? u32(dec[st * 8 + d]) : u32(d);
-                rec |= u64(cnt & 0xffu) << (8 * oct);
-            }
-            a.rec[start + i] = big ? kBigRec : rec;
+        for (int d = 0; d < 8; ++d)
+        {
+            const u32 cnt = (d < 7 ? b[d] : hi) - (d ? b[d - 1] : lo);
+            big |= cnt >= 255u;
+            const u32 oct = Hilbert ? u32(dec[st * 8 + d]) : u32(d);
+            rec |= u64(cnt & 0xffu) << (8 * oct);
         }
+        a.rec[start + i] = big ? kBigRec : rec;
     }
 }
 
-template <bool Rec, bool Hilbert>
+template <bool Hilbert>
 static __global__ void __launch_bounds__(kThreads) expandKernel(Arena a, KeyIndex idx, int l)
 {
     __shared__ __align__(4) unsigned char sDec[48 * 8];
     const Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
-    if constexpr (Rec && Hilbert)
+    if constexpr (Hilbert)
     {
         copyTable(sDec, gHilbert.decOct);
         __syncthreads();
     }
-    expandUnits<Rec, Hilbert>(a, idx, l, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x,
+    expandUnits<Hilbert>(a, idx, l, c.levelStart[l], c.levelCount[l], blockIdx.x * blockDim.x + threadIdx.x,
                               gridDim.x * blockDim.x, sDec);
 }
 
@@ -1048,11 +1183,9 @@ static __global__ void __launch_bounds__(kThreads) unitsToTableKernel(Arena a, r
 // the slots of its new units with one atomic add; the order of the units in
 // a level is free (every later step finds them through the child and parent
 // links, and the placement follows the digits).
-// Forest: the history counts go to the unit's system's bins in global memory
-// (sContrib / sLanded unused); otherwise to the CTA's shared bins.
-// NFCount: the child slots are kept by octant; sSlots[32 * 9] of the warp
-// turns them around and lets the warp write them coalesced.
-template <bool NF, bool Hilbert, bool Forest>
+// The child slots are kept by octant; sSlots[32 * 9] of the warp turns them
+// around and lets the warp write them coalesced.  NFCount builds.
+template <bool Hilbert>
 __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bucket, u32 start, u32 count,
                                               const unsigned char *sNext, const unsigned char *sDec, u32 *sContrib,
                                               u32 *sLanded, u32 *sSlots, u32 rank, u32 size)
@@ -1081,17 +1214,13 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
             b[2] = r1.x; b[3] = r1.y; b[4] = r1.z; b[5] = r1.w;
             b[6] = r2.x; b[7] = r2.y; b[8] = r2.z;
             reg = r2.w;
-            if constexpr (NF)
-            {
-                const uint4 *v4 = reinterpret_cast<const uint4 *>(a.val + size_t(g) * 8);
-                const uint4 v0 = v4[0], v1 = v4[1];
-                x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
-                x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
-            }
+            const uint4 *v4 = reinterpret_cast<const uint4 *>(a.val + size_t(g) * 8);
+            const uint4 v0 = v4[0], v1 = v4[1];
+            x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
+            x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
 #pragma unroll
             for (int d = 0; d < 8; ++d)
             {
-                if constexpr (!NF) x[d] = b[d + 1] - b[d];
                 if (x[d] > bucket && m < kOctLevels) highMask |= 1u << d;
             }
         }
@@ -1107,16 +1236,13 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
         u32 base = 0;
         if (lane == 31 && incl) base = atomicAdd(&c.levelCount[l + 1], incl);
         base = __shfl_sync(0xffffffffu, base, 31);
-        if (!NF && !valid) continue;
         const u32 aR = regionArrival(reg), lR = regionLevel(reg), kR = regionDepth(reg);
         const u32 j = m - lR;  // 1 <= j <= kR
-        const u32 sys = Forest ? a.usys[g] : 0u;
         u32 rank = base + incl - nHigh;
-        u32 slots[8];
 #pragma unroll
         for (int d = 0; d < 8; ++d)
         {
-            if (NF && !valid) break;
+            if (!valid) break;
             u32 slot = kLeaf;
             if (highMask & (1u << d))
             {
@@ -1127,12 +1253,10 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
                     if (j == kR)
                     {
                         // a landed internal node: a leaf in round aR + 1, splitting at once
-                        creg = regionWord(aR + 1, m, splitDepth(NF, x[d], bucket, m));
+                        creg = regionWord(aR + 1, m, splitDepth(true, x[d], bucket, m));
                         if (aR + 2 >= u32(kArrivals)) c.late = 1;
-                        else if (Forest) atomicAdd(a.landed + size_t(sys) * kArrivals + aR + 1, 1ull);
                         else atomicAdd(&sLanded[aR + 1], 1u);
                     }
-                    if constexpr (Forest) a.usys[gc] = sys;
                     // the child's own level and the curve state ordering its children
                     u32 cst = kHilbertStart, oct = u32(d);
                     if constexpr (Hilbert)
@@ -1141,11 +1265,8 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
                         oct = sDec[st * 8 + d];
                         cst = sNext[st * 8 + oct];
                     }
-                    if constexpr (!Forest)
-                    {
-                        a.parent[gc] = g * 8 + oct;
-                        a.offset[gc] = kPending;
-                    }
+                    a.parent[gc] = g * 8 + oct;
+                    a.offset[gc] = kPending;
                     const u64 ck = key + u64(d) * cr;
                     uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
                     crow[0] = make_uint4(u32(ck), u32(ck >> 32), b[d], 0u);
@@ -1157,51 +1278,34 @@ __device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bu
                     c.overflow = 1;
                 }
             }
-            else if constexpr (Forest)
-            {
-                atomicAdd(a.contrib + size_t(sys) * kContribBins + (aR * kJumps + kR) * kJumps + j, 1ull);
-            }
             else
             {
                 atomicAdd(&sContrib[(aR * kJumps + kR) * kJumps + j], 1u);
             }
-            if constexpr (NF && Hilbert) sSlots[lane * 9 + sDec[unitStateOf(reg) * 8 + d]] = slot;
-            else if constexpr (NF) sSlots[lane * 9 + d] = slot;
-            else slots[d] = slot;
+            if constexpr (Hilbert) sSlots[lane * 9 + sDec[unitStateOf(reg) * 8 + d]] = slot;
+            else sSlots[lane * 9 + d] = slot;
         }
-        if constexpr (!Forest)
-        {
-            if (valid) a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
-        }
-        if constexpr (NF)
-        {
-            __syncwarp();
-            const u32 words = min(32u, count - i0) * 8;
-            u32 *out = a.child + size_t(start + i0) * 8;
+        if (valid) a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
+        __syncwarp();
+        const u32 words = min(32u, count - i0) * 8;
+        u32 *out = a.child + size_t(start + i0) * 8;
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-            {
-                const u32 e = u32(k) * 32 + u32(lane);
-                if (e < words) out[e] = sSlots[(e >> 3) * 9 + (e & 7)];
-            }
-            __syncwarp();
-        }
-        else
+        for (int k = 0; k < 8; ++k)
         {
-            uint4 *ch4 = reinterpret_cast<uint4 *>(a.child + size_t(g) * 8);
-            ch4[0] = make_uint4(slots[0], slots[1], slots[2], slots[3]);
-            ch4[1] = make_uint4(slots[4], slots[5], slots[6], slots[7]);
+            const u32 e = u32(k) * 32 + u32(lane);
+            if (e < words) out[e] = sSlots[(e >> 3) * 9 + (e & 7)];
         }
+        __syncwarp();
     }
 }
 
-template <bool NF, bool Hilbert>
+template <bool Hilbert>
 static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l, unsigned bucket)
 {
     __shared__ u32 sContrib[kContribBins];
     __shared__ u32 sLanded[kArrivals];
     __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
-    __shared__ u32 sSlots[NF ? (kThreads / 32) * 32 * 9 : 1];
+    __shared__ u32 sSlots[(kThreads / 32) * 32 * 9];
     Control &c = *a.ctl;
     if (c.overflow | c.late | c.error) return;
     const u32 start = c.levelStart[l], count = c.levelCount[l];
@@ -1215,8 +1319,8 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
     for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
     if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
     __syncthreads();
-    classifyUnits<NF, Hilbert, false>(a, l, bucket, start, count, sNext, sDec, sContrib, sLanded,
-                                      sSlots + (NF ? (threadIdx.x >> 5) * 32 * 9 : 0),
+    classifyUnits<Hilbert>(a, l, bucket, start, count, sNext, sDec, sContrib, sLanded,
+                                      sSlots + (threadIdx.x >> 5) * 32 * 9,
                                       blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     __syncthreads();
     for (int k = threadIdx.x; k < kContribBins; k += kThreads)
@@ -1225,48 +1329,39 @@ static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l
         atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
 }
 
-// Batch of trees: leaves below each unit of a level (the units of the next are done).
-__device__ __forceinline__ void leafCountUnits(const Arena &a, u32 start, u32 count, u32 rank, u32 size)
-{
-    for (u32 i = rank; i < count; i += size)
-    {
-        const u32 g = start + i;
-        u32 s = 0;
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-        {
-            const u32 ch = a.child[size_t(g) * 8 + d];
-            s += ch == kLeaf ? 1u : a.leaves[ch];
-        }
-        a.leaves[g] = s;
-    }
-}
-
-// The leaves below every unit of a single tree, all levels in one launch: a
+// The leaves below every unit, all levels at once (the first `total` units): a
 // unit whose children are all leaves starts (8 leaves) and adds its count to
-// its parent's; the child that comes last takes the parent's total on.  (A
-// kernel per level cost its launch and tail 11 times at 300k particles, 2.5 us
-// and a gap each.)  `levels` is the number of levels the build expanded: units
-// below them mean the build is incomplete, and nothing is counted.
-static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int levels)
+// its parent's; the child that comes last takes the parent's total on.
+template <bool Forest>
+__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
 {
-    const Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    const u32 total = c.levelStart[levels];
     for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
         // (a unit with internal children holds 15 leaves or more when they have come)
         u64 n = sort::ldRelaxed(a.sub + g);
         if (n != 8) continue;
-        for (u32 u = g; u != 0;)
+        for (u32 u = g; Forest || u != 0;)
         {
-            u = a.parent[u] >> 3;
+            const u32 up = a.parent[u];
+            if (Forest && up == kLeaf) break;  // a system's root
+            u = up >> 3;
             const u64 old = atomicAdd(reinterpret_cast<unsigned long long *>(a.sub + u),
                                       (unsigned long long)(n - (u64(1) << kSubShift)));
             if ((old >> kSubShift) != 1) break;
             n += old & ((u64(1) << kSubShift) - 1);
         }
     }
+}
+
+// The subtree counts of an NFCount build.  (A kernel per level cost its launch
+// and tail 11 times at 300k particles, 2.5 us and a gap each.)  `levels` is
+// the number of levels the build expanded: units below them mean the build is
+// incomplete, and nothing is counted.
+static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int levels)
+{
+    const Control &c = *a.ctl;
+    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
+    countSubtrees<false>(a, c.levelStart[levels]);
 }
 
 // Cornerstone entries of the leaf children of the level-l units, and the
@@ -1292,7 +1387,7 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
         const bool valid = e < total;
         const u32 g = start + u32(valid ? e >> 3 : 0);
         u32 ch = valid ? a.child[size_t(g) * 8 + d] : kLeaf;
-        u32 mine = ch == kLeaf ? 1u : Forest ? a.leaves[ch] : u32(a.sub[ch]);
+        u32 mine = ch == kLeaf ? 1u : u32(a.sub[ch]);
         if constexpr (NF && Hilbert)
         {
             // from octants to digits within the unit's 8 lanes
@@ -1308,25 +1403,18 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
             if (d >= off) inc += t;
         }
-        u32 first = 0;  // the unit's first leaf
-        if constexpr (Forest)
+        // the unit's first leaf: placed by its parent, in a chunk handed out before this one
+        u32 first = 0;
+        for (unsigned spins = 0;; ++spins)
         {
-            if (valid) first = a.offset[g];
-        }
-        else
-        {
-            // placed by the unit's parent, in a chunk handed out before this one
-            for (unsigned spins = 0;; ++spins)
+            first = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
+            if (!__any_sync(0xffffffffu, first == kPending)) break;
+            if (spins > kPlaceSpins)
             {
-                first = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
-                if (!__any_sync(0xffffffffu, first == kPending)) break;
-                if (spins > kPlaceSpins)
-                {
-                    c.error = kErrLookback;
-                    return;
-                }
-                if (spins > 64) __nanosleep(64);
+                c.error = kErrLookback;
+                return;
             }
+            if (spins > 64) __nanosleep(64);
         }
         if (!valid) continue;
         const u32 o = first + inc - mine;
@@ -1341,7 +1429,7 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             B[o] = row[2 + d];
             if constexpr (NF) NFo[o] = a.val[size_t(g) * 8 + d];
             if (N) N[o] = row[3 + d] - row[2 + d];
-            if (SEG) SEG[o] = int(a.usys[g]);
+            if constexpr (Forest) SEG[o] = int(a.usys[g]);
         }
         else
         {
@@ -1354,20 +1442,16 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
 // chunks before it).
 constexpr u32 kPlaceChunk = 128;
 
-// The placement of a single tree, all levels in one launch: CTAs take chunks
+// The placement of all levels (the first `levels`) at once: CTAs take chunks
 // of units in level order from a counter; a unit waits for its own place,
 // which its parent's chunk writes.  Chunks are handed out in order to running
 // CTAs and wait for earlier ones only, so the waits end (they are bounded all
 // the same).  A kernel per level: 36 us and 11 gaps at 300k particles.
-template <bool NF, bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels,
-                                                               u32 capacity)
+template <bool NF, bool Hilbert, bool Forest>
+__device__ __forceinline__ void placeChunks(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, int levels,
+                                            u32 capacity, const unsigned char *dec, u32 &sChunk)
 {
-    __shared__ __align__(4) unsigned char sDec[48 * 8];
-    __shared__ u32 sChunk;
     Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    if constexpr (NF && Hilbert) copyTable(sDec, gHilbert.decOct);
     u32 level = 0, levelChunk = 0;  // chunks before `level`
     for (;;)
     {
@@ -1380,27 +1464,35 @@ static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, 
         u32 count = 0;
         for (; level < u32(levels); ++level)
         {
-            count = c.levelCount[level];
+            count = vload(c.levelCount[level]);
             const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
             if (chunk < levelChunk + chunks) break;
             levelChunk += chunks;
         }
         if (level >= u32(levels)) return;
         const u32 base = (chunk - levelChunk) * kPlaceChunk;
-        placeUnits<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, int(level), c.levelStart[level] + base,
-                                       min(kPlaceChunk, count - base), capacity, threadIdx.x, kThreads, sDec);
+        placeUnits<NF, Hilbert, Forest>(a, K, B, NFo, N, SEG, int(level), vload(c.levelStart[level]) + base,
+                                        min(kPlaceChunk, count - base), capacity, threadIdx.x, kThreads, dec);
     }
+}
+
+template <bool NF, bool Hilbert>
+static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels,
+                                                               u32 capacity)
+{
+    __shared__ __align__(4) unsigned char sDec[48 * 8];
+    __shared__ u32 sChunk;
+    const Control &c = *a.ctl;
+    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
+    if constexpr (NF && Hilbert) copyTable(sDec, gHilbert.decOct);
+    placeChunks<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, levels, capacity, sDec, sChunk);
 }
 
 // The finished tree: sentinel boundary and the state of a converged build
 // (finishBuildStateKernel, octree.cu:40-47, after `rounds` changing rounds).
-static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int rounds, int levels, u32 capacity)
+__device__ __forceinline__ void finishState(const rb::TreeBufs &tb, int leaves, int rounds)
 {
     DeviceState *st = tb.st;
-    const Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow | c.late | c.error | c.placeOverflow) return;
-    const int leaves = c.levelCount[0] ? int(u32(a.sub[0])) : 1;
-    if (u32(leaves) > capacity) return;
     tb.K[0][leaves] = kMaxKey;
     tb.B[0][leaves] = st->numActiveParticles;
     st->numLeaves = leaves;
@@ -1413,6 +1505,88 @@ static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int rounds, int le
     st->activeBuffer = 0;
     st->overflow = 0;
     st->dirtyCount = 0;
+}
+
+static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int rounds, int levels, u32 capacity)
+{
+    const Control &c = *a.ctl;
+    if (c.levelCount[levels] | c.overflow | c.late | c.error | c.placeOverflow) return;
+    const int leaves = c.levelCount[0] ? int(u32(a.sub[0])) : 1;
+    if (u32(leaves) <= capacity) finishState(tb, leaves, rounds);
+}
+
+struct LeafBuildArgs
+{
+    Arena a;  // (control block zero on entry)
+    KeyIndex idx;
+    rb::TreeBufs tb;
+    const u64 *P;
+    size_t n;
+    unsigned bucket, maxDepth;
+    u32 capacity;  // leaves the cornerstone buffers hold
+};
+
+// A LeafCount build in one cooperative launch: root, levels, subtree counts,
+// placement and final state.  Bound by the latency of the searches and the
+// barriers on small trees, of the searches on large ones.  With a launch per
+// step and level: 10k particles 74 us in 19 launches, now 49; 1Mi 71 in 15,
+// now 75 without their gaps (build() 212 to 160 and 262 to 238 us).
+//
+// CTAs take the same turns at the barriers: a level's count, and with it the
+// room in the arena, is final once its barrier has opened, while the overflow
+// flag may already be set by the next level's units and is read after the
+// last barrier only.
+static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildArgs p)
+{
+    __shared__ u32 sContrib[kContribBins];
+    __shared__ u32 sLanded[kArrivals];
+    __shared__ u32 sEnds[8];
+    __shared__ u32 sChunk;
+    __shared__ int sRounds;
+    const Arena &a = p.a;
+    Control &c = *a.ctl;
+    for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
+    if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
+    if (threadIdx.x == 0) sRounds = 0;
+    if (blockIdx.x == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, false);
+    if (!gridBarrier(&c.bar)) return;
+    int levels = 0;
+    for (; levels < int(kOctLevels); ++levels)
+    {
+        const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
+        if (count == 0 || count > a.cap - start) break;
+        growUnits<false>(a, p.idx, levels, p.bucket, start, count, sEnds, sContrib, sLanded);
+        if (!gridBarrier(&c.bar)) return;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kContribBins; k += kThreads)
+        if (sContrib[k]) atomicAdd(a.contrib + k, (unsigned long long)sContrib[k]);
+    if (threadIdx.x < kArrivals && sLanded[threadIdx.x])
+        atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
+    countSubtrees<false>(a, levels ? vload(c.levelStart[levels]) : 0u);
+    if (!gridBarrier(&c.bar)) return;
+    if (vload(c.overflow) | vload(c.late)) return;
+    if (blockIdx.x == 0)
+    {
+        for (int k = threadIdx.x; k < kContribBins; k += kThreads)
+            if (vload(a.contrib[k]))
+            {
+                const int j = k % kJumps, kk = (k / kJumps) % kJumps, ai = k / (kJumps * kJumps);
+                atomicMax(&sRounds, ai + 1 + kk - j);
+            }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            const u32 leaves = levels ? u32(vload(a.sub[0])) : 1u;
+            c.leaves = leaves;
+            c.active = p.tb.st->numActiveParticles;
+            c.stateError = p.tb.st->error;
+            if (leaves > p.capacity) c.placeOverflow = 1;
+            else if (sRounds <= int(p.maxDepth)) finishState(p.tb, int(leaves), sRounds);
+        }
+    }
+    placeChunks<false, false, false>(a, p.tb.K[0], p.tb.B[0], nullptr, p.tb.N[0], nullptr, levels, p.capacity, nullptr,
+                                     sChunk);
 }
 }  // namespace lb
 }  // namespace aot
