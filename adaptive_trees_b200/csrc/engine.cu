@@ -35,7 +35,7 @@
 #include "binlevel.cuh"
 #include "levelbuild.cuh"
 #include "rebalance.cuh"
-#include "sort_repair.cuh"
+#include "sort_fused.cuh"
 #include "tree_view.cuh"
 
 namespace aot
@@ -499,27 +499,69 @@ struct SortArena
     u32 *longRuns() const { return reinterpret_cast<u32 *>(at(longAt)); }
 };
 
+// Sorts of at most this many keys run their passes and repair in one launch,
+// unless the stream is being captured: a graph's launches cost less than the
+// grid barriers.  Pair sorts of random keys queued directly, launch by launch
+// and in one: 10k keys 72 and 57 us, 100k 79 and 61, 1M 113 and 99, 4M 202 and
+// 200; from a graph 39 and 46, 48 and 51, 81 and 89, 164 and 190.
+constexpr size_t kFusedSort = size_t(1) << 21;
+
+// The passes and the repair of one launch (sort_fused.cuh), after the plan (or
+// beginSortKernel); hist: with the digit counts.  False (nothing done) where
+// the passes run launch by launch.
+bool launchFusedSort(int cfg, cudaStream_t s, const sort::PassArgs &p, const sort::RepairArgs &r, u32 *hist, u32 *bins,
+                     bool repair)
+{
+    if (p.n > kFusedSort) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    AOT_CHECK(cudaStreamIsCapturing(s, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return false;
+    size_t smem = 0;
+    const void *fn = sort::fusedSort(cfg, smem);
+    if (!fn) return false;
+    AOT_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    int perSm = 0;
+    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, sort::kThreads, smem));
+    if (perSm <= 0) return false;
+    const u32 tiles = u32(configTiles(cfg, p.n));
+    sort::FusedArgs a{p, r, tiles, hist, bins, repair, r.keyMask == ~u64(0)};
+    void *args[] = {&a};
+    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(std::min<unsigned>(tiles, unsigned(perSm) * unsigned(smCount()))),
+                                          dim3(sort::kThreads), args, smem, s));
+    noteLaunch();
+    return true;
+}
+
 // The passes of configuration `cfg` over (k[0], v[0]) -> ... for bits [0,
-// endBit), the input indices as values; the digit starts must be in bins.
+// endBit), the input indices as values; the digit starts must be in bins, or
+// hist: are counted first (the counts zero).
 // Without a plan all passes run, and the index (0/1) of the buffers holding
 // the result is returned; with one, the repair puts it into buffers 0
 // (and writes the sample).
 int runPasses(int cfg, cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int endBit, SortArena &a, int *error, bool plan,
-              u64 *sample = nullptr)
+              bool hist, u64 *sample = nullptr)
 {
     sort::setPassSmemAll();
     const int bitsPer = sort::kSortConfigs[cfg].bits;
     const int passes = (endBit + bitsPer - 1) / bitsPer;
     sort::PassArgs p{k[0], nullptr, {k[0], k[1]}, {v[0], v[1]}, n, a.bins(), a.ctl(), a.status(), error,
                      0, endBit, passes, false};
+    const sort::RepairArgs r{{k[0], k[1]}, {v[0], v[1]}, n, a.ctl(), a.longRuns(), sample, error,
+                             0, passes, ~u64(0), false, true, true};
+    if (launchFusedSort(cfg, s, p, r, hist ? a.hist() : nullptr, a.bins(), plan)) return plan ? 0 : passes & 1;
+    if (hist)
+    {
+        const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
+        sort::launchHistogram(cfg, s, blocks, k[0], n, 0, passes, a.hist(), endBit, a.ctl()), noteLaunch();
+        sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
+        AOT_LAUNCH_CHECK();
+    }
     for (int slot = 0; slot < passes; ++slot)
     {
         sort::launchPass(cfg, s, p, slot), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
     if (!plan) return passes & 1;
-    const sort::RepairArgs r{{k[0], k[1]}, {v[0], v[1]}, n, a.ctl(), a.longRuns(), sample, error,
-                             0, passes, ~u64(0), false, true, true};
     sort::repairKernel<true><<<sort::repairTiles(n), sort::kRepairThreads, 0, s>>>(r), noteLaunch();
     sort::longRunKernel<<<unsigned(smCount()) * 2u, sort::kLongThreads, 0, s>>>(r), noteLaunch();
     AOT_LAUNCH_CHECK();
@@ -533,11 +575,8 @@ int sortWithIndices(cudaStream_t s, u64 *k[2], u32 *v[2], size_t n, int passes, 
     const int cfg = sort::defaultSortConfig(n);
     a.ensure(n, s, false);
     sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
-    const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
-    sort::launchHistogram(cfg, s, blocks, k[0], n, 0, passes, a.hist(), 8 * passes, a.ctl()), noteLaunch();
-    sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
     AOT_LAUNCH_CHECK();
-    return runPasses(cfg, s, k, v, n, 8 * passes, a, error, false);
+    return runPasses(cfg, s, k, v, n, 8 * passes, a, error, false, true);
 }
 
 }  // namespace
@@ -784,22 +823,24 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     {
         sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(ctl, nullptr), noteLaunch();
     }
+    AOT_LAUNCH_CHECK();
+    const sort::PassArgs p{in, valsIn, {out, altK}, {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes,
+                           true};
+    const bool aligned = aligned16(out) && (reinterpret_cast<uintptr_t>(valsOut) & 7u) == 0;
+    const sort::RepairArgs r{{out, altK}, {valsOut, altV}, n, ctl, reinterpret_cast<u32 *>(base + lay.longRuns), nullptr,
+                             error, beginBit, passes, keyMask, true, aligned, false};
+    if (launchFusedSort(cfg, s, p, r, hist, bins, planned)) return;
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
     sort::launchHistogram(cfg, s, blocks, in, n, beginBit, passes, hist, endBit, ctl), noteLaunch();
     sort::binsKernel<<<1, sort::kThreads, 0, s>>>(hist, bins, passes), noteLaunch();
     AOT_LAUNCH_CHECK();
     sort::setPassSmemAll();
-    const sort::PassArgs p{in, valsIn, {out, altK}, {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes,
-                           true};
     for (int slot = 0; slot < passes; ++slot)
     {
         sort::launchPass(cfg, s, p, slot), noteLaunch();
         AOT_LAUNCH_CHECK();
     }
     if (!planned) return;
-    const bool aligned = aligned16(out) && (reinterpret_cast<uintptr_t>(valsOut) & 7u) == 0;
-    const sort::RepairArgs r{{out, altK}, {valsOut, altV}, n, ctl, reinterpret_cast<u32 *>(base + lay.longRuns), nullptr,
-                             error, beginBit, passes, keyMask, true, aligned, false};
     if (keyMask == ~u64(0))
         sort::repairKernel<true><<<sort::repairTiles(n), sort::kRepairThreads, 0, s>>>(r), noteLaunch();
     else
@@ -833,6 +874,15 @@ void TreeEngine::sortPairsPreload()
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::repairKernel<true>));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::repairKernel<false>));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::longRunKernel));
+    for (int c = 0; c < sort::kNumSortConfigs; ++c)
+    {
+        size_t smem = 0;
+        if (const void *fn = sort::fusedSort(c, smem))
+        {
+            AOT_CHECK(cudaFuncGetAttributes(&a, fn));
+            AOT_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        }
+    }
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<8>));
     AOT_CHECK(cudaFuncGetAttributes(&a, sort::histogramKernel<7>));
 #define AOT_CASE(i, B, I) AOT_CHECK(cudaFuncGetAttributes(&a, sort::onesweepKernel<B, I>));
@@ -1257,16 +1307,10 @@ void TreeEngine::sortKeys(int config)
     else
         launchKeygen<double>(cfg_.kind, cfg_.hilbert, static_cast<const double *>(x_), static_cast<const double *>(y_),
                              static_cast<const double *>(z_), n_, m_->kpd, k[0], ks, s);
-    if (!planned)
-    {
-        sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
-        const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n_, sort::kThreads), unsigned(smCount()) * 8u));
-        sort::launchHistogram(config, s, blocks, k[0], n_, 0, passes, a.hist(), 64, a.ctl()), noteLaunch();
-        sort::binsKernel<<<1, sort::kThreads, 0, s>>>(a.hist(), a.bins(), passes), noteLaunch();
-        AOT_LAUNCH_CHECK();
-    }
+    if (!planned) sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(a.ctl(), a.hist()), noteLaunch();
+    AOT_LAUNCH_CHECK();
     // (without a plan the repair finds all passes run and writes the sample alone)
-    runPasses(config, s, k, v, n_, 64, a, &m_->st->error, true, m_->sample.as<u64>());
+    runPasses(config, s, k, v, n_, 64, a, &m_->st->error, true, !planned, m_->sample.as<u64>());
     sortConfig_ = config;
 }
 

@@ -41,6 +41,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "grid_barrier.cuh"
 
 namespace aot
 {
@@ -93,6 +94,7 @@ struct SortControl
     u32 longRuns;   // runs the repair left to the long-run kernel
     u32 keygenDone; // CTAs of the key generation that have added their digit counts
     u32 tileCounters[kPassSlots];
+    GridBarrier bar; // of a sort in one launch (as each barrier leaves it)
 };
 constexpr u32 kEpochStep = 16;  // tags per sort (>= kPassSlots)
 

@@ -187,3 +187,51 @@ def test_planned_pair_sort_is_the_stable_sort(n, offset, kind, begin, end):
         C.check(lib.ao_sort_pairs_check(scratch.data_ptr(), n, stream))
         assert np.array_equal(out_k.cpu().numpy().view(np.uint64), k[order])
         assert np.array_equal(out_v.cpu().numpy(), order.astype(np.int32) * 7)
+
+
+@pytest.mark.parametrize("n", [1, 2047, 4097, 100_003, (1 << 21) + 1])
+@pytest.mark.parametrize("bits", [(0, 64), (0, 16), (5, 46)])
+def test_pair_sort_queued_and_captured(n, bits):
+    """Small sorts run in one launch, or launch by launch under capture: both are the stable sort."""
+    import ctypes
+
+    import torch
+
+    from adaptive_trees_b200 import _capi as C
+    r = np.random.default_rng(n + bits[1])
+    host = r.integers(0, 1 << 63, n, dtype=np.uint64) & ~np.uint64(0x3FF << 20)
+    host[r.integers(0, n, n // 3)] = host[0]  # a stack of equal keys
+    begin, end = bits
+    mask = np.uint64(((1 << (end - begin)) - 1) << begin)
+    order = np.argsort(host & mask, kind="stable")
+    keys = torch.from_numpy(host.view(np.int64)).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    out, out_vals = torch.empty_like(keys), torch.empty_like(vals)
+    size = ctypes.c_size_t()
+    lib = C.load()
+    C.check(lib.ao_sort_pairs(None, ctypes.byref(size), None, None, None, None, n, begin, end, None))
+    scratch = torch.empty(size.value, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.Stream()
+
+    def sort():
+        C.check(lib.ao_sort_pairs(scratch.data_ptr(), ctypes.byref(size), keys.data_ptr(), out.data_ptr(),
+                                  vals.data_ptr(), out_vals.data_ptr(), n, begin, end,
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
+    def check(how):
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), host[order]), how
+        assert np.array_equal(out_vals.cpu().numpy(), order.astype(np.int32)), how
+        out.zero_(), out_vals.zero_()
+        torch.cuda.synchronize()
+
+    with torch.cuda.stream(stream):
+        sort()
+    check("queued")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        sort()
+    graph.replay()
+    check("replayed")
+    graph.replay()
+    check("replayed again")
