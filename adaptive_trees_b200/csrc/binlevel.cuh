@@ -1,4 +1,4 @@
-// binlevel.cuh -- the converged binary (k-d) tree build, level by level.
+// binlevel.cuh -- the converged binary (k-d) tree build, three levels at a time.
 //
 // The reference builds a binary tree from the root by passes until a pass
 // changes nothing (the build loop of kdtree3d.cu:239-249 over
@@ -8,18 +8,22 @@
 // `bucket`.  A leaf's count never grows from a node to its children, so no
 // pair made by a split can merge afterwards, and the tree the passes end with
 // is unique: a node is internal exactly when it holds more than `bucket`
-// particles below maxDepth.  One level of internal nodes ("units") at a time:
-//   level     per unit the lower bound of its midpoint key among its keys
-//             (a warp per unit on levels of few units), then its two
-//             children: those above the bucket become units of the next
-//             level (warp-aggregated slots), the others are leaves;
-//   subtree   subtree leaf counts, bottom-up, all levels in one launch;
-//   place     every leaf's K, B and count, top-down, all levels in one launch.
-// Each pass of the reference splits one level, so the passes that change the
-// tree number the deepest unit's level + 1, and its leaf capacity, grown by
-// 25 % steps to the leaf count of every pass (commitIfLast, rebalance.cuh),
-// ends at the first step of that chain at or above the final leaf count:
-// the counts only grow during a build.
+// particles below maxDepth.
+//
+// A "unit" is an internal node at a depth that is a multiple of three,
+// together with the nodes of the two depths below it: its slots are its 8
+// descendants three depths down.  A slot is an internal node (a unit of the
+// next level), a leaf, or part of a wider leaf of 2 or 4 slots, which starts
+// at the first of them.  One cooperative launch (buildKernel) makes the tree:
+//   levels    the 7 inner slot boundaries of each unit among its keys, then
+//             its slots (warp-aggregated slots of new units), barrier;
+//   subtree   subtree leaf counts, bottom-up, all levels at once;
+//   place     every leaf's K, B and count, top-down, all levels at once.
+// Each pass of the reference splits one depth, so the passes that change the
+// tree number the deepest internal node's depth + 1, and its leaf capacity,
+// grown by 25 % steps to the leaf count of every pass (commitIfLast,
+// rebalance.cuh), ends at the first step of that chain at or above the final
+// leaf count: the counts only grow during a build.
 #pragma once
 
 #include "levelbuild.cuh"
@@ -28,10 +32,11 @@ namespace aot
 {
 namespace bl
 {
-constexpr int kThreads = 256;
-constexpr u32 kLeaf = 0xffffffffu;
-constexpr int kLevels = 64;          // depths 0..63
-constexpr u32 kWideUnits = 2048;     // levels of at most this many units search by warps
+using lb::kLeaf;
+using lb::kThreads;
+constexpr u32 kInside = 0xfffffffeu;  // child slot: inside a leaf that starts before it
+constexpr int kLevels = 21;           // unit depths 0, 3, .. 60
+constexpr u32 kWideUnits = 2048;      // levels of at most this many units search by warps
 
 struct Control
 {
@@ -41,15 +46,19 @@ struct Control
     int placeOverflow;  // more leaves than the leaf arrays hold
     int error;          // a bounded wait gave up
     u32 placeNext;      // next chunk of the placement
+    GridBarrier bar;
+    int depths;         // depths holding internal nodes
+    u32 leaves;         // leaves of the tree
+    u32 active;         // active particles
+    int stateError;     // DeviceState::error
 };
 
 struct Arena
 {
-    uint4 *rows;    // [cap] key lo, key hi, begin, end
-    u32 *mid;       // [cap] first key of the upper child
-    u32 *child;     // [cap][2] unit index of an internal child, or kLeaf
+    u32 *rows;      // [cap][lb::kRow] key (2 words), 9 slot begins, slot masks: leaf or unit starts | units << 8
+    u32 *child;     // [cap][8] unit index of an internal slot, kLeaf or kInside
     u32 *parent;    // [cap] parent unit
-    u64 *sub;       // [cap] leaves counted below the unit | children to come << lb::kSubShift
+    u64 *sub;       // [cap] leaves counted below the unit | units to come << lb::kSubShift
     u32 *offset;    // [cap] leaf index of the unit's first leaf (lb::kPending before it is known)
     Control *ctl;
     u32 cap;
@@ -58,10 +67,10 @@ struct Arena
 // Key range of a node at depth d: 2^(63 - d).
 __device__ __forceinline__ u64 depthRange(int d) { return u64(1) << (63 - d); }
 
-// The root: a unit when it holds more than `bucket` particles (and may
-// split), else the single root leaf, written straight to the leaf arrays.
-static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t n, unsigned bucket,
-                                  unsigned maxDepth)
+// The root (one warp): a unit when it holds more than `bucket` particles (and
+// may split), else the single root leaf, written straight to the leaf arrays.
+__device__ __forceinline__ void rootUnit(const Arena &a, const rb::TreeBufs &tb, const u64 *P, size_t n, unsigned bucket,
+                                         unsigned maxDepth)
 {
     const unsigned active = n ? warpLowerBound(P, 0, u32(n), kMaxKey, int(threadIdx.x & 31)) : 0u;
     if (threadIdx.x != 0) return;
@@ -74,7 +83,8 @@ static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t
     c.levelStart[0] = 0;
     if (active > bucket && maxDepth > 0)
     {
-        a.rows[0] = make_uint4(0u, 0u, 0u, active);
+        a.rows[0] = a.rows[1] = a.rows[2] = 0;
+        a.rows[10] = active;
         a.offset[0] = 0;
         c.levelCount[0] = 1;
     }
@@ -89,129 +99,124 @@ static __global__ void rootKernel(Arena a, rb::TreeBufs tb, const u64 *P, size_t
     }
 }
 
-// The units of depth l: their midpoints, then their children.
-static __global__ void __launch_bounds__(kThreads) levelKernel(Arena a, KeyIndex idx, int l, unsigned bucket,
-                                                               unsigned maxDepth)
+// The slots of units: lanes hold one each, eight to a unit g in key order, of
+// which `valid` ones take part (whole units; all lanes of the warp call).
+// [begin, end): the slot's keys.  deepest: of the CTA.
+__device__ __forceinline__ void growSlots(const Arena &a, int level, unsigned bucket, unsigned maxDepth, u32 next, u32 g,
+                                          bool valid, u32 begin, u32 end, u64 key, int &deepest)
 {
     Control &c = *a.ctl;
-    if (c.overflow) return;
-    const u32 start = c.levelStart[l], count = c.levelCount[l];
+    const int l = 3 * level, lane = threadIdx.x & 31, d = lane & 7;
+    const auto splits = [&](u32 count, int depth) { return count > bucket && unsigned(depth) < maxDepth; };
+    // particles of the slot and of the wider nodes that hold it
+    const u32 x1 = end - begin;
+    const u32 x2 = x1 + __shfl_xor_sync(0xffffffffu, x1, 1);
+    const u32 x4 = x2 + __shfl_xor_sync(0xffffffffu, x2, 2);
+    const bool half = valid && splits(x4, l + 1), quarter = half && splits(x2, l + 2);
+    const bool high = quarter && splits(x1, l + 3);
+    const bool starts = valid && (quarter || (half ? (d & 1) == 0 : (d & 3) == 0));
+    const unsigned highs = __ballot_sync(0xffffffffu, high), starting = __ballot_sync(0xffffffffu, starts);
+    const unsigned halves = __ballot_sync(0xffffffffu, half), quarters = __ballot_sync(0xffffffffu, quarter);
+    if (quarters) deepest = max(deepest, l + 3);
+    else if (halves) deepest = max(deepest, l + 2);
+    else deepest = max(deepest, l + 1);
+    u32 base = 0;
+    if (lane == 0 && highs) base = atomicAdd(&c.levelCount[level + 1], u32(__popc(highs)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (!valid) return;
+    u32 slot = starts ? kLeaf : kInside;
+    if (high)
+    {
+        const u32 gc = next + base + u32(__popc(highs & sort::laneMaskLt()));
+        if (gc < a.cap)
+        {
+            const u64 ck = key + u64(d) * depthRange(l + 3);
+            uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * lb::kRow);
+            crow[0] = make_uint4(u32(ck), u32(ck >> 32), begin, 0u);
+            crow[2] = make_uint4(0u, 0u, end, 0u);
+            a.parent[gc] = g;
+            a.offset[gc] = lb::kPending;
+            slot = gc;
+        }
+        else
+        {
+            c.overflow = 1;
+        }
+    }
+    a.child[size_t(g) * 8 + d] = slot;
+    if (d != 0) return;
+    const u32 s8 = (starting >> lane) & 0xffu, h8 = (highs >> lane) & 0xffu;
+    a.rows[size_t(g) * lb::kRow + 11] = s8 | (h8 << 8);
+    a.sub[g] = (u64(__popc(h8)) << lb::kSubShift) | u32(__popc(s8) - __popc(h8));
+}
+
+// The units of a level, by a whole grid: on levels of few units a CTA per
+// unit, a warp per inner boundary (sEnds: 7 words of the CTA), else a lane per
+// slot.
+__device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, int level, unsigned bucket,
+                                          unsigned maxDepth, u32 start, u32 count, u32 *sEnds, int &deepest)
+{
     const u32 next = start + count;
-    if (blockIdx.x == 0 && threadIdx.x == 0) c.levelStart[l + 1] = next;
-    const u64 half = depthRange(l + 1);
-    const bool deeper = unsigned(l + 1) < maxDepth;  // children at depth l + 1 may split
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u64 range = depthRange(3 * level + 3);
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->levelStart[level + 1] = next;
     if (count <= kWideUnits)
     {
-        // a warp per unit: 33-way searches over the unit's keys
-        const u32 warps = gridDim.x * (blockDim.x >> 5);
-        for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps)
+        static_assert(kThreads / 32 >= 7, "a warp per inner boundary");
+        for (u32 i = blockIdx.x; i < count; i += gridDim.x)
         {
-            const u32 g = start + i;
-            const uint4 r = a.rows[g];
-            const u64 key = (u64(r.y) << 32) | r.x;
-            const u32 m = warpLowerBound(idx.keys, r.z, r.w, key + half, lane);
-            if (lane != 0) continue;
-            a.mid[g] = m;
-            const u32 cnt[2] = {m - r.z, r.w - m};
-            const u32 inner = (cnt[0] > bucket && deeper ? 1u : 0u) + (cnt[1] > bucket && deeper ? 1u : 0u);
-            a.sub[g] = (u64(inner) << lb::kSubShift) | (2u - inner);
-            for (int s = 0; s < 2; ++s)
+            u32 *row = a.rows + size_t(start + i) * lb::kRow;
+            const u32 lo = row[2], hi = row[10];
+            const u64 key = lb::rowKey(row);
+            if (warp < 7)
             {
-                u32 slot = kLeaf;
-                if (cnt[s] > bucket && deeper)
+                const u32 r = lb::warpBoundaryIn(idx, lo, hi, key + u64(warp + 1) * range, lane);
+                if (lane == 0)
                 {
-                    const u32 gc = next + atomicAdd(&c.levelCount[l + 1], 1u);
-                    if (gc < a.cap)
-                    {
-                        const u64 ck = key + u64(s) * half;
-                        a.rows[gc] = make_uint4(u32(ck), u32(ck >> 32), s ? m : r.z, s ? r.w : m);
-                        a.parent[gc] = g;
-                        a.offset[gc] = lb::kPending;
-                        slot = gc;
-                    }
-                    else
-                    {
-                        c.overflow = 1;
-                    }
+                    row[3 + warp] = r;
+                    sEnds[warp] = r;
                 }
-                a.child[size_t(g) * 2 + s] = slot;
             }
+            __syncthreads();
+            if (warp == 0)
+            {
+                const int d = lane & 7;
+                growSlots(a, level, bucket, maxDepth, next, start + i, lane < 8, d ? sEnds[d - 1] : lo,
+                          d < 7 ? sEnds[d] : hi, key, deepest);
+            }
+            __syncthreads();
         }
         return;
     }
-    const u32 stride = gridDim.x * blockDim.x;
-    for (u32 i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < count; i0 += stride)
+    const size_t total = size_t(count) * 8;
+    for (size_t e0 = size_t(blockIdx.x) * kThreads + warp * 32; e0 < total; e0 += size_t(gridDim.x) * kThreads)
     {
-        const u32 i = i0 + u32(lane);
-        const bool valid = i < count;
-        const u32 g = start + (valid ? i : 0);
-        uint4 r = make_uint4(0u, 0u, 0u, 0u);
-        u64 key = 0;
-        u32 m = 0;
-        unsigned high = 0;
-        if (valid)
+        const size_t e = e0 + lane;
+        const bool valid = e < total;
+        const u32 g = start + u32(valid ? e >> 3 : 0);
+        const int d = lane & 7;
+        u32 *row = a.rows + size_t(g) * lb::kRow;
+        const u32 lo = row[2], hi = row[10];
+        const u64 key = lb::rowKey(row);
+        u32 end = hi;
+        if (valid && d < 7)
         {
-            r = a.rows[g];
-            key = (u64(r.y) << 32) | r.x;
-            m = lb::boundaryIn(idx, r.z, r.w, key + half);
-            a.mid[g] = m;
-            if (m - r.z > bucket && deeper) high |= 1u;
-            if (r.w - m > bucket && deeper) high |= 2u;
+            end = lb::boundaryIn(idx, lo, hi, key + u64(d + 1) * range);
+            row[3 + d] = end;
         }
-        // slots of the warp's new units: one atomic add per warp
-        const u32 nHigh = u32(__popc(high));
-        u32 incl = nHigh;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1)
-        {
-            const u32 t = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += t;
-        }
-        u32 base = 0;
-        if (lane == 31 && incl) base = atomicAdd(&c.levelCount[l + 1], incl);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        if (!valid) continue;
-        a.sub[g] = (u64(nHigh) << lb::kSubShift) | (2u - nHigh);
-        u32 rank = base + incl - nHigh;
-        for (int s = 0; s < 2; ++s)
-        {
-            u32 slot = kLeaf;
-            if (high & (1u << s))
-            {
-                const u32 gc = next + rank++;
-                if (gc < a.cap)
-                {
-                    const u64 ck = key + u64(s) * half;
-                    a.rows[gc] = make_uint4(u32(ck), u32(ck >> 32), s ? m : r.z, s ? r.w : m);
-                    a.parent[gc] = g;
-                    a.offset[gc] = lb::kPending;
-                    slot = gc;
-                }
-                else
-                {
-                    c.overflow = 1;
-                }
-            }
-            a.child[size_t(g) * 2 + s] = slot;
-        }
+        const u32 prev = __shfl_up_sync(0xffffffffu, end, 1, 8);
+        growSlots(a, level, bucket, maxDepth, next, g, valid, d ? prev : lo, end, key, deepest);
     }
 }
 
-// The leaves below every unit (lb::subtreeKernel for two children): a unit of
-// two leaves starts, and the child of a unit that comes last takes the total
-// on.  `levels`: the depths the build expanded; units below them mean the
-// build is incomplete, and nothing is counted or placed.
-static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int levels)
+// The leaves below every unit (lb::countSubtrees): a unit without units below
+// it starts, and the unit below another that comes last takes the total on.
+__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
 {
-    const Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow) return;
-    const u32 total = c.levelStart[levels];
     for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
-        // (a unit with internal children holds 3 leaves or more when they have come)
+        if (a.rows[size_t(g) * lb::kRow + 11] >> 8) continue;
         u64 n = sort::ldRelaxed(a.sub + g);
-        if (n != 2) continue;
         for (u32 u = g; u != 0;)
         {
             u = a.parent[u];
@@ -223,48 +228,54 @@ static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int le
     }
 }
 
-// K, B and the count of the leaf children of every unit, and the first leaf
-// index of the internal ones (lb::placeKernel for two children: chunks of one
-// depth's units in order, a thread per unit; a unit waits for its own place,
-// which its parent's chunk writes).
-constexpr u32 kPlaceChunk = kThreads;
-static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, int levels, u32 capacity)
+// K, B and the count of the leaves that start in every unit, and the first
+// leaf index of the units below (lb::placeChunks: chunks of one level's units
+// in order, a lane per slot; a unit waits for its own place, which its
+// parent's chunk writes).
+constexpr u32 kPlaceChunk = kThreads / 8;
+__device__ __forceinline__ void placeChunks(const Arena &a, u64 *K, u32 *B, u32 *N, int levels, u32 capacity, u32 &sChunk)
 {
-    __shared__ u32 sChunk;
     Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow | c.error) return;
+    const int lane = threadIdx.x & 31, d = lane & 7;
     u32 level = 0, levelChunk = 0;  // chunks before `level`
     for (;;)
     {
         __syncthreads();
         // (after a wait that gave up: no more chunks)
-        if (threadIdx.x == 0)
-            sChunk = *static_cast<volatile int *>(&c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
+        if (threadIdx.x == 0) sChunk = vload(c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
         __syncthreads();
         const u32 chunk = sChunk;
         u32 count = 0;
         for (; level < u32(levels); ++level)
         {
-            count = c.levelCount[level];
+            count = vload(c.levelCount[level]);
             const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
             if (chunk < levelChunk + chunks) break;
             levelChunk += chunks;
         }
         if (level >= u32(levels)) return;
-        const u32 i = (chunk - levelChunk) * kPlaceChunk + threadIdx.x;
+        const u32 i = (chunk - levelChunk) * kPlaceChunk + (threadIdx.x >> 3);
         const bool valid = i < count;
-        const u32 g = c.levelStart[level] + (valid ? i : 0);
-        const u64 half = depthRange(int(level) + 1);
-        const uint4 r = a.rows[g];
-        const u64 key = (u64(r.y) << 32) | r.x;
-        const u32 m = a.mid[g];
-        const u32 ch[2] = {a.child[size_t(g) * 2], a.child[size_t(g) * 2 + 1]};
-        const u32 below = ch[0] == kLeaf ? 1u : u32(a.sub[ch[0]]);
-        u32 o = 0;
+        const u32 g = vload(c.levelStart[level]) + (valid ? i : 0);
+        const u32 *row = a.rows + size_t(g) * lb::kRow;
+        const u32 ch = valid ? a.child[size_t(g) * 8 + d] : kInside;
+        const u32 mine = ch == kLeaf ? 1u : ch == kInside ? 0u : u32(a.sub[ch]);
+        const u32 begin = row[2 + d], later = (row[11] & 0xffu) >> (d + 1);  // starts of the slots after d
+        const u32 end = row[2 + (later ? d + __ffs(int(later)) : 8)];
+        const u64 key = lb::rowKey(row) + u64(d) * depthRange(3 * int(level) + 3);
+        // exclusive prefix of the leaf counts within the unit's 8 lanes
+        u32 inc = mine;
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1)
+        {
+            const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
+            if (d >= off) inc += t;
+        }
+        u32 first = 0;
         for (unsigned spins = 0;; ++spins)
         {
-            o = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
-            if (!__any_sync(0xffffffffu, o == lb::kPending)) break;
+            first = valid ? vload(a.offset[g]) : 0u;
+            if (!__any_sync(0xffffffffu, first == lb::kPending)) break;
             if (spins > lb::kPlaceSpins)
             {
                 c.error = kErrLookback;
@@ -272,31 +283,36 @@ static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, 
             }
             if (spins > 64) __nanosleep(64);
         }
-        if (!valid || o == lb::kPending) continue;
-        const u32 lo[2] = {r.z, m}, hi[2] = {m, r.w};
-        for (int s = 0; s < 2; ++s, o += below)
+        if (first == lb::kPending || ch == kInside) continue;
+        const u32 o = first + inc - mine;
+        if (ch != kLeaf)
         {
-            if (ch[s] != kLeaf)
-            {
-                *static_cast<volatile u32 *>(a.offset + ch[s]) = o;
-            }
-            else if (o >= capacity)
-            {
-                c.placeOverflow = 1;  // the host grows the leaf arrays and places again
-            }
-            else
-            {
-                K[o] = key + u64(s) * half;
-                B[o] = lo[s];
-                N[o] = hi[s] - lo[s];
-            }
+            *static_cast<volatile u32 *>(a.offset + ch) = o;
+        }
+        else if (o >= capacity)
+        {
+            c.placeOverflow = 1;  // the host grows the leaf arrays and places again
+        }
+        else
+        {
+            K[o] = key;
+            B[o] = begin;
+            N[o] = end - begin;
         }
     }
 }
 
+static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, u32 capacity)
+{
+    __shared__ u32 sChunk;
+    const Control &c = *a.ctl;
+    if (c.overflow | c.error) return;
+    placeChunks(a, K, B, N, kLevels, capacity, sChunk);
+}
+
 // The finished tree: its sentinel and the state the reference's passes end
 // with (the last pass changes nothing: converged, one more pass counted).
-static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int leaves, int passes, long long logicalCap)
+__device__ __forceinline__ void finishState(const rb::TreeBufs &tb, int leaves, int passes, long long logicalCap)
 {
     DeviceState *st = tb.st;
     tb.K[0][leaves] = kMaxKey;
@@ -312,6 +328,68 @@ static __global__ void finishKernel(Arena a, rb::TreeBufs tb, int leaves, int pa
     st->overflow = 0;
     st->dirtyCount = 0;
     st->logicalCap = logicalCap;
+}
+
+static __global__ void finishKernel(rb::TreeBufs tb, int leaves, int passes, long long logicalCap)
+{
+    finishState(tb, leaves, passes, logicalCap);
+}
+
+// Leaf capacity after a build that ends with `leaves` leaves.
+__host__ __device__ __forceinline__ long long grownCapacity(long long c, long long leaves)
+{
+    if (c < 1) c = 1;
+    while (leaves > c) c += (c + 3) / 4;
+    return c;
+}
+
+struct BuildArgs
+{
+    Arena a;  // (control block zero on entry)
+    KeyIndex idx;
+    rb::TreeBufs tb;
+    const u64 *P;
+    size_t n;
+    unsigned bucket, maxDepth;
+    u32 capacity;           // leaves the leaf arrays hold
+    long long logicalCap;   // the reference's leaf capacity before the build
+};
+
+// The whole build in one cooperative launch.  Bound by the latency of its
+// steps: 33 depths of an 8Mi k-d tree are 11 levels here; with a launch per
+// depth they took 190 us and 34 gaps, the subtree counts 33 us and the
+// placement 28 us, whose chains of dependent steps are a third as long now.
+// (CTAs decide at the barriers as in lb::leafBuildKernel.)
+static __global__ void __launch_bounds__(kThreads, 4) buildKernel(BuildArgs p)
+{
+    __shared__ u32 sEnds[8];
+    __shared__ u32 sChunk;
+    const Arena &a = p.a;
+    Control &c = *a.ctl;
+    if (blockIdx.x == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, p.maxDepth);
+    if (!gridBarrier(&c.bar)) return;
+    int levels = 0, deepest = 0;
+    for (; levels < kLevels; ++levels)
+    {
+        const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
+        if (count == 0 || count > a.cap - start) break;
+        growUnits(a, p.idx, levels, p.bucket, p.maxDepth, start, count, sEnds, deepest);
+        if (!gridBarrier(&c.bar)) return;
+    }
+    if ((threadIdx.x & 31) == 0 && deepest) atomicMax(&c.depths, deepest);
+    countSubtrees(a, levels ? vload(c.levelStart[levels]) : 0u);
+    if (!gridBarrier(&c.bar)) return;
+    if (vload(c.overflow)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        const u32 leaves = levels ? u32(vload(a.sub[0])) : 1u;
+        c.leaves = leaves;
+        c.active = p.tb.st->numActiveParticles;
+        c.stateError = p.tb.st->error;
+        if (leaves > p.capacity) c.placeOverflow = 1;
+        else finishState(p.tb, int(leaves), vload(c.depths), grownCapacity(p.logicalCap, (long long)leaves));
+    }
+    placeChunks(a, p.tb.K[0], p.tb.B[0], p.tb.N[0], levels, p.capacity, sChunk);
 }
 }  // namespace bl
 }  // namespace aot

@@ -922,9 +922,8 @@ struct TreeEngine::Impl
     unsigned char *lvHost = nullptr; // pinned: the level build's one readback
     size_t lvHostBytes = 0;
     // binary tree by levels (binlevel.cuh)
-    DevMem blRows, blMid, blChild, blSub, blParent, blOffset, blCtl;
+    DevMem blRows, blChild, blSub, blParent, blOffset, blCtl;
     size_t blCap = 0;
-    int blLevels = bl::kLevels;      // depths the last binary build needed, with one to spare
     bl::Control *blHost = nullptr;   // pinned readback
     size_t blHostBytes = 0;
     u32 nodeSlots = 0;
@@ -1961,100 +1960,85 @@ bool TreeEngine::binaryLevelBuild()
     if (cfg_.maxDepth > 63) return false;
     cudaStream_t s = cfg_.stream;
     Impl &m = *m_;
-    const unsigned blocks = unsigned(smCount()) * 4u;
-    const KeyIndex idx = m.keyIndex(n_);
-    const u64 *P = m.P[0].as<u64>();
-    size_t cap = std::max<size_t>(m.blCap, 2 * (n_ / std::max(1u, cfg_.bucket)) + 4096);
-    // pinned readback: the control block, then the root's subtree leaf count
-    constexpr size_t kLeavesAt = (sizeof(bl::Control) + 15) & ~size_t(15);
-    if (!m.blHost) m.blHost = static_cast<bl::Control *>(blockcache::takeHost(kLeavesAt + 16, &m.blHostBytes));
+    // a CTA per unit of a typical level (as octreeLevelBuild), as many as fit
+    int perSm = 0;
+    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, bl::buildKernel, bl::kThreads, 0));
+    if (perSm <= 0) return false;
+    const size_t buckets = n_ / std::max<size_t>(cfg_.bucket, 1);
+    const unsigned grid =
+        unsigned(std::min<size_t>(size_t(std::min(perSm, 4)) * size_t(smCount()), buckets / 2 + 16));
+    size_t cap = std::max<size_t>(m.blCap, buckets + 4096);
+    if (!m.blHost) m.blHost = static_cast<bl::Control *>(blockcache::takeHost(sizeof(bl::Control), &m.blHostBytes));
     const bl::Control &hc = *m.blHost;
     for (;;)
     {
         if (cap >= (size_t(1) << 31)) return false;
-        m.blRows.reserve(cap * sizeof(uint4), s);
-        m.blMid.reserve(cap * sizeof(u32), s);
-        m.blChild.reserve(cap * 2 * sizeof(u32), s);
+        m.blRows.reserve(cap * lb::kRow * sizeof(u32), s);
+        m.blChild.reserve(cap * 8 * sizeof(u32), s);
         m.blSub.reserve(cap * sizeof(u64), s);
         m.blParent.reserve(cap * sizeof(u32), s);
         m.blOffset.reserve(cap * sizeof(u32), s);
         m.blCtl.reserve(sizeof(bl::Control), s);
         m.blCap = cap;
-        bl::Arena a{};
-        a.rows = m.blRows.as<uint4>();
-        a.mid = m.blMid.as<u32>();
+        bl::BuildArgs p{};
+        bl::Arena &a = p.a;
+        a.rows = m.blRows.as<u32>();
         a.child = m.blChild.as<u32>();
         a.sub = m.blSub.as<u64>();
         a.parent = m.blParent.as<u32>();
         a.offset = m.blOffset.as<u32>();
         a.ctl = m.blCtl.as<bl::Control>();
         a.cap = u32(cap);
+        p.idx = m.keyIndex(n_);
+        p.tb = m.bufs();
+        p.P = m.P[0].as<u64>();
+        p.n = n_;
+        p.bucket = cfg_.bucket;
+        p.maxDepth = cfg_.maxDepth;
+        p.capacity = u32(physCap_);
+        p.logicalCap = (long long)leafCapacity_;
         AOT_CHECK(cudaMemsetAsync(m.blCtl.p, 0, sizeof(bl::Control), s));
-        bl::rootKernel<<<1, 32, 0, s>>>(a, m.bufs(), P, n_, cfg_.bucket, cfg_.maxDepth), noteLaunch();
-        // as many depths as the last build needed (all 64 the first time);
-        // the readback tells whether the tree went deeper
-        const int levels = std::max(1, std::min(bl::kLevels, m.blLevels));
-        for (int l = 0; l < levels; ++l)
-            bl::levelKernel<<<blocks * 2, bl::kThreads, 0, s>>>(a, idx, l, cfg_.bucket, cfg_.maxDepth), noteLaunch();
-        bl::subtreeKernel<<<blocks, bl::kThreads, 0, s>>>(a, levels), noteLaunch();
-        auto place = [&]() {
-            const rb::TreeBufs tb = m.bufs();
-            bl::placeKernel<<<blocks, bl::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.N[0], levels, u32(physCap_)), noteLaunch();
-            AOT_LAUNCH_CHECK();
-        };
-        place();
+        void *args[] = {&p};
+        AOT_CHECK(cudaLaunchCooperativeKernel(bl::buildKernel, dim3(grid), dim3(bl::kThreads), args, 0, s));
+        noteLaunch();
         AOT_CHECK(cudaMemcpyAsync(m.blHost, m.blCtl.p, sizeof(bl::Control), cudaMemcpyDeviceToHost, s));
-        unsigned char *leavesHost = reinterpret_cast<unsigned char *>(m.blHost) + kLeavesAt;
-        AOT_CHECK(cudaMemcpyAsync(leavesHost, a.sub, sizeof(u32), cudaMemcpyDeviceToHost, s));  // the root's leaves
-        AOT_CHECK(cudaMemcpyAsync(m.hst, m.st, sizeof(DeviceState), cudaMemcpyDeviceToHost, s));
         waitStream(s);
-        u32 rootLeaves = 1;
-        if (m.hst->error | hc.error)
-            throw std::runtime_error("adaptive_octree: a device scan gave up waiting (bounded look-back)");
+        if (hc.bar.error) throw std::runtime_error("adaptive_octree: a grid barrier of the level build gave up waiting");
         if (hc.overflow)
         {
             cap *= 2;
             continue;
         }
-        if (hc.levelCount[levels] != 0)
-        {
-            m.blLevels = bl::kLevels;  // deeper than the last build: all depths again
-            continue;
-        }
-        int deepest = -1;  // deepest depth holding units
-        for (int l = 0; l < levels; ++l)
-            if (hc.levelCount[l]) deepest = l;
-        if (deepest >= 0) std::memcpy(&rootLeaves, leavesHost, sizeof(u32));
+        if (hc.stateError | hc.error)
+            throw std::runtime_error("adaptive_octree: a device scan gave up waiting (bounded look-back)");
+        // one pass per depth of internal nodes
+        const u32 leaves = hc.leaves;
+        const int passes = hc.depths;
+        const long long c = bl::grownCapacity((long long)leafCapacity_, (long long)leaves);
         if (hc.placeOverflow)
         {
-            ensurePhysical(rootLeaves);
+            ensurePhysical(leaves);
+            const rb::TreeBufs tb = m.bufs();
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeNext, 0, sizeof(u32), s));
-            place();
+            bl::placeKernel<<<unsigned(smCount()) * 4u, bl::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.N[0], u32(physCap_)),
+                noteLaunch();
+            bl::finishKernel<<<1, 1, 0, s>>>(tb, int(leaves), passes, c), noteLaunch();
+            AOT_LAUNCH_CHECK();
         }
-        // one pass per depth of units; the capacity's 25 % steps end at the
-        // first step at or above the final leaf count (the counts only grow)
-        const int passes = deepest + 1;
-        long long c = std::max<long long>((long long)leafCapacity_, 1);
-        while ((long long)rootLeaves > c) c += (c + 3) / 4;
-        m.blLevels = std::min(bl::kLevels, deepest + 2);
-        bl::finishKernel<<<1, 1, 0, s>>>(a, m.bufs(), int(rootLeaves), passes, c), noteLaunch();
-        AOT_LAUNCH_CHECK();
         // the host mirror of the finished state
         DeviceState &h = *m.hst;
-        h.numLeaves = h.newNumLeaves = int(rootLeaves);
-        h.numNodes = (int(rootLeaves) - 1) * 2 + 1;
-        h.proposal = (long long)rootLeaves;
+        h = DeviceState{};
+        h.numActiveParticles = hc.active;
+        h.numLeaves = h.newNumLeaves = int(leaves);
+        h.numNodes = (int(leaves) - 1) * 2 + 1;
+        h.proposal = (long long)leaves;
         h.iteration = passes;
         h.rounds = passes + 1;
         h.converged = 1;
-        h.changed = h.needsResize = 0;
-        h.activeBuffer = 0;
-        h.overflow = 0;
-        h.dirtyCount = 0;
         h.logicalCap = c;
         buildRounds_ = passes;
-        hostLeaves_ = rootLeaves;
+        hostLeaves_ = leaves;
         leafCapacity_ = size_t(c);
         ensurePhysical(leafCapacity_);
         return true;
