@@ -45,17 +45,18 @@ struct Control
     int overflow;       // the unit arena is too small
     int placeOverflow;  // more leaves than the leaf arrays hold
     int error;          // a bounded wait gave up
-    u32 placeNext;      // next chunk of the placement
     GridBarrier bar;
     int depths;         // depths holding internal nodes
     u32 leaves;         // leaves of the tree
+    u32 units;
     u32 active;         // active particles
     int stateError;     // DeviceState::error
 };
 
 struct Arena
 {
-    u32 *rows;      // [cap][lb::kRow] key (2 words), 9 slot begins, slot masks: leaf or unit starts | units << 8
+    u32 *rows;      // [cap][lb::kRow] key (2 words), 9 slot begins, slot masks: leaf or unit starts |
+                    // units << 8 | level << 16
     u32 *child;     // [cap][8] unit index of an internal slot, kLeaf or kInside
     u32 *parent;    // [cap] parent unit
     u64 *sub;       // [cap] leaves counted below the unit | units to come << lb::kSubShift
@@ -146,7 +147,7 @@ __device__ __forceinline__ void growSlots(const Arena &a, int level, unsigned bu
     a.child[size_t(g) * 8 + d] = slot;
     if (d != 0) return;
     const u32 s8 = (starting >> lane) & 0xffu, h8 = (highs >> lane) & 0xffu;
-    a.rows[size_t(g) * lb::kRow + 11] = s8 | (h8 << 8);
+    a.rows[size_t(g) * lb::kRow + 11] = s8 | (h8 << 8) | (u32(level) << 16);
     a.sub[g] = (u64(__popc(h8)) << lb::kSubShift) | u32(__popc(s8) - __popc(h8));
 }
 
@@ -215,7 +216,7 @@ __device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
 {
     for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
-        if (a.rows[size_t(g) * lb::kRow + 11] >> 8) continue;
+        if (a.rows[size_t(g) * lb::kRow + 11] & 0xff00u) continue;
         u64 n = sort::ldRelaxed(a.sub + g);
         for (u32 u = g; u != 0;)
         {
@@ -229,40 +230,23 @@ __device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
 }
 
 // K, B and the count of the leaves that start in every unit, and the first
-// leaf index of the units below (lb::placeChunks: chunks of one level's units
-// in order, a lane per slot; a unit waits for its own place, which its
-// parent's chunk writes).
-constexpr u32 kPlaceChunk = kThreads / 8;
-__device__ __forceinline__ void placeChunks(const Arena &a, u64 *K, u32 *B, u32 *N, int levels, u32 capacity, u32 &sChunk)
+// leaf index of the units below (lb::placeUnits with a lane per slot; by a
+// grid of resident CTAs).
+__device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *N, u32 total, u32 capacity)
 {
     Control &c = *a.ctl;
     const int lane = threadIdx.x & 31, d = lane & 7;
-    u32 level = 0, levelChunk = 0;  // chunks before `level`
-    for (;;)
+    const u32 stride = gridDim.x * (kThreads / 8);
+    for (u32 g0 = blockIdx.x * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
     {
-        __syncthreads();
-        // (after a wait that gave up: no more chunks)
-        if (threadIdx.x == 0) sChunk = vload(c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
-        __syncthreads();
-        const u32 chunk = sChunk;
-        u32 count = 0;
-        for (; level < u32(levels); ++level)
-        {
-            count = vload(c.levelCount[level]);
-            const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
-            if (chunk < levelChunk + chunks) break;
-            levelChunk += chunks;
-        }
-        if (level >= u32(levels)) return;
-        const u32 i = (chunk - levelChunk) * kPlaceChunk + (threadIdx.x >> 3);
-        const bool valid = i < count;
-        const u32 g = vload(c.levelStart[level]) + (valid ? i : 0);
+        const u32 g = min(g0 + (lane >> 3), total - 1);
+        bool done = g0 + (lane >> 3) >= total;
         const u32 *row = a.rows + size_t(g) * lb::kRow;
-        const u32 ch = valid ? a.child[size_t(g) * 8 + d] : kInside;
+        const u32 word = row[11], begin = row[2 + d], later = (word & 0xffu) >> (d + 1);  // starts of the slots after d
+        const u32 ch = a.child[size_t(g) * 8 + d];
         const u32 mine = ch == kLeaf ? 1u : ch == kInside ? 0u : u32(a.sub[ch]);
-        const u32 begin = row[2 + d], later = (row[11] & 0xffu) >> (d + 1);  // starts of the slots after d
         const u32 end = row[2 + (later ? d + __ffs(int(later)) : 8)];
-        const u64 key = lb::rowKey(row) + u64(d) * depthRange(3 * int(level) + 3);
+        const u64 key = lb::rowKey(row) + u64(d) * depthRange(3 * int(word >> 16) + 3);
         // exclusive prefix of the leaf counts within the unit's 8 lanes
         u32 inc = mine;
 #pragma unroll
@@ -271,43 +255,49 @@ __device__ __forceinline__ void placeChunks(const Arena &a, u64 *K, u32 *B, u32 
             const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
             if (d >= off) inc += t;
         }
-        u32 first = 0;
         for (unsigned spins = 0;; ++spins)
         {
-            first = valid ? vload(a.offset[g]) : 0u;
-            if (!__any_sync(0xffffffffu, first == lb::kPending)) break;
-            if (spins > lb::kPlaceSpins)
+            if (!done)
+            {
+                const u32 first = vload(a.offset[g]);
+                if (first != lb::kPending)
+                {
+                    done = true;
+                    const u32 o = first + inc - mine;
+                    if (ch == kLeaf && o >= capacity)
+                    {
+                        c.placeOverflow = 1;  // the host grows the leaf arrays and places again
+                    }
+                    else if (ch == kLeaf)
+                    {
+                        K[o] = key;
+                        B[o] = begin;
+                        N[o] = end - begin;
+                    }
+                    else if (ch != kInside)
+                    {
+                        *static_cast<volatile u32 *>(a.offset + ch) = o;
+                    }
+                }
+            }
+            if (__all_sync(0xffffffffu, done)) break;
+            if (spins < 64) continue;
+            if (spins > lb::kPlaceSpins || vload(c.error))
             {
                 c.error = kErrLookback;
-                break;
+                return;
             }
-            if (spins > 64) __nanosleep(64);
-        }
-        if (first == lb::kPending || ch == kInside) continue;
-        const u32 o = first + inc - mine;
-        if (ch != kLeaf)
-        {
-            *static_cast<volatile u32 *>(a.offset + ch) = o;
-        }
-        else if (o >= capacity)
-        {
-            c.placeOverflow = 1;  // the host grows the leaf arrays and places again
-        }
-        else
-        {
-            K[o] = key;
-            B[o] = begin;
-            N[o] = end - begin;
+            __nanosleep(64);
         }
     }
 }
 
-static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, u32 capacity)
+// (cooperative)
+static __global__ void __launch_bounds__(kThreads, 4) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, u32 total, u32 capacity)
 {
-    __shared__ u32 sChunk;
     const Control &c = *a.ctl;
     if (c.overflow | c.error) return;
-    placeChunks(a, K, B, N, kLevels, capacity, sChunk);
+    placeUnits(a, K, B, N, total, capacity);
 }
 
 // The finished tree: its sentinel and the state the reference's passes end
@@ -363,7 +353,6 @@ struct BuildArgs
 static __global__ void __launch_bounds__(kThreads, 4) buildKernel(BuildArgs p)
 {
     __shared__ u32 sEnds[8];
-    __shared__ u32 sChunk;
     const Arena &a = p.a;
     Control &c = *a.ctl;
     if (blockIdx.x == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, p.maxDepth);
@@ -377,19 +366,21 @@ static __global__ void __launch_bounds__(kThreads, 4) buildKernel(BuildArgs p)
         if (!gridBarrier(&c.bar)) return;
     }
     if ((threadIdx.x & 31) == 0 && deepest) atomicMax(&c.depths, deepest);
-    countSubtrees(a, levels ? vload(c.levelStart[levels]) : 0u);
+    const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
+    countSubtrees(a, total);
     if (!gridBarrier(&c.bar)) return;
     if (vload(c.overflow)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         const u32 leaves = levels ? u32(vload(a.sub[0])) : 1u;
         c.leaves = leaves;
+        c.units = total;
         c.active = p.tb.st->numActiveParticles;
         c.stateError = p.tb.st->error;
         if (leaves > p.capacity) c.placeOverflow = 1;
         else finishState(p.tb, int(leaves), vload(c.depths), grownCapacity(p.logicalCap, (long long)leaves));
     }
-    placeChunks(a, p.tb.K[0], p.tb.B[0], p.tb.N[0], levels, p.capacity, sChunk);
+    placeUnits(a, p.tb.K[0], p.tb.B[0], p.tb.N[0], total, p.capacity);
 }
 }  // namespace bl
 }  // namespace aot

@@ -1715,6 +1715,19 @@ void TreeEngine::setBuildMode(int mode)
     buildMode_ = mode;
 }
 
+namespace
+{
+// A cooperative launch of at most `want` CTAs, as many as fit at once.
+void launchResident(const void *fn, void **args, int threads, unsigned want, cudaStream_t s)
+{
+    int perSm = 0;
+    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, threads, 0));
+    const unsigned grid = std::max(1u, std::min(want, unsigned(perSm) * unsigned(smCount())));
+    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(unsigned(threads)), args, 0, s));
+    noteLaunch();
+}
+}  // namespace
+
 // The converged octree, level by level (levelbuild.cuh).  The tree is the
 // one the reference's build rounds converge to; the round history (leaves
 // after each round that changed the tree) comes from the per-region counts.
@@ -1760,20 +1773,15 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         // placement; one readback at the end checks that no deeper level
         // was left out.
         const int levels = nf ? std::max(1, std::min(int(kOctLevels), m.lvLevels)) : int(kOctLevels);
-        auto place = [&]() {
-            const rb::TreeBufs tb = m.bufs();
-            const u32 room = u32(physCap_);
-            const unsigned grid = blocks * wide;
-            if (nf && cfg_.hilbert)
-                lb::placeKernel<true, true><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0], levels, room),
-                    noteLaunch();
-            else if (nf)
-                lb::placeKernel<true, false><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.NF[0], tb.N[0], levels, room),
-                    noteLaunch();
-            else
-                lb::placeKernel<false, false><<<grid, lb::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], nullptr, tb.N[0], levels, room),
-                    noteLaunch();
-            AOT_LAUNCH_CHECK();
+        auto place = [&](int expanded) {
+            rb::TreeBufs tb = m.bufs();
+            u32 room = u32(physCap_);
+            lb::Arena arena = a;
+            const void *fn = nf && cfg_.hilbert ? reinterpret_cast<const void *>(&lb::placeKernel<true, true>)
+                             : nf               ? reinterpret_cast<const void *>(&lb::placeKernel<true, false>)
+                                                : reinterpret_cast<const void *>(&lb::placeKernel<false, false>);
+            void *args[] = {&arena, &tb.K[0], &tb.B[0], &tb.NF[0], &tb.N[0], &expanded, &room};
+            launchResident(fn, args, lb::kThreads, unsigned(smCount()) * 8u, s);
         };
         u32 rootLeaves = 1;
         if (nf)
@@ -1796,7 +1804,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
             }
             lb::subtreeKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
             AOT_LAUNCH_CHECK();
-            place();
+            place(levels);
             // the round history is needed before finishKernel writes it; read
             // everything once
             // (with the device state: its active count, set by the root kernel)
@@ -1867,8 +1875,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         {
             ensurePhysical(rootLeaves);
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
-            AOT_CHECK(cudaMemsetAsync(&a.ctl->placeNext, 0, sizeof(u32), s));
-            place();
+            place(deepest + 1);
         }
         hostLeaves_ = rootLeaves;
         m.lvLevels = std::min(int(kOctLevels), deepest + 2);
@@ -2018,11 +2025,10 @@ bool TreeEngine::binaryLevelBuild()
         if (hc.placeOverflow)
         {
             ensurePhysical(leaves);
-            const rb::TreeBufs tb = m.bufs();
-            AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
-            AOT_CHECK(cudaMemsetAsync(&a.ctl->placeNext, 0, sizeof(u32), s));
-            bl::placeKernel<<<unsigned(smCount()) * 4u, bl::kThreads, 0, s>>>(a, tb.K[0], tb.B[0], tb.N[0], u32(physCap_)),
-                noteLaunch();
+            rb::TreeBufs tb = m.bufs();
+            u32 units = hc.units, room = u32(physCap_);
+            void *again[] = {&a, &tb.K[0], &tb.B[0], &tb.N[0], &units, &room};
+            launchResident(reinterpret_cast<const void *>(&bl::placeKernel), again, bl::kThreads, unsigned(smCount()) * 4u, s);
             bl::finishKernel<<<1, 1, 0, s>>>(tb, int(leaves), passes, c), noteLaunch();
             AOT_LAUNCH_CHECK();
         }

@@ -56,10 +56,10 @@ struct LevelArgs
     int maxDepth;
 };
 
-static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArgs p)
+static __global__ void __launch_bounds__(lb::kThreads, 4) levelBuildKernel(LevelArgs p)
 {
     using namespace lb;
-    __shared__ u32 sEnds[8], sChunk;
+    __shared__ u32 sEnds[8];
     __shared__ u32 sBin[kContribBins];
     __shared__ unsigned long long sVal[kContribBins];
     __shared__ int sBins, sRounds;
@@ -113,7 +113,8 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         if (!gridBarrier(&ls->bar)) return;
     }
     if (vload(c.overflow) | vload(c.late)) return;
-    countSubtrees<true>(a, levels ? vload(c.levelStart[levels]) : 0u);
+    const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
+    countSubtrees<true>(a, total);
     if (!gridBarrier(&ls->bar)) return;
     // layout (CTA 0): systems one after the other, each followed by its sentinel
     if (blockIdx.x == 0)
@@ -227,8 +228,7 @@ static __global__ void __launch_bounds__(lb::kThreads) levelBuildKernel(LevelArg
         __syncthreads();
     }
     // placement (a unit's first entry comes from its parent)
-    placeChunks<false, false, true>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], levels, p.capacity, nullptr,
-                                    sChunk);
+    placeUnits<false, false, true>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], total, p.capacity, nullptr);
     if (!gridBarrier(&ls->bar)) return;
     const i64 E = vload(ls->entries);
     for (i64 i = rank; i < E; i += size)

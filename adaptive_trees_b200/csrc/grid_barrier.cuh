@@ -6,22 +6,27 @@
 
 namespace aot
 {
-// Barrier words (zeroed before the launch).
+// Barrier words (zeroed before the first launch; each barrier leaves them as it
+// found them, but for the generation).
+constexpr unsigned kBarrierGroups = 8, kBarrierFlat = 192;
 struct GridBarrier
 {
-    u32 arrived;     // CTAs at the current barrier
     u32 generation;  // barriers passed
     int error;       // a wait gave up
-    int pad;
+    u32 arrived;     // CTAs (or groups) at the current barrier
+    u32 pad[13];
+    u32 group[kBarrierGroups][16];  // CTAs of each group, a word per 64 bytes
 };
 
 constexpr u32 kBarrierSpins = 1u << 22;  // polls of about 128 ns: well over 0.5 s
-constexpr u32 kBarrierHot = 64;          // polls without a pause: most barriers open within a few hundred ns
+constexpr u32 kBarrierHot = 64;          // polls without a pause: most barriers open within a microsecond
 
-// Every CTA of the grid arrives; the last one opens the next generation.  A
-// CTA that polls more than kBarrierSpins times (or sees another CTA's error)
-// records the error and leaves; the result is false for it and for every CTA
-// that reads the error after the barrier, and the kernel returns.
+// Every CTA of the grid arrives; the last one opens the next generation.  CTAs
+// of a large grid arrive in groups, the last of a group for the group: the
+// atomics on one word pass one by one, 592 of them in about 3 us.  A CTA that polls more than
+// kBarrierSpins times (or sees another CTA's error) records the error and
+// leaves; the result is false for it and for every CTA that reads the error
+// after the barrier, and the kernel returns.
 __device__ __forceinline__ bool gridBarrier(GridBarrier *b)
 {
     __shared__ int sOk;
@@ -32,7 +37,24 @@ __device__ __forceinline__ bool gridBarrier(GridBarrier *b)
         volatile int *err = &b->error;
         const u32 g = *gen;
         __threadfence();
-        if (atomicAdd(&b->arrived, 1u) == gridDim.x - 1)
+        bool last;
+        if (gridDim.x <= kBarrierFlat)
+        {
+            last = atomicAdd(&b->arrived, 1u) == gridDim.x - 1;
+        }
+        else
+        {
+            const u32 mine = blockIdx.x % kBarrierGroups;
+            const u32 members = (gridDim.x - mine + kBarrierGroups - 1) / kBarrierGroups;
+            last = atomicAdd(&b->group[mine][0], 1u) == members - 1;
+            if (last)
+            {
+                atomicExch(&b->group[mine][0], 0u);
+                __threadfence();
+                last = atomicAdd(&b->arrived, 1u) == kBarrierGroups - 1;
+            }
+        }
+        if (last)
         {
             atomicExch(&b->arrived, 0u);
             __threadfence();

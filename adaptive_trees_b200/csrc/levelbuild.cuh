@@ -65,9 +65,7 @@ struct Control
     int late;           // an arrival round beyond the tracked ones
     int error;          // a bounded wait gave up
     int placeOverflow;  // the tree has more leaves than the cornerstone buffers hold
-    u32 placeNext;      // next chunk of the placement
-    // one-launch build:
-    GridBarrier bar;
+    GridBarrier bar;    // one-launch build
     u32 leaves;         // leaves of the tree
     u32 active;         // active particles
     int stateError;     // DeviceState::error
@@ -1364,34 +1362,48 @@ static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int le
     countSubtrees<false>(a, c.levelStart[levels]);
 }
 
-// Cornerstone entries of the leaf children of the level-l units, and the
-// first leaf index of their internal children.  Eight lanes per unit, one per
-// child: a segmented scan of the children's leaf counts gives each child's
-// position, so a warp writes the entries of four units at once.
+// Cornerstone entries of the leaf children of every unit (the first `total`),
+// and the first leaf index of their internal children.  Eight lanes per unit,
+// one per child: a segmented scan of the children's leaf counts gives each
+// child's position, so a warp writes the entries of four units at once.
 // K, B (and NF, N, SEG where given) are the cornerstone arrays written: N the
 // leaf counts, SEG each leaf's tree (system) in a batch of trees.  dec: the
 // digit -> octant table of the Hilbert curve (NFCount trees keep their
 // children by octant).
+//
+// A unit waits for its own place, which its parent's warp writes; parents come
+// before their children in the arena.  The warps of the grid, all resident
+// (cooperative launches), take units in increasing order, and a warp writes
+// what is ready before it polls again (parent and child may share it), so the
+// first unit not placed is always being worked on and the waits end (they are
+// bounded all the same).  Bound by the latency of a step: child, its leaf
+// count, the poll.  Chunks of units handed out by a counter, with their levels
+// looked up, took 43 us for the 32k units of 300k NFCount particles, 166 us for
+// the 1.8 M of 16Mi and 51 us for the 133k of an 8Mi k-d tree (a kernel per
+// level before that: 36 us and 11 gaps at 300k).
 template <bool NF, bool Hilbert, bool Forest>
-__device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, int l,
-                                           u32 start, u32 count, u32 capacity, u32 rank, u32 size,
-                                           const unsigned char *dec)
+__device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, u32 total,
+                                           u32 capacity, const unsigned char *dec)
 {
     Control &c = *a.ctl;
-    const u64 cr = octRange(unsigned(l) + 1);
     const int lane = threadIdx.x & 31, d = lane & 7;
-    const size_t total = size_t(count) * 8;
-    for (size_t e0 = rank & ~31u; e0 < total; e0 += size)
+    const u32 stride = gridDim.x * (kThreads / 8);
+    for (u32 g0 = blockIdx.x * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
     {
-        const size_t e = e0 + size_t(lane);
-        const bool valid = e < total;
-        const u32 g = start + u32(valid ? e >> 3 : 0);
-        u32 ch = valid ? a.child[size_t(g) * 8 + d] : kLeaf;
+        const u32 g = min(g0 + (lane >> 3), total - 1);
+        bool done = g0 + (lane >> 3) >= total;
+        const u32 *row = a.rows + size_t(g) * kRow;
+        const u32 reg = row[11], begin = row[2 + d], end = row[3 + d];
+        const u64 key = rowKey(row) + u64(d) * octRange(unitLevelOf(reg) + 1);
+        u32 ch = a.child[size_t(g) * 8 + d];
+        u32 val = 0, sys = 0;
+        if constexpr (NF) val = a.val[size_t(g) * 8 + d];
+        if constexpr (Forest) sys = a.usys[g];
         u32 mine = ch == kLeaf ? 1u : u32(a.sub[ch]);
         if constexpr (NF && Hilbert)
         {
             // from octants to digits within the unit's 8 lanes
-            const int from = valid ? (lane & 24) | dec[unitStateOf(a.rows[size_t(g) * kRow + 11]) * 8 + d] : lane;
+            const int from = (lane & 24) | dec[unitStateOf(reg) * 8 + d];
             ch = __shfl_sync(0xffffffffu, ch, from);
             mine = __shfl_sync(0xffffffffu, mine, from);
         }
@@ -1403,89 +1415,60 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             const u32 t = __shfl_up_sync(0xffffffffu, inc, off);
             if (d >= off) inc += t;
         }
-        // the unit's first leaf: placed by its parent, in a chunk handed out before this one
-        u32 first = 0;
         for (unsigned spins = 0;; ++spins)
         {
-            first = valid ? *static_cast<volatile const u32 *>(a.offset + g) : 0u;
-            if (!__any_sync(0xffffffffu, first == kPending)) break;
-            if (spins > kPlaceSpins)
+            if (!done)
+            {
+                const u32 first = vload(a.offset[g]);  // the unit's first leaf
+                if (first != kPending)
+                {
+                    done = true;
+                    const u32 o = first + inc - mine;
+                    if (ch != kLeaf)
+                    {
+                        *static_cast<volatile u32 *>(a.offset + ch) = o;
+                    }
+                    else if (o >= capacity)
+                    {
+                        c.placeOverflow = 1;  // the host grows the buffers and places again
+                    }
+                    else
+                    {
+                        K[o] = key;
+                        B[o] = begin;
+                        if constexpr (NF) NFo[o] = val;
+                        if (N) N[o] = end - begin;
+                        if constexpr (Forest) SEG[o] = int(sys);
+                    }
+                }
+            }
+            if (__all_sync(0xffffffffu, done)) break;
+            if (spins < 64) continue;
+            if (spins > kPlaceSpins || vload(c.error))
             {
                 c.error = kErrLookback;
                 return;
             }
-            if (spins > 64) __nanosleep(64);
-        }
-        if (!valid) continue;
-        const u32 o = first + inc - mine;
-        if (ch == kLeaf && o >= capacity)
-        {
-            c.placeOverflow = 1;  // the host grows the buffers and places again
-        }
-        else if (ch == kLeaf)
-        {
-            const u32 *row = a.rows + size_t(g) * kRow;
-            K[o] = rowKey(row) + u64(d) * cr;
-            B[o] = row[2 + d];
-            if constexpr (NF) NFo[o] = a.val[size_t(g) * 8 + d];
-            if (N) N[o] = row[3 + d] - row[2 + d];
-            if constexpr (Forest) SEG[o] = int(a.usys[g]);
-        }
-        else
-        {
-            *static_cast<volatile u32 *>(a.offset + ch) = o;
+            __nanosleep(64);
         }
     }
 }
 
-// Units of a placement chunk (one level's, so a chunk's parents lie in
-// chunks before it).
-constexpr u32 kPlaceChunk = 128;
-
-// The placement of all levels (the first `levels`) at once: CTAs take chunks
-// of units in level order from a counter; a unit waits for its own place,
-// which its parent's chunk writes.  Chunks are handed out in order to running
-// CTAs and wait for earlier ones only, so the waits end (they are bounded all
-// the same).  A kernel per level: 36 us and 11 gaps at 300k particles.
-template <bool NF, bool Hilbert, bool Forest>
-__device__ __forceinline__ void placeChunks(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, int levels,
-                                            u32 capacity, const unsigned char *dec, u32 &sChunk)
-{
-    Control &c = *a.ctl;
-    u32 level = 0, levelChunk = 0;  // chunks before `level`
-    for (;;)
-    {
-        __syncthreads();
-        // (after a wait that gave up: no more chunks)
-        if (threadIdx.x == 0)
-            sChunk = *static_cast<volatile int *>(&c.error) ? 0xffffffffu : atomicAdd(&c.placeNext, 1u);
-        __syncthreads();
-        const u32 chunk = sChunk;
-        u32 count = 0;
-        for (; level < u32(levels); ++level)
-        {
-            count = vload(c.levelCount[level]);
-            const u32 chunks = (count + kPlaceChunk - 1) / kPlaceChunk;
-            if (chunk < levelChunk + chunks) break;
-            levelChunk += chunks;
-        }
-        if (level >= u32(levels)) return;
-        const u32 base = (chunk - levelChunk) * kPlaceChunk;
-        placeUnits<NF, Hilbert, Forest>(a, K, B, NFo, N, SEG, int(level), vload(c.levelStart[level]) + base,
-                                        min(kPlaceChunk, count - base), capacity, threadIdx.x, kThreads, dec);
-    }
-}
-
+// (cooperative)  `levels`: the levels the build expanded.
 template <bool NF, bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels,
-                                                               u32 capacity)
+static __global__ void __launch_bounds__(kThreads, 4)
+    placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels, u32 capacity)
 {
     __shared__ __align__(4) unsigned char sDec[48 * 8];
-    __shared__ u32 sChunk;
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    if constexpr (NF && Hilbert) copyTable(sDec, gHilbert.decOct);
-    placeChunks<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, levels, capacity, sDec, sChunk);
+    if constexpr (NF && Hilbert)
+    {
+        copyTable(sDec, gHilbert.decOct);
+        __syncthreads();
+    }
+    const u32 total = c.levelCount[0] ? c.levelStart[levels] : 0u;
+    placeUnits<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, total, capacity, sDec);
 }
 
 // The finished tree: sentinel boundary and the state of a converged build
@@ -1541,7 +1524,6 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
     __shared__ u32 sContrib[kContribBins];
     __shared__ u32 sLanded[kArrivals];
     __shared__ u32 sEnds[8];
-    __shared__ u32 sChunk;
     __shared__ int sRounds;
     const Arena &a = p.a;
     Control &c = *a.ctl;
@@ -1563,7 +1545,8 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
         if (sContrib[k]) atomicAdd(a.contrib + k, (unsigned long long)sContrib[k]);
     if (threadIdx.x < kArrivals && sLanded[threadIdx.x])
         atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
-    countSubtrees<false>(a, levels ? vload(c.levelStart[levels]) : 0u);
+    const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
+    countSubtrees<false>(a, total);
     if (!gridBarrier(&c.bar)) return;
     if (vload(c.overflow) | vload(c.late)) return;
     if (blockIdx.x == 0)
@@ -1585,8 +1568,7 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
             else if (sRounds <= int(p.maxDepth)) finishState(p.tb, int(leaves), sRounds);
         }
     }
-    placeChunks<false, false, false>(a, p.tb.K[0], p.tb.B[0], nullptr, p.tb.N[0], nullptr, levels, p.capacity, nullptr,
-                                     sChunk);
+    placeUnits<false, false, false>(a, p.tb.K[0], p.tb.B[0], nullptr, p.tb.N[0], nullptr, total, p.capacity, nullptr);
 }
 }  // namespace lb
 }  // namespace aot
