@@ -900,8 +900,10 @@ struct TreeEngine::Impl
     DevMem P[2], Perm[2], sample;
     SortArena sortArena;
     // state
-    DevMem stMem;
+    DevMem stMem;                // DeviceState, then the barrier
     DeviceState *st = nullptr;   // device (stMem)
+    GridBarrier *updateBar = nullptr;
+    static constexpr size_t kBarAt = (sizeof(DeviceState) + 255) & ~size_t(255);
     DeviceState *hst = nullptr;  // pinned mirror (block cache)
     size_t hstBytes = 0;
     cudaStream_t d2h = nullptr;
@@ -1084,9 +1086,10 @@ TreeEngine::TreeEngine(const void *x, const void *y, const void *z, size_t n, co
     prepared_ = cfg.views;
 
     // stream-ordered set-up: nothing here synchronises the device
-    m_->stMem.reserve(sizeof(DeviceState));
+    m_->stMem.reserve(Impl::kBarAt + sizeof(GridBarrier));
+    m_->updateBar = reinterpret_cast<GridBarrier *>(m_->stMem.as<unsigned char>() + Impl::kBarAt);
     m_->st = m_->stMem.as<DeviceState>();
-    AOT_CHECK(cudaMemsetAsync(m_->st, 0, sizeof(DeviceState), cfg.stream));
+    AOT_CHECK(cudaMemsetAsync(m_->st, 0, Impl::kBarAt + sizeof(GridBarrier), cfg.stream));
     m_->hst = static_cast<DeviceState *>(blockcache::takeHost(sizeof(DeviceState), &m_->hstBytes));
     std::memset(m_->hst, 0, sizeof(DeviceState));
     AOT_CHECK(cudaGetDevice(&m_->device));
@@ -2051,21 +2054,54 @@ bool TreeEngine::binaryLevelBuild()
     }
 }
 
+// Trees of at most this many leaves (their capacity) pass in one launch.  An
+// update() queued directly, launch by launch and in one, and the same from a
+// graph: octrees of 1.2k leaves 109 and 81 us (graph 69 and 69), 33k 150 and
+// 127 (125 and 114), 262k 274 and 253 (228 and 228), 2.1M 495 and 516 (440 and
+// 494); k-d trees of 1.3k leaves 152 and 85 (118 and 80), 354k 516 and 463 (451
+// and 439).
+constexpr size_t kFusedPasses = size_t(1) << 19;
+
+// The refresh, the passes and the counts of an update() in one launch
+// (rb::updateKernel).  False (nothing done) where they run launch by launch:
+// NFCount trees, and while stages are timed.
+bool TreeEngine::passesFused()
+{
+    if (cfg_.nf || profiling_) return false;
+    if (leafCapacity_ > kFusedPasses) return false;
+    const void *fn = cfg_.kind == 0 ? reinterpret_cast<const void *>(&rb::updateKernel<false>)
+                                    : reinterpret_cast<const void *>(&rb::updateKernel<true>);
+    int perSm = 0;
+    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, rb::kScanThreads, 0));
+    if (perSm <= 0) return false;
+    rb::UpdateArgs u{m_->bufs(), m_->keyIndex(n_), m_->P[0].as<u64>(), n_, m_->scanTiles + 1, cfg_.bucket, cfg_.maxDepth,
+                     cfg_.iterations, (long long)leafCapacity_, m_->updateBar};
+    // a thread per leaf, as many CTAs as fit; few meet at a barrier sooner
+    const unsigned grid = std::min(gridFor(leafCapacity_ + 1, rb::kScanThreads), unsigned(std::min(perSm, 4)) * unsigned(smCount()));
+    void *args[] = {&u};
+    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(rb::kScanThreads), args, 0, cfg_.stream));
+    noteLaunch();
+    return true;
+}
+
 void TreeEngine::update()
 {
     if (!built_) throw std::logic_error("adaptive_octree: call build() before update()");
     mark(MarkStart, 2);
     sortParticles();
     mark(MarkSorted);
-    refreshAll();
-    mark(MarkRefreshed);
-    for (unsigned i = 0; i < cfg_.iterations; ++i)
+    if (!passesFused())
     {
-        if (cfg_.kind == 0) octreePass(false, (long long)leafCapacity_);
-        else binaryPass(false, (long long)leafCapacity_);
+        refreshAll();
+        mark(MarkRefreshed);
+        for (unsigned i = 0; i < cfg_.iterations; ++i)
+        {
+            if (cfg_.kind == 0) octreePass(false, (long long)leafCapacity_);
+            else binaryPass(false, (long long)leafCapacity_);
+        }
+        mark(MarkPassed);
+        materializeCounts();
     }
-    mark(MarkPassed);
-    materializeCounts();
     buildViews(cfg_.views);
     mark(MarkEnd);
 }

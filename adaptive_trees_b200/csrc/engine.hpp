@@ -248,6 +248,7 @@ private:
     void octreePass(bool buildMode, long long limit);
     void binaryPass(bool buildMode, long long limit);
     void refreshAll();
+    bool passesFused();
     void refreshCounts(bool all, unsigned blocks);
     void refreshUnits();
     bool refreshByUnits() const;

@@ -19,6 +19,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include "sfc.cuh"
 
 namespace aot
@@ -166,12 +167,14 @@ struct DecideShared
     int changed;
 };
 
+// False (nothing done) when there is no tile left or no pass to make; a
+// persistent CTA calls it, with a __syncthreads between, until then.
 template <class Op>
-__device__ void decideScan(const Op &op, TreeBufs tb, const u64 *K, const u32 *V, const u8 *G)
+__device__ bool decideScan(const Op &op, const TreeBufs &tb, const u64 *K, const u32 *V, const u8 *G)
 {
     __shared__ DecideShared<Op> sm;
     DeviceState *st = tb.st;
-    if (halted(st) || st->needsResize) return;
+    if (halted(st) || st->needsResize) return false;
     const int L = st->numLeaves;
     const size_t entries = size_t(L) + 1;
     const u32 numTiles = u32((entries + kScanTile - 1) / kScanTile);
@@ -182,7 +185,7 @@ __device__ void decideScan(const Op &op, TreeBufs tb, const u64 *K, const u32 *V
     }
     __syncthreads();
     const u32 tile = sm.tile;
-    if (tile >= numTiles) return;
+    if (tile >= numTiles) return false;
     const long long base = (long long)tile * kScanTile, origin = base - Op::kBack;  // leaf of window position 0
     {
         // all loads in flight together (positions outside the tree repeat its ends)
@@ -195,9 +198,9 @@ __device__ void decideScan(const Op &op, TreeBufs tb, const u64 *K, const u32 *V
         {
             const long long i = origin + int(threadIdx.x) + r * kScanThreads;
             const int at = i < 0 ? 0 : i > L ? L : int(i);
-            k[r] = __ldg(K + at);
-            v[r] = __ldg(V + at);
-            if constexpr (Op::kFlags) f[r] = __ldg(G + at);
+            k[r] = K[at];
+            v[r] = V[at];
+            if constexpr (Op::kFlags) f[r] = G[at];
         }
 #pragma unroll
         for (int r = 0; r < kRounds; ++r)
@@ -267,6 +270,7 @@ __device__ void decideScan(const Op &op, TreeBufs tb, const u64 *K, const u32 *V
         for (int j = 0; j < kScanItems; ++j)
             if (first + j <= L) tb.offs[first + j] = out[j];
     }
+    return true;
 }
 
 // Warp-aggregated append of `count` consecutive items to a list; returns the
@@ -542,8 +546,7 @@ __device__ __forceinline__ void octScatterLeaf(const TreeBufs &tb, DeviceState *
 // warp of kept leaves is done then; loads behind the op code and the flag took
 // 127 instead of 92 us for 12.7 M leaves.
 template <bool NF>
-static __global__ void __launch_bounds__(kScatterThreads)
-    octScatterKernel(TreeBufs tb, long long limit, int mode, long long *history)
+__device__ __forceinline__ void octScatter(const TreeBufs &tb, long long limit, int mode, long long *history)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;  // uniform: the state does not change before the last CTA
@@ -559,6 +562,13 @@ static __global__ void __launch_bounds__(kScatterThreads)
         for (int base = w0 * 32; base < L; base += warpsTotal * 32) octScatterLeaf<NF>(tb, st, base + lane, L, a, b, total);
     }
     commitIfLast(st, limit, mode, false, history);
+}
+
+template <bool NF>
+static __global__ void __launch_bounds__(kScatterThreads)
+    octScatterKernel(TreeBufs tb, long long limit, int mode, long long *history)
+{
+    octScatter<NF>(tb, limit, mode, history);
 }
 
 // Lower bound of v in the sorted keys when `lo` is already a lower bound of a
@@ -590,7 +600,7 @@ __device__ __forceinline__ u32 lowerFrom(const KeyIndex &idx, u32 lo, u64 v)
 // the end sentinel).  This is the whole count refresh of LeafCount trees: the
 // counts are differences of B.
 template <bool All>
-static __global__ void __launch_bounds__(kRefreshThreads) octBeginKernel(TreeBufs tb, KeyIndex idx)
+__device__ __forceinline__ void octBegins(const TreeBufs &tb, const KeyIndex &idx)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;
@@ -605,6 +615,12 @@ static __global__ void __launch_bounds__(kRefreshThreads) octBeginKernel(TreeBuf
         const int i = All ? j : tb.dirty[j];
         B[i] = u32(idx.lower(K[i]));
     }
+}
+
+template <bool All>
+static __global__ void __launch_bounds__(kRefreshThreads) octBeginKernel(TreeBufs tb, KeyIndex idx)
+{
+    octBegins<All>(tb, idx);
 }
 
 // The begin index of every leaf (and B[L] = the active count) by merging the
@@ -1323,7 +1339,7 @@ static __global__ void __launch_bounds__(kRefreshThreads, 4)
 }
 
 // N[i] = B[i+1] - B[i] on the active buffer.
-static __global__ void materializeCountsKernel(TreeBufs tb)
+__device__ __forceinline__ void materializeCounts(const TreeBufs &tb)
 {
     const DeviceState *st = tb.st;
     const int a = st->activeBuffer, L = st->numLeaves;
@@ -1331,6 +1347,8 @@ static __global__ void materializeCountsKernel(TreeBufs tb)
     u32 *N = tb.n(a);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) N[i] = B[i + 1] - B[i];
 }
+
+static __global__ void materializeCountsKernel(TreeBufs tb) { materializeCounts(tb); }
 
 // --------------------------------------------------------------------------
 // Binary (kdtree3d_rebalance.cuh:61-125)
@@ -1362,8 +1380,7 @@ static __global__ void __launch_bounds__(kScanThreads) binDecideScanKernel(TreeB
     decideScan(op, tb, tb.k(a), tb.b(a), static_cast<const u8 *>(nullptr));
 }
 
-static __global__ void __launch_bounds__(kScatterThreads)
-    binScatterKernel(TreeBufs tb, long long limit, int mode)
+__device__ __forceinline__ void binScatter(const TreeBufs &tb, long long limit, int mode)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;
@@ -1409,6 +1426,12 @@ static __global__ void __launch_bounds__(kScatterThreads)
     commitIfLast(st, limit, mode, true, nullptr);
 }
 
+static __global__ void __launch_bounds__(kScatterThreads)
+    binScatterKernel(TreeBufs tb, long long limit, int mode)
+{
+    binScatter(tb, limit, mode);
+}
+
 // Binary count refresh: B of new split points (All: every boundary).  The
 // reference counts over the active prefix of P (binaryLeafCountsKernel,
 // kdtree3d_rebalance.cuh:127-138); lower bounds of keys below 2^63 agree.
@@ -1432,7 +1455,7 @@ static __global__ void binRefreshKernel(TreeBufs tb, KeyIndex idx)
 // Reset at the start of update() (resetRebalanceStateKernel,
 // octree_rebalance.cuh:62-73): changed, converged and the active count.
 // One warp (the active count by a warp-wide search).
-static __global__ void resetForUpdateKernel(DeviceState *st, const u64 *P, size_t n)
+__device__ __forceinline__ void resetForUpdate(DeviceState *st, const u64 *P, size_t n)
 {
     const unsigned active = n ? warpLowerBound(P, 0, u32(n), kMaxKey, int(threadIdx.x & 31)) : 0u;
     if (threadIdx.x != 0) return;
@@ -1443,11 +1466,83 @@ static __global__ void resetForUpdateKernel(DeviceState *st, const u64 *P, size_
     st->updatePasses = 0;
 }
 
+static __global__ void resetForUpdateKernel(DeviceState *st, const u64 *P, size_t n) { resetForUpdate(st, P, n); }
+
 // Per-pass reset of the flags the decision accumulates.
 static __global__ void beginPassKernel(DeviceState *st)
 {
     st->changed = 0;
     st->dirtyCount = 0;
+}
+
+// All of an update() after the sort in one cooperative launch, for octrees
+// that refine by leaf counts and binary trees: the reset, the begin index of
+// every leaf, `iterations` passes (decide and scan, scatter, new begins) and
+// the counts, with a grid barrier between.  A pass of its own launches is five
+// of them, each too short to pay for its launch: 30k particles 56 us and 13
+// launches after the sort.
+struct UpdateArgs
+{
+    TreeBufs tb;
+    KeyIndex idx;
+    const u64 *P;
+    size_t n, scanWords;  // scanWords: status words and tile counter of the scan
+    unsigned bucket, maxDepth, iterations;
+    long long limit;      // the reference's leaf capacity
+    GridBarrier *bar;
+};
+
+template <bool Binary>
+static __global__ void __launch_bounds__(kScanThreads, 4) updateKernel(UpdateArgs u)
+{
+    const TreeBufs &tb = u.tb;
+    DeviceState *st = tb.st;
+    const size_t rank = size_t(blockIdx.x) * blockDim.x + threadIdx.x, size = size_t(gridDim.x) * blockDim.x;
+    const auto clearScan = [&] {
+        for (size_t i = rank; i < u.scanWords; i += size) tb.scanStatus[i] = 0;
+    };
+    // (the barrier's failure is the host's to report: the state's error word)
+    const auto barrier = [&] {
+        const bool ok = gridBarrier(u.bar);
+        if (!ok && threadIdx.x == 0) atomicExch(&st->error, kErrLookback);
+        return ok;
+    };
+    if (blockIdx.x == 0 && threadIdx.x < 32) resetForUpdate(st, u.P, u.n);
+    clearScan();
+    if (!barrier()) return;
+    octBegins<true>(tb, u.idx);
+    if (!barrier()) return;
+    for (unsigned pass = 0; pass < u.iterations; ++pass)
+    {
+        if (halted(st))
+        {
+            // the passes left only reset what a decision accumulates
+            if (rank == 0) st->changed = st->dirtyCount = 0;
+            if (!barrier()) return;
+            break;
+        }
+        if (rank == 0) st->dirtyCount = 0;  // (filled by the scatter)
+        const int a = st->activeBuffer;
+        if constexpr (Binary)
+        {
+            const BinaryOp op{u.bucket, u.maxDepth};
+            while (decideScan(op, tb, tb.k(a), tb.b(a), static_cast<const u8 *>(nullptr))) __syncthreads();
+        }
+        else
+        {
+            const OctreeOp<false> op{u.bucket};
+            while (decideScan(op, tb, tb.k(a), tb.b(a), static_cast<const u8 *>(nullptr))) __syncthreads();
+        }
+        if (!barrier()) return;
+        clearScan();
+        if constexpr (Binary) binScatter(tb, u.limit, kModeUpdate);
+        else octScatter<false>(tb, u.limit, kModeUpdate, nullptr);
+        if (!barrier()) return;
+        octBegins<false>(tb, u.idx);
+        if (rank == 0 && pass + 1 < u.iterations) st->changed = 0;
+        if (!barrier()) return;
+    }
+    materializeCounts(tb);
 }
 
 }  // namespace rb
