@@ -1741,9 +1741,6 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
     Impl &m = *m_;
     const bool nf = cfg_.nf;
     const unsigned blocks = unsigned(smCount()) * 4u;
-    // deep levels of many units classify, count and place with 8 CTAs per SM
-    // (an A/B at 16 Mi: 3.49 ms with 4, 3.40 ms with 8, 3.42 ms with 16)
-    const unsigned wide = 2u;
     unsigned leafGrid = 0;
     if (!nf)
     {
@@ -1796,16 +1793,12 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
                 if (cfg_.hilbert) lb::expandKernel<true><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
                 else lb::expandKernel<false><<<blocks * 2, lb::kThreads, 0, s>>>(a, idx, l), noteLaunch();
                 markNearField(true);
-                if (cfg_.hilbert) lb::nearFieldKernel<true, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
-                else lb::nearFieldKernel<false, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, 0u), noteLaunch();
+                if (cfg_.hilbert) lb::nearFieldKernel<true, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, cfg_.bucket), noteLaunch();
+                else lb::nearFieldKernel<false, true><<<blocks, lb::kThreads, 0, s>>>(a, idx, l, rb::TreeBufs{}, cfg_.bucket), noteLaunch();
                 markNearField(false);
-                if (cfg_.hilbert)
-                    lb::classifyKernel<true><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
-                else
-                    lb::classifyKernel<false><<<blocks * wide, lb::kThreads, 0, s>>>(a, l, cfg_.bucket), noteLaunch();
                 AOT_LAUNCH_CHECK();
             }
-            lb::subtreeKernel<<<blocks * wide, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
+            lb::subtreeKernel<<<blocks * 2, lb::kThreads, 0, s>>>(a, levels), noteLaunch();
             AOT_LAUNCH_CHECK();
             place(levels);
             // the round history is needed before finishKernel writes it; read

@@ -18,13 +18,14 @@
 //             counts of the unit's children;
 //   classify  the children whose value exceeds the bucket become the units of
 //             level l + 1 (slots taken by warp-aggregated atomics); the
-//             others are leaves of the tree;
+//             others are leaves of the tree (with the near field, or with
+//             expand where the value is the count);
 //   subtree, place: subtree leaf counts bottom-up, then every leaf's
 //             position in the cornerstone array top-down.
 // A LeafCount build is one cooperative launch (leafBuildKernel): a unit's
 // counts are differences of its begins, so expand and classify are one step
-// (growUnits) with a grid barrier per level.  An NFCount build is a launch per
-// step and level, and one each for the subtree counts and the placement.
+// (growUnits) with a grid barrier per level.  An NFCount build has two launches
+// per level, and one each for the subtree counts and the placement.
 //
 // The capacity the reference ends with depends on how many leaves each round
 // proposed (resizeWithHeadroom history, octree.cu:159-180 and 453-457).  That
@@ -37,8 +38,8 @@
 // arrive at round a + 1; every leaf f of the final tree in that region, at
 // relative depth j <= k, is then represented by its 8^(k-j) descendants at
 // the landing level, which merge up one level per round, so f stands for
-// 8^max(0, k - (t - a - 1) - j) leaves at round t >= a + 1.  The classify
-// kernel counts the final leaves per (a, k, j) and the landed internal nodes
+// 8^max(0, k - (t - a - 1) - j) leaves at round t >= a + 1.  Classify
+// counts the final leaves per (a, k, j) and the landed internal nodes
 // per round; the host sums the leaf counts of every round from them.
 #pragma once
 
@@ -304,22 +305,25 @@ __device__ __forceinline__ u32 warpBoundaryIn(const KeyIndex &idx, u32 lo, u32 h
     return warpLowerBound(idx.keys, wlo, whi, t, lane);
 }
 
-// The children of units (LeafCount): lanes hold a child each, eight to a unit
-// g in digit order, of which `valid` ones take part (whole units; all lanes of
-// the warp call).  A child of more than `bucket` keys below level 21 becomes a
-// unit of level l + 1 (slots by an atomic add per warp; the order of a level's
-// units is free), the others are leaves, counted into the round history by
-// (arrival, depth, relative level): of the CTA (sContrib, sLanded) or, Forest,
-// of the unit's system.  key and reg: the unit's key and region word;
-// [begin, end): the child's keys; next: first unit of level l + 1.
-template <bool Forest>
-__device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned bucket, u32 next, u32 g, bool valid,
-                                             u32 begin, u32 end, u64 key, u32 reg, u32 *sContrib, u32 *sLanded)
+// The children of units: lanes hold a child each, eight to a unit g in digit
+// order, of which `valid` ones take part (whole units; all lanes of the warp
+// call).  A child whose value x (its keys, or NF: its near-field count) exceeds
+// `bucket` below level 21 becomes a unit of level l + 1 (slots by an atomic add
+// per warp; the order of a level's units is free: every later step finds them
+// through the child and parent links, and the placement follows the digits),
+// the others are leaves, counted into the round history by (arrival, depth,
+// relative level): of the CTA (sContrib, sLanded) or, Forest, of the unit's
+// system.  key and reg: the unit's key and region word; [begin, end): the
+// child's keys; next: first unit of level l + 1.  NFCount units keep their
+// children by octant (dec, encNext: the curve's tables).
+template <bool NF, bool Hilbert, bool Forest>
+__device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned bucket, u32 next, u32 g, bool valid, u32 x,
+                                             u32 begin, u32 end, u64 key, u32 reg, const unsigned char *dec,
+                                             const unsigned char *encNext, u32 *sContrib, u32 *sLanded)
 {
     Control &c = *a.ctl;
     const unsigned m = unsigned(l) + 1;
     const int lane = threadIdx.x & 31, d = lane & 7;
-    const u32 x = end - begin;
     const bool high = valid && x > bucket && m < kOctLevels;
     const unsigned ballot = __ballot_sync(0xffffffffu, high);
     u32 base = 0;
@@ -330,6 +334,8 @@ __device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned buc
     const u32 j = m - lR;  // 1 <= j <= kR
     const u32 nHigh = u32(__popc((ballot >> (lane & 24)) & 0xffu));
     const u32 sys = Forest ? a.usys[g] : 0u;
+    const u32 state = Hilbert ? unitStateOf(reg) : 0u;
+    const u32 oct = Hilbert ? u32(dec[state * 8 + d]) : u32(d);
     u32 slot = kLeaf;
     if (high)
     {
@@ -338,14 +344,14 @@ __device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned buc
         {
             u32 creg = reg;
             // a landed internal node: a leaf in round aR + 1, splitting at once
-            if (j == kR) creg = regionWord(min(aR + 1, u32(kArrivals) - 1), m, splitDepth(false, x, bucket, m));
+            if (j == kR) creg = regionWord(min(aR + 1, u32(kArrivals) - 1), m, splitDepth(NF, x, bucket, m));
             if constexpr (Forest) a.usys[gc] = sys;
-            a.parent[gc] = g * 8 + u32(d);
+            a.parent[gc] = g * 8 + oct;
             a.offset[gc] = kPending;
             const u64 ck = key + u64(d) * octRange(m);
             uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
             crow[0] = make_uint4(u32(ck), u32(ck >> 32), begin, 0u);
-            crow[2] = make_uint4(0u, 0u, end, withUnit(creg, m, kHilbertStart));
+            crow[2] = make_uint4(0u, 0u, end, withUnit(creg, m, Hilbert ? u32(encNext[state * 8 + oct]) : u32(kHilbertStart)));
             slot = gc;
         }
         else
@@ -353,7 +359,7 @@ __device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned buc
             c.overflow = 1;
         }
     }
-    a.child[size_t(g) * 8 + d] = slot;
+    a.child[size_t(g) * 8 + oct] = slot;
     if (d != 0) return;
     a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
     const u32 bin = (aR * kJumps + kR) * kJumps + j;
@@ -402,8 +408,9 @@ __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, i
             if (warp == 0)
             {
                 const int d = lane & 7;
-                growChildren<Forest>(a, l, bucket, next, start + i, lane < 8, d ? sEnds[d - 1] : lo, d < 7 ? sEnds[d] : hi,
-                                     key, reg, sContrib, sLanded);
+                const u32 b = d ? sEnds[d - 1] : lo, e = d < 7 ? sEnds[d] : hi;
+                growChildren<false, false, Forest>(a, l, bucket, next, start + i, lane < 8, e - b, b, e, key, reg, nullptr,
+                                                   nullptr, sContrib, sLanded);
             }
             __syncthreads();
         }
@@ -426,7 +433,9 @@ __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, i
             row[3 + d] = end;
         }
         const u32 prev = __shfl_up_sync(0xffffffffu, end, 1, 8);
-        growChildren<Forest>(a, l, bucket, next, g, valid, d ? prev : lo, end, key, reg, sContrib, sLanded);
+        const u32 begin = d ? prev : lo;
+        growChildren<false, false, Forest>(a, l, bucket, next, g, valid, end - begin, begin, end, key, reg, nullptr, nullptr,
+                                           sContrib, sLanded);
     }
 }
 
@@ -793,8 +802,11 @@ __device__ __forceinline__ u64 countedRec(const u64 *P, u32 lo, u32 hi, u64 qKey
     return rec;
 }
 
-// Build: the values of a build's units; else the near-field counts and group
-// flags of the leaves of a standing tree (treeUnitsKernel).
+// Build: the values of a build's units, and with them the units of the next
+// level and the round history (growChildren; a launch per level that read the
+// rows and values back took 178 us at 16Mi and 48 us in 11 launches at 300k);
+// else the near-field counts and group flags of the leaves of a standing tree
+// (treeUnitsKernel).
 template <bool Hilbert, bool Build>
 static __global__ void __launch_bounds__(kThreads, 4)
     nearFieldKernel(Arena a, KeyIndex idx, int l, rb::TreeBufs tb, unsigned bucket)
@@ -802,9 +814,11 @@ static __global__ void __launch_bounds__(kThreads, 4)
     using rb::kUnitBatch;
     __shared__ NearTables t;
     __shared__ NearScratch sWarp[kThreads / 32];
-    const Control &c = *a.ctl;
-    if (c.overflow | c.late | c.error) return;
+    __shared__ u32 sContrib[Build ? kContribBins : 1], sLanded[Build ? kArrivals : 1];
+    Control &c = *a.ctl;
+    if (c.overflow | c.late | c.error) return;  // (set by this level's CTAs too: what is left out then does not matter)
     const u32 start = c.levelStart[l], count = c.levelCount[l];
+    if (Build && blockIdx.x == 0 && threadIdx.x == 0) c.levelStart[l + 1] = start + count;
     NearOut out{};
     if constexpr (!Build)
     {
@@ -825,6 +839,11 @@ static __global__ void __launch_bounds__(kThreads, 4)
         const int qp = ((tx + 2) / 2) + 3 * ((ty + 2) / 2) + 9 * ((tz + 2) / 2);  // offset around the parent
         t.step[k] = (unsigned char)(qp << 3 | ((tx & 1) << 2) | ((ty & 1) << 1) | (tz & 1));
     }
+    if constexpr (Build)
+    {
+        for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
+        if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
+    }
     __syncthreads();
     constexpr int kRounds = (kUnitBatch * 27 + 31) / 32;
     const int lane = threadIdx.x & 31;
@@ -835,6 +854,19 @@ static __global__ void __launch_bounds__(kThreads, 4)
     // levels that do not fill the warps' batches: fewer units per warp, shorter chains
     const u32 per = min(u32(kUnitBatch), (count + warpsTotal - 1) / warpsTotal);
     const u32 w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // (a level of few units spreads over the SMs)
+    // the units [first, first + nb), whose values are written, four at a time
+    const auto classify = [&](u32 first, int nb) {
+        for (int e = lane; e < ((nb * 8 + 31) & ~31); e += 32)
+        {
+            const bool valid = e < nb * 8;
+            const u32 g = first + u32(valid ? e >> 3 : 0);
+            const int d = e & 7;
+            const u32 *row = a.rows + size_t(g) * kRow;
+            growChildren<true, Hilbert, false>(a, l, bucket, start + count, g, valid, a.val[size_t(g) * 8 + d], row[2 + d],
+                                               row[3 + d], rowKey(row), row[11], t.dec, t.next, sContrib, sLanded);
+        }
+        __syncwarp();
+    };
     for (u32 base = w0 * per; base < count; base += warpsTotal * per)
     {
         const int nb = int(min(per, count - base)), items = nb * 27;
@@ -928,6 +960,7 @@ static __global__ void __launch_bounds__(kThreads, 4)
         if (big)
         {
             nearFieldByRows<Hilbert, Build>(a, idx, l, first, nb, sWarp[threadIdx.x >> 5].rows, t, out);
+            if constexpr (Build) classify(first, nb);
             continue;
         }
         // Four lanes a unit: lane (x0, y0) sums the children (x0, y0, 0) and
@@ -994,6 +1027,15 @@ static __global__ void __launch_bounds__(kThreads, 4)
             }
         }
         __syncwarp();
+        if constexpr (Build) classify(first, nb);
+    }
+    if constexpr (Build)
+    {
+        __syncthreads();
+        for (int k = threadIdx.x; k < kContribBins; k += kThreads)
+            if (sContrib[k]) atomicAdd(a.contrib + k, (unsigned long long)sContrib[k]);
+        if (threadIdx.x < kArrivals && sLanded[threadIdx.x])
+            atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
     }
 }
 
@@ -1173,158 +1215,6 @@ static __global__ void __launch_bounds__(kThreads) unitsToTableKernel(Arena a, r
         *reinterpret_cast<uint2 *>(to + 6) = make_uint2(r2.x, r2.y);
         to[8] = r2.z;
     }
-}
-
-// Children of the level-l units: those whose value exceeds the bucket (below
-// level 21) become the units of level l + 1, the others are leaves, counted
-// into the round history by (arrival, depth, relative level).  A warp takes
-// the slots of its new units with one atomic add; the order of the units in
-// a level is free (every later step finds them through the child and parent
-// links, and the placement follows the digits).
-// The child slots are kept by octant; sSlots[32 * 9] of the warp turns them
-// around and lets the warp write them coalesced.  NFCount builds.
-template <bool Hilbert>
-__device__ __forceinline__ void classifyUnits(const Arena &a, int l, unsigned bucket, u32 start, u32 count,
-                                              const unsigned char *sNext, const unsigned char *sDec, u32 *sContrib,
-                                              u32 *sLanded, u32 *sSlots, u32 rank, u32 size)
-{
-    Control &c = *a.ctl;
-    const u32 next = start + count;
-    if (rank == 0) c.levelStart[l + 1] = next;
-    const unsigned m = unsigned(l) + 1;
-    const u64 cr = octRange(m);
-    const int lane = threadIdx.x & 31;
-    for (u32 i0 = rank & ~31u; i0 < count; i0 += size)
-    {
-        const u32 i = i0 + u32(lane);
-        const bool valid = i < count;
-        const u32 g = start + (valid ? i : 0);
-        const uint4 *row4 = reinterpret_cast<const uint4 *>(a.rows + size_t(g) * kRow);
-        u32 b[rb::kGroupBegins], x[8];
-        u32 reg = 0;
-        u64 key = 0;
-        unsigned highMask = 0;
-        if (valid)
-        {
-            const uint4 r0 = row4[0], r1 = row4[1], r2 = row4[2];
-            key = (u64(r0.y) << 32) | r0.x;
-            b[0] = r0.z; b[1] = r0.w;
-            b[2] = r1.x; b[3] = r1.y; b[4] = r1.z; b[5] = r1.w;
-            b[6] = r2.x; b[7] = r2.y; b[8] = r2.z;
-            reg = r2.w;
-            const uint4 *v4 = reinterpret_cast<const uint4 *>(a.val + size_t(g) * 8);
-            const uint4 v0 = v4[0], v1 = v4[1];
-            x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
-            x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
-#pragma unroll
-            for (int d = 0; d < 8; ++d)
-            {
-                if (x[d] > bucket && m < kOctLevels) highMask |= 1u << d;
-            }
-        }
-        // slots of the warp's new units: one atomic add per warp
-        const u32 nHigh = u32(__popc(highMask));
-        u32 incl = nHigh;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1)
-        {
-            const u32 t = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += t;
-        }
-        u32 base = 0;
-        if (lane == 31 && incl) base = atomicAdd(&c.levelCount[l + 1], incl);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        const u32 aR = regionArrival(reg), lR = regionLevel(reg), kR = regionDepth(reg);
-        const u32 j = m - lR;  // 1 <= j <= kR
-        u32 rank = base + incl - nHigh;
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-        {
-            if (!valid) break;
-            u32 slot = kLeaf;
-            if (highMask & (1u << d))
-            {
-                const u32 gc = next + rank++;
-                if (gc < a.cap)
-                {
-                    u32 creg = reg;
-                    if (j == kR)
-                    {
-                        // a landed internal node: a leaf in round aR + 1, splitting at once
-                        creg = regionWord(aR + 1, m, splitDepth(true, x[d], bucket, m));
-                        if (aR + 2 >= u32(kArrivals)) c.late = 1;
-                        else atomicAdd(&sLanded[aR + 1], 1u);
-                    }
-                    // the child's own level and the curve state ordering its children
-                    u32 cst = kHilbertStart, oct = u32(d);
-                    if constexpr (Hilbert)
-                    {
-                        const u32 st = unitStateOf(reg);
-                        oct = sDec[st * 8 + d];
-                        cst = sNext[st * 8 + oct];
-                    }
-                    a.parent[gc] = g * 8 + oct;
-                    a.offset[gc] = kPending;
-                    const u64 ck = key + u64(d) * cr;
-                    uint4 *crow = reinterpret_cast<uint4 *>(a.rows + size_t(gc) * kRow);
-                    crow[0] = make_uint4(u32(ck), u32(ck >> 32), b[d], 0u);
-                    crow[2] = make_uint4(0u, 0u, b[d + 1], withUnit(creg, m, cst));
-                    slot = gc;
-                }
-                else
-                {
-                    c.overflow = 1;
-                }
-            }
-            else
-            {
-                atomicAdd(&sContrib[(aR * kJumps + kR) * kJumps + j], 1u);
-            }
-            if constexpr (Hilbert) sSlots[lane * 9 + sDec[unitStateOf(reg) * 8 + d]] = slot;
-            else sSlots[lane * 9 + d] = slot;
-        }
-        if (valid) a.sub[g] = (u64(nHigh) << kSubShift) | (8u - nHigh);
-        __syncwarp();
-        const u32 words = min(32u, count - i0) * 8;
-        u32 *out = a.child + size_t(start + i0) * 8;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-        {
-            const u32 e = u32(k) * 32 + u32(lane);
-            if (e < words) out[e] = sSlots[(e >> 3) * 9 + (e & 7)];
-        }
-        __syncwarp();
-    }
-}
-
-template <bool Hilbert>
-static __global__ void __launch_bounds__(kThreads) classifyKernel(Arena a, int l, unsigned bucket)
-{
-    __shared__ u32 sContrib[kContribBins];
-    __shared__ u32 sLanded[kArrivals];
-    __shared__ __align__(4) unsigned char sNext[48 * 8], sDec[48 * 8];
-    __shared__ u32 sSlots[(kThreads / 32) * 32 * 9];
-    Control &c = *a.ctl;
-    if (c.overflow | c.late | c.error) return;
-    const u32 start = c.levelStart[l], count = c.levelCount[l];
-    if (blockIdx.x == 0 && threadIdx.x == 0) c.levelStart[l + 1] = start + count;
-    if (count <= blockIdx.x * blockDim.x) return;
-    if constexpr (Hilbert)
-    {
-        copyTable(sNext, gHilbert.encNext);
-        copyTable(sDec, gHilbert.decOct);
-    }
-    for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
-    if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
-    __syncthreads();
-    classifyUnits<Hilbert>(a, l, bucket, start, count, sNext, sDec, sContrib, sLanded,
-                                      sSlots + (threadIdx.x >> 5) * 32 * 9,
-                                      blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-    __syncthreads();
-    for (int k = threadIdx.x; k < kContribBins; k += kThreads)
-        if (sContrib[k]) atomicAdd(a.contrib + k, (unsigned long long)sContrib[k]);
-    if (threadIdx.x < kArrivals && sLanded[threadIdx.x])
-        atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
 }
 
 // The leaves below every unit, all levels at once (the first `total` units): a
