@@ -16,7 +16,7 @@ the reference algorithm on a bounded sample (the reference has no CPU
 implementation of this path); the reference library's own GPU time on this
 box is reported by the default run under "reference_gpu", CUB's pair sort on
 the same keys under "roofline" (the build's dominant kernel, the sort pass;
-"roofline_update" is update()'s, the full near-field refresh), and bit-exact
+"roofline_update" is update()'s, the full near-field refresh by units), and bit-exact
 parity of the timed tree with the reference library under "parity".  A single-GPU default run then
 adds the metric's other configurations under "configs": c1 (2^20 uniform fp64
 LeafCount octree), c3 (8Mi binary k-d tree), c4 (512 batched octrees against
@@ -44,18 +44,20 @@ N_DEFAULT = 1 << 24
 BUCKET = 512
 METRIC = "particles/s (octree build, 16Mi Plummer fp32, Hilbert, NFCount 512)"
 WORKLOAD = "octree build + graph-replayed update, 16Mi Plummer fp32 (a=0.05, r<=0.5), Hilbert keys, NFCount 512"
-# DRAM bytes (read + write) of one 16Mi-key onesweep pass, measured by ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum) on that pass: 204.9 MB + 162.7 MB.
-ONESWEEP_TRAFFIC_BYTES = 367.6e6
+# DRAM bytes (read + write) per key of one onesweep pass, measured by ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum) over the 8 passes of a build
+# and an update of 8 Mi particles: 742.3 MB + 351.7 MB (less than the 24 bytes
+# a key moves: a part stays in L2).
+ONESWEEP_TRAFFIC_BYTES_PER_KEY = (742.3e6 + 351.7e6) / (8 * 8388608)
 # Algorithmic bytes of the near-field refresh per leaf: K[i] read (8), the
 # begin index B[i] read (4), NF[i] written (4), and the group flag, one byte
 # per sibling group (1/8).
 NF_BYTES_PER_LEAF = 16.125
 # DRAM bytes (read + write) per leaf of the full near-field refresh, measured
-# by ncu on that launch at 8 Mi particles (6,678,211 leaves); the traffic
-# reported for the 16 Mi launch is this times its leaves (scaled, not
+# by ncu on its launches (one per level) at 8 Mi particles (6,678,974 leaves);
+# the traffic reported for 16 Mi is this times its leaves (scaled, not
 # re-measured in the run).
-NF_TRAFFIC_BYTES_PER_LEAF = (292337664 + 30597888) / 6678211
+NF_TRAFFIC_BYTES_PER_LEAF = (155.2e6 + 53.4e6) / 6678974
 # The arrays compared with the reference library in the line's parity record.
 PARITY_ARRAYS = ("particleKeys", "perm", "cornerstone", "leafCounts", "nearFieldCounts")
 
@@ -999,9 +1001,12 @@ def main():
         keys_in = ab.compute_sfc_keys(0, *xs, sfc_kind=ab.SfcKind.Hilbert, stream=s)
         s.synchronize()
         rig = SortRig(keys_in, s)
+        # (sorts of one and two digits run every pass: one pass apart, with one
+        # more digit counted; the 64-bit sort's plan leaves passes out)
         t64 = graph_ms(lambda: rig(64), s, 7)
+        t16 = graph_ms(lambda: rig(16), s, 7)
         t8 = graph_ms(lambda: rig(8), s, 7)
-        pass_ms = (t64 - t8) / 7.0
+        pass_ms = t16 - t8
         keygen_ms = graph_ms(lambda: ab.compute_sfc_keys(0, *xs, sfc_kind=ab.SfcKind.Hilbert, stream=s), s, 7)
     barrier()
 
@@ -1012,12 +1017,14 @@ def main():
     hbm, peak_kind = peaks()
     pass_bytes = 24.0 * n
     achieved = pass_bytes / (pass_ms * 1e-3) / 1e9
-    # the dominant kernel of the timed step: one build runs 8 onesweep passes,
-    # 38 % of its device time, more than any other kernel
+    # the sort pass is the kernel the path has most of: the build's plan runs 4
+    # of 8, a quarter of its device time (the near field, over 13 levels, is
+    # nearly a third)
     roof_sort = {"bound": "hbm", "kernel": "onesweepKernel (one 8-bit pass of the 64-bit key + 32-bit value sort)",
-                 "why": "the build's dominant kernel: 8 launches per build, 1.33 of 3.61 ms serialised device time",
+                 "why": "the plan of the build's sort runs 4 of 8 passes, 0.48 of 1.91 ms device time",
                  "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind,
-                 "traffic": ONESWEEP_TRAFFIC_BYTES, "traffic_kind": "ncu capture of one 16Mi pass, not re-measured",
+                 "traffic": ONESWEEP_TRAFFIC_BYTES_PER_KEY * n,
+                 "traffic_kind": "ncu on the passes of 8Mi keys, scaled, not re-measured",
                  "algorithmic_bytes_per_launch": pass_bytes,
                  "launch_ms": pass_ms, "sort_64bit_ms": t64,
                  "keygen": {"ms": keygen_ms, "achieved_gbs": (20.0 * n) / (keygen_ms * 1e-3) / 1e9}}
@@ -1036,17 +1043,18 @@ def main():
     def med(rows, key):
         return statistics.median(r[key] for r in rows)
 
-    # the dominant kernel of update(): the near-field refresh.  Its full
-    # launch covers every leaf, so its algorithmic bytes are known exactly.
+    # the dominant kernel of update(): the near-field refresh.  Its full run
+    # (a launch per level) covers every leaf, so its algorithmic bytes are known
+    # exactly.
     nf_ms = max_over_ranks(med(update_stages, "near_field_first_ms"), world, dev)
     nf_bytes = NF_BYTES_PER_LEAF * nf_leaves
     nf_achieved = nf_bytes / (nf_ms * 1e-3) / 1e9
-    roof = {"bound": "hbm", "kernel": "octNearFieldKernel<Hilbert, All> (the full near-field refresh of update())",
+    roof = {"bound": "hbm", "kernel": "lb::nearFieldKernel<Hilbert> by units (the full near-field refresh of update(), all levels)",
             "achieved": nf_achieved, "peak": hbm, "unit": "GB/s", "frac": nf_achieved / hbm, "peak_kind": peak_kind,
             "traffic": (NF_TRAFFIC_BYTES_PER_LEAF * nf_leaves) if NF_TRAFFIC_BYTES_PER_LEAF else None,
             "algorithmic_bytes_per_launch": nf_bytes, "launch_ms": nf_ms, "leaves": nf_leaves,
-            "note": "search-bound: 27 neighbour-cell populations per parent cell come from hash tables or "
-                    "searches of the sorted keys; HBM is the roof, not the limit"}
+            "note": "latency-bound: the 27 cells around every internal node are found through the parent's and "
+                    "summed from byte records; HBM is the roof, not the limit"}
     stages = {
         "build": {k: med(build_stages, k) for k in ("keys_and_sort_ms", "passes_ms", "finish_ms", "total_ms",
                                                      "near_field_ms")},
@@ -1055,7 +1063,8 @@ def main():
         "build_near_field_launches": build_stages[-1]["near_field_launches"],
         "update_near_field_launches": update_stages[-1]["near_field_launches"],
         "how": "CUDA events on the tree's stream around each stage (ao_tree_set_profiling), direct calls"}
-    # the whole build on the byte model of the path: per particle the
+    # the whole build on the byte model of a build whose sort runs all 8 passes
+    # (the plan runs 4, so this figure can pass the peak): per particle the
     # coordinates read (3 x 4 B), key + index written (12 B), the upfront
     # histogram read (8 B), 24 B per radix pass (8 passes), one streaming read
     # of the sorted keys (8 B); per leaf K and N written (12 B)
