@@ -4,7 +4,9 @@
 // (octree.cu:427-551, kdtree3d.cu:227-297, tree_view.cu:814-1134) with
 // B200-specific choices:
 //   * keygen + onesweep sort replace computeSfcKeys + CUB SortPairs;
-//   * the octree build runs its split/merge rounds on the device without a
+//   * builds make the converged tree by levels (levelbuild.cuh, binlevel.cuh);
+//   * where that does not apply, the octree build runs its split/merge rounds
+//     on the device without a
 //     host round-trip per round: rounds are issued in batches, every kernel
 //     stops as soon as the device state says the tree converged, and the host
 //     reads the state once per batch; the reference's vector capacity growth,

@@ -1,6 +1,7 @@
 // rebalance.cuh -- device kernels of the split/merge rebalance passes.
 //
-// One pass (octree or binary) is three kernels, all reading sizes and the
+// One pass (octree or binary) is three kernels (or, trees of few leaves, three
+// steps of updateKernel, which runs a whole update), all reading sizes and the
 // A/B selection from DeviceState so a captured CUDA graph stays valid while
 // the topology changes (the reference's graph path, octree_rebalance.cuh:
 // 1177-1322 and kdtree3d_rebalance.cuh:160-245):

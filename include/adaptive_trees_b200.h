@@ -123,15 +123,17 @@ AO_API ao_status ao_tree_update(ao_tree *tree);
  * reference's NVTX ranges behind ADAPTIVE_OCTREE_PROFILING (config.hpp:20-28,
  * octree.cu:287-306).  With profiling on, each octree build() and update()
  * not made under stream capture records events at its stage boundaries and
- * around every near-field launch on the tree's stream, and pushes one NVTX
- * range per stage. */
+ * around every near-field refresh on the tree's stream, and pushes one NVTX
+ * range per stage.  (A profiled update() runs its passes launch by launch;
+ * otherwise LeafCount and binary trees of up to 2^19 leaves run them in one
+ * launch.  The results are the same.) */
 typedef struct ao_stage_times {
-    double keys_and_sort_ms; /* key generation, the 8 sort passes and the key sample */
+    double keys_and_sort_ms; /* key generation, the sort and the key sample */
     double refresh_ms;       /* update: the full per-leaf refresh (begin indices, cell table, near field) */
     double passes_ms;        /* the rebalance passes (build: its rounds, with the host's checks between them) */
     double finish_ms;        /* leaf counts and views (build: and the final copies) */
     double total_ms;
-    double near_field_ms;    /* all near-field kernel launches of the call (0 without NFCount) */
+    double near_field_ms;    /* all near-field refreshes of the call (0 without NFCount; build: with the classification) */
     double near_field_first_ms; /* the first of them (update(): the full refresh of every leaf) */
     int near_field_launches;
     int call;                /* 1 build, 2 update */
