@@ -453,13 +453,13 @@ bool ForestEngine::sortPersistent(int config)
 
 namespace
 {
-template <int Tile>
+template <int Tile, int Parts>
 void launchSegmentRepair(unsigned numTiles, const sort::RepairArgs &r, const sort::SegmentTiles &tiles,
                          const forest::System *systems, cudaStream_t s)
 {
     constexpr int smem = int(sizeof(sort::RepairShared<Tile>));
-    AOT_CHECK(cudaFuncSetAttribute(forest::segmentRepairKernel<Tile>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    forest::segmentRepairKernel<Tile><<<numTiles, sort::kRepairThreads, smem, s>>>(r, tiles, systems), noteLaunch();
+    AOT_CHECK(cudaFuncSetAttribute(forest::segmentRepairKernel<Tile, Parts>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    forest::segmentRepairKernel<Tile, Parts><<<numTiles * Parts, sort::kRepairThreads, smem, s>>>(r, tiles, systems), noteLaunch();
 }
 }  // namespace
 
@@ -512,9 +512,9 @@ void ForestEngine::sortKeys(int config)
     const forest::System *systems = m.systemsD.as<forest::System>();
     switch (sort::kSortConfigs[config].items)
     {
-    case 8: launchSegmentRepair<sort::kThreads * 8>(m.numTiles, r, tiles, systems, s); break;
-    case 10: launchSegmentRepair<sort::kThreads * 10>(m.numTiles, r, tiles, systems, s); break;
-    case 16: launchSegmentRepair<sort::kThreads * 16>(m.numTiles, r, tiles, systems, s); break;
+    case 8: launchSegmentRepair<sort::kThreads * 8, 1>(m.numTiles, r, tiles, systems, s); break;
+    case 10: launchSegmentRepair<sort::kThreads * 10, 1>(m.numTiles, r, tiles, systems, s); break;
+    case 16: launchSegmentRepair<sort::kThreads * 8, 2>(m.numTiles, r, tiles, systems, s); break;
     default: throw std::logic_error("forest: no repair for the sort configuration's tiles");
     }
     sort::longRunKernel<<<unsigned(smCount()) * 2u, sort::kLongThreads, 0, s>>>(r), noteLaunch();

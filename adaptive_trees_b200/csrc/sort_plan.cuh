@@ -30,7 +30,7 @@ constexpr int kPlanMaxPasses = 6;
 constexpr int kPlanSets = kPlanMaxPasses - kPlanMinPasses + 2;  // a set of prefixes per choice, one of whole keys
 // Cost in passes: the repair's fixed part and its part per key of the mean
 // run.  Measured at 16Mi keys (a pass 120 us): repairs of mean runs of 3.8,
-// 4.7 and 14.4 keys took 116, 130 and 272 us.
+// 4.7 and 14.4 keys took 116, 130 and 272 us (the first takes 109 now).
 constexpr float kRepairCost = 0.55f;
 constexpr float kRunCost = 0.11f;
 // Mean run of equal keys above which all passes run: they share their run with

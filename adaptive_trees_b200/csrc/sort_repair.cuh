@@ -210,11 +210,11 @@ __device__ __forceinline__ void repairTile(const RepairArgs &a, RepairShared<Til
                 if (First >= 1 && First <= 4)
                 {
                     // at most 32 bits are left: the low words order the run
-                    for (int j = h; j < e; ++j)
-                    {
-                        const u32 o = sm.lo[j];
-                        to += (o < lo || (o == lo && j < w)) ? 1 : 0;
-                    }
+                    // (with the place as one 64-bit compare; 16Mi keys: 116 us
+                    // by two 32-bit ones, 109)
+                    const u64 mine = (u64(lo) << 32) | u32(w);
+#pragma unroll 2
+                    for (int j = h; j < e; ++j) to += ((u64(sm.lo[j]) << 32) | u32(j)) < mine ? 1 : 0;
                 }
                 else
                 {
