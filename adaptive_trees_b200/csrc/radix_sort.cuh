@@ -145,22 +145,26 @@ static __global__ void __launch_bounds__(kThreads) histogramKernel(const u64 *__
 
 // Exclusive scan of each pass' 256 digit counts (a narrower radix leaves the
 // upper counts zero, so their starts are unused).  A warp per pass, eight
-// counts per lane.  __ldcg: the counts may come from other CTAs' atomics.
+// counts per lane, two an access: the counts and the starts of a pair sort lie
+// in the caller's scratch, of which 8-byte alignment is all that is asked.
+// __ldcg: the counts may come from other CTAs' atomics.
 __device__ __forceinline__ void scanBins(const u32 *hist, u32 *bins, int firstPass, int passes)
 {
     static_assert(kRadix == 256, "eight counts per lane");
     const int lane = threadIdx.x & 31;
     for (int p = firstPass + int(threadIdx.x >> 5); p < passes; p += int(blockDim.x >> 5))
     {
-        const uint4 *h = reinterpret_cast<const uint4 *>(hist + p * kRadix) + lane * 2;
-        const uint4 a = __ldcg(h), b = __ldcg(h + 1);
-        const u32 c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const uint2 *h = reinterpret_cast<const uint2 *>(hist + p * kRadix) + lane * 4;
+        uint2 c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c[i] = __ldcg(h + i);
         u32 sum = 0, e[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
         {
-            e[i] = sum;
-            sum += c[i];
+            e[2 * i] = sum;
+            e[2 * i + 1] = sum + c[i].x;
+            sum += c[i].x + c[i].y;
         }
         u32 inc = sum;
 #pragma unroll
@@ -170,9 +174,9 @@ __device__ __forceinline__ void scanBins(const u32 *hist, u32 *bins, int firstPa
             if (lane >= off) inc += t;
         }
         const u32 base = inc - sum;
-        uint4 *o = reinterpret_cast<uint4 *>(bins + p * kRadix) + lane * 2;
-        o[0] = make_uint4(base + e[0], base + e[1], base + e[2], base + e[3]);
-        o[1] = make_uint4(base + e[4], base + e[5], base + e[6], base + e[7]);
+        uint2 *o = reinterpret_cast<uint2 *>(bins + p * kRadix) + lane * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = make_uint2(base + e[2 * i], base + e[2 * i + 1]);
     }
 }
 

@@ -211,7 +211,8 @@ AO_API ao_status ao_compute_sfc_keys(int kind, int real_type, const void *x, con
  * end_bit, stream) as called at octree.cu:301-304 and kdtree3d.cu:168-170:
  * stable LSD sort of 64-bit keys carrying 32-bit values by bits
  * [begin_bit, end_bit), onesweep with decoupled look-back.  With scratch ==
- * NULL only *scratch_bytes is set.  values_in == NULL sorts the indices
+ * NULL only *scratch_bytes is set; scratch needs the alignment of its 64-bit
+ * words, 8 bytes, no more.  values_in == NULL sorts the indices
  * 0..n-1 (the identity permutation).  keys_in/values_in are not modified and
  * must not alias the outputs.  No allocation; capturable.  The sort uses
  * the configuration the sort tuner holds for n (below); the size query
