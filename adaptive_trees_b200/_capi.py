@@ -88,6 +88,8 @@ PROTOTYPES = {
     "ao_sort_pairs_check": [vp, sz, vp],
     "ao_sort_pairs_noalloc_check": [sz, vp],
     "ao_selftest_bounded_wait": [ci, cu, ctypes.POINTER(ci)],
+    "ao_selftest_team_wait": [ci, cu, ctypes.POINTER(ci)],
+    "ao_selftest_hold_sms": [ci, ci, vp],
     "ao_sort_config_count": [ctypes.POINTER(ci)],
     "ao_sort_config_info": [ci, ctypes.POINTER(ci), ctypes.POINTER(ci)],
     "ao_sort_tuning": [ci, sz, ctypes.POINTER(ci), ctypes.POINTER(ci), ctypes.POINTER(ci), ctypes.POINTER(ci)],

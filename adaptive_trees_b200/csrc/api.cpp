@@ -557,6 +557,21 @@ ao_status ao_selftest_bounded_wait(int which, unsigned spin_limit, int *error_wo
     });
 }
 
+ao_status ao_selftest_team_wait(int which, unsigned spin_limit, int *error_word)
+{
+    return guarded([&] {
+        const int e = aot::TreeEngine::teamWaitProbe(which, spin_limit);
+        if (error_word) *error_word = e;
+        if (e != 0)
+            throw std::runtime_error("ao_selftest_team_wait: the wait gave up after its limit and the kernel returned");
+    });
+}
+
+ao_status ao_selftest_hold_sms(int sms, int milliseconds, void *stream)
+{
+    return guarded([&] { aot::TreeEngine::holdSms(sms, milliseconds, static_cast<cudaStream_t>(stream)); });
+}
+
 ao_status ao_sort_config_count(int *count)
 {
     return guarded([&] {

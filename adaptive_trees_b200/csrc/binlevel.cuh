@@ -14,7 +14,8 @@
 // together with the nodes of the two depths below it: its slots are its 8
 // descendants three depths down.  A slot is an internal node (a unit of the
 // next level), a leaf, or part of a wider leaf of 2 or 4 slots, which starts
-// at the first of them.  One cooperative launch (buildKernel) makes the tree:
+// at the first of them.  One launch by team (buildKernel, grid_barrier.cuh)
+// makes the tree:
 //   levels    the 7 inner slot boundaries of each unit among its keys, then
 //             its slots (warp-aggregated slots of new units), barrier;
 //   subtree   subtree leaf counts, bottom-up, all levels at once;
@@ -151,20 +152,21 @@ __device__ __forceinline__ void growSlots(const Arena &a, int level, unsigned bu
     a.sub[g] = (u64(__popc(h8)) << lb::kSubShift) | u32(__popc(s8) - __popc(h8));
 }
 
-// The units of a level, by a whole grid: on levels of few units a CTA per
+// The units of a level, by a team: on levels of few units a CTA per
 // unit, a warp per inner boundary (sEnds: 7 words of the CTA), else a lane per
 // slot.
 __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, int level, unsigned bucket,
-                                          unsigned maxDepth, u32 start, u32 count, u32 *sEnds, int &deepest)
+                                          unsigned maxDepth, u32 start, u32 count, const Team &team, u32 *sEnds,
+                                          int &deepest)
 {
     const u32 next = start + count;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 range = depthRange(3 * level + 3);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->levelStart[level + 1] = next;
+    if (team.rank == 0 && threadIdx.x == 0) a.ctl->levelStart[level + 1] = next;
     if (count <= kWideUnits)
     {
         static_assert(kThreads / 32 >= 7, "a warp per inner boundary");
-        for (u32 i = blockIdx.x; i < count; i += gridDim.x)
+        for (u32 i = team.rank; i < count; i += team.size)
         {
             u32 *row = a.rows + size_t(start + i) * lb::kRow;
             const u32 lo = row[2], hi = row[10];
@@ -190,7 +192,7 @@ __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, i
         return;
     }
     const size_t total = size_t(count) * 8;
-    for (size_t e0 = size_t(blockIdx.x) * kThreads + warp * 32; e0 < total; e0 += size_t(gridDim.x) * kThreads)
+    for (size_t e0 = size_t(team.rank) * kThreads + warp * 32; e0 < total; e0 += size_t(team.size) * kThreads)
     {
         const size_t e = e0 + lane;
         const bool valid = e < total;
@@ -212,9 +214,9 @@ __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, i
 
 // The leaves below every unit (lb::countSubtrees): a unit without units below
 // it starts, and the unit below another that comes last takes the total on.
-__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
+__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total, const Team &team)
 {
-    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
+    for (u32 g = team.rank * blockDim.x + threadIdx.x; g < total; g += team.size * blockDim.x)
     {
         if (a.rows[size_t(g) * lb::kRow + 11] & 0xff00u) continue;
         u64 n = sort::ldRelaxed(a.sub + g);
@@ -230,14 +232,14 @@ __device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
 }
 
 // K, B and the count of the leaves that start in every unit, and the first
-// leaf index of the units below (lb::placeUnits with a lane per slot; by a
-// grid of resident CTAs).
-__device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *N, u32 total, u32 capacity)
+// leaf index of the units below (lb::placeUnits with a lane per slot).
+__device__ __forceinline__ void placeUnits(const Arena &a, const Team &team, u64 *K, u32 *B, u32 *N, u32 total,
+                                           u32 capacity, unsigned spinLimit = lb::kPlaceSpins)
 {
     Control &c = *a.ctl;
     const int lane = threadIdx.x & 31, d = lane & 7;
-    const u32 stride = gridDim.x * (kThreads / 8);
-    for (u32 g0 = blockIdx.x * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
+    const u32 stride = team.size * (kThreads / 8);
+    for (u32 g0 = team.rank * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
     {
         const u32 g = min(g0 + (lane >> 3), total - 1);
         bool done = g0 + (lane >> 3) >= total;
@@ -282,7 +284,7 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             }
             if (__all_sync(0xffffffffu, done)) break;
             if (spins < 64) continue;
-            if (spins > lb::kPlaceSpins || vload(c.error))
+            if (spins > spinLimit || vload(c.error))
             {
                 c.error = kErrLookback;
                 return;
@@ -292,12 +294,20 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
     }
 }
 
-// (cooperative)
+// (by team)
 static __global__ void __launch_bounds__(kThreads, 4) placeKernel(Arena a, u64 *K, u32 *B, u32 *N, u32 total, u32 capacity)
 {
-    const Control &c = *a.ctl;
-    if (c.overflow | c.error) return;
-    placeUnits(a, K, B, N, total, capacity);
+    Control &c = *a.ctl;
+    if (c.overflow | c.error) return;  // (c.error: this launch's, too)
+    Team team{enterRoll(&c.bar), 0};
+    if (team.rank == kLeftOut) return;
+    team.size = closeRoll(&c.bar);
+    if (!team.size)
+    {
+        if (threadIdx.x == 0) c.error = kErrLookback;
+        return;
+    }
+    placeUnits(a, team, K, B, N, total, capacity);
 }
 
 // The finished tree: its sentinel and the state the reference's passes end
@@ -345,7 +355,7 @@ struct BuildArgs
     long long logicalCap;   // the reference's leaf capacity before the build
 };
 
-// The whole build in one cooperative launch.  Bound by the latency of its
+// The whole build in one launch by team.  Bound by the latency of its
 // steps: 33 depths of an 8Mi k-d tree are 11 levels here; with a launch per
 // depth they took 190 us and 34 gaps, the subtree counts 33 us and the
 // placement 28 us, whose chains of dependent steps are a third as long now.
@@ -355,22 +365,25 @@ static __global__ void __launch_bounds__(kThreads, 4) buildKernel(BuildArgs p)
     __shared__ u32 sEnds[8];
     const Arena &a = p.a;
     Control &c = *a.ctl;
-    if (blockIdx.x == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, p.maxDepth);
-    if (!gridBarrier(&c.bar)) return;
+    Team team{enterRoll(&c.bar), 0};
+    if (team.rank == kLeftOut) return;
+    if (team.rank == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, p.maxDepth);
+    team.size = closeRoll(&c.bar);
+    if (!team.size || !gridBarrier(&c.bar, team)) return;
     int levels = 0, deepest = 0;
     for (; levels < kLevels; ++levels)
     {
         const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
         if (count == 0 || count > a.cap - start) break;
-        growUnits(a, p.idx, levels, p.bucket, p.maxDepth, start, count, sEnds, deepest);
-        if (!gridBarrier(&c.bar)) return;
+        growUnits(a, p.idx, levels, p.bucket, p.maxDepth, start, count, team, sEnds, deepest);
+        if (!gridBarrier(&c.bar, team)) return;
     }
     if ((threadIdx.x & 31) == 0 && deepest) atomicMax(&c.depths, deepest);
     const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
-    countSubtrees(a, total);
-    if (!gridBarrier(&c.bar)) return;
+    countSubtrees(a, total, team);
+    if (!gridBarrier(&c.bar, team)) return;
     if (vload(c.overflow)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
+    if (team.rank == 0 && threadIdx.x == 0)
     {
         const u32 leaves = levels ? u32(vload(a.sub[0])) : 1u;
         c.leaves = leaves;
@@ -380,7 +393,7 @@ static __global__ void __launch_bounds__(kThreads, 4) buildKernel(BuildArgs p)
         if (leaves > p.capacity) c.placeOverflow = 1;
         else finishState(p.tb, int(leaves), vload(c.depths), grownCapacity(p.logicalCap, (long long)leaves));
     }
-    placeUnits(a, p.tb.K[0], p.tb.B[0], p.tb.N[0], total, p.capacity);
+    placeUnits(a, team, p.tb.K[0], p.tb.B[0], p.tb.N[0], total, p.capacity);
 }
 }  // namespace bl
 }  // namespace aot

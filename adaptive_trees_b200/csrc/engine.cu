@@ -528,8 +528,8 @@ bool launchFusedSort(int cfg, cudaStream_t s, const sort::PassArgs &p, const sor
     const u32 tiles = u32(configTiles(cfg, p.n));
     sort::FusedArgs a{p, r, tiles, hist, bins, repair, r.keyMask == ~u64(0)};
     void *args[] = {&a};
-    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(std::min<unsigned>(tiles, unsigned(perSm) * unsigned(smCount()))),
-                                          dim3(sort::kThreads), args, smem, s));
+    AOT_CHECK(cudaLaunchKernel(fn, dim3(std::min<unsigned>(tiles, unsigned(perSm) * unsigned(smCount()))),
+                               dim3(sort::kThreads), args, smem, s));
     noteLaunch();
     return true;
 }
@@ -902,10 +902,8 @@ struct TreeEngine::Impl
     DevMem P[2], Perm[2], sample;
     SortArena sortArena;
     // state
-    DevMem stMem;                // DeviceState, then the barrier
+    DevMem stMem;
     DeviceState *st = nullptr;   // device (stMem)
-    GridBarrier *updateBar = nullptr;
-    static constexpr size_t kBarAt = (sizeof(DeviceState) + 255) & ~size_t(255);
     DeviceState *hst = nullptr;  // pinned mirror (block cache)
     size_t hstBytes = 0;
     cudaStream_t d2h = nullptr;
@@ -1088,10 +1086,9 @@ TreeEngine::TreeEngine(const void *x, const void *y, const void *z, size_t n, co
     prepared_ = cfg.views;
 
     // stream-ordered set-up: nothing here synchronises the device
-    m_->stMem.reserve(Impl::kBarAt + sizeof(GridBarrier));
-    m_->updateBar = reinterpret_cast<GridBarrier *>(m_->stMem.as<unsigned char>() + Impl::kBarAt);
+    m_->stMem.reserve(sizeof(DeviceState));
     m_->st = m_->stMem.as<DeviceState>();
-    AOT_CHECK(cudaMemsetAsync(m_->st, 0, Impl::kBarAt + sizeof(GridBarrier), cfg.stream));
+    AOT_CHECK(cudaMemsetAsync(m_->st, 0, sizeof(DeviceState), cfg.stream));
     m_->hst = static_cast<DeviceState *>(blockcache::takeHost(sizeof(DeviceState), &m_->hstBytes));
     std::memset(m_->hst, 0, sizeof(DeviceState));
     AOT_CHECK(cudaGetDevice(&m_->device));
@@ -1722,14 +1719,19 @@ void TreeEngine::setBuildMode(int mode)
 
 namespace
 {
-// A cooperative launch of at most `want` CTAs, as many as fit at once.
-void launchResident(const void *fn, void **args, int threads, unsigned want, cudaStream_t s)
+// A launch by team (grid_barrier.cuh); grid: as many CTAs as fit at once on an
+// idle GPU, or fewer.
+void launchTeam(const void *fn, void **args, int threads, unsigned grid, cudaStream_t s)
+{
+    AOT_CHECK(cudaLaunchKernel(fn, dim3(grid), dim3(unsigned(threads)), args, 0, s));
+    noteLaunch();
+}
+// The grid of a placement: all that fits.
+unsigned placeGrid(const void *fn)
 {
     int perSm = 0;
-    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, threads, 0));
-    const unsigned grid = std::max(1u, std::min(want, unsigned(perSm) * unsigned(smCount())));
-    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(unsigned(threads)), args, 0, s));
-    noteLaunch();
+    AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, lb::kThreads, 0));
+    return unsigned(std::max(1, perSm)) * unsigned(smCount());
 }
 }  // namespace
 
@@ -1746,7 +1748,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
     unsigned leafGrid = 0;
     if (!nf)
     {
-        // one cooperative launch: a CTA per unit of a typical level (2.5
+        // one launch by team: a CTA per unit of a typical level (2.5
         // leaves per bucket of particles, 7 leaves per unit), as many as fit;
         // few CTAs meet at a barrier sooner
         int perSm = 0;
@@ -1783,7 +1785,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
                              : nf               ? reinterpret_cast<const void *>(&lb::placeKernel<true, false>)
                                                 : reinterpret_cast<const void *>(&lb::placeKernel<false, false>);
             void *args[] = {&arena, &tb.K[0], &tb.B[0], &tb.NF[0], &tb.N[0], &expanded, &room};
-            launchResident(fn, args, lb::kThreads, unsigned(smCount()) * 8u, s);
+            launchTeam(fn, args, lb::kThreads, placeGrid(fn), s);
         };
         u32 rootLeaves = 1;
         if (nf)
@@ -1816,8 +1818,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         {
             lb::LeafBuildArgs p{a, idx, m.bufs(), P, n_, cfg_.bucket, cfg_.maxDepth, u32(physCap_)};
             void *args[] = {&p};
-            AOT_CHECK(cudaLaunchCooperativeKernel(lb::leafBuildKernel, dim3(leafGrid), dim3(lb::kThreads), args, 0, s));
-            noteLaunch();
+            launchTeam(reinterpret_cast<const void *>(&lb::leafBuildKernel), args, lb::kThreads, leafGrid, s);
             AOT_CHECK(cudaMemcpyAsync(host, m.lvCtl.p, kCtlBytes, cudaMemcpyDeviceToHost, s));
             waitStream(s);
             if (hc.bar.error) throw std::runtime_error("adaptive_octree: a grid barrier of the level build gave up waiting");
@@ -1873,6 +1874,7 @@ bool TreeEngine::octreeLevelBuild(std::vector<long long> &proposals)
         {
             ensurePhysical(rootLeaves);
             AOT_CHECK(cudaMemsetAsync(&a.ctl->placeOverflow, 0, sizeof(int), s));
+            AOT_CHECK(cudaMemsetAsync(&a.ctl->bar, 0, sizeof(GridBarrier), s));
             place(deepest + 1);
         }
         hostLeaves_ = rootLeaves;
@@ -2004,8 +2006,7 @@ bool TreeEngine::binaryLevelBuild()
         p.logicalCap = (long long)leafCapacity_;
         AOT_CHECK(cudaMemsetAsync(m.blCtl.p, 0, sizeof(bl::Control), s));
         void *args[] = {&p};
-        AOT_CHECK(cudaLaunchCooperativeKernel(bl::buildKernel, dim3(grid), dim3(bl::kThreads), args, 0, s));
-        noteLaunch();
+        launchTeam(reinterpret_cast<const void *>(&bl::buildKernel), args, bl::kThreads, grid, s);
         AOT_CHECK(cudaMemcpyAsync(m.blHost, m.blCtl.p, sizeof(bl::Control), cudaMemcpyDeviceToHost, s));
         waitStream(s);
         if (hc.bar.error) throw std::runtime_error("adaptive_octree: a grid barrier of the level build gave up waiting");
@@ -2026,7 +2027,9 @@ bool TreeEngine::binaryLevelBuild()
             rb::TreeBufs tb = m.bufs();
             u32 units = hc.units, room = u32(physCap_);
             void *again[] = {&a, &tb.K[0], &tb.B[0], &tb.N[0], &units, &room};
-            launchResident(reinterpret_cast<const void *>(&bl::placeKernel), again, bl::kThreads, unsigned(smCount()) * 4u, s);
+            AOT_CHECK(cudaMemsetAsync(&a.ctl->bar, 0, sizeof(GridBarrier), s));
+            const void *fn = reinterpret_cast<const void *>(&bl::placeKernel);
+            launchTeam(fn, again, bl::kThreads, placeGrid(fn), s);
             bl::finishKernel<<<1, 1, 0, s>>>(tb, int(leaves), passes, c), noteLaunch();
             AOT_LAUNCH_CHECK();
         }
@@ -2059,10 +2062,10 @@ constexpr size_t kFusedPasses = size_t(1) << 19;
 
 // The refresh, the passes and the counts of an update() in one launch
 // (rb::updateKernel).  False (nothing done) where they run launch by launch:
-// NFCount trees, and while stages are timed.
+// NFCount trees, trees without particles, and while stages are timed.
 bool TreeEngine::passesFused()
 {
-    if (cfg_.nf || profiling_) return false;
+    if (cfg_.nf || profiling_ || n_ == 0) return false;  // (the sort clears the barrier)
     if (leafCapacity_ > kFusedPasses) return false;
     const void *fn = cfg_.kind == 0 ? reinterpret_cast<const void *>(&rb::updateKernel<false>)
                                     : reinterpret_cast<const void *>(&rb::updateKernel<true>);
@@ -2070,12 +2073,11 @@ bool TreeEngine::passesFused()
     AOT_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, rb::kScanThreads, 0));
     if (perSm <= 0) return false;
     rb::UpdateArgs u{m_->bufs(), m_->keyIndex(n_), m_->P[0].as<u64>(), n_, m_->scanTiles + 1, cfg_.bucket, cfg_.maxDepth,
-                     cfg_.iterations, (long long)leafCapacity_, m_->updateBar};
+                     cfg_.iterations, (long long)leafCapacity_, &m_->sortArena.ctl()->afterBar};
     // a thread per leaf, as many CTAs as fit; few meet at a barrier sooner
     const unsigned grid = std::min(gridFor(leafCapacity_ + 1, rb::kScanThreads), unsigned(std::min(perSm, 4)) * unsigned(smCount()));
     void *args[] = {&u};
-    AOT_CHECK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(rb::kScanThreads), args, 0, cfg_.stream));
-    noteLaunch();
+    launchTeam(fn, args, rb::kScanThreads, grid, cfg_.stream);
     return true;
 }
 

@@ -182,6 +182,12 @@ public:
     // publishes, with `spinLimit` polls allowed; returns the kernel's error
     // word (kErrLookback when the wait ran out and the kernel returned)
     static int boundedWaitProbe(int which, unsigned spinLimit);
+    // the same of the waits of launches by team (0: the grid barrier, 1: the
+    // roll, 2: the octree's placement, 3: the binary tree's)
+    static int teamWaitProbe(int which, unsigned spinLimit);
+    // keeps `sms` SMs busy for some time (at most 2000 ms), as another
+    // program's long kernel would
+    static void holdSms(int sms, int milliseconds, cudaStream_t s);
     // the same with sort configuration `config` (its own scratch size)
     static void sortPairsWith(int config, void *scratch, size_t *scratchBytes, const unsigned long long *keysIn,
                               unsigned long long *keysOut, const unsigned *valsIn, unsigned *valsOut, size_t n,

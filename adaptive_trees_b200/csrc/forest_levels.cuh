@@ -101,7 +101,7 @@ static __global__ void __launch_bounds__(lb::kThreads, 4) levelBuildKernel(Level
         }
         a.sysRoot[s] = root;
     }
-    if (!gridBarrier(&ls->bar)) return;
+    if (!gridBarrier(&ls->bar, wholeGrid())) return;
     // levels: every CTA reads the same counts after a barrier (a flag may
     // already be set by the next level's units)
     int levels = 0;
@@ -109,13 +109,13 @@ static __global__ void __launch_bounds__(lb::kThreads, 4) levelBuildKernel(Level
     {
         const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
         if (count == 0 || count > a.cap - start) break;
-        growUnits<true>(a, p.idx, levels, p.bucket, start, count, sEnds, nullptr, nullptr);
-        if (!gridBarrier(&ls->bar)) return;
+        growUnits<true>(a, p.idx, levels, p.bucket, start, count, wholeGrid(), sEnds, nullptr, nullptr);
+        if (!gridBarrier(&ls->bar, wholeGrid())) return;
     }
     if (vload(c.overflow) | vload(c.late)) return;
     const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
-    countSubtrees<true>(a, total);
-    if (!gridBarrier(&ls->bar)) return;
+    countSubtrees<true>(a, total, wholeGrid());
+    if (!gridBarrier(&ls->bar, wholeGrid())) return;
     // layout (CTA 0): systems one after the other, each followed by its sentinel
     if (blockIdx.x == 0)
     {
@@ -178,7 +178,7 @@ static __global__ void __launch_bounds__(lb::kThreads, 4) levelBuildKernel(Level
             st.proposal = entries;
         }
     }
-    if (!gridBarrier(&ls->bar)) return;
+    if (!gridBarrier(&ls->bar, wholeGrid())) return;
     if (vload(ls->entriesOverflow)) return;
     // each system's leaves after every round that changes it: a final leaf at
     // (arrival a, region depth k, relative level j) stands for
@@ -228,8 +228,9 @@ static __global__ void __launch_bounds__(lb::kThreads, 4) levelBuildKernel(Level
         __syncthreads();
     }
     // placement (a unit's first entry comes from its parent)
-    placeUnits<false, false, true>(a, p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], total, p.capacity, nullptr);
-    if (!gridBarrier(&ls->bar)) return;
+    placeUnits<false, false, true>(a, wholeGrid(), p.f.K[0], p.f.B[0], nullptr, nullptr, p.f.SEG[0], total, p.capacity,
+                                   nullptr);
+    if (!gridBarrier(&ls->bar, wholeGrid())) return;
     const i64 E = vload(ls->entries);
     for (i64 i = rank; i < E; i += size)
         p.f.N[i] = p.f.K[0][i] == kMaxKey ? 0u : p.f.B[0][i + 1] - p.f.B[0][i];

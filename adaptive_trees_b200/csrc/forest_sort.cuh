@@ -109,7 +109,7 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     }
     for (int sys = blockIdx.x; sys < p.f.numSystems; sys += gridDim.x)
         systemBins(p.f.systems, p.f.numSystems, sys, p.hist, p.bins, kCountedFrom, sort::kMaxPasses);
-    if (!gridBarrier(p.bar)) return fail(p);
+    if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
     u32 repeats[sort::kPlanSets];
 #pragma unroll
     for (int k = 0; k < sort::kPlanSets; ++k) repeats[k] = vload(p.plan.counters->repeats[k]);
@@ -117,10 +117,10 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     if (first < kCountedFrom)
     {
         countLowDigits(p, first, sm.hist);
-        if (!gridBarrier(p.bar)) return fail(p);
+        if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
         for (int sys = blockIdx.x; sys < p.f.numSystems; sys += gridDim.x)
             systemBins(p.f.systems, p.f.numSystems, sys, p.hist, p.bins, first, kCountedFrom);
-        if (!gridBarrier(p.bar)) return fail(p);
+        if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
     }
     for (int pass = first; pass < sort::kMaxPasses; ++pass)
     {
@@ -134,7 +134,7 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
             p.r.ctl->tileCounters + slot, p.status, sort::passTag(epoch + u32(slot)), p.error, sort::kRadixBits,
             sort::kLookbackSpins, p.numTiles))
             __syncthreads();
-        if (!gridBarrier(p.bar)) return fail(p);
+        if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
     }
     if (first > 0)
     {
@@ -144,12 +144,12 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
             __syncthreads();
             repairSystemTile<kTile>(p.r, sm.repair, u32(first), p.tiles, p.f.systems, t);
         }
-        if (!gridBarrier(p.bar)) return fail(p);
+        if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
         const u32 runs = vload(p.r.ctl->longRuns);
         if (runs)
         {
-            sort::sortLongRuns(p.r, sm.longRun, first, runs);
-            if (!gridBarrier(p.bar)) return fail(p);
+            sort::sortLongRuns(p.r, sm.longRun, first, runs, wholeGrid());
+            if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->epoch = epoch;

@@ -22,9 +22,9 @@
 //             expand where the value is the count);
 //   subtree, place: subtree leaf counts bottom-up, then every leaf's
 //             position in the cornerstone array top-down.
-// A LeafCount build is one cooperative launch (leafBuildKernel): a unit's
-// counts are differences of its begins, so expand and classify are one step
-// (growUnits) with a grid barrier per level.  An NFCount build has two launches
+// A LeafCount build is one launch by team (leafBuildKernel, grid_barrier.cuh):
+// a unit's counts are differences of its begins, so expand and classify are
+// one step (growUnits) with a grid barrier per level.  An NFCount build has two launches
 // per level, and one each for the subtree counts and the placement.
 //
 // The capacity the reference ends with depends on how many leaves each round
@@ -44,6 +44,7 @@
 #pragma once
 
 #include "grid_barrier.cuh"
+#include "radix_sort.cuh"
 #include "rebalance.cuh"
 
 namespace aot
@@ -66,7 +67,7 @@ struct Control
     int late;           // an arrival round beyond the tracked ones
     int error;          // a bounded wait gave up
     int placeOverflow;  // the tree has more leaves than the cornerstone buffers hold
-    GridBarrier bar;    // one-launch build
+    GridBarrier bar;    // of the one-launch build, or of the placement
     u32 leaves;         // leaves of the tree
     u32 active;         // active particles
     int stateError;     // DeviceState::error
@@ -376,21 +377,21 @@ __device__ __forceinline__ void growChildren(const Arena &a, int l, unsigned buc
     }
 }
 
-// Expand and classify of a LeafCount level in one step, by a whole grid: on
+// Expand and classify of a LeafCount level in one step, by a team: on
 // levels of few units a CTA per unit, a warp per inner child boundary (sEnds:
 // 7 words of the CTA), else a lane per child.
 template <bool Forest>
 __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, int l, unsigned bucket, u32 start,
-                                          u32 count, u32 *sEnds, u32 *sContrib, u32 *sLanded)
+                                          u32 count, const Team &team, u32 *sEnds, u32 *sContrib, u32 *sLanded)
 {
     const u32 next = start + count;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 cr = octRange(unsigned(l) + 1);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->levelStart[l + 1] = next;
+    if (team.rank == 0 && threadIdx.x == 0) a.ctl->levelStart[l + 1] = next;
     if (count <= kWideUnits)
     {
         static_assert(kThreads / 32 >= 7, "a warp per inner boundary");
-        for (u32 i = blockIdx.x; i < count; i += gridDim.x)
+        for (u32 i = team.rank; i < count; i += team.size)
         {
             u32 *row = a.rows + size_t(start + i) * kRow;
             const u32 lo = row[2], hi = row[10], reg = row[11];
@@ -417,7 +418,7 @@ __device__ __forceinline__ void growUnits(const Arena &a, const KeyIndex &idx, i
         return;
     }
     const size_t total = size_t(count) * 8;
-    for (size_t e0 = size_t(blockIdx.x) * kThreads + warp * 32; e0 < total; e0 += size_t(gridDim.x) * kThreads)
+    for (size_t e0 = size_t(team.rank) * kThreads + warp * 32; e0 < total; e0 += size_t(team.size) * kThreads)
     {
         const size_t e = e0 + lane;
         const bool valid = e < total;
@@ -1221,9 +1222,9 @@ static __global__ void __launch_bounds__(kThreads) unitsToTableKernel(Arena a, r
 // unit whose children are all leaves starts (8 leaves) and adds its count to
 // its parent's; the child that comes last takes the parent's total on.
 template <bool Forest>
-__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total)
+__device__ __forceinline__ void countSubtrees(const Arena &a, u32 total, const Team &team)
 {
-    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
+    for (u32 g = team.rank * blockDim.x + threadIdx.x; g < total; g += team.size * blockDim.x)
     {
         // (a unit with internal children holds 15 leaves or more when they have come)
         u64 n = sort::ldRelaxed(a.sub + g);
@@ -1249,7 +1250,7 @@ static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int le
 {
     const Control &c = *a.ctl;
     if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
-    countSubtrees<false>(a, c.levelStart[levels]);
+    countSubtrees<false>(a, c.levelStart[levels], wholeGrid());
 }
 
 // Cornerstone entries of the leaf children of every unit (the first `total`),
@@ -1262,9 +1263,8 @@ static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int le
 // children by octant).
 //
 // A unit waits for its own place, which its parent's warp writes; parents come
-// before their children in the arena.  The warps of the grid, all resident
-// (cooperative launches), take units in increasing order, and a warp writes
-// what is ready before it polls again (parent and child may share it), so the
+// before their children in the arena.  The warps of the team, all resident,
+// take units in increasing order, and a warp writes what is ready before it polls again (parent and child may share it), so the
 // first unit not placed is always being worked on and the waits end (they are
 // bounded all the same).  Bound by the latency of a step: child, its leaf
 // count, the poll.  Chunks of units handed out by a counter, with their levels
@@ -1272,13 +1272,14 @@ static __global__ void __launch_bounds__(kThreads) subtreeKernel(Arena a, int le
 // the 1.8 M of 16Mi and 51 us for the 133k of an 8Mi k-d tree (a kernel per
 // level before that: 36 us and 11 gaps at 300k).
 template <bool NF, bool Hilbert, bool Forest>
-__device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG, u32 total,
-                                           u32 capacity, const unsigned char *dec)
+__device__ __forceinline__ void placeUnits(const Arena &a, const Team &team, u64 *K, u32 *B, u32 *NFo, u32 *N, int *SEG,
+                                           u32 total, u32 capacity, const unsigned char *dec,
+                                           unsigned spinLimit = kPlaceSpins)
 {
     Control &c = *a.ctl;
     const int lane = threadIdx.x & 31, d = lane & 7;
-    const u32 stride = gridDim.x * (kThreads / 8);
-    for (u32 g0 = blockIdx.x * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
+    const u32 stride = team.size * (kThreads / 8);
+    for (u32 g0 = team.rank * (kThreads / 8) + (threadIdx.x >> 5) * 4; g0 < total; g0 += stride)
     {
         const u32 g = min(g0 + (lane >> 3), total - 1);
         bool done = g0 + (lane >> 3) >= total;
@@ -1334,7 +1335,7 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
             }
             if (__all_sync(0xffffffffu, done)) break;
             if (spins < 64) continue;
-            if (spins > kPlaceSpins || vload(c.error))
+            if (spins > spinLimit || vload(c.error))
             {
                 c.error = kErrLookback;
                 return;
@@ -1344,21 +1345,29 @@ __device__ __forceinline__ void placeUnits(const Arena &a, u64 *K, u32 *B, u32 *
     }
 }
 
-// (cooperative)  `levels`: the levels the build expanded.
+// (by team)  `levels`: the levels the build expanded.
 template <bool NF, bool Hilbert>
 static __global__ void __launch_bounds__(kThreads, 4)
     placeKernel(Arena a, u64 *K, u32 *B, u32 *NFo, u32 *N, int levels, u32 capacity)
 {
     __shared__ __align__(4) unsigned char sDec[48 * 8];
-    const Control &c = *a.ctl;
-    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;
+    Control &c = *a.ctl;
+    if (c.levelCount[levels] | c.overflow | c.late | c.error) return;  // (c.error: this launch's, too)
+    Team team{enterRoll(&c.bar), 0};
+    if (team.rank == kLeftOut) return;
     if constexpr (NF && Hilbert)
     {
         copyTable(sDec, gHilbert.decOct);
         __syncthreads();
     }
     const u32 total = c.levelCount[0] ? c.levelStart[levels] : 0u;
-    placeUnits<NF, Hilbert, false>(a, K, B, NFo, N, nullptr, total, capacity, sDec);
+    team.size = closeRoll(&c.bar);
+    if (!team.size)
+    {
+        if (threadIdx.x == 0) c.error = kErrLookback;
+        return;
+    }
+    placeUnits<NF, Hilbert, false>(a, team, K, B, NFo, N, nullptr, total, capacity, sDec);
 }
 
 // The finished tree: sentinel boundary and the state of a converged build
@@ -1399,7 +1408,7 @@ struct LeafBuildArgs
     u32 capacity;  // leaves the cornerstone buffers hold
 };
 
-// A LeafCount build in one cooperative launch: root, levels, subtree counts,
+// A LeafCount build in one launch by team: root, levels, subtree counts,
 // placement and final state.  Bound by the latency of the searches and the
 // barriers on small trees, of the searches on large ones.  With a launch per
 // step and level: 10k particles 74 us in 19 launches, now 49; 1Mi 71 in 15,
@@ -1420,15 +1429,18 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
     for (int k = threadIdx.x; k < kContribBins; k += kThreads) sContrib[k] = 0;
     if (threadIdx.x < kArrivals) sLanded[threadIdx.x] = 0;
     if (threadIdx.x == 0) sRounds = 0;
-    if (blockIdx.x == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, false);
-    if (!gridBarrier(&c.bar)) return;
+    Team team{enterRoll(&c.bar), 0};
+    if (team.rank == kLeftOut) return;
+    if (team.rank == 0 && threadIdx.x < 32) rootUnit(a, p.tb, p.P, p.n, p.bucket, false);
+    team.size = closeRoll(&c.bar);
+    if (!team.size || !gridBarrier(&c.bar, team)) return;
     int levels = 0;
     for (; levels < int(kOctLevels); ++levels)
     {
         const u32 start = vload(c.levelStart[levels]), count = vload(c.levelCount[levels]);
         if (count == 0 || count > a.cap - start) break;
-        growUnits<false>(a, p.idx, levels, p.bucket, start, count, sEnds, sContrib, sLanded);
-        if (!gridBarrier(&c.bar)) return;
+        growUnits<false>(a, p.idx, levels, p.bucket, start, count, team, sEnds, sContrib, sLanded);
+        if (!gridBarrier(&c.bar, team)) return;
     }
     __syncthreads();
     for (int k = threadIdx.x; k < kContribBins; k += kThreads)
@@ -1436,10 +1448,10 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
     if (threadIdx.x < kArrivals && sLanded[threadIdx.x])
         atomicAdd(a.landed + threadIdx.x, (unsigned long long)sLanded[threadIdx.x]);
     const u32 total = levels ? vload(c.levelStart[levels]) : 0u;
-    countSubtrees<false>(a, total);
-    if (!gridBarrier(&c.bar)) return;
+    countSubtrees<false>(a, total, team);
+    if (!gridBarrier(&c.bar, team)) return;
     if (vload(c.overflow) | vload(c.late)) return;
-    if (blockIdx.x == 0)
+    if (team.rank == 0)
     {
         for (int k = threadIdx.x; k < kContribBins; k += kThreads)
             if (vload(a.contrib[k]))
@@ -1458,7 +1470,7 @@ static __global__ void __launch_bounds__(kThreads, 4) leafBuildKernel(LeafBuildA
             else if (sRounds <= int(p.maxDepth)) finishState(p.tb, int(leaves), sRounds);
         }
     }
-    placeUnits<false, false, false>(a, p.tb.K[0], p.tb.B[0], nullptr, p.tb.N[0], nullptr, total, p.capacity, nullptr);
+    placeUnits<false, false, false>(a, team, p.tb.K[0], p.tb.B[0], nullptr, p.tb.N[0], nullptr, total, p.capacity, nullptr);
 }
 }  // namespace lb
 }  // namespace aot

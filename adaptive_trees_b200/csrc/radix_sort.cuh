@@ -94,9 +94,22 @@ struct SortControl
     u32 longRuns;   // runs the repair left to the long-run kernel
     u32 keygenDone; // CTAs of the key generation that have added their digit counts
     u32 tileCounters[kPassSlots];
-    GridBarrier bar; // of a sort in one launch (as each barrier leaves it)
+    GridBarrier sortBar;   // of the passes and the repair in one launch
+    GridBarrier afterBar;  // of what follows the sort in one launch (update())
 };
 constexpr u32 kEpochStep = 16;  // tags per sort (>= kPassSlots)
+
+// Zeroes the barriers of a sort and of what follows it (one CTA, before them).
+__device__ __forceinline__ void clearBarriers(SortControl *ctl)
+{
+    static_assert(sizeof(GridBarrier) % sizeof(u32) == 0, "words");
+    constexpr u32 kWords = sizeof(GridBarrier) / sizeof(u32);
+    for (u32 i = threadIdx.x; i < kWords; i += blockDim.x)
+    {
+        reinterpret_cast<u32 *>(&ctl->sortBar)[i] = 0;
+        reinterpret_cast<u32 *>(&ctl->afterBar)[i] = 0;
+    }
+}
 
 // Start of a sort without a plan: every pass runs.
 static __global__ void __launch_bounds__(kThreads) beginSortKernel(SortControl *ctl, u32 *hist)
@@ -104,6 +117,7 @@ static __global__ void __launch_bounds__(kThreads) beginSortKernel(SortControl *
     if (hist)
         for (int i = threadIdx.x; i < kPassSlots * kRadix; i += blockDim.x) hist[i] = 0;
     if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
+    clearBarriers(ctl);
     if (threadIdx.x == 0)
     {
         ctl->first = 0;

@@ -303,14 +303,14 @@ __device__ __forceinline__ int warpAppend(int *counter, int count)
 // proposal fits, as its build loop does through needsResize/growBuffers
 // (kdtree3d.cu:239-249).
 __device__ __forceinline__ void commitIfLast(DeviceState *st, long long limit, int mode, bool binary,
-                                             long long *history)
+                                             long long *history, const Team &team)
 {
     __shared__ bool sLast;
     __syncthreads();
     if (threadIdx.x == 0)
     {
         __threadfence();
-        sLast = atomicAdd(&st->doneBlocks, 1) == int(gridDim.x) - 1;
+        sLast = atomicAdd(&st->doneBlocks, 1) == int(team.size) - 1;
     }
     __syncthreads();
     if (!sLast || threadIdx.x != 0) return;
@@ -547,7 +547,8 @@ __device__ __forceinline__ void octScatterLeaf(const TreeBufs &tb, DeviceState *
 // warp of kept leaves is done then; loads behind the op code and the flag took
 // 127 instead of 92 us for 12.7 M leaves.
 template <bool NF>
-__device__ __forceinline__ void octScatter(const TreeBufs &tb, long long limit, int mode, long long *history)
+__device__ __forceinline__ void octScatter(const TreeBufs &tb, long long limit, int mode, long long *history,
+                                           const Team &team)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;  // uniform: the state does not change before the last CTA
@@ -558,18 +559,18 @@ __device__ __forceinline__ void octScatter(const TreeBufs &tb, long long limit, 
         const int L = st->numLeaves;
         const int a = st->activeBuffer, b = a ^ 1;
         const int lane = threadIdx.x & 31;
-        const int warpsTotal = gridDim.x * (blockDim.x / 32);
-        const int w0 = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        const int warpsTotal = team.size * (blockDim.x / 32);
+        const int w0 = team.rank * (blockDim.x / 32) + (threadIdx.x >> 5);
         for (int base = w0 * 32; base < L; base += warpsTotal * 32) octScatterLeaf<NF>(tb, st, base + lane, L, a, b, total);
     }
-    commitIfLast(st, limit, mode, false, history);
+    commitIfLast(st, limit, mode, false, history, team);
 }
 
 template <bool NF>
 static __global__ void __launch_bounds__(kScatterThreads)
     octScatterKernel(TreeBufs tb, long long limit, int mode, long long *history)
 {
-    octScatter<NF>(tb, limit, mode, history);
+    octScatter<NF>(tb, limit, mode, history, wholeGrid());
 }
 
 // Lower bound of v in the sorted keys when `lo` is already a lower bound of a
@@ -601,7 +602,7 @@ __device__ __forceinline__ u32 lowerFrom(const KeyIndex &idx, u32 lo, u64 v)
 // the end sentinel).  This is the whole count refresh of LeafCount trees: the
 // counts are differences of B.
 template <bool All>
-__device__ __forceinline__ void octBegins(const TreeBufs &tb, const KeyIndex &idx)
+__device__ __forceinline__ void octBegins(const TreeBufs &tb, const KeyIndex &idx, const Team &team)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;
@@ -609,9 +610,9 @@ __device__ __forceinline__ void octBegins(const TreeBufs &tb, const KeyIndex &id
     const int L = st->numLeaves;
     const u64 *K = tb.k(a);
     u32 *B = tb.b(a);
-    if (All && blockIdx.x == 0 && threadIdx.x == 0) B[L] = st->numActiveParticles;
+    if (All && team.rank == 0 && threadIdx.x == 0) B[L] = st->numActiveParticles;
     const int count = All ? L : st->dirtyCount;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
+    for (int j = team.rank * blockDim.x + threadIdx.x; j < count; j += team.size * blockDim.x)
     {
         const int i = All ? j : tb.dirty[j];
         B[i] = u32(idx.lower(K[i]));
@@ -621,7 +622,7 @@ __device__ __forceinline__ void octBegins(const TreeBufs &tb, const KeyIndex &id
 template <bool All>
 static __global__ void __launch_bounds__(kRefreshThreads) octBeginKernel(TreeBufs tb, KeyIndex idx)
 {
-    octBegins<All>(tb, idx);
+    octBegins<All>(tb, idx, wholeGrid());
 }
 
 // The begin index of every leaf (and B[L] = the active count) by merging the
@@ -1340,16 +1341,16 @@ static __global__ void __launch_bounds__(kRefreshThreads, 4)
 }
 
 // N[i] = B[i+1] - B[i] on the active buffer.
-__device__ __forceinline__ void materializeCounts(const TreeBufs &tb)
+__device__ __forceinline__ void materializeCounts(const TreeBufs &tb, const Team &team)
 {
     const DeviceState *st = tb.st;
     const int a = st->activeBuffer, L = st->numLeaves;
     const u32 *B = tb.b(a);
     u32 *N = tb.n(a);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) N[i] = B[i + 1] - B[i];
+    for (int i = team.rank * blockDim.x + threadIdx.x; i < L; i += team.size * blockDim.x) N[i] = B[i + 1] - B[i];
 }
 
-static __global__ void materializeCountsKernel(TreeBufs tb) { materializeCounts(tb); }
+static __global__ void materializeCountsKernel(TreeBufs tb) { materializeCounts(tb, wholeGrid()); }
 
 // --------------------------------------------------------------------------
 // Binary (kdtree3d_rebalance.cuh:61-125)
@@ -1381,7 +1382,7 @@ static __global__ void __launch_bounds__(kScanThreads) binDecideScanKernel(TreeB
     decideScan(op, tb, tb.k(a), tb.b(a), static_cast<const u8 *>(nullptr));
 }
 
-__device__ __forceinline__ void binScatter(const TreeBufs &tb, long long limit, int mode)
+__device__ __forceinline__ void binScatter(const TreeBufs &tb, long long limit, int mode, const Team &team)
 {
     DeviceState *st = tb.st;
     if (halted(st)) return;
@@ -1392,8 +1393,8 @@ __device__ __forceinline__ void binScatter(const TreeBufs &tb, long long limit, 
         const int L = st->numLeaves;
         const int a = st->activeBuffer, b = a ^ 1;
         const int lane = threadIdx.x & 31;
-        const int warpsTotal = gridDim.x * (blockDim.x / 32);
-        const int w0 = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        const int warpsTotal = team.size * (blockDim.x / 32);
+        const int w0 = team.rank * (blockDim.x / 32) + (threadIdx.x >> 5);
         for (int base = w0 * 32; base < L; base += warpsTotal * 32)
         {
             const int i = base + lane;
@@ -1424,13 +1425,13 @@ __device__ __forceinline__ void binScatter(const TreeBufs &tb, long long limit, 
             if (nDirty) tb.dirty[d0] = int(ni) + 1;
         }
     }
-    commitIfLast(st, limit, mode, true, nullptr);
+    commitIfLast(st, limit, mode, true, nullptr, team);
 }
 
 static __global__ void __launch_bounds__(kScatterThreads)
     binScatterKernel(TreeBufs tb, long long limit, int mode)
 {
-    binScatter(tb, limit, mode);
+    binScatter(tb, limit, mode, wholeGrid());
 }
 
 // Binary count refresh: B of new split points (All: every boundary).  The
@@ -1464,6 +1465,7 @@ __device__ __forceinline__ void resetForUpdate(DeviceState *st, const u64 *P, si
     st->converged = 0;
     st->numActiveParticles = active;
     st->dirtyCount = 0;
+    st->doneBlocks = 0;
     st->updatePasses = 0;
 }
 
@@ -1476,12 +1478,12 @@ static __global__ void beginPassKernel(DeviceState *st)
     st->dirtyCount = 0;
 }
 
-// All of an update() after the sort in one cooperative launch, for octrees
-// that refine by leaf counts and binary trees: the reset, the begin index of
-// every leaf, `iterations` passes (decide and scan, scatter, new begins) and
-// the counts, with a grid barrier between.  A pass of its own launches is five
-// of them, each too short to pay for its launch: 30k particles 56 us and 13
-// launches after the sort.
+// All of an update() after the sort in one launch by team (grid_barrier.cuh),
+// for octrees that refine by leaf counts and binary trees: the reset, the
+// begin index of every leaf, `iterations` passes (decide and scan, scatter,
+// new begins) and the counts, with a grid barrier between.  A pass of its own
+// launches is five of them, each too short to pay for its launch: 30k
+// particles 56 us and 13 launches after the sort.
 struct UpdateArgs
 {
     TreeBufs tb;
@@ -1490,7 +1492,7 @@ struct UpdateArgs
     size_t n, scanWords;  // scanWords: status words and tile counter of the scan
     unsigned bucket, maxDepth, iterations;
     long long limit;      // the reference's leaf capacity
-    GridBarrier *bar;
+    GridBarrier *bar;       // zero on entry
 };
 
 template <bool Binary>
@@ -1498,31 +1500,35 @@ static __global__ void __launch_bounds__(kScanThreads, 4) updateKernel(UpdateArg
 {
     const TreeBufs &tb = u.tb;
     DeviceState *st = tb.st;
-    const size_t rank = size_t(blockIdx.x) * blockDim.x + threadIdx.x, size = size_t(gridDim.x) * blockDim.x;
+    Team team{enterRoll(u.bar), 0};
+    if (team.rank == kLeftOut) return;
+    if (team.rank == 0 && threadIdx.x < 32) resetForUpdate(st, u.P, u.n);
+    team.size = closeRoll(u.bar);
+    const bool first = team.rank == 0 && threadIdx.x == 0;
     const auto clearScan = [&] {
-        for (size_t i = rank; i < u.scanWords; i += size) tb.scanStatus[i] = 0;
+        for (size_t i = size_t(team.rank) * blockDim.x + threadIdx.x; i < u.scanWords; i += size_t(team.size) * blockDim.x)
+            tb.scanStatus[i] = 0;
     };
     // (the barrier's failure is the host's to report: the state's error word)
     const auto barrier = [&] {
-        const bool ok = gridBarrier(u.bar);
+        const bool ok = team.size && gridBarrier(u.bar, team);
         if (!ok && threadIdx.x == 0) atomicExch(&st->error, kErrLookback);
         return ok;
     };
-    if (blockIdx.x == 0 && threadIdx.x < 32) resetForUpdate(st, u.P, u.n);
-    clearScan();
     if (!barrier()) return;
-    octBegins<true>(tb, u.idx);
+    clearScan();
+    octBegins<true>(tb, u.idx, team);
     if (!barrier()) return;
     for (unsigned pass = 0; pass < u.iterations; ++pass)
     {
         if (halted(st))
         {
             // the passes left only reset what a decision accumulates
-            if (rank == 0) st->changed = st->dirtyCount = 0;
+            if (first) st->changed = st->dirtyCount = 0;
             if (!barrier()) return;
             break;
         }
-        if (rank == 0) st->dirtyCount = 0;  // (filled by the scatter)
+        if (first) st->dirtyCount = 0;  // (filled by the scatter)
         const int a = st->activeBuffer;
         if constexpr (Binary)
         {
@@ -1536,14 +1542,14 @@ static __global__ void __launch_bounds__(kScanThreads, 4) updateKernel(UpdateArg
         }
         if (!barrier()) return;
         clearScan();
-        if constexpr (Binary) binScatter(tb, u.limit, kModeUpdate);
-        else octScatter<false>(tb, u.limit, kModeUpdate, nullptr);
+        if constexpr (Binary) binScatter(tb, u.limit, kModeUpdate, team);
+        else octScatter<false>(tb, u.limit, kModeUpdate, nullptr, team);
         if (!barrier()) return;
-        octBegins<false>(tb, u.idx);
-        if (rank == 0 && pass + 1 < u.iterations) st->changed = 0;
+        octBegins<false>(tb, u.idx, team);
+        if (first && pass + 1 < u.iterations) st->changed = 0;
         if (!barrier()) return;
     }
-    materializeCounts(tb);
+    materializeCounts(tb, team);
 }
 
 }  // namespace rb

@@ -12,12 +12,21 @@
 //            starting at 1, so the CTAs take tiles 1..3;
 //   which 1: the decide+scan look-back of tiles 1..3 over a zeroed status
 //            array.
+// The launches by team (grid_barrier.cuh) wait for the CTAs of their team and,
+// in the placements, for a parent's place; teamWaitProbe runs one CTA of them
+// where nobody else comes:
+//   which 0: a grid barrier of a team of 2, then (a small and a large team
+//            count their arrivals in different words) of 400;
+//   which 1: the roll of a launch, with nobody on it and no limit but the wait's;
+//   which 2: the octree's placement of a unit whose parent never places it;
+//   which 3: the same of the binary tree.
 // Every index stays inside its buffer (a tile that gave up writes its keys at
 // the prefix it has, below the prefix of the full input), and every wait is
 // bounded by `spinLimit`, so the probes neither fault nor hang.
 #include <stdexcept>
 #include <string>
 
+#include "binlevel.cuh"
 #include "engine_util.cuh"
 #include "radix_sort.cuh"
 #include "rebalance.cuh"
@@ -42,6 +51,47 @@ __global__ void scanWaitProbeKernel(u64 *status, int *error, unsigned spinLimit,
 {
     const i64 p = rb::lookback(status, blockIdx.x + 1, 1, error, spinLimit);
     if (threadIdx.x == 0) prefix[blockIdx.x] = p;
+}
+
+__global__ void __launch_bounds__(lb::kThreads) barrierProbeKernel(GridBarrier *bar, u32 size, unsigned spinLimit, int *error)
+{
+    if (!gridBarrier(bar, Team{0, size}, spinLimit) && threadIdx.x == 0) *error = kErrLookback;
+}
+
+__global__ void __launch_bounds__(lb::kThreads) rollProbeKernel(GridBarrier *bar, unsigned spinLimit, int *error)
+{
+    if (!closeRoll(bar, spinLimit, 0xffffffffu) && threadIdx.x == 0) *error = kErrLookback;
+}
+
+__global__ void __launch_bounds__(lb::kThreads) placeProbeKernel(lb::Arena a, u64 *K, u32 *B, u32 *N, unsigned spinLimit, int *error)
+{
+    lb::placeUnits<false, false, false>(a, Team{0, 1}, K, B, nullptr, N, nullptr, 1, 8, nullptr, spinLimit);
+    __syncthreads();
+    if (threadIdx.x == 0) *error = a.ctl->error;
+}
+
+__global__ void __launch_bounds__(lb::kThreads) binaryPlaceProbeKernel(bl::Arena a, u64 *K, u32 *B, u32 *N, unsigned spinLimit, int *error)
+{
+    bl::placeUnits(a, Team{0, 1}, K, B, N, 1, 8, spinLimit);
+    __syncthreads();
+    if (threadIdx.x == 0) *error = a.ctl->error;
+}
+
+// A CTA that fills its SM's shared memory and waits (bounded by the clock and by polls).
+constexpr size_t kHoldBytes = 200 * 1024;
+constexpr int kHoldMilliseconds = 2000;
+__global__ void __launch_bounds__(32) holdKernel(unsigned long long nanoseconds)
+{
+    extern __shared__ u32 held[];
+    unsigned long long start, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(start));
+    u32 polls = 0;
+    do
+    {
+        __nanosleep(1000);
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    } while (now - start < nanoseconds && ++polls < (1u << 22));
+    if (threadIdx.x == 0) held[0] = polls;
 }
 
 // Device allocations of the probe, freed on every exit path.
@@ -101,5 +151,73 @@ int TreeEngine::boundedWaitProbe(int which, unsigned spinLimit)
     int error = 0;
     AOT_CHECK(cudaMemcpy(&error, err.p, sizeof(int), cudaMemcpyDeviceToHost));
     return error;
+}
+
+int TreeEngine::teamWaitProbe(int which, unsigned spinLimit)
+{
+    if (which < 0 || which > 3) throw std::invalid_argument("ao_selftest_team_wait: which must be 0 to 3");
+    if (spinLimit == 0 || spinLimit > (1u << 16))
+        throw std::invalid_argument("ao_selftest_team_wait: spin_limit must be in [1, 65536]");
+    ProbeStream ps;
+    const cudaStream_t s = ps.s;
+    ProbeMem err(2 * sizeof(int)), bar(sizeof(GridBarrier));
+    AOT_CHECK(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), s));
+    AOT_CHECK(cudaMemsetAsync(bar.p, 0, sizeof(GridBarrier), s));
+    // one unit of 8 leaves, whose first leaf's index never comes
+    ProbeMem rows(lb::kRow * sizeof(u32)), child(8 * sizeof(u32)), sub(sizeof(u64)), offset(sizeof(u32));
+    ProbeMem ctl(std::max(sizeof(lb::Control), sizeof(bl::Control)));
+    ProbeMem K(8 * sizeof(u64)), B(8 * sizeof(u32)), N(8 * sizeof(u32));
+    AOT_CHECK(cudaMemsetAsync(rows.p, 0, lb::kRow * sizeof(u32), s));
+    AOT_CHECK(cudaMemsetAsync(child.p, 0xff, 8 * sizeof(u32), s));  // kLeaf
+    AOT_CHECK(cudaMemsetAsync(offset.p, 0xff, sizeof(u32), s));     // kPending
+    AOT_CHECK(cudaMemsetAsync(ctl.p, 0, std::max(sizeof(lb::Control), sizeof(bl::Control)), s));
+    int *error = err.as<int>();
+    if (which == 0)
+    {
+        barrierProbeKernel<<<1, lb::kThreads, 0, s>>>(bar.as<GridBarrier>(), 2, spinLimit, error);
+        AOT_CHECK(cudaMemsetAsync(bar.p, 0, sizeof(GridBarrier), s));
+        barrierProbeKernel<<<1, lb::kThreads, 0, s>>>(bar.as<GridBarrier>(), 400, spinLimit, error + 1);
+    }
+    else if (which == 1)
+    {
+        rollProbeKernel<<<1, lb::kThreads, 0, s>>>(bar.as<GridBarrier>(), spinLimit, error);
+    }
+    else if (which == 2)
+    {
+        lb::Arena a{};
+        a.rows = rows.as<u32>();
+        a.child = child.as<u32>();
+        a.sub = sub.as<u64>();
+        a.offset = offset.as<u32>();
+        a.ctl = ctl.as<lb::Control>();
+        a.cap = 1;
+        placeProbeKernel<<<1, lb::kThreads, 0, s>>>(a, K.as<u64>(), B.as<u32>(), N.as<u32>(), spinLimit, error);
+    }
+    else
+    {
+        bl::Arena a{};
+        a.rows = rows.as<u32>();
+        a.child = child.as<u32>();
+        a.sub = sub.as<u64>();
+        a.offset = offset.as<u32>();
+        a.ctl = ctl.as<bl::Control>();
+        a.cap = 1;
+        binaryPlaceProbeKernel<<<1, lb::kThreads, 0, s>>>(a, K.as<u64>(), B.as<u32>(), N.as<u32>(), spinLimit, error);
+    }
+    AOT_LAUNCH_CHECK();
+    AOT_CHECK(cudaStreamSynchronize(s));
+    int e[2] = {0, 0};
+    AOT_CHECK(cudaMemcpy(e, err.p, sizeof(e), cudaMemcpyDeviceToHost));
+    return which == 0 && e[0] != e[1] ? 0 : e[0];
+}
+
+void TreeEngine::holdSms(int sms, int milliseconds, cudaStream_t s)
+{
+    if (sms < 1 || sms > smCount()) throw std::invalid_argument("ao_selftest_hold_sms: sms must be in [1, the device's]");
+    if (milliseconds < 1 || milliseconds > kHoldMilliseconds)
+        throw std::invalid_argument("ao_selftest_hold_sms: milliseconds must be in [1, 2000]");
+    AOT_CHECK(cudaFuncSetAttribute(holdKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kHoldBytes)));
+    holdKernel<<<unsigned(sms), 32, kHoldBytes, s>>>((unsigned long long)milliseconds * 1000000ull);
+    AOT_LAUNCH_CHECK();
 }
 }  // namespace aot

@@ -1,15 +1,17 @@
 // sort_fused.cuh -- the passes and the repair of a contiguous sort in one
-// cooperative launch.
+// launch by team (grid_barrier.cuh).
 //
 // Small sorts are bound by launches: 10k keys in 3 passes spend 5 us in each
 // pass, 1 us and a launch in each of the 5 passes the plan leaves out, and two
 // launches in the repair.  Here the CTAs go through the same tiles phase by
 // phase, with a grid barrier between:
-//   counts     (optional) digit counts of the passes that run, and their bins;
+//   counts     (optional) digit counts of the passes that run, tiles taken
+//              from a counter, and their bins;
 //   passes     the onesweep passes; in each, CTAs take tiles from the pass's
 //              counter until it runs out.  A tile's look-back waits only for
 //              tiles taken before it, by CTAs that are resident and do not
-//              wait for later tiles, so every wait ends;
+//              wait for later tiles, so every wait ends.  The roll of the team
+//              closes behind the first phase: whoever takes a tile is on it;
 //   repair     the runs of equal high digits (sort_repair.cuh), tile by tile,
 //              then the long ones.
 #pragma once
@@ -52,31 +54,46 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
     extern __shared__ __align__(16) unsigned char smemRaw[];
     FusedShared<Items> &sm = *reinterpret_cast<FusedShared<Items> *>(smemRaw);
     const PassArgs &p = a.p;
-    GridBarrier *bar = &p.ctl->bar;
+    GridBarrier *bar = &p.ctl->sortBar;
+    Team team{enterRoll(bar), 0};
+    if (team.rank == kLeftOut) return;
     const auto fail = [&] {
         if (threadIdx.x == 0) atomicExch(p.error, kErrLookback);
+    };
+    const auto barrier = [&] {
+        if (!team.size) team.size = closeRoll(bar);
+        return team.size && gridBarrier(bar, team);
     };
     const int first = int(p.ctl->first);
     if (a.hist)
     {
+        constexpr int kCountSlot = kPassSlots - 1;  // no pass' tile counter
+        static_assert(kMaxPasses <= kCountSlot, "a counter to spare");
+        __shared__ u32 sTile;
         for (int i = threadIdx.x; i < kPassSlots * kRadix; i += kThreads) sm.hist[i] = 0;
-        __syncthreads();
-        for (size_t g = size_t(blockIdx.x) * kThreads + threadIdx.x; g < p.n; g += size_t(gridDim.x) * kThreads)
+        for (;;)
         {
-            const u64 k = p.keysIn[g];
-            for (int q = first; q < p.passes; ++q)
+            __syncthreads();
+            if (threadIdx.x == 0) sTile = atomicAdd(p.ctl->tileCounters + kCountSlot, 1u);
+            __syncthreads();
+            if (sTile >= a.tiles) break;
+            const size_t begin = size_t(sTile) * kTile, end = min(p.n, begin + kTile);
+            for (size_t g = begin + threadIdx.x; g < end; g += kThreads)
             {
-                const int shift = p.beginBit + q * kRadixBits;
-                const int bits = min(kRadixBits, p.endBit - shift);
-                atomicAdd(&sm.hist[q * kRadix + int((k >> shift) & ((1u << bits) - 1))], 1u);
+                const u64 k = p.keysIn[g];
+                for (int q = first; q < p.passes; ++q)
+                {
+                    const int shift = p.beginBit + q * kRadixBits;
+                    const int bits = min(kRadixBits, p.endBit - shift);
+                    atomicAdd(&sm.hist[q * kRadix + int((k >> shift) & ((1u << bits) - 1))], 1u);
+                }
             }
         }
-        __syncthreads();
         for (int i = first * kRadix + threadIdx.x; i < p.passes * kRadix; i += kThreads)
             if (sm.hist[i]) atomicAdd(a.hist + i, sm.hist[i]);
-        if (!gridBarrier(bar)) return fail();
-        if (blockIdx.x == 0) scanBins(a.hist, a.binsOut, first, p.passes);
-        if (!gridBarrier(bar)) return fail();
+        if (!barrier()) return fail();
+        if (team.rank == 0) scanBins(a.hist, a.binsOut, first, p.passes);
+        if (!barrier()) return fail();
     }
     for (int pass = first; pass < p.passes; ++pass)
     {
@@ -90,7 +107,7 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
                                                p.ctl->tileCounters + slot, p.status, passTag(p.ctl->epoch + u32(slot)),
                                                p.error, min(kRadixBits, p.endBit - shift), kLookbackSpins, a.tiles))
             __syncthreads();
-        if (!gridBarrier(bar)) return fail();
+        if (!barrier()) return fail();
     }
     if (!a.repair) return;
     const RepairArgs &r = a.r;
@@ -98,14 +115,14 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
     {
         // every pass has run; only the sample is left
         if (r.sample)
-            for (size_t j = size_t(blockIdx.x) * kThreads + threadIdx.x; (j << kSampleShift) < r.n;
-                 j += size_t(gridDim.x) * kThreads)
+            for (size_t j = size_t(team.rank) * kThreads + threadIdx.x; (j << kSampleShift) < r.n;
+                 j += size_t(team.size) * kThreads)
                 r.sample[j] = r.k[0][j << kSampleShift];
         return;
     }
     if (vload(*p.error)) return;
     const bool inPlace = r.endsIn0 || ((u32(r.passes) - u32(first)) & 1u) == 0;
-    for (u32 t = blockIdx.x; t < a.tiles; t += gridDim.x)
+    for (u32 t = team.rank; t < a.tiles; t += team.size)
     {
         __syncthreads();
         const size_t begin = size_t(t) * kTile;
@@ -113,9 +130,9 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
         else if (a.whole && first < 4) repairTile<3>(r, sm.repair, u32(first), inPlace, begin, 0, r.n);
         else repairTile<0>(r, sm.repair, u32(first), inPlace, begin, 0, r.n);
     }
-    if (!gridBarrier(bar)) return fail();
+    if (!barrier()) return fail();
     const u32 runs = vload(p.ctl->longRuns);
-    if (runs) sortLongRuns(r, sm.longRun, first, runs);
+    if (runs) sortLongRuns(r, sm.longRun, first, runs, team);
 }
 
 // The kernel of a configuration (nullptr: none) and its shared memory.

@@ -180,6 +180,7 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
         a.counters->repeats[threadIdx.x] = 0;
     }
     if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
+    clearBarriers(ctl);
     __syncthreads();
     if (threadIdx.x == 0)
     {

@@ -289,13 +289,14 @@ struct LongShared
 // of them equal, took 267 us with a digit counted to see that it is shared and
 // a key per thread and step; 17k such keys take 122 now, 50k 327.
 template <int Threads>
-__device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Threads> &sm, int first, u32 runs)
+__device__ __forceinline__ void sortLongRuns(const RepairArgs &a, LongShared<Threads> &sm, int first, u32 runs,
+                                             const Team &team)
 {
     constexpr int W = Threads / 32;
     constexpr int kLongItems = Threads == kLongThreads ? 4 : 2;  // keys per thread and step (2: no spills in the forest's sort)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int prefix = a.beginBit + first * kRadixBits;
-    for (u32 r = blockIdx.x; r < runs; r += gridDim.x)
+    for (u32 r = team.rank; r < runs; r += team.size)
     {
         const u32 h = a.longList[2 * r], limit = a.longList[2 * r + 1];
         if (warp == 0)
@@ -464,7 +465,7 @@ static __global__ void __launch_bounds__(kLongThreads) longRunKernel(RepairArgs 
 {
     __shared__ LongShared<kLongThreads> sm;
     if (*a.error) return;
-    sortLongRuns(a, sm, int(a.ctl->first), a.ctl->longRuns);
+    sortLongRuns(a, sm, int(a.ctl->first), a.ctl->longRuns, wholeGrid());
 }
 
 // The repair of a planned sort (after its passes).

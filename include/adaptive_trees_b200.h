@@ -236,6 +236,17 @@ AO_API ao_status ao_sort_pairs_check(const void *scratch, size_t n, void *stream
  * code when the wait gave up and the kernel returned, the designed outcome;
  * the device stays usable.  Uses its own small allocations and stream. */
 AO_API ao_status ao_selftest_bounded_wait(int which, unsigned spin_limit, int *error_word);
+/* The same of the waits between the CTAs of a build, a small update or a
+ * small sort in one launch -- which 0: the grid barrier, 1: the roll of the
+ * CTAs that take part, 2: the octree's placement, 3: the binary tree's -- run
+ * by one CTA that waits for what never comes. */
+AO_API ao_status ao_selftest_team_wait(int which, unsigned spin_limit, int *error_word);
+/* Queues a kernel that holds `sms` SMs of the device for `milliseconds` (at
+ * most 2000) on `stream`: what another program's long kernel leaves of the
+ * GPU, for tests.  Builds, updates and sorts of single trees on other streams
+ * run on the SMs that are free (no call waits for the whole GPU but a batch's
+ * build). */
+AO_API ao_status ao_selftest_hold_sms(int sms, int milliseconds, void *stream);
 
 /* The sort tuner (no counterpart in the reference; it picks what the
  * reference leaves to CUB's fixed policy).  The radix sort is compiled in a
