@@ -101,6 +101,7 @@ PROTOTYPES = {
     "ao_batch_destroy": [vp],
     "ao_batch_build": [vp],
     "ao_batch_set_build_mode": [vp, ci],
+    "ao_selftest_batch_error": [vp, ci],
     "ao_batch_build_path": [vp, ctypes.POINTER(ci)],
     "ao_batch_update": [vp, vp],
     "ao_batch_update_until_converged": [vp, vp, ci, ctypes.POINTER(ci)],

@@ -661,6 +661,14 @@ ao_status ao_batch_set_build_mode(ao_batch *batch, int mode)
     });
 }
 
+ao_status ao_selftest_batch_error(ao_batch *batch, int value)
+{
+    return guarded([&] {
+        if (!batch) throw std::invalid_argument("ao_selftest_batch_error: null batch");
+        batch->engine->setError(value);
+    });
+}
+
 ao_status ao_batch_build_path(ao_batch *batch, int *by_levels)
 {
     return guarded([&] {

@@ -249,6 +249,11 @@ ForestEngine::~ForestEngine()
 
 int ForestEngine::numSystems() const { return m_->S; }
 size_t ForestEngine::numParticles() const { return m_->total; }
+void ForestEngine::setError(int value)
+{
+    AOT_CHECK(cudaMemcpyAsync(&m_->st.as<forest::State>()->error, &value, sizeof(int), cudaMemcpyHostToDevice, m_->cfg.stream));
+    waitStream(m_->cfg.stream);
+}
 
 void ForestEngine::setCoordinates(int s, const void *x, const void *y, const void *z)
 {

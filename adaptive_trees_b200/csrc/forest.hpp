@@ -56,6 +56,8 @@ public:
     };
     SystemInfo info(int s) const;
     int numSystems() const;
+    // sets the device's error word, as a wait that gave up does (self-tests)
+    void setError(int value);
     size_t numParticles() const;
 
 private:

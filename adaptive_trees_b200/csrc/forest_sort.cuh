@@ -98,7 +98,7 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     static_assert(sort::kThreads == sort::kPlanThreads && sort::kThreads == sort::kRepairThreads, "one CTA shape");
     extern __shared__ __align__(16) unsigned char smemRaw[];
     SortShared<Items> &sm = *reinterpret_cast<SortShared<Items> *>(smemRaw);
-    const u32 epoch = vload(p.r.ctl->epoch) + sort::kEpochStep;  // stored at the end
+    const u32 epoch = vload(p.r.ctl->epoch) + sort::kEpochStep;
     if (blockIdx.x * blockDim.x < p.plan.samples)
     {
         const auto keyAt = [&](size_t g, u32 &group) {
@@ -110,6 +110,11 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     for (int sys = blockIdx.x; sys < p.f.numSystems; sys += gridDim.x)
         systemBins(p.f.systems, p.f.numSystems, sys, p.hist, p.bins, kCountedFrom, sort::kMaxPasses);
     if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
+    // every CTA has read it; stored before the first word that carries a tag of
+    // it, so that the next sort has other tags however this one ends (with the
+    // tags of a sort that gave up, its words would be taken for published
+    // counts, and the places made of them can lie outside the buffers)
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->epoch = epoch;
     u32 repeats[sort::kPlanSets];
 #pragma unroll
     for (int k = 0; k < sort::kPlanSets; ++k) repeats[k] = vload(p.plan.counters->repeats[k]);
@@ -152,7 +157,6 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
             if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->epoch = epoch;
     activeAndSample(p.f, p.sample, p.ns, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
                     size_t(gridDim.x) * blockDim.x);
 }

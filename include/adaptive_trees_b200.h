@@ -329,6 +329,10 @@ AO_API ao_status ao_batch_build(ao_batch *batch);
  * system's rounds would not converge within max_depth; mode 1: always the
  * rounds.  Both give the same trees, counts and capacities. */
 AO_API ao_status ao_batch_set_build_mode(ao_batch *batch, int mode);
+/* Sets the batch's device error word, as a wait that gave up does (0 clears
+ * it): calls report it, and the sort of a build ends before its repair.  For
+ * tests. */
+AO_API ao_status ao_selftest_batch_error(ao_batch *batch, int value);
 /* *by_levels = 1 when the last build() used the level builder. */
 AO_API ao_status ao_batch_build_path(ao_batch *batch, int *by_levels);
 /* update() of every system (octree.cu:459-496); capturable when frozen is
