@@ -84,14 +84,17 @@ __host__ __device__ inline unsigned octDigit(u64 key, unsigned level)
 }
 
 // First index in a[0, n) whose key is >= v (lowerBound, helpers.cuh:65-85).
-// Branch-free halving; `a` is read through the read-only path.
-__device__ __forceinline__ size_t lowerBoundDev(const u64 *__restrict__ a, size_t n, u64 v)
+// Branch-free halving.  `a` is read through the read-only path, which is
+// defined only for memory that the whole launch leaves alone; Written: keys
+// that this launch has written (before a grid barrier), read from L2.
+template <bool Written = false>
+__device__ __forceinline__ size_t lowerBoundDev(const u64 *a, size_t n, u64 v)
 {
     size_t lo = 0;
     while (n > 0)
     {
         const size_t half = n >> 1;
-        const u64 m = __ldg(a + lo + half);
+        const u64 m = Written ? __ldcg(a + lo + half) : __ldg(a + lo + half);
         const bool less = m < v;
         lo = less ? lo + half + 1 : lo;
         n = less ? n - half - 1 : half;

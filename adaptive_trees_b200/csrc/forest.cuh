@@ -329,21 +329,23 @@ static __global__ void __launch_bounds__(sort::kRepairThreads)
 }
 
 // With a sample array: also every 32nd key of the concatenated sorted keys
-// (the key index of a build by levels).
+// (the key index of a build by levels).  Written: the launch that calls it has
+// sorted the keys itself.
+template <bool Written>
 __device__ __forceinline__ void activeAndSample(const Bufs &f, u64 *sample, size_t ns, size_t r, size_t size)
 {
     for (size_t s = r; s < size_t(f.numSystems); s += size)
     {
         const System sy = f.systems[s];
-        f.sys[s].active = sy.n ? u32(lowerBoundDev(f.P + sy.base, sy.n, kMaxKey)) : 0u;
+        f.sys[s].active = sy.n ? u32(lowerBoundDev<Written>(f.P + sy.base, sy.n, kMaxKey)) : 0u;
     }
     if (sample)
-        for (size_t j = r; j < ns; j += size) sample[j] = f.P[j << kSampleShift];
+        for (size_t j = r; j < ns; j += size) sample[j] = Written ? __ldcg(f.P + (j << kSampleShift)) : f.P[j << kSampleShift];
 }
 
 static __global__ void activeKernel(Bufs f, u64 *sample, size_t ns)
 {
-    activeAndSample(f, sample, ns, size_t(blockIdx.x) * blockDim.x + threadIdx.x, size_t(gridDim.x) * blockDim.x);
+    activeAndSample<false>(f, sample, ns, size_t(blockIdx.x) * blockDim.x + threadIdx.x, size_t(gridDim.x) * blockDim.x);
 }
 
 // --------------------------------------------------------------------------

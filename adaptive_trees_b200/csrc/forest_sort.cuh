@@ -157,8 +157,8 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
             if (!gridBarrier(p.bar, wholeGrid())) return fail(p);
         }
     }
-    activeAndSample(p.f, p.sample, p.ns, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
-                    size_t(gridDim.x) * blockDim.x);
+    activeAndSample<true>(p.f, p.sample, p.ns, size_t(blockIdx.x) * blockDim.x + threadIdx.x,
+                          size_t(gridDim.x) * blockDim.x);
 }
 
 }  // namespace forest
