@@ -102,6 +102,10 @@ PROTOTYPES = {
     "ao_batch_build": [vp],
     "ao_batch_set_build_mode": [vp, ci],
     "ao_selftest_batch_error": [vp, ci],
+    "ao_selftest_batch_sort_plan": [vp, ci, ctypes.POINTER(ci), ctypes.POINTER(ci)],
+    "ao_selftest_tree_sort_plan": [vp, ci, ctypes.POINTER(ci), ctypes.POINTER(ci)],
+    "ao_selftest_sort_pairs": [vp, ctypes.POINTER(sz), vp, vp, vp, vp, sz, ci, ci, ci, ci, vp],
+    "ao_selftest_sort_pairs_plan": [vp, sz, ctypes.POINTER(ci), ctypes.POINTER(ci), vp],
     "ao_batch_build_path": [vp, ctypes.POINTER(ci)],
     "ao_batch_update": [vp, vp],
     "ao_batch_update_until_converged": [vp, vp, ci, ctypes.POINTER(ci)],

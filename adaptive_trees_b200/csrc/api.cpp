@@ -557,6 +557,38 @@ ao_status ao_selftest_bounded_wait(int which, unsigned spin_limit, int *error_wo
     });
 }
 
+ao_status ao_selftest_tree_sort_plan(ao_tree *tree, int force_first, int *first, int *long_runs)
+{
+    return guarded([&] {
+        if (!tree) throw std::invalid_argument("ao_selftest_tree_sort_plan: null tree");
+        tree->engine->forceSortPlan(force_first);
+        const aot::TreeEngine::SortPlan p = tree->engine->sortPlan();
+        if (first) *first = p.first;
+        if (long_runs) *long_runs = p.longRuns;
+    });
+}
+
+ao_status ao_selftest_sort_pairs(void *scratch, size_t *scratch_bytes, const unsigned long long *keys_in,
+                                 unsigned long long *keys_out, const unsigned *values_in, unsigned *values_out,
+                                 size_t n, int begin_bit, int end_bit, int config, int force_first, void *stream)
+{
+    return guarded([&] {
+        if (force_first < 0 || force_first > 7)
+            throw std::invalid_argument("ao_selftest_sort_pairs: force_first must be 0 to 7");
+        aot::TreeEngine::sortPairsWith(config, scratch, scratch_bytes, keys_in, keys_out, values_in, values_out, n,
+                                       begin_bit, end_bit, static_cast<cudaStream_t>(stream), force_first);
+    });
+}
+
+ao_status ao_selftest_sort_pairs_plan(const void *scratch, size_t n, int *first, int *long_runs, void *stream)
+{
+    return guarded([&] {
+        const aot::TreeEngine::SortPlan p = aot::TreeEngine::sortPairsPlan(scratch, n, static_cast<cudaStream_t>(stream));
+        if (first) *first = p.first;
+        if (long_runs) *long_runs = p.longRuns;
+    });
+}
+
 ao_status ao_selftest_team_wait(int which, unsigned spin_limit, int *error_word)
 {
     return guarded([&] {
@@ -658,6 +690,17 @@ ao_status ao_batch_set_build_mode(ao_batch *batch, int mode)
     return guarded([&] {
         if (!batch) throw std::invalid_argument("ao_batch_set_build_mode: null batch");
         batch->engine->setBuildMode(mode);
+    });
+}
+
+ao_status ao_selftest_batch_sort_plan(ao_batch *batch, int force_first, int *first, int *long_runs)
+{
+    return guarded([&] {
+        if (!batch) throw std::invalid_argument("ao_selftest_batch_sort_plan: null batch");
+        batch->engine->forceSortPlan(force_first);
+        const aot::TreeEngine::SortPlan p = batch->engine->sortPlan();
+        if (first) *first = p.first;
+        if (long_runs) *long_runs = p.longRuns;
     });
 }
 

@@ -768,7 +768,7 @@ void TreeEngine::sortPairs(void *scratch, size_t *scratchBytes, const unsigned l
 
 void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, const unsigned long long *keysIn,
                                unsigned long long *keysOut, const unsigned *valsIn, unsigned *valsOut, size_t n,
-                               int beginBit, int endBit, cudaStream_t s)
+                               int beginBit, int endBit, cudaStream_t s, int forcePlan)
 {
     if (!scratchBytes) throw std::invalid_argument("ao_sort_pairs: scratch_bytes must not be null");
     if (beginBit < 0 || endBit > 64 || beginBit > endBit)
@@ -817,7 +817,7 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     {
         const sort::PlanArgs plan{reinterpret_cast<u64 *>(base + lay.table),
                                   reinterpret_cast<sort::PlanCounters *>(planCounters), sort::planSamples(n),
-                                  sort::planSlotBits(n)};
+                                  sort::planSlotBits(n), std::min(forcePlan, passes - 1)};
         sort::planPairsKernel<<<ceilDiv(plan.samples, sort::kPlanThreads), sort::kPlanThreads, 0, s>>>(
             in, n, beginBit, passes, keyMask, plan, ctl), noteLaunch();
     }
@@ -862,6 +862,27 @@ bool TreeEngine::sortPairsFailed(const void *scratch, size_t n, cudaStream_t s)
                               sizeof(int), cudaMemcpyDeviceToHost, s));
     AOT_CHECK(cudaStreamSynchronize(s));
     return error != 0;
+}
+
+namespace
+{
+TreeEngine::SortPlan readSortPlan(const sort::SortControl *ctl, cudaStream_t s)
+{
+    u32 words[3];  // epoch, first, longRuns
+    static_assert(offsetof(sort::SortControl, longRuns) == 2 * sizeof(u32), "the leading words");
+    AOT_CHECK(cudaMemcpyAsync(words, ctl, sizeof(words), cudaMemcpyDeviceToHost, s));
+    waitStream(s);
+    return {int(words[1]), int(words[2])};
+}
+}  // namespace
+
+TreeEngine::SortPlan TreeEngine::sortPairsPlan(const void *scratch, size_t n, cudaStream_t s)
+{
+    if (!scratch) throw std::invalid_argument("ao_selftest_sort_pairs: null scratch");
+    return readSortPlan(reinterpret_cast<const sort::SortControl *>(
+                            static_cast<const char *>(scratch) + PairSortLayout::countersOffset(n) +
+                            PairSortLayout::kCounterHead * sizeof(u32)),
+                        s);
 }
 
 // Loads every kernel a pair sort with the default configuration can launch
@@ -1114,6 +1135,18 @@ TreeEngine::TreeEngine(const void *x, const void *y, const void *z, size_t n, co
 }
 
 size_t TreeEngine::deviceBytes() const { return m_->bytes(); }
+
+void TreeEngine::forceSortPlan(int first)
+{
+    if (first < -1 || first >= sort::kMaxPasses) throw std::invalid_argument("sort plan: first pass must be -1 to 7");
+    m_->sortArena.plan.force = first;
+}
+
+TreeEngine::SortPlan TreeEngine::sortPlan() const
+{
+    if (n_ == 0) return {0, 0};
+    return readSortPlan(m_->sortArena.ctl(), cfg_.stream);
+}
 
 namespace
 {

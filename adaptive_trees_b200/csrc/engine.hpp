@@ -185,13 +185,23 @@ public:
     // the same of the waits of launches by team (0: the grid barrier, 1: the
     // roll, 2: the octree's placement, 3: the binary tree's)
     static int teamWaitProbe(int which, unsigned spinLimit);
+    // Self-tests of the planned sort: a plan that runs the passes from `first`
+    // on whatever the keys are (-1: the sample decides again), and the last
+    // sort's first pass and number of long runs (waits for the stream).
+    struct SortPlan
+    {
+        int first, longRuns;
+    };
+    void forceSortPlan(int first);
+    SortPlan sortPlan() const;
+    static SortPlan sortPairsPlan(const void *scratch, size_t n, cudaStream_t s);
     // keeps `sms` SMs busy for some time (at most 2000 ms), as another
     // program's long kernel would
     static void holdSms(int sms, int milliseconds, cudaStream_t s);
     // the same with sort configuration `config` (its own scratch size)
     static void sortPairsWith(int config, void *scratch, size_t *scratchBytes, const unsigned long long *keysIn,
                               unsigned long long *keysOut, const unsigned *valsIn, unsigned *valsOut, size_t n,
-                              int beginBit, int endBit, cudaStream_t s);
+                              int beginBit, int endBit, cudaStream_t s, int forcePlan = -1);
     // dst[i] = src[perm[i]] for the numParticles() elements of elemBytes
     // each: per-particle data in key order (device pointers, the tree's stream)
     void gather(const void *src, void *dst, size_t elemBytes) const;

@@ -249,6 +249,18 @@ ForestEngine::~ForestEngine()
 
 int ForestEngine::numSystems() const { return m_->S; }
 size_t ForestEngine::numParticles() const { return m_->total; }
+void ForestEngine::forceSortPlan(int first)
+{
+    if (first < -1 || first >= sort::kMaxPasses) throw std::invalid_argument("sort plan: first pass must be -1 to 7");
+    m_->plan.force = first;
+}
+TreeEngine::SortPlan ForestEngine::sortPlan() const
+{
+    sort::SortControl c;
+    AOT_CHECK(cudaMemcpyAsync(&c, m_->ctl(), sizeof(c), cudaMemcpyDeviceToHost, m_->cfg.stream));
+    waitStream(m_->cfg.stream);
+    return {int(c.first), int(c.longRuns)};
+}
 void ForestEngine::setError(int value)
 {
     AOT_CHECK(cudaMemcpyAsync(&m_->st.as<forest::State>()->error, &value, sizeof(int), cudaMemcpyHostToDevice, m_->cfg.stream));

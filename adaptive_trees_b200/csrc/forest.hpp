@@ -58,6 +58,9 @@ public:
     int numSystems() const;
     // sets the device's error word, as a wait that gave up does (self-tests)
     void setError(int value);
+    // as TreeEngine's
+    void forceSortPlan(int first);
+    TreeEngine::SortPlan sortPlan() const;
     size_t numParticles() const;
 
 private:

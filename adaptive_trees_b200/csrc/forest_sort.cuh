@@ -118,7 +118,8 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     u32 repeats[sort::kPlanSets];
 #pragma unroll
     for (int k = 0; k < sort::kPlanSets; ++k) repeats[k] = vload(p.plan.counters->repeats[k]);
-    const int first = int(sort::planFirst(repeats, p.plan.samples, p.r.n));
+    const int first = p.plan.force >= 0 ? p.plan.force : int(sort::planFirst(repeats, p.plan.samples, p.r.n));
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->first = u32(first);  // (for who asks)
     if (first < kCountedFrom)
     {
         countLowDigits(p, first, sm.hist);

@@ -79,6 +79,7 @@ struct PlanArgs
     u64 *table;  // [kPlanSets][1 << slotBits]: sort number << 32 | the last prefix hashed there
     PlanCounters *counters;
     u32 samples, slotBits;
+    int force = -1;  // first pass to run whatever the sample says (self-tests), or -1
 };
 
 // The first pass to run (0: all `passes`) for n keys, from the repeats in each
@@ -185,7 +186,7 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     if (threadIdx.x == 0)
     {
         a.counters->done = 0;
-        ctl->first = planFirst(sTotal, a.samples, n, passes);
+        ctl->first = a.force >= 0 ? u32(a.force) : planFirst(sTotal, a.samples, n, passes);
         ctl->epoch = epoch;
         ctl->longRuns = 0;
         ctl->keygenDone = 0;

@@ -241,6 +241,21 @@ AO_API ao_status ao_selftest_bounded_wait(int which, unsigned spin_limit, int *e
  * CTAs that take part, 2: the octree's placement, 3: the binary tree's -- run
  * by one CTA that waits for what never comes. */
 AO_API ao_status ao_selftest_team_wait(int which, unsigned spin_limit, int *error_word);
+/* Self-tests of the planned sort (a sort passes over the keys' high digits
+ * from a first pass on, 0 for all of them, and a repair orders the runs that
+ * share them).  The first two make the sorts of the tree or batch that follow
+ * start at pass force_first (0 to 7; -1: the plan decides again) and report
+ * the last sort's first pass and the number of runs too long for the tiles
+ * of its repair (outputs may be NULL; the call waits for the stream).  The
+ * others are ao_sort_pairs with configuration `config` and a given first pass
+ * (at most the sort's last one), and the same report.  Sorts that make no
+ * plan (7-bit digits, pair sorts of one or two passes) run every pass. */
+AO_API ao_status ao_selftest_tree_sort_plan(ao_tree *tree, int force_first, int *first, int *long_runs);
+AO_API ao_status ao_selftest_sort_pairs(void *scratch, size_t *scratch_bytes, const unsigned long long *keys_in,
+                                        unsigned long long *keys_out, const unsigned *values_in,
+                                        unsigned *values_out, size_t n, int begin_bit, int end_bit, int config,
+                                        int force_first, void *stream);
+AO_API ao_status ao_selftest_sort_pairs_plan(const void *scratch, size_t n, int *first, int *long_runs, void *stream);
 /* Queues a kernel that holds `sms` SMs of the device for `milliseconds` (at
  * most 2000) on `stream`: what another program's long kernel leaves of the
  * GPU, for tests.  Builds, updates and sorts of single trees on other streams
@@ -329,6 +344,8 @@ AO_API ao_status ao_batch_build(ao_batch *batch);
  * system's rounds would not converge within max_depth; mode 1: always the
  * rounds.  Both give the same trees, counts and capacities. */
 AO_API ao_status ao_batch_set_build_mode(ao_batch *batch, int mode);
+/* As ao_selftest_tree_sort_plan. */
+AO_API ao_status ao_selftest_batch_sort_plan(ao_batch *batch, int force_first, int *first, int *long_runs);
 /* Sets the batch's device error word, as a wait that gave up does (0 clears
  * it): calls report it, and the sort of a build ends before its repair.  For
  * tests. */
