@@ -993,7 +993,8 @@ struct TreeEngine::Impl
                                &vLvVals[1],  &vLayKeys[0], &vLayKeys[1],    &vLayVals[0],  &vLayVals[1],
                                &vIntStartSfc, &vIntLevelSfc, &vIntM,        &vIntStartLay, &vIntLevelLay,
                                &viewSort.mem, &nodeRows, &lvRows, &lvVal, &lvChild,
-                               &lvSub, &lvOffset, &lvCtl, &lvNbr, &lvParent, &lvRec};
+                               &lvSub, &lvOffset, &lvCtl, &lvNbr, &lvParent, &lvRec,
+                               &blRows, &blChild, &blSub, &blParent, &blOffset, &blCtl, &mergeSplits};
         size_t s = 0;
         for (const DevMem *d : all) s += d->bytes;
         return s;
