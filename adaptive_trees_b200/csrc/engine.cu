@@ -1256,8 +1256,10 @@ void TreeEngine::ensurePhysical(size_t capacity)
             m_->nodeSlots = u32(slots);
             m_->nodeStale = true;
         }
-        // the refresh of update() takes a large tree's internal nodes as units
-        if (refreshByUnits() && c > 4096) ensureUnits(std::max(c / 7 + 1, n_ / 4 + 4096));
+        // the refresh of update() takes a large tree's internal nodes as units: a
+        // seventh of its leaves less one.  (Not a unit more: a build that places
+        // again, in larger leaf arrays, keeps its units, however full the arena.)
+        if (refreshByUnits() && c > 4096) ensureUnits(std::max((c - 1) / 7, n_ / 4 + 4096));
     }
     physCap_ = c;
 }
