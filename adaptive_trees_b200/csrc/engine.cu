@@ -507,6 +507,15 @@ struct SortArena
 // and in one: 10k keys 72 and 57 us, 100k 79 and 61, 1M 113 and 99, 4M 202 and
 // 200; from a graph 39 and 46, 48 and 51, 81 and 89, 164 and 190.
 constexpr size_t kFusedSort = size_t(1) << 21;
+// Sorts that make no plan run every pass, and count their digits first, which
+// the few CTAs of a small sort do slowly.  Random keys queued directly, launch by
+// launch and in one: one digit, 10k keys 21 and 26 us, 50k 24 and 27, 2M 48 and
+// 51; four digits 45 and 49, 49 and 51, 200k 62 and 56, 700k 80 and 75, 2M 113
+// and 120; eight digits 78 and 79, 84 and 83, 101 and 91, 128 and 128, 197 and
+// 210.
+constexpr int kFusedPasses = 4;
+constexpr unsigned kFusedCounting = 32;
+constexpr size_t kFusedUnplannedFrom = size_t(1) << 17, kFusedUnplannedTo = size_t(1) << 20;
 
 // The passes and the repair of one launch (sort_fused.cuh), after the plan (or
 // beginSortKernel); hist: with the digit counts.  False (nothing done) where
@@ -515,6 +524,7 @@ bool launchFusedSort(int cfg, cudaStream_t s, const sort::PassArgs &p, const sor
                      bool repair)
 {
     if (p.n > kFusedSort) return false;
+    if (!repair && (p.passes < kFusedPasses || p.n < kFusedUnplannedFrom || p.n > kFusedUnplannedTo)) return false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     AOT_CHECK(cudaStreamIsCapturing(s, &capture));
     if (capture != cudaStreamCaptureStatusNone) return false;
@@ -528,8 +538,10 @@ bool launchFusedSort(int cfg, cudaStream_t s, const sort::PassArgs &p, const sor
     const u32 tiles = u32(configTiles(cfg, p.n));
     sort::FusedArgs a{p, r, tiles, hist, bins, repair, r.keyMask == ~u64(0)};
     void *args[] = {&a};
-    AOT_CHECK(cudaLaunchKernel(fn, dim3(std::min<unsigned>(tiles, unsigned(perSm) * unsigned(smCount()))),
-                               dim3(sort::kThreads), args, smem, s));
+    // (a sort of few tiles counts with more CTAs than pass)
+    const unsigned most = hist ? std::max(tiles, std::min(ceilDiv(p.n, 1024), kFusedCounting)) : tiles;
+    AOT_CHECK(cudaLaunchKernel(fn, dim3(std::min(most, unsigned(perSm) * unsigned(smCount()))), dim3(sort::kThreads), args,
+                               smem, s));
     noteLaunch();
     return true;
 }
@@ -811,8 +823,8 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     const u64 *in = reinterpret_cast<const u64 *>(keysIn);
     u64 *out = reinterpret_cast<u64 *>(keysOut);
     const u64 keyMask = (endBit - beginBit == 64 ? ~u64(0) : ((u64(1) << (endBit - beginBit)) - 1)) << beginBit;
-    // a plan for 8-bit digits, where it can leave passes out
-    const bool planned = bitsPer == sort::kRadixBits && passes > sort::kPlanMinPasses;
+    // a plan for 8-bit digits, where it can leave passes enough out
+    const bool planned = bitsPer == sort::kRadixBits && (passes > sort::kUnplannedPasses || forcePlan >= 0);
     if (planned)
     {
         const sort::PlanArgs plan{reinterpret_cast<u64 *>(base + lay.table),
@@ -821,10 +833,7 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
         sort::planPairsKernel<<<ceilDiv(plan.samples, sort::kPlanThreads), sort::kPlanThreads, 0, s>>>(
             in, n, beginBit, passes, keyMask, plan, ctl), noteLaunch();
     }
-    else
-    {
-        sort::beginSortKernel<<<1, sort::kThreads, 0, s>>>(ctl, nullptr), noteLaunch();
-    }
+    // (without a plan every pass runs, and the cleared control block says so)
     AOT_LAUNCH_CHECK();
     const sort::PassArgs p{in, valsIn, {out, altK}, {valsOut, altV}, n, bins, ctl, status, error, beginBit, endBit, passes,
                            true};
@@ -2094,7 +2103,7 @@ bool TreeEngine::binaryLevelBuild()
 // 127 (125 and 114), 262k 274 and 253 (228 and 228), 2.1M 495 and 516 (440 and
 // 494); k-d trees of 1.3k leaves 152 and 85 (118 and 80), 354k 516 and 463 (451
 // and 439).
-constexpr size_t kFusedPasses = size_t(1) << 19;
+constexpr size_t kFusedLeaves = size_t(1) << 19;
 
 // The refresh, the passes and the counts of an update() in one launch
 // (rb::updateKernel).  False (nothing done) where they run launch by launch:
@@ -2102,7 +2111,7 @@ constexpr size_t kFusedPasses = size_t(1) << 19;
 bool TreeEngine::passesFused()
 {
     if (cfg_.nf || profiling_ || n_ == 0) return false;  // (the sort clears the barrier)
-    if (leafCapacity_ > kFusedPasses) return false;
+    if (leafCapacity_ > kFusedLeaves) return false;
     const void *fn = cfg_.kind == 0 ? reinterpret_cast<const void *>(&rb::updateKernel<false>)
                                     : reinterpret_cast<const void *>(&rb::updateKernel<true>);
     int perSm = 0;

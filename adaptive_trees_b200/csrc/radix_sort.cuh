@@ -64,8 +64,9 @@ constexpr u64 kFlagMask = u64(3) << 62;
 // sort without being cleared between them: a word of another pass reads as
 // not published.  (Cleared arrays of 8 passes were 107 MB of writes and 28 us
 // of a 16Mi sort; one pass' words are 13 MB and stay in L2.)
+// (The first number is 1: a cleared word carries no pass' tag.)
 constexpr u64 kTagMask = ((u64(1) << 30) - 1) << 32;
-__host__ __device__ constexpr u64 passTag(u32 number) { return (u64(number) << 32) & kTagMask; }
+__host__ __device__ constexpr u64 passTag(u32 number) { return (u64(number + 1) << 32) & kTagMask; }
 constexpr unsigned kLookbackSpins = 1u << 22;
 constexpr int kLookbackWindow = 8;
 
@@ -98,6 +99,7 @@ struct SortControl
     GridBarrier afterBar;  // of what follows the sort in one launch (update())
 };
 constexpr u32 kEpochStep = 16;  // tags per sort (>= kPassSlots)
+static_assert(kEpochStep >= kPassSlots && (u64(1) << 30) % kEpochStep == 0, "a tag per pass slot");
 
 // Zeroes the barriers of a sort and of what follows it (one CTA, before them).
 __device__ __forceinline__ void clearBarriers(SortControl *ctl)

@@ -5,13 +5,13 @@
 // pass, 1 us and a launch in each of the 5 passes the plan leaves out, and two
 // launches in the repair.  Here the CTAs go through the same tiles phase by
 // phase, with a grid barrier between:
-//   counts     (optional) digit counts of the passes that run, tiles taken
-//              from a counter, and their bins;
+//   counts     (optional) digit counts of the passes that run, and their bins;
 //   passes     the onesweep passes; in each, CTAs take tiles from the pass's
 //              counter until it runs out.  A tile's look-back waits only for
 //              tiles taken before it, by CTAs that are resident and do not
-//              wait for later tiles, so every wait ends.  The roll of the team
-//              closes behind the first phase: whoever takes a tile is on it;
+//              wait for later tiles, so every wait ends.  (Without counts the
+//              roll of the team closes behind the first pass: whoever takes a
+//              tile is on it);
 //   repair     the runs of equal high digits (sort_repair.cuh), tile by tile,
 //              then the long ones.
 #pragma once
@@ -55,6 +55,9 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
     FusedShared<Items> &sm = *reinterpret_cast<FusedShared<Items> *>(smemRaw);
     const PassArgs &p = a.p;
     GridBarrier *bar = &p.ctl->sortBar;
+    const int first = int(p.ctl->first);
+    if (a.hist)
+        for (int i = threadIdx.x; i < kPassSlots * kRadix; i += kThreads) sm.hist[i] = 0;
     Team team{enterRoll(bar), 0};
     if (team.rank == kLeftOut) return;
     const auto fail = [&] {
@@ -64,31 +67,21 @@ static __global__ void __launch_bounds__(kThreads, 3) fusedSortKernel(FusedArgs 
         if (!team.size) team.size = closeRoll(bar);
         return team.size && gridBarrier(bar, team);
     };
-    const int first = int(p.ctl->first);
     if (a.hist)
     {
-        constexpr int kCountSlot = kPassSlots - 1;  // no pass' tile counter
-        static_assert(kMaxPasses <= kCountSlot, "a counter to spare");
-        __shared__ u32 sTile;
-        for (int i = threadIdx.x; i < kPassSlots * kRadix; i += kThreads) sm.hist[i] = 0;
-        for (;;)
+        team.size = closeRoll(bar);
+        if (!team.size) return fail();
+        for (size_t g = size_t(team.rank) * kThreads + threadIdx.x; g < p.n; g += size_t(team.size) * kThreads)
         {
-            __syncthreads();
-            if (threadIdx.x == 0) sTile = atomicAdd(p.ctl->tileCounters + kCountSlot, 1u);
-            __syncthreads();
-            if (sTile >= a.tiles) break;
-            const size_t begin = size_t(sTile) * kTile, end = min(p.n, begin + kTile);
-            for (size_t g = begin + threadIdx.x; g < end; g += kThreads)
+            const u64 k = p.keysIn[g];
+            for (int q = first; q < p.passes; ++q)
             {
-                const u64 k = p.keysIn[g];
-                for (int q = first; q < p.passes; ++q)
-                {
-                    const int shift = p.beginBit + q * kRadixBits;
-                    const int bits = min(kRadixBits, p.endBit - shift);
-                    atomicAdd(&sm.hist[q * kRadix + int((k >> shift) & ((1u << bits) - 1))], 1u);
-                }
+                const int shift = p.beginBit + q * kRadixBits;
+                const int bits = min(kRadixBits, p.endBit - shift);
+                atomicAdd(&sm.hist[q * kRadix + int((k >> shift) & ((1u << bits) - 1))], 1u);
             }
         }
+        __syncthreads();
         for (int i = first * kRadix + threadIdx.x; i < p.passes * kRadix; i += kThreads)
             if (sm.hist[i]) atomicAdd(a.hist + i, sm.hist[i]);
         if (!barrier()) return fail();

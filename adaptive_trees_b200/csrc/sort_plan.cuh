@@ -27,6 +27,13 @@ constexpr int kPlanThreads = 256;      // a sampled key per thread
 constexpr u32 kPlanMaxSamples = 8192;
 constexpr int kPlanMinPasses = 2;
 constexpr int kPlanMaxPasses = 6;
+// Pair sorts of at most this many digits make no plan: it can leave out two
+// passes of them at best, and costs a launch and a repair.  Random keys, four
+// digits, with a plan and without: replayed 10k keys 33 and 31 us, 700k 68 and
+// 66, 5M 187 and 186, queued 2M 132 and 113; three digits 33 and 25, 62 and 53,
+// 154 and 145, 103 and 93.  Five digits: 35 and 35, 72 and 76, 189 and 225, 132
+// and 135.
+constexpr int kUnplannedPasses = 4;
 constexpr int kPlanSets = kPlanMaxPasses - kPlanMinPasses + 2;  // a set of prefixes per choice, one of whole keys
 // Cost in passes: the repair's fixed part and its part per key of the mean
 // run.  Measured at 16Mi keys (a pass 120 us): repairs of mean runs of 3.8,
