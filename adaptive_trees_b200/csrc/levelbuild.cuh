@@ -1171,7 +1171,9 @@ static __global__ void __launch_bounds__(kThreads) treeUnitsKernel(Arena a, rb::
         const u32 g = start + (act ? e >> 3 : 0);
         const u32 *row = a.rows + size_t(g) * kRow;
         const u64 key = rowKey(row);
-        const u32 i0 = row[3], i1 = row[4], bEnd = row[10], st = unitStateOf(row[11]);
+        // (lanes without a child look at no unit's leaves: its own warp replaces
+        // the two words by begin indices)
+        const u32 i0 = act ? row[3] : 0u, i1 = act ? row[4] : 0u, bEnd = row[10], st = unitStateOf(row[11]);
         // first leaf of child d
         u32 j = i0;
         if (d > 0)
