@@ -63,6 +63,7 @@ struct SortShared
         sort::SharedPass<sort::kRadixBits, Items> pass;
         sort::RepairShared<sort::kThreads * Items> repair;
         sort::LongShared<sort::kThreads> longRun;
+        sort::PlanShared plan;
         u32 hist[sort::kMaxPasses * sort::kRadix];
     };
 };
@@ -105,7 +106,7 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
             group = systemOf(p.tiles.segBase, p.f.numSystems, u32(g));
             return p.r.k[0][g];
         };
-        sort::planSample(keyAt, p.r.n, p.plan, epoch);
+        sort::planSample(keyAt, p.r.n, p.plan, epoch, sm.plan);
     }
     for (int sys = blockIdx.x; sys < p.f.numSystems; sys += gridDim.x)
         systemBins(p.f.systems, p.f.numSystems, sys, p.hist, p.bins, kCountedFrom, sort::kMaxPasses);
@@ -115,10 +116,14 @@ static __global__ void __launch_bounds__(sort::kThreads, 3) sortKernel(SortArgs 
     // tags of a sort that gave up, its words would be taken for published
     // counts, and the places made of them can lie outside the buffers)
     if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->epoch = epoch;
-    u32 repeats[sort::kPlanSets];
+    u32 repeats[sort::kPlanSets], more[sort::kPlanSets];
 #pragma unroll
-    for (int k = 0; k < sort::kPlanSets; ++k) repeats[k] = vload(p.plan.counters->repeats[k]);
-    const int first = p.plan.force >= 0 ? p.plan.force : int(sort::planFirst(repeats, p.plan.samples, p.r.n));
+    for (int k = 0; k < sort::kPlanSets; ++k)
+    {
+        repeats[k] = vload(p.plan.counters->repeats[k]);
+        more[k] = vload(p.plan.counters->more[k]);
+    }
+    const int first = p.plan.force >= 0 ? p.plan.force : int(sort::planFirst(repeats, more, p.plan.samples, p.r.n));
     if (blockIdx.x == 0 && threadIdx.x == 0) p.r.ctl->first = u32(first);  // (for who asks)
     if (first < kCountedFrom)
     {

@@ -15,6 +15,13 @@
 // of equal keys need no repair and are taken off (also positions drawn
 // twice); keys that repeat so often that their runs would be long send the
 // sort to all passes.
+//
+// The sample counts the keys that find an earlier one of their prefix.  That is
+// the pairs where a prefix is drawn twice, but k - 1 of k (k - 1) / 2 where it is
+// drawn k times, and a run that holds a share p of the keys is drawn p M times:
+// R_D has n p^2 of it.  So each CTA also counts the pairs beyond among its own
+// keys.  (Without them a tenth of 130k keys in one cell looked like a mean run
+// of 34 instead of 1300 keys, and a CTA sorted it: 248 us, all passes take 110.)
 #pragma once
 
 #include "radix_sort.cuh"
@@ -56,8 +63,8 @@ __host__ __device__ __forceinline__ u64 mix64(u64 x)
     return x ^ (x >> 31);
 }
 
-// Keys sampled of n: about n / 4 pairs, so that a mean run of one key more
-// is seen two or three times (n up to 16Mi).
+// Keys sampled of n: about 2 n pairs, so that a mean run of one key more is
+// seen about twice (n up to 16Mi).
 inline u32 planSamples(size_t n)
 {
     u32 m = 64;
@@ -77,6 +84,7 @@ inline size_t planTableBytes(size_t n) { return (size_t(kPlanSets) << planSlotBi
 struct PlanCounters
 {
     u32 repeats[kPlanSets];  // sampled keys whose prefix another one holds already
+    u32 more[kPlanSets];     // pairs beyond them among the keys of a CTA
     u32 done;                // CTAs that have counted
 };
 
@@ -89,19 +97,34 @@ struct PlanArgs
     int force = -1;  // first pass to run whatever the sample says (self-tests), or -1
 };
 
-// The first pass to run (0: all `passes`) for n keys, from the repeats in each
-// set (set 0: whole keys; set s: prefixes of kPlanMinPasses + s - 1 digits).
-__device__ __forceinline__ u32 planFirst(const u32 *repeats, u32 m, size_t n, int passes = kMaxPasses)
+// The prefixes of a CTA's sampled keys, for the pairs beyond.
+constexpr u32 kPlanLocalBits = 9;
+struct PlanShared
 {
-    const float perPair = 2.f * float(n) / (float(m) * float(m));  // mean run per repeated key
-    const u32 equal = repeats[0];
-    if (float(equal) * perPair > kMaxRepeats) return 0;
+    u32 word[kPlanSets][1u << kPlanLocalBits];   // the last prefix hashed there
+    u32 finds[kPlanSets][1u << kPlanLocalBits];  // keys that found their prefix there
+    u32 repeats[kPlanSets], more[kPlanSets];
+};
+
+// The first pass to run (0: all `passes`) for n keys, from the counts of each
+// set (set 0: whole keys; set s: prefixes of kPlanMinPasses + s - 1 digits).
+__host__ __device__ __forceinline__ u32 planFirst(const u32 *repeats, const u32 *more, u32 m, size_t n,
+                                                  int passes = kMaxPasses)
+{
+    const float perPair = 2.f * float(n) / (float(m) * float(m));  // mean run per pair
+    if (float(repeats[0]) * perPair > kMaxRepeats) return 0;
+    // pairs of sampled keys for each pair within a CTA
+    const u32 whole = m / kPlanThreads, rest = m % kPlanThreads;
+    const float scale = float(m) * float(m - 1) /
+                        (float(whole) * kPlanThreads * (kPlanThreads - 1) + float(rest) * float(rest ? rest - 1 : 0));
+    const float equal = float(repeats[0]) + float(more[0]) * scale;
     float best = float(passes);
     u32 first = 0;
     for (int d = kPlanMinPasses; d <= kPlanMaxPasses && d < passes; ++d)
     {
-        const u32 r = repeats[d - kPlanMinPasses + 1];
-        const float run = float(r > equal ? r - equal : 0u) * perPair;
+        const int set = d - kPlanMinPasses + 1;
+        const float pairs = float(repeats[set]) + float(more[set]) * scale;
+        const float run = pairs > equal ? (pairs - equal) * perPair : 0.f;
         const float cost = float(d) + kRepairCost + kRunCost * run;
         if (cost < best)
         {
@@ -130,11 +153,11 @@ __device__ __forceinline__ size_t planPosition(u32 i, size_t n)
 // earlier sorts (epoch: the number of this one) match no prefix of this one,
 // so nothing is cleared.
 template <class KeyAt>
-__device__ __forceinline__ void planSample(const KeyAt &keyAt, size_t n, const PlanArgs &a, u32 epoch)
+__device__ __forceinline__ void planSample(const KeyAt &keyAt, size_t n, const PlanArgs &a, u32 epoch, PlanShared &sm)
 {
-    __shared__ u32 sRepeats[kPlanSets];
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (threadIdx.x < kPlanSets) sRepeats[threadIdx.x] = 0;
+    static_assert(sizeof(PlanShared) % sizeof(u32) == 0, "words");
+    for (u32 k = threadIdx.x; k < sizeof(PlanShared) / sizeof(u32); k += blockDim.x) reinterpret_cast<u32 *>(&sm)[k] = 0;
     __syncthreads();
     u32 group = 0;
     u64 key = 0;
@@ -153,15 +176,44 @@ __device__ __forceinline__ void planSample(const KeyAt &keyAt, size_t n, const P
                 reinterpret_cast<unsigned long long *>(a.table + (size_t(set) << a.slotBits) + (h >> (64 - a.slotBits))),
                 (unsigned long long)word[set]);
     }
+    // (while the exchanges are on their way)
+    static_assert(kPlanSets % 2 == 0 && kPlanThreads <= 256, "two sets' pairs of a warp in a word");
+    u32 more[kPlanSets / 2] = {};
+#pragma unroll
+    for (int set = 0; set < kPlanSets; ++set)
+    {
+        const u32 mine = u32(word[set]) | 1u, at = mine >> (32 - kPlanLocalBits);
+        if (valid && atomicExch(&sm.word[set][at], mine) == mine)
+            more[set / 2] += atomicAdd(&sm.finds[set][at], 1u) << (16 * (set % 2));
+    }
+    u32 any = 0;
+#pragma unroll
+    for (int k = 0; k < kPlanSets / 2; ++k) any |= more[k];
+    if (__any_sync(0xffffffffu, any))
+    {
+#pragma unroll
+        for (int k = 0; k < kPlanSets / 2; ++k)
+        {
+            const u32 pairs = __reduce_add_sync(0xffffffffu, more[k]);
+            if ((threadIdx.x & 31) == 0 && pairs)
+            {
+                atomicAdd(&sm.more[2 * k], pairs & 0xffffu);
+                atomicAdd(&sm.more[2 * k + 1], pairs >> 16);
+            }
+        }
+    }
 #pragma unroll
     for (int set = 0; set < kPlanSets; ++set)
     {
         const u32 c = u32(__popc(__ballot_sync(0xffffffffu, old[set] == word[set])));
-        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sRepeats[set], c);
+        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sm.repeats[set], c);
     }
     __syncthreads();
-    if (threadIdx.x < kPlanSets && sRepeats[threadIdx.x])
-        atomicAdd(&a.counters->repeats[threadIdx.x], sRepeats[threadIdx.x]);
+    if (threadIdx.x < kPlanSets)
+    {
+        if (sm.repeats[threadIdx.x]) atomicAdd(&a.counters->repeats[threadIdx.x], sm.repeats[threadIdx.x]);
+        if (sm.more[threadIdx.x]) atomicAdd(&a.counters->more[threadIdx.x], sm.more[threadIdx.x]);
+    }
 }
 
 // Start of a sort of n keys: the digit counts are cleared and the keys
@@ -170,12 +222,13 @@ template <class KeyAt>
 __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const PlanArgs &a, SortControl *ctl, u32 *hist,
                                          size_t histWords, int passes = kMaxPasses)
 {
-    __shared__ u32 sTotal[kPlanSets];
+    __shared__ PlanShared sm;
+    __shared__ u32 sRepeats[kPlanSets], sMore[kPlanSets];
     __shared__ bool sLast;
     const u32 epoch = ctl->epoch + kEpochStep;  // this sort's number (set at the end)
     for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < histWords; k += size_t(gridDim.x) * blockDim.x)
         hist[k] = 0;
-    planSample(keyAt, n, a, epoch);
+    planSample(keyAt, n, a, epoch, sm);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) sLast = atomicAdd(&a.counters->done, 1u) == gridDim.x - 1;
@@ -184,8 +237,9 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     __threadfence();
     if (threadIdx.x < kPlanSets)
     {
-        sTotal[threadIdx.x] = __ldcg(&a.counters->repeats[threadIdx.x]);
-        a.counters->repeats[threadIdx.x] = 0;
+        sRepeats[threadIdx.x] = __ldcg(&a.counters->repeats[threadIdx.x]);
+        sMore[threadIdx.x] = __ldcg(&a.counters->more[threadIdx.x]);
+        a.counters->repeats[threadIdx.x] = a.counters->more[threadIdx.x] = 0;
     }
     if (threadIdx.x < kPassSlots) ctl->tileCounters[threadIdx.x] = 0;
     clearBarriers(ctl);
@@ -193,7 +247,7 @@ __device__ __forceinline__ void planSort(const KeyAt &keyAt, size_t n, const Pla
     if (threadIdx.x == 0)
     {
         a.counters->done = 0;
-        ctl->first = a.force >= 0 ? u32(a.force) : planFirst(sTotal, a.samples, n, passes);
+        ctl->first = a.force >= 0 ? u32(a.force) : planFirst(sRepeats, sMore, a.samples, n, passes);
         ctl->epoch = epoch;
         ctl->longRuns = 0;
         ctl->keygenDone = 0;
