@@ -19,7 +19,9 @@ namespace aot
 // --------------------------------------------------------------------------
 // Morton (iMorton / decodeMorton, sfc_keys.cuh:174-237)
 // --------------------------------------------------------------------------
-// The 10 low bits of v, three places apart.  A multiplication adds the
+// The 10 low bits of v, three places apart: the expansion by multiplications
+// and masks of T. Karras, "Thinking Parallel, Part III: Tree Construction on
+// the GPU" (NVIDIA developer blog, 2012).  A multiplication adds the
 // shifted copy (the bits do not overlap), which leaves half of the work to the
 // multiply-add pipe: key generation is bound by the integer ALU, and 64-bit
 // spreads by shifts took half of its instructions.

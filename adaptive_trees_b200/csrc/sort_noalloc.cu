@@ -39,16 +39,15 @@ namespace aot
 namespace
 {
 // Scratch of the pair sort for kNoAllocMaxItems items: alternate keys
-// (8 B/item) and values (4 B/item), counters, look-back status, plan table and
-// list of long runs, about 14.3 MB; the array keeps the room that look-back
-// words for 8 passes took.  The call checks the sort's own size query against
-// this before using the array.
+// (8 B/item) and values (4 B/item), the look-back status of a pass (256 x 8 B a
+// tile), and within half a megabyte the control block, the digit counts and
+// starts (18 KB), the plan's table (393 KB) and the list of long runs (33 KB).
+// The call checks the sort's own size query (13.87 MB) against this before
+// using the array.
 constexpr size_t kNoAllocMaxItems = size_t(1) << 20;
-constexpr size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kNoAllocTiles = (kNoAllocMaxItems + kSortTileItems - 1) / kSortTileItems;
 constexpr size_t kNoAllocScratchBytes =
-    up256(up256(up256(up256(kNoAllocMaxItems * 8) + kNoAllocMaxItems * 4) + (4 + 2 * 8 * 256 + 8) * 4) +
-          size_t(8) * kNoAllocTiles * 256 * 8);  // 19,316,992 bytes
+    kNoAllocMaxItems * 12 + kNoAllocTiles * 256 * 8 + (size_t(512) << 10);  // 13,946,880 bytes
 
 static __device__ __align__(256) unsigned char g_noAllocScratch[kNoAllocScratchBytes];
 

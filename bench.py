@@ -818,6 +818,19 @@ def reference_parity(tree, xs, frames, stream):
                    "sm_100a (oracle/_ref/ref_driver), same coordinates, build then update(N(0,1e-3) jitter)"}
 
 
+def sort_passes(tree, n):
+    """(passes the tree's last sort ran, passes of its digits over 64 bits)."""
+    import ctypes
+
+    import adaptive_trees_b200 as ab
+    from adaptive_trees_b200 import _capi as C
+    bits = ab.sort_tuning(n)["digit_bits"]
+    of = -(-64 // bits)
+    first = ctypes.c_int()
+    C.check(C.load().ao_selftest_tree_sort_plan(tree.handle, -1, ctypes.byref(first), None))
+    return (of - first.value if bits == 8 else of), of
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1017,11 +1030,12 @@ def main():
     hbm, peak_kind = peaks()
     pass_bytes = 24.0 * n
     achieved = pass_bytes / (pass_ms * 1e-3) / 1e9
-    # the sort pass is the kernel the path has most of: the build's plan runs 4
-    # of 8, a quarter of its device time (the near field, over 13 levels, is
-    # nearly a third)
+    # the sort pass is the kernel the path has most of: a quarter of the build's
+    # device time (the near field, over 13 levels, is nearly a third)
+    passes, of = sort_passes(tree, n)
     roof_sort = {"bound": "hbm", "kernel": "onesweepKernel (one 8-bit pass of the 64-bit key + 32-bit value sort)",
-                 "why": "the plan of the build's sort runs 4 of 8 passes, 0.48 of 1.91 ms device time",
+                 "why": f"the timed tree's last sort ran {passes} of {of} passes, {passes * pass_ms:.2f} ms of a "
+                        f"{step_ms:.2f} ms build",
                  "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind,
                  "traffic": ONESWEEP_TRAFFIC_BYTES_PER_KEY * n,
                  "traffic_kind": "ncu on the passes of 8Mi keys, scaled, not re-measured",
@@ -1063,15 +1077,14 @@ def main():
         "build_near_field_launches": build_stages[-1]["near_field_launches"],
         "update_near_field_launches": update_stages[-1]["near_field_launches"],
         "how": "CUDA events on the tree's stream around each stage (ao_tree_set_profiling), direct calls"}
-    # the whole build on the byte model of a build whose sort runs all 8 passes
-    # (the plan runs 4, so this figure can pass the peak): per particle the
-    # coordinates read (3 x 4 B), key + index written (12 B), the upfront
-    # histogram read (8 B), 24 B per radix pass (8 passes), one streaming read
-    # of the sorted keys (8 B); per leaf K and N written (12 B)
-    model_bytes = n * (3 * 4 + 12 + 8 + 24 * 8 + 8) + 12 * leaves
+    # the whole build by the bytes its stages have to move: per particle the
+    # coordinates read (3 x 4 B), the key written (8 B; the first pass makes the
+    # index), 24 B for each pass that ran, the repair's read (12 B), one
+    # streaming read of the sorted keys (8 B); per leaf K and N written (12 B)
+    model_bytes = n * (3 * 4 + 8 + 24 * passes + 12 + 8) + 12 * leaves
     model_gbs = model_bytes / (step_ms * 1e-3) / 1e9
-    roof_build = {"bound": "hbm", "what": "whole build() on the byte model N(3 s_r + 12 + 8 + 24 R + 8) + 12 L "
-                                          "(s_r = 4, R = 8)", "bytes": model_bytes, "ms": step_ms,
+    roof_build = {"bound": "hbm", "what": "whole build() by the bytes of its stages, N(3 s_r + 8 + 24 R + 12 + 8) + 12 L "
+                                          f"(s_r = 4, R = {passes} passes run of {of})", "bytes": model_bytes, "ms": step_ms,
                   "achieved": model_gbs, "peak": hbm, "unit": "GB/s", "frac": model_gbs / hbm, "peak_kind": peak_kind}
     line = {"metric": METRIC, "value": total / (step_ms * 1e-3), "unit": "particles/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
