@@ -507,12 +507,14 @@ struct SortArena
 // and in one: 10k keys 72 and 57 us, 100k 79 and 61, 1M 113 and 99, 4M 202 and
 // 200; from a graph 39 and 46, 48 and 51, 81 and 89, 164 and 190.
 constexpr size_t kFusedSort = size_t(1) << 21;
-// Sorts that make no plan run every pass, and count their digits first, which
+// Pair sorts that make no plan run every pass, and count their digits first, which
 // the few CTAs of a small sort do slowly.  Random keys queued directly, launch by
 // launch and in one: one digit, 10k keys 21 and 26 us, 50k 24 and 27, 2M 48 and
 // 51; four digits 45 and 49, 49 and 51, 200k 62 and 56, 700k 80 and 75, 2M 113
 // and 120; eight digits 78 and 79, 84 and 83, 101 and 91, 128 and 128, 197 and
-// 210.
+// 210.  (The sorts of views wait for their launches more than for their keys:
+// computeViews() of k-d trees of 500, 5k and 50k particles, bucket 64, launch by launch
+// 109, 121 and 127 us, in one 97, 102 and 111.)
 constexpr int kFusedPasses = 4;
 constexpr unsigned kFusedCounting = 32;
 constexpr size_t kFusedUnplannedFrom = size_t(1) << 17, kFusedUnplannedTo = size_t(1) << 20;
@@ -524,7 +526,6 @@ bool launchFusedSort(int cfg, cudaStream_t s, const sort::PassArgs &p, const sor
                      bool repair)
 {
     if (p.n > kFusedSort) return false;
-    if (!repair && (p.passes < kFusedPasses || p.n < kFusedUnplannedFrom || p.n > kFusedUnplannedTo)) return false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     AOT_CHECK(cudaStreamIsCapturing(s, &capture));
     if (capture != cudaStreamCaptureStatusNone) return false;
@@ -840,7 +841,8 @@ void TreeEngine::sortPairsWith(int cfg, void *scratch, size_t *scratchBytes, con
     const bool aligned = aligned16(out) && (reinterpret_cast<uintptr_t>(valsOut) & 7u) == 0;
     const sort::RepairArgs r{{out, altK}, {valsOut, altV}, n, ctl, reinterpret_cast<u32 *>(base + lay.longRuns), nullptr,
                              error, beginBit, passes, keyMask, true, aligned, false};
-    if (launchFusedSort(cfg, s, p, r, hist, bins, planned)) return;
+    const bool fuse = planned || (passes >= kFusedPasses && n >= kFusedUnplannedFrom && n <= kFusedUnplannedTo);
+    if (fuse && launchFusedSort(cfg, s, p, r, hist, bins, planned)) return;
     const unsigned blocks = std::max(1u, std::min<unsigned>(ceilDiv(n, sort::kThreads), unsigned(smCount()) * 8u));
     sort::launchHistogram(cfg, s, blocks, in, n, beginBit, passes, hist, endBit, ctl), noteLaunch();
     sort::binsKernel<<<1, sort::kThreads, 0, s>>>(hist, bins, passes), noteLaunch();
